@@ -2,11 +2,12 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 
-#include "fft_device.cuh"
 #include "fft_engine.cuh"
+#include "fft_stages.cuh"
 
 namespace fdr {
 
@@ -210,11 +211,236 @@ static PassDesc blank_pass() {
   return d;
 }
 
+
+// ------------------------------------------------------------------------------------
+// Passes over lengths whose prime factors are at most 13 (in-place stages of fft_stages.cuh).
+// ------------------------------------------------------------------------------------
+namespace {
+
+// Fewest stages for every length up to kStageElems; of equal plans the one with the smaller
+// sum of radices.  first[n]: the radix to take from n, largest first.
+struct StagePlans {
+  std::vector<unsigned char> count, first;
+  std::vector<int> cost;
+  StagePlans() : count(kStageElems + 1, 0xff), first(kStageElems + 1, 0), cost(kStageElems + 1, 0) {
+    static const int radices[] = {16, 13, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+    count[1] = 0;
+    for (int n = 2; n <= kStageElems; ++n)
+      for (int r : radices) {
+        if (n % r || count[n / r] == 0xff) continue;
+        const int c = count[n / r] + 1, w = cost[n / r] + r;
+        if (c < count[n] || (c == count[n] && w < cost[n])) {
+          count[n] = (unsigned char)c;
+          cost[n] = w;
+          first[n] = (unsigned char)r;
+        }
+      }
+  }
+};
+
+unsigned magic_of(int d) { return d == 1 ? 0u : (unsigned)(((1ULL << 32) + d - 1) / d); }
+
+}  // namespace
+
+bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, StageDesc* d) {
+  static const StagePlans plans;
+  if (L < 2 || L > kStageElems || plans.count[L] == 0xff || plans.count[L] > kStageMax) return false;
+  memset(d, 0, sizeof(*d));
+  d->L = (int)L;
+  int Ns = 1;
+  for (int n = (int)L; n > 1; n /= plans.first[n]) d->radix[d->nst++] = plans.first[n];
+  std::sort(d->radix, d->radix + d->nst, [](int a, int b) { return a > b; });
+  for (int s = 0; s < d->nst; ++s) {
+    const int R = d->radix[s];
+    d->nbf[s] = (int)L / R;
+    d->Ns[s] = Ns;
+    d->nbf_magic[s] = magic_of(d->nbf[s]);
+    d->Ns_magic[s] = magic_of(Ns);
+    d->tw_step[s] = (int)L / (Ns * R);
+    Ns *= R;
+  }
+  // as many transforms as the buffer holds, fewer when the grid would not reach two CTAs an SM
+  int lg = 0;
+  while ((L << (lg + 1)) <= kStageElems && lg < 8 && (int64_t(1) << lg) < nb) ++lg;
+  while (lg > (rows ? 3 : 0) && cdiv(nb, int64_t(1) << lg) * groups < 2LL * sm_count()) --lg;
+  d->bpc_log2 = lg;
+  d->bpc = 1 << lg;
+  d->SS = (padlen((int)L) / 16 + 1) * 16 + (d->bpc >= 16 ? 1 : 16 / d->bpc);
+  return true;
+}
+
+// Threads of a CTA: every butterfly of the widest stage at once, up to kStageThreads.
+int stage_threads(const StageDesc& d) {
+  const int want = d.nbf[d.nst - 1] << d.bpc_log2;
+  return std::max(64, std::min(kStageThreads, (want + 31) / 32 * 32));
+}
+size_t stage_smem(const StageDesc& d) { return sizeof(float2) * (size_t)d.bpc * d.SS; }
+
+namespace {
+
+enum { kInComplex, kInRealPair, kInHalfPair };
+enum { kOutComplex, kOutTwiddle, kOutRealPair };
+
+struct StageArgs {
+  StageDesc d;
+  const void* in;
+  void* out;
+  const float2* mul;  // kOutComplex: pointwise factor addressed like the output, or NULL
+  long long is0, is1, isl, os0, os1, osl;
+  long long nb0, nb1;
+  long long N, K;     // transform length of the columns and N/2 + 1
+  long long p0, ncol;   // column pairs: first pair, columns in all
+  long long ldi, ldo;   // column strides of the real columns or half spectra
+  int pair_b1;        // the pair index is b1 (whole column in one CTA), else b0
+  int in_lane_i, out_lane_i;
+  float scale;
+};
+
+// Four-step twiddle exp(SIGN 2 pi i l b / N) of the CTA's transforms b, as the product of a
+// factor for l / 32 (rounded value and its residue) and one for l mod 32 (its difference from
+// 1): within 0.2 ulp of the correctly rounded value for L >= 160, since the second factor's
+// angle is below 2 pi / 32 there.  All values come from float64, once per CTA.
+struct TwiddleTables {
+  float4* hi;
+  float2* lo;
+  int nh;
+};
+__host__ __device__ constexpr int tw_rows(int L) { return ((L + 31) / 32) | 1; }
+__host__ __device__ inline size_t tw_bytes(int L, int bpc) {
+  return 16 + (size_t)bpc * (sizeof(float4) * tw_rows(L) + sizeof(float2) * 33);
+}
+
+template <int SIGN>
+__device__ __forceinline__ void fill_twiddles(const TwiddleTables& t, int bpc, int L, long long b1_0, double inv2N) {
+  const int nh = (L + 31) / 32, per = nh + 32;
+  for (int e = threadIdx.x; e < bpc * per; e += blockDim.x) {
+    const int i = e / per, m = e - i * per;
+    const long long l = m < nh ? 32LL * m : m - nh;
+    double s, c;
+    sincospi((double)(l * (b1_0 + i)) * inv2N, &s, &c);
+    s *= SIGN;
+    if (m < nh) {
+      const float x = (float)c, y = (float)s;
+      t.hi[i * t.nh + m] = make_float4(x, y, (float)(c - x), (float)(s - y));
+    } else {
+      t.lo[i * 33 + m - nh] = make_float2((float)(c - 1.0), (float)s);
+    }
+  }
+}
+__device__ __forceinline__ float2 twiddle_at(const TwiddleTables& t, int i, int l) {
+  const float4 h = t.hi[i * t.nh + (l >> 5)];
+  const float2 e = t.lo[i * 33 + (l & 31)];
+  return make_float2(h.x + fmaf(h.x, e.x, fmaf(-h.y, e.y, h.z)), h.y + fmaf(h.x, e.y, fmaf(h.y, e.x, h.w)));
+}
+
+template <int SIGN, int IN, int OUT>
+__global__ void __launch_bounds__(kStageThreads, 2) fft_stage_kernel(const __grid_constant__ StageArgs a) {
+  extern __shared__ float4 sm4[];
+  float2* const sm = reinterpret_cast<float2*>(sm4);
+  const StageDesc& d = a.d;
+  const long long b1_0 = (long long)blockIdx.x << d.bpc_log2;
+  const int nb = (int)min((long long)d.bpc, a.nb1 - b1_0);
+  TwiddleTables tw;
+  if (OUT == kOutTwiddle) {
+    tw.hi = sm4 + (d.bpc * d.SS + 1) / 2;
+    tw.nh = tw_rows(d.L);
+    tw.lo = reinterpret_cast<float2*>(tw.hi + d.bpc * tw.nh);
+    fill_twiddles<SIGN>(tw, d.bpc, d.L, b1_0, 2.0 / (double)a.N);
+    if (d.nst == 1) __syncthreads();  // otherwise the first stage's barrier covers them
+  }
+  for (long long b0 = blockIdx.y; b0 < a.nb0; b0 += gridDim.y) {
+    const float2* const in = static_cast<const float2*>(a.in) + b0 * a.is0 + b1_0 * a.is1;
+    float2* const out = static_cast<float2*>(a.out) + b0 * a.os0 + b1_0 * a.os1;
+    const float2* const mul = a.mul ? a.mul + b0 * a.os0 + b1_0 * a.os1 : nullptr;
+    auto get = [&](int i, int l) -> float2 {
+      if (i >= nb) return make_float2(0.f, 0.f);
+      if (IN == kInComplex) return in[i * a.is1 + l * a.isl];
+      const long long n = (b1_0 + i) * a.is1 + l * a.isl;
+      const long long c = 2 * (a.p0 + (a.pair_b1 ? b1_0 + i : b0));
+      if (IN == kInRealPair) {
+        const float* p = static_cast<const float*>(a.in) + n + c * a.ldi;
+        return make_float2(p[0], c + 1 < a.ncol ? p[a.ldi] : 0.f);
+      }
+      // S_a + i S_b of bin n, from the conjugates of bin N - n above K; the imaginary parts of
+      // bin 0 and, for even N, bin N/2 do not enter
+      const bool upper = n >= a.K;
+      const long long k = upper ? a.N - n : n;
+      const float2* p = static_cast<const float2*>(a.in) + k + c * a.ldi;
+      float2 u = p[0], w = c + 1 < a.ncol ? p[a.ldi] : make_float2(0.f, 0.f);
+      if (k == 0 || 2 * k == a.N) u.y = w.y = 0.f;
+      if (upper) { u.y = -u.y; w.y = -w.y; }
+      return make_float2(u.x - w.y, u.y + w.x);
+    };
+    auto put = [&](int i, int l, float2 v) {
+      if (i >= nb) return;
+      if (OUT == kOutRealPair) {
+        const long long n = (b1_0 + i) * a.os1 + l * a.osl;
+        const long long c = 2 * (a.p0 + (a.pair_b1 ? b1_0 + i : b0));
+        float* p = static_cast<float*>(a.out) + n + c * a.ldo;
+        v = cscale(v, a.scale);
+        p[0] = v.x;
+        if (c + 1 < a.ncol) p[a.ldo] = v.y;
+        return;
+      }
+      if (OUT == kOutTwiddle) {
+        v = cmul(v, twiddle_at(tw, i, l));
+      } else {
+        if (mul) v = cmul(v, mul[i * a.os1 + l * a.osl]);
+        v = cscale(v, a.scale);
+      }
+      out[i * a.os1 + l * a.osl] = v;
+    };
+    stages_run<SIGN>(d, a.in_lane_i, a.out_lane_i, sm, get, put);
+    if (b0 + gridDim.y < a.nb0) __syncthreads();  // the last stage has read shared memory
+  }
+}
+
+template <int SIGN, int IN, int OUT>
+int launch_stages(StageArgs& a, cudaStream_t s) {
+  if (a.nb0 <= 0 || a.nb1 <= 0) return FDR_OK;
+  FDR_TRY(get_roots(a.d.L, &a.d.roots));
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  FDR_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !attr_set[dev]) {
+    FDR_CUDA(cudaFuncSetAttribute(fft_stage_kernel<SIGN, IN, OUT>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
+    if (dev < 64) attr_set[dev] = true;
+  }
+  const size_t smem = stage_smem(a.d) + (OUT == kOutTwiddle ? tw_bytes(a.d.L, a.d.bpc) : 0);
+  const dim3 grid((unsigned)cdiv(a.nb1, a.d.bpc), (unsigned)std::min(a.nb0, 65535LL));
+  fft_stage_kernel<SIGN, IN, OUT><<<grid, stage_threads(a.d), smem, s>>>(a);
+  FDR_LAUNCH_CHECK("fft_stage_kernel");
+  return FDR_OK;
+}
+
+StageArgs blank_stages() {
+  StageArgs a;
+  memset(&a, 0, sizeof(a));
+  a.nb0 = 1;
+  a.scale = 1.f;
+  return a;
+}
+
+}  // namespace
+
 int fft_strided_inplace(float2* buf, long long L, long long sl, long long nb, long long sb,
                         int sign, float scale, const float2* mul, cudaStream_t s) {
   if (L > kMaxCtaElems) {
     set_error(FDR_ERR_UNSUPPORTED_SIZE, "strided FFT length %lld exceeds %d", L, kMaxCtaElems);
     return FDR_ERR_UNSUPPORTED_SIZE;
+  }
+  StageArgs a = blank_stages();
+  if (stage_plan(L, nb, 1, true, &a.d)) {
+    a.in = a.out = buf;
+    a.mul = mul;
+    a.nb1 = nb;
+    a.is1 = a.os1 = sb;
+    a.isl = a.osl = sl;
+    a.in_lane_i = a.out_lane_i = sb == 1;
+    a.scale = scale;
+    return sign < 0 ? launch_stages<-1, kInComplex, kOutComplex>(a, s)
+                    : launch_stages<+1, kInComplex, kOutComplex>(a, s);
   }
   PassDesc d = blank_pass();
   d.in = buf; d.out = buf; d.mul = mul;
@@ -362,6 +588,70 @@ static unsigned grid_for(long long total) {
   return (unsigned)max(1LL, min(b, cap));
 }
 
+// The two passes of a real transform of `np` column pairs starting at pair p0 whose packing
+// and unpacking happen in the passes' own loads and stores (rfft: real columns -> the packed
+// spectra Z in `z`, tmp in between; irfft: half spectra -> real columns, tmp in between).
+// *done is false when a factor of N has a prime above 13: the caller takes the generic passes.
+static int real_stages(bool forward, const void* in, long long ldin, void* out, long long ldout,
+                       long long N, long long ncol, long long p0, long long np, float2* tmp,
+                       cudaStream_t s, bool* done) {
+  *done = false;
+  StageArgs a = blank_stages();
+  a.in = in;
+  a.N = N;
+  a.K = N / 2 + 1;
+  a.p0 = p0;
+  a.ncol = ncol;
+  a.ldi = ldin;
+  a.ldo = ldout;
+  if (N <= kMaxCtaElems) {
+    if (!stage_plan(N, np, 1, false, &a.d)) return FDR_OK;
+    a.nb1 = np;
+    a.isl = a.osl = 1;
+    a.pair_b1 = 1;
+    a.out = out;
+    *done = true;
+    if (forward) {
+      a.os1 = N;
+      return launch_stages<-1, kInRealPair, kOutComplex>(a, s);
+    }
+    a.scale = 1.f / (float)N;
+    return launch_stages<+1, kInHalfPair, kOutRealPair>(a, s);
+  }
+  long long L1, L2;
+  split_len(N, &L1, &L2);
+  StageArgs b = a;
+  if (L1 == 0 || !stage_plan(L1, L2, np, true, &a.d) || !stage_plan(L2, L1, np, true, &b.d)) return FDR_OK;
+  *done = true;
+  // Pass 1: n = n2 + L2*n1, DFT over n1 for each n2, twiddle, tmp[k1*L2 + n2]
+  a.out = tmp;
+  a.nb0 = np;
+  a.nb1 = L2;
+  a.is1 = 1;
+  a.isl = L2;
+  a.os0 = N;
+  a.os1 = 1;
+  a.osl = L2;
+  a.in_lane_i = a.out_lane_i = 1;
+  FDR_TRY((forward ? launch_stages<-1, kInRealPair, kOutTwiddle>(a, s)
+                   : launch_stages<+1, kInHalfPair, kOutTwiddle>(a, s)));
+  // Pass 2: for each k1, DFT over n2 (contiguous), bin or channel k1 + L1*k2
+  b.in = tmp;
+  b.out = out;
+  b.nb0 = np;
+  b.nb1 = L1;
+  b.is0 = N;
+  b.is1 = L2;
+  b.isl = 1;
+  b.os0 = N;
+  b.os1 = 1;
+  b.osl = L1;
+  b.out_lane_i = 1;
+  if (forward) return launch_stages<-1, kInComplex, kOutComplex>(b, s);
+  b.scale = 1.f / (float)N;
+  return launch_stages<+1, kInComplex, kOutRealPair>(b, s);
+}
+
 int rfft_columns(const float* in, long long ldin, long long ncol, long long N, float2* F,
                  long long ldF, float2* scratch, long long pairs_per_chunk, cudaStream_t s) {
   const long long K = N / 2 + 1;
@@ -375,9 +665,13 @@ int rfft_columns(const float* in, long long ldin, long long ncol, long long N, f
     float2* zo = (N <= kMaxCtaElems) ? scratch : scratch + N * np;
     float2* tmp = z;
     (void)per;
-    pack_real_pairs<<<grid_for(N * np), 256, 0, s>>>(in, ldin, ncol, N, p0, np, z);
-    FDR_LAUNCH_CHECK("pack_real_pairs");
-    FDR_TRY(fft_contig(z, N, zo, N, N, np, -1, 1.f, tmp, s));
+    bool done;
+    FDR_TRY(real_stages(true, in, ldin, zo, N, N, ncol, p0, np, tmp, s, &done));
+    if (!done) {
+      pack_real_pairs<<<grid_for(N * np), 256, 0, s>>>(in, ldin, ncol, N, p0, np, z);
+      FDR_LAUNCH_CHECK("pack_real_pairs");
+      FDR_TRY(fft_contig(z, N, zo, N, N, np, -1, 1.f, tmp, s));
+    }
     unpack_r2c<<<grid_for(K * np), 256, 0, s>>>(zo, N, K, ncol, p0, np, F, ldF);
     FDR_LAUNCH_CHECK("unpack_r2c");
   }
@@ -393,6 +687,9 @@ int irfft_columns(const float2* S, long long ldS, long long ncol, long long N, f
     float2* c = scratch;
     float2* co = (N <= kMaxCtaElems) ? scratch : scratch + N * np;
     float2* tmp = c;
+    bool done;
+    FDR_TRY(real_stages(false, S, ldS, out, ldout, N, ncol, p0, np, tmp, s, &done));
+    if (done) continue;
     pack_c2r<<<grid_for(N * np), 256, 0, s>>>(S, ldS, ncol, N, K, p0, np, c);
     FDR_LAUNCH_CHECK("pack_c2r");
     FDR_TRY(fft_contig(c, N, co, N, N, np, +1, 1.f / (float)N, tmp, s));

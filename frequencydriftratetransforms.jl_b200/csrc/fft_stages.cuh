@@ -1,0 +1,225 @@
+// Register DFTs of the radices that the pass kernels use beside the ones of fft_device.cuh,
+// and the in-place mixed-radix Stockham stages of one CTA (several transforms of one runtime
+// length in shared memory).
+#pragma once
+#include "fft_device.cuh"
+
+namespace fdr {
+
+// DFT of an odd prime length from the sums and differences of the mirrored inputs:
+// X[q], X[R-q] = (v0 + sum_m cos(2 pi q m / R) (v[m] + v[R-m]))
+//                +- i sign (sum_m sin(2 pi q m / R) (v[m] - v[R-m])).
+template <int R, class Table>
+struct DftPrime {
+  __device__ __forceinline__ static void run(float2* v, int sign) {
+    constexpr int H = (R - 1) / 2;
+    constexpr Table tab{};
+    float2 t[H], d[H];
+    float2 x0 = v[0];
+#pragma unroll
+    for (int m = 0; m < H; ++m) {
+      t[m] = cadd(v[m + 1], v[R - 1 - m]);
+      d[m] = csub(v[m + 1], v[R - 1 - m]);
+      x0 = cadd(x0, t[m]);
+    }
+    const float2 v0 = v[0];
+    v[0] = x0;
+#pragma unroll
+    for (int q = 1; q <= H; ++q) {
+      float2 a = v0, b = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int m = 0; m < H; ++m) {
+        const float c = tab.c[(q * (m + 1)) % R], s = tab.s[(q * (m + 1)) % R];
+        a = make_float2(fmaf(c, t[m].x, a.x), fmaf(c, t[m].y, a.y));
+        b = make_float2(fmaf(s, d[m].x, b.x), fmaf(s, d[m].y, b.y));
+      }
+      const float2 ib = cmul_i(b, sign);
+      v[q] = cadd(a, ib);
+      v[R - q] = csub(a, ib);
+    }
+  }
+};
+
+// DFT of R1 * R2 points: R2-point DFTs over r = r1 + R1 * r2, the twiddles, R1-point DFTs.
+template <int R1, int R2, class Table>
+struct DftComposite {
+  __device__ __forceinline__ static void run(float2* v, int sign) {
+    constexpr Table tab{};
+    float2 y[R1][R2];
+#pragma unroll
+    for (int r1 = 0; r1 < R1; ++r1) {
+      float2 t[R2];
+#pragma unroll
+      for (int r2 = 0; r2 < R2; ++r2) t[r2] = v[r1 + R1 * r2];
+      Dft<R2>::run(t, sign);
+#pragma unroll
+      for (int m2 = 0; m2 < R2; ++m2)
+        y[r1][m2] = (r1 * m2) == 0 ? t[m2]
+                                   : cmul(t[m2], make_float2(tab.c[r1 * m2], (float)sign * tab.s[r1 * m2]));
+    }
+#pragma unroll
+    for (int m2 = 0; m2 < R2; ++m2) {
+      float2 t[R1];
+#pragma unroll
+      for (int r1 = 0; r1 < R1; ++r1) t[r1] = y[r1][m2];
+      Dft<R1>::run(t, sign);
+#pragma unroll
+      for (int m1 = 0; m1 < R1; ++m1) v[m2 + R2 * m1] = t[m1];
+    }
+  }
+};
+
+// cos and sin of 2 pi m / n
+struct CosSin6 {
+  float c[6] = {1.00000000000000000f, 0.50000000000000011f, -0.49999999999999978f, -1.00000000000000000f, -0.50000000000000044f, 0.50000000000000011f};
+  float s[6] = {0.00000000000000000f, 0.86602540378443860f, 0.86602540378443871f, 0.00000000000000012f, -0.86602540378443837f, -0.86602540378443860f};
+};
+struct CosSin7 {
+  float c[7] = {1.00000000000000000f, 0.62348980185873359f, -0.22252093395631434f, -0.90096886790241903f, -0.90096886790241915f, -0.22252093395631459f, 0.62348980185873337f};
+  float s[7] = {0.00000000000000000f, 0.78183148246802980f, 0.97492791218182362f, 0.43388373911755823f, -0.43388373911755801f, -0.97492791218182362f, -0.78183148246802991f};
+};
+struct CosSin9 {
+  float c[9] = {1.00000000000000000f, 0.76604444311897801f, 0.17364817766693041f, -0.49999999999999978f, -0.93969262078590832f, -0.93969262078590843f, -0.50000000000000044f, 0.17364817766692997f, 0.76604444311897779f};
+  float s[9] = {0.00000000000000000f, 0.64278760968653925f, 0.98480775301220802f, 0.86602540378443871f, 0.34202014332566888f, -0.34202014332566866f, -0.86602540378443837f, -0.98480775301220813f, -0.64278760968653958f};
+};
+struct CosSin10 {
+  float c[10] = {1.00000000000000000f, 0.80901699437494745f, 0.30901699437494745f, -0.30901699437494734f, -0.80901699437494734f, -1.00000000000000000f, -0.80901699437494756f, -0.30901699437494756f, 0.30901699437494723f, 0.80901699437494734f};
+  float s[10] = {0.00000000000000000f, 0.58778525229247314f, 0.95105651629515353f, 0.95105651629515364f, 0.58778525229247325f, 0.00000000000000012f, -0.58778525229247303f, -0.95105651629515353f, -0.95105651629515364f, -0.58778525229247336f};
+};
+struct CosSin11 {
+  float c[11] = {1.00000000000000000f, 0.84125353283118121f, 0.41541501300188644f, -0.14231483827328500f, -0.65486073394528499f, -0.95949297361449737f, -0.95949297361449748f, -0.65486073394528521f, -0.14231483827328523f, 0.41541501300188605f, 0.84125353283118121f};
+  float s[11] = {0.00000000000000000f, 0.54064081745559756f, 0.90963199535451833f, 0.98982144188093280f, 0.75574957435425827f, 0.28173255684142967f, -0.28173255684142939f, -0.75574957435425816f, -0.98982144188093268f, -0.90963199535451855f, -0.54064081745559744f};
+};
+struct CosSin13 {
+  float c[13] = {1.00000000000000000f, 0.88545602565320991f, 0.56806474673115592f, 0.12053668025532301f, -0.35460488704253545f, -0.74851074817110119f, -0.97094181742605201f, -0.97094181742605212f, -0.74851074817110130f, -0.35460488704253590f, 0.12053668025532320f, 0.56806474673115481f, 0.88545602565321002f};
+  float s[13] = {0.00000000000000000f, 0.46472317204376851f, 0.82298386589365635f, 0.99270887409805397f, 0.93501624268541483f, 0.66312265824079519f, 0.23931566428755768f, -0.23931566428755743f, -0.66312265824079497f, -0.93501624268541472f, -0.99270887409805397f, -0.82298386589365702f, -0.46472317204376840f};
+};
+
+template <> struct Dft<6> : DftComposite<2, 3, CosSin6> {};
+template <> struct Dft<7> : DftPrime<7, CosSin7> {};
+template <> struct Dft<9> : DftComposite<3, 3, CosSin9> {};
+template <> struct Dft<10> : DftComposite<2, 5, CosSin10> {};
+template <> struct Dft<11> : DftPrime<11, CosSin11> {};
+template <> struct Dft<13> : DftPrime<13, CosSin13> {};
+
+// ------------------------------------------------------------------------------------
+// In-place Stockham stages over `bpc` transforms of one length L in shared memory, at most
+// kStageElems points in all.  A thread takes whole butterflies into registers (at most
+// ceil(32 / R) of radix R), the block synchronises, and the outputs replace the inputs, so
+// one buffer is enough and two CTAs share an SM.  The first stage takes its inputs straight
+// from global memory and the last one hands its outputs to global memory: a transform of n
+// stages crosses shared memory n - 1 times.
+// Element l of transform i is at i * SS + pidx(l).  SS = 16 / bpc (mod 16) (1 from bpc = 16
+// on): a half-warp of neighbouring transforms (lanes over i) and one of neighbouring elements
+// (lanes over l) both meet 16 different 8-byte banks.
+// ------------------------------------------------------------------------------------
+constexpr int kStageThreads = 256;
+constexpr int kStageElems = 32 * kStageThreads;
+constexpr int kStageMax = 12;  // stages of a plan (2^12 < kStageElems, radix 2 only once)
+
+struct StageDesc {
+  int L, nst, bpc, bpc_log2, SS;
+  int radix[kStageMax];
+  int nbf[kStageMax];            // L / radix: butterflies of one transform
+  int Ns[kStageMax];             // product of the earlier radices
+  unsigned nbf_magic[kStageMax]; // ceil(2^32 / nbf): exact quotients of numbers below 2^16
+  unsigned Ns_magic[kStageMax];
+  int tw_step[kStageMax];        // L / (Ns * radix)
+  const float2* roots;           // exp(-2 pi i m / L), m < L
+};
+
+// n / d for n < 2^13 from magic = ceil(2^32 / d) (0 stands for d = 1): the excess of the
+// product, below 2^13 / 2^32, is less than the 1 / d that separates it from the next integer.
+__device__ __forceinline__ int div_magic(int n, unsigned magic) {
+  return magic ? (int)__umulhi((unsigned)n, magic) : n;
+}
+
+// Reads, transforms and hands on the butterflies of stage s.  get(i, l, n) gives the value of
+// element l of transform i at the first stage (n: the butterfly's first element, l = n + r *
+// nbf), put(i, l, v) takes it at the last.  lane_i: neighbouring threads take neighbouring
+// transforms (else neighbouring elements).
+template <int R, int SIGN, class Get, class Put>
+__device__ __forceinline__ void stage_run(const StageDesc& d, int s, bool lane_i, bool first, bool last,
+                                          float2* sm, Get get, Put put) {
+  constexpr int PER = (32 + R - 1) / R;
+  const int nbf = d.nbf[s], Ns = d.Ns[s], SS = d.SS;
+  const int total = nbf << d.bpc_log2;
+  float2 v[PER][R];
+#pragma unroll
+  for (int p = 0; p < PER; ++p) {
+    const int j = threadIdx.x + p * blockDim.x;
+    if (j < total) {
+      const int i = lane_i ? j & (d.bpc - 1) : div_magic(j, d.nbf_magic[s]);
+      const int jj = lane_i ? j >> d.bpc_log2 : j - i * nbf;
+      if (first) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[p][r] = get(i, jj + r * nbf);
+      } else {
+        const float2* a = sm + i * SS;
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[p][r] = a[pidx(jj + r * nbf)];
+      }
+    } else {  // no value may live on from the stage before
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[p][r] = make_float2(0.f, 0.f);
+    }
+  }
+  if (!first && !last) __syncthreads();  // every input is read before an output replaces it
+#pragma unroll
+  for (int p = 0; p < PER; ++p) {
+    const int j = threadIdx.x + p * blockDim.x;
+    if (j < total) {
+      const int i = lane_i ? j & (d.bpc - 1) : div_magic(j, d.nbf_magic[s]);
+      const int jj = lane_i ? j >> d.bpc_log2 : j - i * nbf;
+      const int b = div_magic(jj, d.Ns_magic[s]);
+      const int k = jj - b * Ns;
+      if (!first) {
+        const float2* w = d.roots;
+        const int step = k * d.tw_step[s];
+#pragma unroll
+        for (int r = 1; r < R; ++r) {
+          float2 t = __ldg(w + r * step);
+          if (SIGN > 0) t.y = -t.y;
+          v[p][r] = cmul(v[p][r], t);
+        }
+      }
+      Dft<R>::run(v[p], SIGN);
+      if (last) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) put(i, jj + r * nbf, v[p][r]);
+      } else {
+        float2* o = sm + i * SS;
+        const int base = b * Ns * R + k;
+#pragma unroll
+        for (int r = 0; r < R; ++r) o[pidx(base + r * Ns)] = v[p][r];
+      }
+    }
+  }
+  if (!last) __syncthreads();
+}
+
+#define FDR_FOR_RADIX(X) X(16) X(13) X(11) X(10) X(9) X(8) X(7) X(6) X(5) X(4) X(3) X(2)
+
+// All stages of d; the block must be synchronised before if shared memory is still being read.
+template <int SIGN, class Get, class Put>
+__device__ __forceinline__ void stages_run(const StageDesc& d, bool first_lane_i, bool last_lane_i,
+                                           float2* sm, Get get, Put put) {
+  for (int s = 0; s < d.nst; ++s) {
+    const bool first = s == 0, last = s == d.nst - 1;
+    const bool lane_i = first ? first_lane_i : (last ? last_lane_i : d.bpc >= 8);
+    switch (d.radix[s]) {
+#define FDR_STAGE(R) case R: stage_run<R, SIGN>(d, s, lane_i, first, last, sm, get, put); break;
+      FDR_FOR_RADIX(FDR_STAGE)
+#undef FDR_STAGE
+    }
+  }
+}
+
+// Fills d for `groups` sets of `nb` transforms of length L, neighbouring transforms of a set at
+// neighbouring addresses (rows: CTAs then take at least 8 of them, 64 bytes a row); false if L
+// has a prime factor above 13 or exceeds kStageElems.
+bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, StageDesc* d);
+size_t stage_smem(const StageDesc& d);
+int stage_threads(const StageDesc& d);
+
+}  // namespace fdr
