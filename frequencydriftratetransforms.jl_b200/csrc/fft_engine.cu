@@ -240,6 +240,20 @@ struct StagePlans {
 
 unsigned magic_of(int d) { return d == 1 ? 0u : (unsigned)(((1ULL << 32) + d - 1) / d); }
 
+// The fields that follow from L and the radices.
+void fill_stages(StageDesc* d) {
+  int Ns = 1;
+  for (int s = 0; s < d->nst; ++s) {
+    const int R = d->radix[s];
+    d->nbf[s] = d->L / R;
+    d->Ns[s] = Ns;
+    d->nbf_magic[s] = magic_of(d->nbf[s]);
+    d->Ns_magic[s] = magic_of(Ns);
+    d->tw_step[s] = d->L / (Ns * R);
+    Ns *= R;
+  }
+}
+
 }  // namespace
 
 bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, StageDesc* d) {
@@ -247,18 +261,9 @@ bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, StageDesc* d) 
   if (L < 2 || L > kStageElems || plans.count[L] == 0xff || plans.count[L] > kStageMax) return false;
   memset(d, 0, sizeof(*d));
   d->L = (int)L;
-  int Ns = 1;
   for (int n = (int)L; n > 1; n /= plans.first[n]) d->radix[d->nst++] = plans.first[n];
   std::sort(d->radix, d->radix + d->nst, [](int a, int b) { return a > b; });
-  for (int s = 0; s < d->nst; ++s) {
-    const int R = d->radix[s];
-    d->nbf[s] = (int)L / R;
-    d->Ns[s] = Ns;
-    d->nbf_magic[s] = magic_of(d->nbf[s]);
-    d->Ns_magic[s] = magic_of(Ns);
-    d->tw_step[s] = (int)L / (Ns * R);
-    Ns *= R;
-  }
+  fill_stages(d);
   // as many transforms as the buffer holds, fewer when the grid would not reach two CTAs an SM
   int lg = 0;
   while ((L << (lg + 1)) <= kStageElems && lg < 8 && (int64_t(1) << lg) < nb) ++lg;
@@ -269,12 +274,19 @@ bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, StageDesc* d) 
   return true;
 }
 
+StageDesc stage_reversed(const StageDesc& d) {
+  StageDesc r = d;
+  std::reverse(r.radix, r.radix + r.nst);
+  fill_stages(&r);
+  return r;
+}
+
 // Threads of a CTA: every butterfly of the widest stage at once, up to kStageThreads.
 int stage_threads(const StageDesc& d) {
-  const int want = d.nbf[d.nst - 1] << d.bpc_log2;
+  const int want = std::max(d.nbf[0], d.nbf[d.nst - 1]) << d.bpc_log2;
   return std::max(64, std::min(kStageThreads, (want + 31) / 32 * 32));
 }
-size_t stage_smem(const StageDesc& d) { return sizeof(float2) * (size_t)d.bpc * d.SS; }
+size_t stage_smem_bytes(const StageDesc& d) { return sizeof(float2) * (size_t)d.bpc * d.SS; }
 
 namespace {
 
@@ -333,7 +345,7 @@ __device__ __forceinline__ float2 twiddle_at(const TwiddleTables& t, int i, int 
   return make_float2(h.x + fmaf(h.x, e.x, fmaf(-h.y, e.y, h.z)), h.y + fmaf(h.x, e.y, fmaf(h.y, e.x, h.w)));
 }
 
-template <int SIGN, int IN, int OUT>
+template <int SIGN, int IN, int OUT, bool PAD>
 __global__ void __launch_bounds__(kStageThreads, 2) fft_stage_kernel(const __grid_constant__ StageArgs a) {
   extern __shared__ float4 sm4[];
   float2* const sm = reinterpret_cast<float2*>(sm4);
@@ -352,50 +364,68 @@ __global__ void __launch_bounds__(kStageThreads, 2) fft_stage_kernel(const __gri
     const float2* const in = static_cast<const float2*>(a.in) + b0 * a.is0 + b1_0 * a.is1;
     float2* const out = static_cast<float2*>(a.out) + b0 * a.os0 + b1_0 * a.os1;
     const float2* const mul = a.mul ? a.mul + b0 * a.os0 + b1_0 * a.os1 : nullptr;
-    auto get = [&](int i, int l) -> float2 {
-      if (i >= nb) return make_float2(0.f, 0.f);
-      if (IN == kInComplex) return in[i * a.is1 + l * a.isl];
-      const long long n = (b1_0 + i) * a.is1 + l * a.isl;
+    // rows past the last transform read the last one's values and write nothing
+    auto get = [&](int i0) {
+      const int i = min(i0, nb - 1);
       const long long c = 2 * (a.p0 + (a.pair_b1 ? b1_0 + i : b0));
-      if (IN == kInRealPair) {
-        const float* p = static_cast<const float*>(a.in) + n + c * a.ldi;
-        return make_float2(p[0], c + 1 < a.ncol ? p[a.ldi] : 0.f);
-      }
-      // S_a + i S_b of bin n, from the conjugates of bin N - n above K; the imaginary parts of
-      // bin 0 and, for even N, bin N/2 do not enter
-      const bool upper = n >= a.K;
-      const long long k = upper ? a.N - n : n;
-      const float2* p = static_cast<const float2*>(a.in) + k + c * a.ldi;
-      float2 u = p[0], w = c + 1 < a.ncol ? p[a.ldi] : make_float2(0.f, 0.f);
-      if (k == 0 || 2 * k == a.N) u.y = w.y = 0.f;
-      if (upper) { u.y = -u.y; w.y = -w.y; }
-      return make_float2(u.x - w.y, u.y + w.x);
+      const int n0 = a.pair_b1 ? 0 : (int)b1_0 + i, N = (int)a.N, K = (int)a.K, isl = (int)a.isl;
+      const bool has1 = c + 1 < a.ncol;
+      const float2* const row = in + i * a.is1;
+      const float* const ra = static_cast<const float*>(a.in) + c * a.ldi;
+      const float* const rb = has1 ? ra + a.ldi : ra;
+      const float2* const sa = static_cast<const float2*>(a.in) + c * a.ldi;
+      const float2* const sb = has1 ? sa + a.ldi : sa;
+      return [=](int l) -> float2 {
+        if (IN == kInComplex) return row[l * (long long)isl];
+        const int n = n0 + l * isl;
+        if (IN == kInRealPair) {
+          const float x = __ldg(ra + n), y = __ldg(rb + n);
+          return make_float2(x, has1 ? y : 0.f);
+        }
+        // S_a + i S_b of bin n, from the conjugates of bin N - n above K; the imaginary parts
+        // of bin 0 and, for even N, bin N/2 do not enter
+        const bool upper = n >= K;
+        const int k = upper ? N - n : n;
+        const float2 u = __ldg(sa + k), w = __ldg(sb + k);
+        const bool real = k == 0 || 2 * k == N;
+        const float uy = real ? 0.f : (upper ? -u.y : u.y);
+        const float wy = real || !has1 ? 0.f : (upper ? -w.y : w.y);
+        return make_float2(u.x - wy, uy + (has1 ? w.x : 0.f));
+      };
     };
-    auto put = [&](int i, int l, float2 v) {
-      if (i >= nb) return;
-      if (OUT == kOutRealPair) {
-        const long long n = (b1_0 + i) * a.os1 + l * a.osl;
-        const long long c = 2 * (a.p0 + (a.pair_b1 ? b1_0 + i : b0));
-        float* p = static_cast<float*>(a.out) + n + c * a.ldo;
-        v = cscale(v, a.scale);
-        p[0] = v.x;
-        if (c + 1 < a.ncol) p[a.ldo] = v.y;
-        return;
-      }
-      if (OUT == kOutTwiddle) {
-        v = cmul(v, twiddle_at(tw, i, l));
-      } else {
-        if (mul) v = cmul(v, mul[i * a.os1 + l * a.osl]);
-        v = cscale(v, a.scale);
-      }
-      out[i * a.os1 + l * a.osl] = v;
+    auto put = [&](int i) {
+      const bool live = i < nb;
+      const long long c = 2 * (a.p0 + (a.pair_b1 ? b1_0 + i : b0));
+      const int n0 = a.pair_b1 ? 0 : (int)b1_0 + i, osl = (int)a.osl;
+      const bool has1 = live && c + 1 < a.ncol;
+      float2* const row = out + i * a.os1;
+      const float2* const mrow = mul ? mul + i * a.os1 : nullptr;
+      float* const ra = static_cast<float*>(a.out) + c * a.ldo;
+      const float scale = a.scale;
+      const TwiddleTables t = tw;
+      return [=](int l, float2 v) {
+        if (OUT == kOutRealPair) {
+          v = cscale(v, scale);
+          if (live) ra[n0 + l * osl] = v.x;
+          if (has1) ra[n0 + l * osl + a.ldo] = v.y;
+          return;
+        }
+        if (OUT == kOutTwiddle) {
+          v = cmul(v, twiddle_at(t, i, l));
+        } else {
+          if (mrow && live) v = cmul(v, __ldg(mrow + l * (long long)osl));
+          v = cscale(v, scale);
+        }
+        if (live) row[l * (long long)osl] = v;
+      };
     };
-    stages_run<SIGN>(d, a.in_lane_i, a.out_lane_i, sm, get, put);
+    stages_run<SIGN, PAD>(d, a.in_lane_i, a.out_lane_i, sm, get, put);
     if (b0 + gridDim.y < a.nb0) __syncthreads();  // the last stage has read shared memory
   }
 }
 
-template <int SIGN, int IN, int OUT>
+// PAD: a stage runs with neighbouring threads on neighbouring elements.
+template <int SIGN, int IN, int OUT, bool PAD>
 int launch_stages(StageArgs& a, cudaStream_t s) {
   if (a.nb0 <= 0 || a.nb1 <= 0) return FDR_OK;
   FDR_TRY(get_roots(a.d.L, &a.d.roots));
@@ -403,13 +433,13 @@ int launch_stages(StageArgs& a, cudaStream_t s) {
   int dev = 0;
   FDR_CUDA(cudaGetDevice(&dev));
   if (dev >= 64 || !attr_set[dev]) {
-    FDR_CUDA(cudaFuncSetAttribute(fft_stage_kernel<SIGN, IN, OUT>,
+    FDR_CUDA(cudaFuncSetAttribute(fft_stage_kernel<SIGN, IN, OUT, PAD>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
     if (dev < 64) attr_set[dev] = true;
   }
-  const size_t smem = stage_smem(a.d) + (OUT == kOutTwiddle ? tw_bytes(a.d.L, a.d.bpc) : 0);
+  const size_t smem = stage_smem_bytes(a.d) + (OUT == kOutTwiddle ? tw_bytes(a.d.L, a.d.bpc) : 0);
   const dim3 grid((unsigned)cdiv(a.nb1, a.d.bpc), (unsigned)std::min(a.nb0, 65535LL));
-  fft_stage_kernel<SIGN, IN, OUT><<<grid, stage_threads(a.d), smem, s>>>(a);
+  fft_stage_kernel<SIGN, IN, OUT, PAD><<<grid, stage_threads(a.d), smem, s>>>(a);
   FDR_LAUNCH_CHECK("fft_stage_kernel");
   return FDR_OK;
 }
@@ -437,10 +467,10 @@ int fft_strided_inplace(float2* buf, long long L, long long sl, long long nb, lo
     a.nb1 = nb;
     a.is1 = a.os1 = sb;
     a.isl = a.osl = sl;
-    a.in_lane_i = a.out_lane_i = sb == 1;
+    a.in_lane_i = a.out_lane_i = 1;
     a.scale = scale;
-    return sign < 0 ? launch_stages<-1, kInComplex, kOutComplex>(a, s)
-                    : launch_stages<+1, kInComplex, kOutComplex>(a, s);
+    return sign < 0 ? launch_stages<-1, kInComplex, kOutComplex, false>(a, s)
+                    : launch_stages<+1, kInComplex, kOutComplex, false>(a, s);
   }
   PassDesc d = blank_pass();
   d.in = buf; d.out = buf; d.mul = mul;
@@ -613,10 +643,10 @@ static int real_stages(bool forward, const void* in, long long ldin, void* out, 
     *done = true;
     if (forward) {
       a.os1 = N;
-      return launch_stages<-1, kInRealPair, kOutComplex>(a, s);
+      return launch_stages<-1, kInRealPair, kOutComplex, true>(a, s);
     }
     a.scale = 1.f / (float)N;
-    return launch_stages<+1, kInHalfPair, kOutRealPair>(a, s);
+    return launch_stages<+1, kInHalfPair, kOutRealPair, true>(a, s);
   }
   long long L1, L2;
   split_len(N, &L1, &L2);
@@ -633,8 +663,8 @@ static int real_stages(bool forward, const void* in, long long ldin, void* out, 
   a.os1 = 1;
   a.osl = L2;
   a.in_lane_i = a.out_lane_i = 1;
-  FDR_TRY((forward ? launch_stages<-1, kInRealPair, kOutTwiddle>(a, s)
-                   : launch_stages<+1, kInHalfPair, kOutTwiddle>(a, s)));
+  FDR_TRY((forward ? launch_stages<-1, kInRealPair, kOutTwiddle, false>(a, s)
+                   : launch_stages<+1, kInHalfPair, kOutTwiddle, false>(a, s)));
   // Pass 2: for each k1, DFT over n2 (contiguous), bin or channel k1 + L1*k2
   b.in = tmp;
   b.out = out;
@@ -647,9 +677,9 @@ static int real_stages(bool forward, const void* in, long long ldin, void* out, 
   b.os1 = 1;
   b.osl = L1;
   b.out_lane_i = 1;
-  if (forward) return launch_stages<-1, kInComplex, kOutComplex>(b, s);
+  if (forward) return launch_stages<-1, kInComplex, kOutComplex, true>(b, s);
   b.scale = 1.f / (float)N;
-  return launch_stages<+1, kInComplex, kOutRealPair>(b, s);
+  return launch_stages<+1, kInComplex, kOutRealPair, true>(b, s);
 }
 
 int rfft_columns(const float* in, long long ldin, long long ncol, long long N, float2* F,

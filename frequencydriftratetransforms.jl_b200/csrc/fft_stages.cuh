@@ -109,7 +109,8 @@ template <> struct Dft<13> : DftPrime<13, CosSin13> {};
 // one buffer is enough and two CTAs share an SM.  The first stage takes its inputs straight
 // from global memory and the last one hands its outputs to global memory: a transform of n
 // stages crosses shared memory n - 1 times.
-// Element l of transform i is at i * SS + pidx(l).  SS = 16 / bpc (mod 16) (1 from bpc = 16
+// Element l of transform i is at i * SS + l, or i * SS + pidx(l) when a stage runs with
+// neighbouring threads on neighbouring elements (PAD).  SS = 16 / bpc (mod 16) (1 from bpc = 16
 // on): a half-warp of neighbouring transforms (lanes over i) and one of neighbouring elements
 // (lanes over l) both meet 16 different 8-byte banks.
 // ------------------------------------------------------------------------------------
@@ -134,11 +135,13 @@ __device__ __forceinline__ int div_magic(int n, unsigned magic) {
   return magic ? (int)__umulhi((unsigned)n, magic) : n;
 }
 
-// Reads, transforms and hands on the butterflies of stage s.  get(i, l, n) gives the value of
-// element l of transform i at the first stage (n: the butterfly's first element, l = n + r *
-// nbf), put(i, l, v) takes it at the last.  lane_i: neighbouring threads take neighbouring
-// transforms (else neighbouring elements).
-template <int R, int SIGN, class Get, class Put>
+template <bool PAD>
+__device__ __forceinline__ int sidx(int l) { return PAD ? pidx(l) : l; }
+
+// Reads, transforms and hands on the butterflies of stage s.  get(i)(l) gives element l of
+// transform i at the first stage, put(i)(l, v) takes it at the last.  lane_i: neighbouring
+// threads take neighbouring transforms (else neighbouring elements).
+template <int R, int SIGN, bool PAD, class Get, class Put>
 __device__ __forceinline__ void stage_run(const StageDesc& d, int s, bool lane_i, bool first, bool last,
                                           float2* sm, Get get, Put put) {
   constexpr int PER = (32 + R - 1) / R;
@@ -152,12 +155,13 @@ __device__ __forceinline__ void stage_run(const StageDesc& d, int s, bool lane_i
       const int i = lane_i ? j & (d.bpc - 1) : div_magic(j, d.nbf_magic[s]);
       const int jj = lane_i ? j >> d.bpc_log2 : j - i * nbf;
       if (first) {
+        auto row = get(i);
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[p][r] = get(i, jj + r * nbf);
+        for (int r = 0; r < R; ++r) v[p][r] = row(jj + r * nbf);
       } else {
         const float2* a = sm + i * SS;
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[p][r] = a[pidx(jj + r * nbf)];
+        for (int r = 0; r < R; ++r) v[p][r] = a[sidx<PAD>(jj + r * nbf)];
       }
     } else {  // no value may live on from the stage before
 #pragma unroll
@@ -185,13 +189,14 @@ __device__ __forceinline__ void stage_run(const StageDesc& d, int s, bool lane_i
       }
       Dft<R>::run(v[p], SIGN);
       if (last) {
+        auto row = put(i);
 #pragma unroll
-        for (int r = 0; r < R; ++r) put(i, jj + r * nbf, v[p][r]);
+        for (int r = 0; r < R; ++r) row(jj + r * nbf, v[p][r]);
       } else {
         float2* o = sm + i * SS;
         const int base = b * Ns * R + k;
 #pragma unroll
-        for (int r = 0; r < R; ++r) o[pidx(base + r * Ns)] = v[p][r];
+        for (int r = 0; r < R; ++r) o[sidx<PAD>(base + r * Ns)] = v[p][r];
       }
     }
   }
@@ -201,14 +206,100 @@ __device__ __forceinline__ void stage_run(const StageDesc& d, int s, bool lane_i
 #define FDR_FOR_RADIX(X) X(16) X(13) X(11) X(10) X(9) X(8) X(7) X(6) X(5) X(4) X(3) X(2)
 
 // All stages of d; the block must be synchronised before if shared memory is still being read.
-template <int SIGN, class Get, class Put>
+template <int SIGN, bool PAD, class Get, class Put>
 __device__ __forceinline__ void stages_run(const StageDesc& d, bool first_lane_i, bool last_lane_i,
                                            float2* sm, Get get, Put put) {
   for (int s = 0; s < d.nst; ++s) {
     const bool first = s == 0, last = s == d.nst - 1;
-    const bool lane_i = first ? first_lane_i : (last ? last_lane_i : d.bpc >= 8);
+    const bool lane_i = first ? first_lane_i : (last ? last_lane_i : !PAD || d.bpc >= 8);
     switch (d.radix[s]) {
-#define FDR_STAGE(R) case R: stage_run<R, SIGN>(d, s, lane_i, first, last, sm, get, put); break;
+#define FDR_STAGE(R) case R: stage_run<R, SIGN, PAD>(d, s, lane_i, first, last, sm, get, put); break;
+      FDR_FOR_RADIX(FDR_STAGE)
+#undef FDR_STAGE
+    }
+  }
+}
+
+// One stage within shared memory, neighbouring threads on neighbouring transforms.  TURN: the
+// last forward stage, the product with factor(i)(l) and the first backward stage of a plan
+// whose radices run the other way, which takes the same elements (a convolution's middle).
+template <int R, int SIGN, bool TURN, class Factor>
+__device__ __forceinline__ void stage_smem(const StageDesc& d, int s, float2* sm, Factor factor) {
+  constexpr int PER = (32 + R - 1) / R;
+  const int nbf = d.nbf[s], Ns = d.Ns[s], SS = d.SS;
+  const int total = nbf << d.bpc_log2;
+  float2 v[PER][R];
+#pragma unroll
+  for (int p = 0; p < PER; ++p) {
+    const int j = threadIdx.x + p * blockDim.x;
+    if (j < total) {
+      const float2* a = sm + (j & (d.bpc - 1)) * SS + (j >> d.bpc_log2);
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[p][r] = a[r * nbf];
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[p][r] = make_float2(0.f, 0.f);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int p = 0; p < PER; ++p) {
+    const int j = threadIdx.x + p * blockDim.x;
+    if (j < total) {
+      const int i = j & (d.bpc - 1), jj = j >> d.bpc_log2;
+      const int b = div_magic(jj, d.Ns_magic[s]);
+      const int k = jj - b * Ns;
+      float2 f[TURN ? R : 1];
+      if (TURN) {
+        auto row = factor(i);
+#pragma unroll
+        for (int r = 0; r < R; ++r) f[r] = row(jj + r * nbf);
+      }
+      if (Ns > 1) {
+        const int step = k * d.tw_step[s];
+#pragma unroll
+        for (int r = 1; r < R; ++r) {
+          float2 t = __ldg(d.roots + r * step);
+          if (SIGN > 0) t.y = -t.y;
+          v[p][r] = cmul(v[p][r], t);
+        }
+      }
+      Dft<R>::run(v[p], SIGN);
+      if (TURN) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[p][r] = cmul(v[p][r], f[r]);
+        Dft<R>::run(v[p], -SIGN);
+      }
+      float2* o = sm + i * SS + (TURN ? jj * R : b * Ns * R + k);
+      const int ostep = TURN ? 1 : Ns;
+#pragma unroll
+      for (int r = 0; r < R; ++r) o[r * ostep] = v[p][r];
+    }
+  }
+  __syncthreads();
+}
+
+// Circular convolution of the transforms in shared memory (element l of transform i at
+// i * SS + l) with the spectrum factor(i)(l), unnormalised: the stages of fwd, the turn, the
+// remaining stages of inv, whose radices are fwd's in reverse.
+template <class Factor>
+__device__ __forceinline__ void convolve_smem(const StageDesc& fwd, const StageDesc& inv, float2* sm,
+                                              Factor factor) {
+  for (int s = 0; s + 1 < fwd.nst; ++s) {
+    switch (fwd.radix[s]) {
+#define FDR_STAGE(R) case R: stage_smem<R, -1, false>(fwd, s, sm, factor); break;
+      FDR_FOR_RADIX(FDR_STAGE)
+#undef FDR_STAGE
+    }
+  }
+  switch (fwd.radix[fwd.nst - 1]) {
+#define FDR_STAGE(R) case R: stage_smem<R, -1, true>(fwd, fwd.nst - 1, sm, factor); break;
+    FDR_FOR_RADIX(FDR_STAGE)
+#undef FDR_STAGE
+  }
+  for (int s = 1; s < inv.nst; ++s) {
+    switch (inv.radix[s]) {
+#define FDR_STAGE(R) case R: stage_smem<R, +1, false>(inv, s, sm, factor); break;
       FDR_FOR_RADIX(FDR_STAGE)
 #undef FDR_STAGE
     }
@@ -219,7 +310,9 @@ __device__ __forceinline__ void stages_run(const StageDesc& d, bool first_lane_i
 // neighbouring addresses (rows: CTAs then take at least 8 of them, 64 bytes a row); false if L
 // has a prime factor above 13 or exceeds kStageElems.
 bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, StageDesc* d);
-size_t stage_smem(const StageDesc& d);
+// The plan whose stages run in the reverse order.
+StageDesc stage_reversed(const StageDesc& d);
+size_t stage_smem_bytes(const StageDesc& d);
 int stage_threads(const StageDesc& d);
 
 }  // namespace fdr

@@ -32,23 +32,40 @@ __device__ __forceinline__ float2 phasor_ref(long long k, long long t, float r, 
   return cispif(x);
 }
 
-// S[k + jj*K] = sum_t F[k, t] * phasor(k, t, r_jj)
-__global__ void phasor_sum_kernel(const float2* __restrict__ F, long long K, long long Nt,
-                                  long long Nf, int nr, float2* __restrict__ S,
-                                  const __grid_constant__ RateParams rp) {
-  const long long total = K * nr;
-  const float Nf_f = __ll2float_rn(Nf);
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long jj = e / K, k = e - jj * K;
-    const float r = rp.r[jj];
-    float2 acc = make_float2(0.f, 0.f);
-    for (long long t = 0; t < Nt; ++t) {
-      float2 p = cmul_rn(F[k + t * K], phasor_ref(k, t, r, Nf_f));
-      acc = make_float2(__fadd_rn(acc.x, p.x), __fadd_rn(acc.y, p.y));
+// S[k + jj*K] = sum_t F[k, t] * phasor(k, t, r_jj).  A thread takes one bin and kRatesPerThread
+// rates, so F is read once for all of them; the time goes to sincospif, one for each (k, t, r).
+// The phasor's argument is formed by the same rounded operations as phasor_ref with cheaper
+// instructions where they give the same value: for MULT (2k and t exact in Float32) the rounded
+// product Float32(2k) * Float32(t) is Float32(2kt), and for a power-of-two Nf the quotient is
+// the product with 1 / Nf.
+constexpr int kRatesPerThread = 8;
+
+template <bool MULT, bool POW2>
+__global__ void __launch_bounds__(256) phasor_sum_kernel(const float2* __restrict__ F, long long K, int Nt,
+                                                         long long Nf, int nr, float2* __restrict__ S,
+                                                         const __grid_constant__ RateParams rp) {
+  const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (k >= K) return;
+  const int j0 = blockIdx.y * kRatesPerThread;
+  const float Nf_f = __ll2float_rn(Nf), inv = 1.f / Nf_f, k2 = __ll2float_rn(2 * k);
+  float2 acc[kRatesPerThread];
+#pragma unroll
+  for (int q = 0; q < kRatesPerThread; ++q) acc[q] = make_float2(0.f, 0.f);
+  for (int t = 0; t < Nt; ++t) {
+    const float2 f = __ldg(F + k + t * K);
+    const float kt = MULT ? __fmul_rn(k2, (float)t) : __ll2float_rn(2 * k * t);
+#pragma unroll
+    for (int q = 0; q < kRatesPerThread; ++q) {
+      if (j0 + q < nr) {
+        const float x = __fmul_rn(kt, rp.r[j0 + q]);
+        const float2 p = cmul_rn(f, cispif(POW2 ? __fmul_rn(x, inv) : __fdiv_rn(x, Nf_f)));
+        acc[q] = make_float2(__fadd_rn(acc[q].x, p.x), __fadd_rn(acc[q].y, p.y));
+      }
     }
-    S[e] = acc;
   }
+#pragma unroll
+  for (int q = 0; q < kRatesPerThread; ++q)
+    if (j0 + q < nr) S[k + (j0 + q) * K] = acc[q];
 }
 
 // P[k, t] = F[k, t] * phasor(k, t, r)
@@ -158,7 +175,11 @@ int fdr_fftfdr(fdr_fft_ws* ws, const float* rates, int64_t Nr, float* fdr, fdr_s
     const int nr = (int)std::min<int64_t>(kRateChunk, Nr - j0);
     memset(&rp, 0, sizeof(rp));
     for (int i = 0; i < nr; ++i) rp.r[i] = rates[j0 + i];
-    phasor_sum_kernel<<<grid_1d(ws->K * nr), 256, 0, s>>>(ws->F, ws->K, ws->Nt, ws->Nf, nr, ws->S, rp);
+    const bool mult = 2 * ws->K < (1LL << 24) && ws->Nt < (1LL << 24);
+    const dim3 grid((unsigned)cdiv(ws->K, 256), (unsigned)cdiv(nr, kRatesPerThread));
+    auto kernel = mult ? (is_pow2(ws->Nf) ? phasor_sum_kernel<true, true> : phasor_sum_kernel<true, false>)
+                       : (is_pow2(ws->Nf) ? phasor_sum_kernel<false, true> : phasor_sum_kernel<false, false>);
+    kernel<<<grid, 256, 0, s>>>(ws->F, ws->K, (int)ws->Nt, ws->Nf, nr, ws->S, rp);
     FDR_LAUNCH_CHECK("phasor_sum_kernel");
     FDR_TRY(irfft_columns(ws->S, ws->K, nr, ws->Nf, fdr + j0 * ws->Nf, ws->Nf, ws->rscratch,
                           ws->rscratch_pairs, s));

@@ -12,6 +12,7 @@
 #include <string.h>
 
 #include "fft_engine.cuh"
+#include "fft_stages.cuh"
 #include "zdt_ws.cuh"
 
 namespace fdr {
@@ -85,7 +86,24 @@ __global__ void zdt_vinit_kernel(float2* __restrict__ V, long long K, long long 
   }
 }
 
-// window: 0 rect, 1 hamming, 2 custom (float64 values w[k])
+// Ys * cispi(...) * w(k, Nf).  window: 0 rect, 1 hamming, 2 custom (float64 values w[k])
+__device__ __forceinline__ float2 postprocess_value(float2 y, float2 ph, long long k, long long Nf, int window,
+                                                    const double* wk) {
+  if (window == 0) return cmul_rn(y, ph);
+  // cispi(...)::ComplexF32 * w(k, Nf)::Float64 promotes to ComplexF64 and the product
+  // with Ys is rounded to ComplexF32 on store (zdtfdr.jl:268-270, :299-300).
+  double w;
+  if (window == 1) {
+    double x = 2.0 * (double)k / (double)Nf;
+    w = 0.53836 + 0.46164 * cospi(x);
+  } else {
+    w = wk[k];
+  }
+  double cr = (double)ph.x * w, ci = (double)ph.y * w;
+  double yr = (double)y.x, yi = (double)y.y;
+  return make_float2((float)(yr * cr - yi * ci), (float)(yr * ci + yi * cr));
+}
+
 __global__ void zdt_postprocess_kernel(float2* __restrict__ Y, long long K, long long Nr,
                                        long long Nf, float dr, int exact, int window,
                                        const double* __restrict__ wk) {
@@ -95,23 +113,60 @@ __global__ void zdt_postprocess_kernel(float2* __restrict__ Y, long long K, long
        e += (long long)gridDim.x * blockDim.x) {
     const long long l = e / K, k = e - l * K;
     float2 ph = exact ? postphase_exact(k, l, dr, (double)Nf) : postphase_ref(k, l, dr, Nf_f);
-    float2 y = Y[e];
-    if (window == 0) {
-      Y[e] = cmul_rn(y, ph);
-    } else {
-      // cispi(...)::ComplexF32 * w(k, Nf)::Float64 promotes to ComplexF64 and the product
-      // with Ys is rounded to ComplexF32 on store (zdtfdr.jl:268-270, :299-300).
-      double w;
-      if (window == 1) {
-        double x = 2.0 * (double)k / (double)Nf;
-        w = 0.53836 + 0.46164 * cospi(x);
-      } else {
-        w = wk[k];
-      }
-      double cr = (double)ph.x * w, ci = (double)ph.y * w;
-      double yr = (double)y.x, yi = (double)y.y;
-      Y[e] = make_float2((float)(yr * cr - yi * ci), (float)(yr * ci + yi * cr));
+    Y[e] = postprocess_value(Y[e], ph, k, Nf, window, wk);
+  }
+}
+
+// preprocess!, convolve! and postprocess! of a block of bins in one CTA: each bin's Nl values
+// stay in shared memory between the prephase and the postphase, where the staged functions move
+// all of Y through device memory six times.  Per element the same rounded operations as
+// zdt_preprocess_kernel, the convolution's two transforms and zdt_postprocess_kernel; columns
+// past Nr receive what convolve! leaves there.
+struct ConvArgs {
+  StageDesc fwd, inv;
+  const float2* F;
+  const float2* V;
+  float2* Y;
+  const double* wk;
+  long long K, Nf;
+  int Nt, Nr, Nl, exact, window;
+  float r0, dr;
+};
+
+__global__ void __launch_bounds__(kStageThreads, 2) zdt_conv_kernel(const __grid_constant__ ConvArgs a) {
+  extern __shared__ float2 sm[];
+  const StageDesc& d = a.fwd;
+  const int bpc = d.bpc, lg = d.bpc_log2, SS = d.SS;
+  const long long k0 = (long long)blockIdx.x << lg, K = a.K;
+  const int nb = (int)min((long long)bpc, K - k0);
+  const float Nf_f = __ll2float_rn(a.Nf);
+  // the last bin stands in for bins past it, which are not stored
+#pragma unroll 4
+  for (int e = threadIdx.x; e < a.Nt << lg; e += blockDim.x) {
+    const int i = e & (bpc - 1), l = e >> lg;
+    const long long k = k0 + min(i, nb - 1);
+    const float2 ph = a.exact ? prephase_exact(k, l, a.r0, a.dr, (double)a.Nf)
+                              : prephase_ref(k, l, a.r0, a.dr, Nf_f);
+    sm[i * SS + l] = cmul_rn(__ldg(a.F + k + l * K), ph);
+  }
+  for (int e = (a.Nt << lg) + threadIdx.x; e < a.Nl << lg; e += blockDim.x)
+    sm[(e & (bpc - 1)) * SS + (e >> lg)] = make_float2(0.f, 0.f);
+  __syncthreads();
+  convolve_smem(a.fwd, a.inv, sm, [&](int i) {
+    const float2* const v = a.V + k0 + min(i, nb - 1);
+    return [=](int l) { return __ldg(v + l * K); };
+  });
+  const float scale = 1.f / (float)a.Nl;
+#pragma unroll 4
+  for (int e = threadIdx.x; e < a.Nl << lg; e += blockDim.x) {
+    const int i = e & (bpc - 1), l = e >> lg;
+    const long long k = k0 + i;
+    float2 y = cscale(sm[i * SS + l], scale);
+    if (l < a.Nr) {
+      const float2 ph = a.exact ? postphase_exact(k, l, a.dr, (double)a.Nf) : postphase_ref(k, l, a.dr, Nf_f);
+      y = postprocess_value(y, ph, i < nb ? k : 0, a.Nf, a.window, a.wk);
     }
+    if (i < nb) a.Y[k + l * K] = y;
   }
 }
 
@@ -225,14 +280,46 @@ static int zdt_compute_V(fdr_zdt* ws, cudaStream_t s) {
   return fft_strided_inplace(ws->V, ws->Nl, ws->K, ws->K, 1, -1, 1.f, nullptr, s);
 }
 
+// preprocess!, convolve! and postprocess! in one kernel (*done); a chirp length with a prime
+// factor above 13 takes the three functions.
+static int zdt_conv(fdr_zdt* ws, float r0, int window, const double* wk, cudaStream_t s, bool* done) {
+  *done = false;
+  ConvArgs a;
+  memset(&a, 0, sizeof(a));
+  if (!stage_plan(ws->Nl, ws->K, 1, true, &a.fwd)) return FDR_OK;
+  FDR_TRY(zdt_ensure_staged(ws, s));
+  FDR_TRY(zdt_ensure_F(ws, s));
+  FDR_TRY(get_roots(ws->Nl, &a.fwd.roots));
+  a.inv = stage_reversed(a.fwd);
+  a.F = ws->F; a.V = ws->V; a.Y = ws->Y; a.wk = wk;
+  a.K = ws->K; a.Nf = ws->Nf;
+  a.Nt = (int)ws->Nt; a.Nr = (int)ws->Nr; a.Nl = (int)ws->Nl;
+  a.exact = (ws->flags & FDR_ZDT_EXACT_PHASE) ? 1 : 0;
+  a.window = window;
+  a.r0 = r0; a.dr = ws->dr;
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  FDR_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !attr_set[dev]) {
+    FDR_CUDA(cudaFuncSetAttribute(zdt_conv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
+    if (dev < 64) attr_set[dev] = true;
+  }
+  zdt_conv_kernel<<<(unsigned)cdiv(ws->K, a.fwd.bpc), stage_threads(a.fwd), stage_smem_bytes(a.fwd), s>>>(a);
+  FDR_LAUNCH_CHECK("zdt_conv_kernel");
+  *done = true;
+  return FDR_OK;
+}
+
 // One staged ZDT (zdtfdr.jl:355-358) for a given r0 into dest.
 int zdt_staged_run(fdr_zdt* ws, float r0, float* dest, int window, const double* wk, double* acc,
                    cudaStream_t s) {
-  FDR_TRY(zdt_preprocess(ws, r0, s));
-  zdt_mark(ws, "preprocess", s);
-  FDR_TRY(zdt_convolve(ws, s));
+  bool done;
+  FDR_TRY(zdt_conv(ws, r0, window, wk, s, &done));
+  if (!done) FDR_TRY(zdt_preprocess(ws, r0, s));
+  zdt_mark(ws, "preprocess", s);  // with convolve! and postprocess! where one kernel runs all
+  if (!done) FDR_TRY(zdt_convolve(ws, s));
   zdt_mark(ws, "convolve", s);
-  FDR_TRY(zdt_postprocess(ws, window, wk, s));
+  if (!done) FDR_TRY(zdt_postprocess(ws, window, wk, s));
   zdt_mark(ws, "postprocess", s);
   FDR_TRY(zdt_output(ws, dest, s));
   if (acc) FDR_TRY(moments_accumulate(dest, ws->Nf, ws->Nr, acc, s));
