@@ -240,20 +240,6 @@ struct StagePlans {
 
 unsigned magic_of(int d) { return d == 1 ? 0u : (unsigned)(((1ULL << 32) + d - 1) / d); }
 
-// The fields that follow from L and the radices.
-void fill_stages(StageDesc* d) {
-  int Ns = 1;
-  for (int s = 0; s < d->nst; ++s) {
-    const int R = d->radix[s];
-    d->nbf[s] = d->L / R;
-    d->Ns[s] = Ns;
-    d->nbf_magic[s] = magic_of(d->nbf[s]);
-    d->Ns_magic[s] = magic_of(Ns);
-    d->tw_step[s] = d->L / (Ns * R);
-    Ns *= R;
-  }
-}
-
 }  // namespace
 
 bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, StageDesc* d) {
@@ -263,27 +249,31 @@ bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, StageDesc* d) 
   d->L = (int)L;
   for (int n = (int)L; n > 1; n /= plans.first[n]) d->radix[d->nst++] = plans.first[n];
   std::sort(d->radix, d->radix + d->nst, [](int a, int b) { return a > b; });
-  fill_stages(d);
+  int Ns = 1;
+  for (int s = 0; s < d->nst; ++s) {
+    const int R = d->radix[s];
+    d->nbf[s] = d->L / R;
+    d->Ns[s] = Ns;
+    d->step[s] = d->L / (Ns * R);
+    d->digit[s] = d->step[s];
+    d->radix_magic[s] = magic_of(R);
+    d->nbf_magic[s] = magic_of(d->nbf[s]);
+    Ns *= R;
+  }
+  d->pitch = d->digit[0] = d->nbf[0] | 1;
   // as many transforms as the buffer holds, fewer when the grid would not reach two CTAs an SM
   int lg = 0;
   while ((L << (lg + 1)) <= kStageElems && lg < 8 && (int64_t(1) << lg) < nb) ++lg;
   while (lg > (rows ? 3 : 0) && cdiv(nb, int64_t(1) << lg) * groups < 2LL * sm_count()) --lg;
   d->bpc_log2 = lg;
   d->bpc = 1 << lg;
-  d->SS = (padlen((int)L) / 16 + 1) * 16 + (d->bpc >= 16 ? 1 : 16 / d->bpc);
+  d->SS = (d->radix[0] * d->pitch + 15) / 16 * 16 + (d->bpc >= 16 ? 1 : 16 / d->bpc);
   return true;
 }
 
-StageDesc stage_reversed(const StageDesc& d) {
-  StageDesc r = d;
-  std::reverse(r.radix, r.radix + r.nst);
-  fill_stages(&r);
-  return r;
-}
-
-// Threads of a CTA: every butterfly of the widest stage at once, up to kStageThreads.
+// Threads of a CTA: two rounds of butterflies of the widest stage, up to kStageThreads.
 int stage_threads(const StageDesc& d) {
-  const int want = std::max(d.nbf[0], d.nbf[d.nst - 1]) << d.bpc_log2;
+  const int want = (d.nbf[d.nst - 1] << d.bpc_log2) / 2;
   return std::max(64, std::min(kStageThreads, (want + 31) / 32 * 32));
 }
 size_t stage_smem_bytes(const StageDesc& d) { return sizeof(float2) * (size_t)d.bpc * d.SS; }
@@ -345,8 +335,8 @@ __device__ __forceinline__ float2 twiddle_at(const TwiddleTables& t, int i, int 
   return make_float2(h.x + fmaf(h.x, e.x, fmaf(-h.y, e.y, h.z)), h.y + fmaf(h.x, e.y, fmaf(h.y, e.x, h.w)));
 }
 
-template <int SIGN, int IN, int OUT, bool PAD>
-__global__ void __launch_bounds__(kStageThreads, 2) fft_stage_kernel(const __grid_constant__ StageArgs a) {
+template <int SIGN, int IN, int OUT>
+__global__ void __launch_bounds__(kStageThreads, kStageCtas) fft_stage_kernel(const __grid_constant__ StageArgs a) {
   extern __shared__ float4 sm4[];
   float2* const sm = reinterpret_cast<float2*>(sm4);
   const StageDesc& d = a.d;
@@ -357,8 +347,7 @@ __global__ void __launch_bounds__(kStageThreads, 2) fft_stage_kernel(const __gri
     tw.hi = sm4 + (d.bpc * d.SS + 1) / 2;
     tw.nh = tw_rows(d.L);
     tw.lo = reinterpret_cast<float2*>(tw.hi + d.bpc * tw.nh);
-    fill_twiddles<SIGN>(tw, d.bpc, d.L, b1_0, 2.0 / (double)a.N);
-    if (d.nst == 1) __syncthreads();  // otherwise the first stage's barrier covers them
+    fill_twiddles<SIGN>(tw, d.bpc, d.L, b1_0, 2.0 / (double)a.N);  // the first stage's barrier follows
   }
   for (long long b0 = blockIdx.y; b0 < a.nb0; b0 += gridDim.y) {
     const float2* const in = static_cast<const float2*>(a.in) + b0 * a.is0 + b1_0 * a.is1;
@@ -419,13 +408,12 @@ __global__ void __launch_bounds__(kStageThreads, 2) fft_stage_kernel(const __gri
         if (live) row[l * (long long)osl] = v;
       };
     };
-    stages_run<SIGN, PAD>(d, a.in_lane_i, a.out_lane_i, sm, get, put);
+    stages_run<SIGN>(d, a.in_lane_i, a.out_lane_i, sm, get, put);
     if (b0 + gridDim.y < a.nb0) __syncthreads();  // the last stage has read shared memory
   }
 }
 
-// PAD: a stage runs with neighbouring threads on neighbouring elements.
-template <int SIGN, int IN, int OUT, bool PAD>
+template <int SIGN, int IN, int OUT>
 int launch_stages(StageArgs& a, cudaStream_t s) {
   if (a.nb0 <= 0 || a.nb1 <= 0) return FDR_OK;
   FDR_TRY(get_roots(a.d.L, &a.d.roots));
@@ -433,13 +421,13 @@ int launch_stages(StageArgs& a, cudaStream_t s) {
   int dev = 0;
   FDR_CUDA(cudaGetDevice(&dev));
   if (dev >= 64 || !attr_set[dev]) {
-    FDR_CUDA(cudaFuncSetAttribute(fft_stage_kernel<SIGN, IN, OUT, PAD>,
+    FDR_CUDA(cudaFuncSetAttribute(fft_stage_kernel<SIGN, IN, OUT>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
     if (dev < 64) attr_set[dev] = true;
   }
   const size_t smem = stage_smem_bytes(a.d) + (OUT == kOutTwiddle ? tw_bytes(a.d.L, a.d.bpc) : 0);
   const dim3 grid((unsigned)cdiv(a.nb1, a.d.bpc), (unsigned)std::min(a.nb0, 65535LL));
-  fft_stage_kernel<SIGN, IN, OUT, PAD><<<grid, stage_threads(a.d), smem, s>>>(a);
+  fft_stage_kernel<SIGN, IN, OUT><<<grid, stage_threads(a.d), smem, s>>>(a);
   FDR_LAUNCH_CHECK("fft_stage_kernel");
   return FDR_OK;
 }
@@ -469,8 +457,8 @@ int fft_strided_inplace(float2* buf, long long L, long long sl, long long nb, lo
     a.isl = a.osl = sl;
     a.in_lane_i = a.out_lane_i = 1;
     a.scale = scale;
-    return sign < 0 ? launch_stages<-1, kInComplex, kOutComplex, false>(a, s)
-                    : launch_stages<+1, kInComplex, kOutComplex, false>(a, s);
+    return sign < 0 ? launch_stages<-1, kInComplex, kOutComplex>(a, s)
+                    : launch_stages<+1, kInComplex, kOutComplex>(a, s);
   }
   PassDesc d = blank_pass();
   d.in = buf; d.out = buf; d.mul = mul;
@@ -643,10 +631,10 @@ static int real_stages(bool forward, const void* in, long long ldin, void* out, 
     *done = true;
     if (forward) {
       a.os1 = N;
-      return launch_stages<-1, kInRealPair, kOutComplex, true>(a, s);
+      return launch_stages<-1, kInRealPair, kOutComplex>(a, s);
     }
     a.scale = 1.f / (float)N;
-    return launch_stages<+1, kInHalfPair, kOutRealPair, true>(a, s);
+    return launch_stages<+1, kInHalfPair, kOutRealPair>(a, s);
   }
   long long L1, L2;
   split_len(N, &L1, &L2);
@@ -663,8 +651,8 @@ static int real_stages(bool forward, const void* in, long long ldin, void* out, 
   a.os1 = 1;
   a.osl = L2;
   a.in_lane_i = a.out_lane_i = 1;
-  FDR_TRY((forward ? launch_stages<-1, kInRealPair, kOutTwiddle, false>(a, s)
-                   : launch_stages<+1, kInHalfPair, kOutTwiddle, false>(a, s)));
+  FDR_TRY((forward ? launch_stages<-1, kInRealPair, kOutTwiddle>(a, s)
+                   : launch_stages<+1, kInHalfPair, kOutTwiddle>(a, s)));
   // Pass 2: for each k1, DFT over n2 (contiguous), bin or channel k1 + L1*k2
   b.in = tmp;
   b.out = out;
@@ -677,9 +665,9 @@ static int real_stages(bool forward, const void* in, long long ldin, void* out, 
   b.os1 = 1;
   b.osl = L1;
   b.out_lane_i = 1;
-  if (forward) return launch_stages<-1, kInComplex, kOutComplex, true>(b, s);
+  if (forward) return launch_stages<-1, kInComplex, kOutComplex>(b, s);
   b.scale = 1.f / (float)N;
-  return launch_stages<+1, kInComplex, kOutRealPair, true>(b, s);
+  return launch_stages<+1, kInComplex, kOutRealPair>(b, s);
 }
 
 int rfft_columns(const float* in, long long ldin, long long ncol, long long N, float2* F,

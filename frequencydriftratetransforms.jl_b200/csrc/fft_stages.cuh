@@ -1,6 +1,6 @@
 // Register DFTs of the radices that the pass kernels use beside the ones of fft_device.cuh,
-// and the in-place mixed-radix Stockham stages of one CTA (several transforms of one runtime
-// length in shared memory).
+// and the in-place mixed-radix stages of one CTA (several transforms of one runtime length in
+// shared memory).
 #pragma once
 #include "fft_device.cuh"
 
@@ -103,30 +103,34 @@ template <> struct Dft<11> : DftPrime<11, CosSin11> {};
 template <> struct Dft<13> : DftPrime<13, CosSin13> {};
 
 // ------------------------------------------------------------------------------------
-// In-place Stockham stages over `bpc` transforms of one length L in shared memory, at most
-// kStageElems points in all.  A thread takes whole butterflies into registers (at most
-// ceil(32 / R) of radix R), the block synchronises, and the outputs replace the inputs, so
-// one buffer is enough and two CTAs share an SM.  The first stage takes its inputs straight
-// from global memory and the last one hands its outputs to global memory: a transform of n
-// stages crosses shared memory n - 1 times.
-// Element l of transform i is at i * SS + l, or i * SS + pidx(l) when a stage runs with
-// neighbouring threads on neighbouring elements (PAD).  SS = 16 / bpc (mod 16) (1 from bpc = 16
-// on): a half-warp of neighbouring transforms (lanes over i) and one of neighbouring elements
-// (lanes over l) both meet 16 different 8-byte banks.
+// In-place stages over `bpc` transforms of one length L = R_0 R_1 ... in shared memory, at most
+// kStageElems points in all (decimation in frequency).  Stage s transforms R_s elements n_s / R_s
+// apart of every block of n_s = L / (R_0 .. R_{s-1}) elements and leaves output m, times
+// exp(-+ 2 pi i jj m / n_s), in the place of input m, so that a butterfly reads and writes the
+// same places: one buffer, one barrier a stage, a loop over butterflies whose code is one
+// butterfly long.  (Stages that first take all of a thread's butterflies into registers spent
+// most of their time on instruction fetches: their code ran once per CTA.)  The first stage takes
+// its inputs straight from global memory; the last one, whose butterfly j in digit order
+// m_0 + R_0 m_1 + ... holds the outputs j + m L / R, hands them to global memory.
+// Element (m_0, rest) of transform i is at i * SS + m_0 * pitch + rest with pitch odd and
+// SS = 16 / bpc (mod 16) (1 from bpc = 16 on): a half-warp of neighbouring transforms (lanes over
+// i) and one of neighbouring butterflies both meet 16 different 8-byte banks.
 // ------------------------------------------------------------------------------------
 constexpr int kStageThreads = 256;
+constexpr int kStageCtas = 3;  // per SM: up to 85 registers a thread, 72 KB of shared memory
 constexpr int kStageElems = 32 * kStageThreads;
-constexpr int kStageMax = 12;  // stages of a plan (2^12 < kStageElems, radix 2 only once)
+constexpr int kStageMax = 8;
 
 struct StageDesc {
-  int L, nst, bpc, bpc_log2, SS;
+  int L, nst, bpc, bpc_log2, SS, pitch;
   int radix[kStageMax];
-  int nbf[kStageMax];            // L / radix: butterflies of one transform
-  int Ns[kStageMax];             // product of the earlier radices
-  unsigned nbf_magic[kStageMax]; // ceil(2^32 / nbf): exact quotients of numbers below 2^16
-  unsigned Ns_magic[kStageMax];
-  int tw_step[kStageMax];        // L / (Ns * radix)
-  const float2* roots;           // exp(-2 pi i m / L), m < L
+  int nbf[kStageMax];              // L / radix: butterflies of one transform
+  int Ns[kStageMax];               // product of the earlier radices
+  int step[kStageMax];             // n_s / radix: distance of a butterfly's elements
+  int digit[kStageMax];            // place value of digit m_s of a position
+  unsigned radix_magic[kStageMax]; // of div_magic
+  unsigned nbf_magic[kStageMax];
+  const float2* roots;             // exp(-2 pi i m / L), m < L
 };
 
 // n / d for n < 2^13 from magic = ceil(2^32 / d) (0 stands for d = 1): the excess of the
@@ -135,174 +139,179 @@ __device__ __forceinline__ int div_magic(int n, unsigned magic) {
   return magic ? (int)__umulhi((unsigned)n, magic) : n;
 }
 
-template <bool PAD>
-__device__ __forceinline__ int sidx(int l) { return PAD ? pidx(l) : l; }
+// Position of butterfly j of stage s (j in digit order, the element jj within the block last);
+// *jj receives that element.
+__device__ __forceinline__ int stage_pos(const StageDesc& d, int s, int j, int* jj) {
+  int pos = 0;
+  for (int t = 0; t < s; ++t) {
+    const int q = div_magic(j, d.radix_magic[t]);
+    pos += (j - q * d.radix[t]) * d.digit[t];
+    j = q;
+  }
+  *jj = j;
+  return pos + j;
+}
 
-// Reads, transforms and hands on the butterflies of stage s.  get(i)(l) gives element l of
-// transform i at the first stage, put(i)(l, v) takes it at the last.  lane_i: neighbouring
-// threads take neighbouring transforms (else neighbouring elements).
-template <int R, int SIGN, bool PAD, class Get, class Put>
-__device__ __forceinline__ void stage_run(const StageDesc& d, int s, bool lane_i, bool first, bool last,
-                                          float2* sm, Get get, Put put) {
-  constexpr int PER = (32 + R - 1) / R;
-  const int nbf = d.nbf[s], Ns = d.Ns[s], SS = d.SS;
-  const int total = nbf << d.bpc_log2;
-  float2 v[PER][R];
+// exp(SIGN 2 pi i jj m / n_s) on the elements m of a butterfly of stage s.
+template <int R, int SIGN>
+__device__ __forceinline__ void stage_twiddle(const StageDesc& d, int s, int jj, float2* v) {
+  const int step = jj * d.Ns[s];
 #pragma unroll
-  for (int p = 0; p < PER; ++p) {
-    const int j = threadIdx.x + p * blockDim.x;
-    if (j < total) {
-      const int i = lane_i ? j & (d.bpc - 1) : div_magic(j, d.nbf_magic[s]);
-      const int jj = lane_i ? j >> d.bpc_log2 : j - i * nbf;
-      if (first) {
-        auto row = get(i);
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[p][r] = row(jj + r * nbf);
-      } else {
-        const float2* a = sm + i * SS;
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[p][r] = a[sidx<PAD>(jj + r * nbf)];
-      }
-    } else {  // no value may live on from the stage before
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[p][r] = make_float2(0.f, 0.f);
-    }
+  for (int m = 1; m < R; ++m) {
+    float2 t = __ldg(d.roots + m * step);
+    if (SIGN > 0) t.y = -t.y;
+    v[m] = cmul(v[m], t);
   }
-  if (!first && !last) __syncthreads();  // every input is read before an output replaces it
+}
+
+// First stage.  get(i)(l): element l of transform i.  lane_i: neighbouring threads take
+// neighbouring transforms (else neighbouring elements).
+template <int R, int SIGN, class Get>
+__device__ __forceinline__ void stage_first(const StageDesc& d, bool lane_i, float2* sm, Get get) {
+  const int nbf = d.nbf[0], total = nbf << d.bpc_log2;
+  for (int j = threadIdx.x; j < total; j += blockDim.x) {
+    const int i = lane_i ? j & (d.bpc - 1) : div_magic(j, d.nbf_magic[0]);
+    const int jj = lane_i ? j >> d.bpc_log2 : j - i * nbf;
+    float2 v[R];
+    auto row = get(i);
 #pragma unroll
-  for (int p = 0; p < PER; ++p) {
-    const int j = threadIdx.x + p * blockDim.x;
-    if (j < total) {
-      const int i = lane_i ? j & (d.bpc - 1) : div_magic(j, d.nbf_magic[s]);
-      const int jj = lane_i ? j >> d.bpc_log2 : j - i * nbf;
-      const int b = div_magic(jj, d.Ns_magic[s]);
-      const int k = jj - b * Ns;
-      if (!first) {
-        const float2* w = d.roots;
-        const int step = k * d.tw_step[s];
+    for (int r = 0; r < R; ++r) v[r] = row(jj + r * nbf);
+    Dft<R>::run(v, SIGN);
+    if (d.nst > 1) stage_twiddle<R, SIGN>(d, 0, jj, v);
+    float2* o = sm + i * d.SS + jj;
 #pragma unroll
-        for (int r = 1; r < R; ++r) {
-          float2 t = __ldg(w + r * step);
-          if (SIGN > 0) t.y = -t.y;
-          v[p][r] = cmul(v[p][r], t);
-        }
-      }
-      Dft<R>::run(v[p], SIGN);
-      if (last) {
-        auto row = put(i);
-#pragma unroll
-        for (int r = 0; r < R; ++r) row(jj + r * nbf, v[p][r]);
-      } else {
-        float2* o = sm + i * SS;
-        const int base = b * Ns * R + k;
-#pragma unroll
-        for (int r = 0; r < R; ++r) o[sidx<PAD>(base + r * Ns)] = v[p][r];
-      }
-    }
+    for (int m = 0; m < R; ++m) o[m * d.pitch] = v[m];
   }
-  if (!last) __syncthreads();
+}
+
+// A stage within shared memory.  TIME: the mirrored stage of a transform that takes its input in
+// the order this one leaves (decimation in time: twiddles before the butterfly).
+template <int R, int SIGN, bool TIME>
+__device__ __forceinline__ void stage_mid(const StageDesc& d, int s, float2* sm) {
+  const int total = d.nbf[s] << d.bpc_log2;
+  const int step = s == 0 ? d.pitch : d.step[s];
+  for (int j = threadIdx.x; j < total; j += blockDim.x) {
+    int jj;
+    float2* const o = sm + (j & (d.bpc - 1)) * d.SS + stage_pos(d, s, j >> d.bpc_log2, &jj);
+    float2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = o[r * step];
+    if (TIME) stage_twiddle<R, SIGN>(d, s, jj, v);
+    Dft<R>::run(v, SIGN);
+    if (!TIME) stage_twiddle<R, SIGN>(d, s, jj, v);
+#pragma unroll
+    for (int r = 0; r < R; ++r) o[r * step] = v[r];
+  }
+}
+
+// Last stage.  put(i)(l, v) takes output l of transform i.
+template <int R, int SIGN, class Put>
+__device__ __forceinline__ void stage_last(const StageDesc& d, bool lane_i, const float2* sm, Put put) {
+  const int s = d.nst - 1, nbf = d.nbf[s], total = nbf << d.bpc_log2;
+  const int step = s == 0 ? d.pitch : 1;
+  for (int j = threadIdx.x; j < total; j += blockDim.x) {
+    const int i = lane_i ? j & (d.bpc - 1) : div_magic(j, d.nbf_magic[s]);
+    const int jj = lane_i ? j >> d.bpc_log2 : j - i * nbf;
+    int within;
+    const float2* const o = sm + i * d.SS + stage_pos(d, s, jj, &within);
+    float2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = o[r * step];
+    Dft<R>::run(v, SIGN);
+    auto row = put(i);
+#pragma unroll
+    for (int m = 0; m < R; ++m) row(jj + m * nbf, v[m]);
+  }
+}
+
+// Last forward stage, the product with factor(i)(l) and the first backward stage.
+template <int R, class Factor>
+__device__ __forceinline__ void stage_turn(const StageDesc& d, float2* sm, Factor factor) {
+  const int s = d.nst - 1, nbf = d.nbf[s], total = nbf << d.bpc_log2;
+  const int step = s == 0 ? d.pitch : 1;
+  for (int j = threadIdx.x; j < total; j += blockDim.x) {
+    const int i = j & (d.bpc - 1), jj = j >> d.bpc_log2;
+    auto row = factor(i);
+    float2 f[R], v[R];
+#pragma unroll
+    for (int m = 0; m < R; ++m) f[m] = row(jj + m * nbf);
+    int within;
+    float2* const o = sm + i * d.SS + stage_pos(d, s, jj, &within);
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = o[r * step];
+    Dft<R>::run(v, -1);
+#pragma unroll
+    for (int m = 0; m < R; ++m) v[m] = cmul(v[m], f[m]);
+    Dft<R>::run(v, +1);
+#pragma unroll
+    for (int r = 0; r < R; ++r) o[r * step] = v[r];
+  }
 }
 
 #define FDR_FOR_RADIX(X) X(16) X(13) X(11) X(10) X(9) X(8) X(7) X(6) X(5) X(4) X(3) X(2)
 
-// All stages of d; the block must be synchronised before if shared memory is still being read.
-template <int SIGN, bool PAD, class Get, class Put>
+// All stages of d (nst >= 2: a single stage passes through shared memory all the same); the
+// block must be synchronised before if shared memory is still being read.
+template <int SIGN, class Get, class Put>
 __device__ __forceinline__ void stages_run(const StageDesc& d, bool first_lane_i, bool last_lane_i,
                                            float2* sm, Get get, Put put) {
-  for (int s = 0; s < d.nst; ++s) {
-    const bool first = s == 0, last = s == d.nst - 1;
-    const bool lane_i = first ? first_lane_i : (last ? last_lane_i : !PAD || d.bpc >= 8);
+  if (d.nst == 1) {  // L <= 16: the butterfly is the transform
+    for (int e = threadIdx.x; e < d.L << d.bpc_log2; e += blockDim.x)
+      sm[(e & (d.bpc - 1)) * d.SS + (e >> d.bpc_log2) * d.pitch] = get(e & (d.bpc - 1))(e >> d.bpc_log2);
+  } else {
+    switch (d.radix[0]) {
+#define FDR_STAGE(R) case R: stage_first<R, SIGN>(d, first_lane_i, sm, get); break;
+      FDR_FOR_RADIX(FDR_STAGE)
+#undef FDR_STAGE
+    }
+  }
+  __syncthreads();
+  for (int s = 1; s + 1 < d.nst; ++s) {
     switch (d.radix[s]) {
-#define FDR_STAGE(R) case R: stage_run<R, SIGN, PAD>(d, s, lane_i, first, last, sm, get, put); break;
+#define FDR_STAGE(R) case R: stage_mid<R, SIGN, false>(d, s, sm); break;
       FDR_FOR_RADIX(FDR_STAGE)
 #undef FDR_STAGE
     }
+    __syncthreads();
   }
-}
-
-// One stage within shared memory, neighbouring threads on neighbouring transforms.  TURN: the
-// last forward stage, the product with factor(i)(l) and the first backward stage of a plan
-// whose radices run the other way, which takes the same elements (a convolution's middle).
-template <int R, int SIGN, bool TURN, class Factor>
-__device__ __forceinline__ void stage_smem(const StageDesc& d, int s, float2* sm, Factor factor) {
-  constexpr int PER = (32 + R - 1) / R;
-  const int nbf = d.nbf[s], Ns = d.Ns[s], SS = d.SS;
-  const int total = nbf << d.bpc_log2;
-  float2 v[PER][R];
-#pragma unroll
-  for (int p = 0; p < PER; ++p) {
-    const int j = threadIdx.x + p * blockDim.x;
-    if (j < total) {
-      const float2* a = sm + (j & (d.bpc - 1)) * SS + (j >> d.bpc_log2);
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[p][r] = a[r * nbf];
-    } else {
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[p][r] = make_float2(0.f, 0.f);
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int p = 0; p < PER; ++p) {
-    const int j = threadIdx.x + p * blockDim.x;
-    if (j < total) {
-      const int i = j & (d.bpc - 1), jj = j >> d.bpc_log2;
-      const int b = div_magic(jj, d.Ns_magic[s]);
-      const int k = jj - b * Ns;
-      float2 f[TURN ? R : 1];
-      if (TURN) {
-        auto row = factor(i);
-#pragma unroll
-        for (int r = 0; r < R; ++r) f[r] = row(jj + r * nbf);
-      }
-      if (Ns > 1) {
-        const int step = k * d.tw_step[s];
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-          float2 t = __ldg(d.roots + r * step);
-          if (SIGN > 0) t.y = -t.y;
-          v[p][r] = cmul(v[p][r], t);
-        }
-      }
-      Dft<R>::run(v[p], SIGN);
-      if (TURN) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[p][r] = cmul(v[p][r], f[r]);
-        Dft<R>::run(v[p], -SIGN);
-      }
-      float2* o = sm + i * SS + (TURN ? jj * R : b * Ns * R + k);
-      const int ostep = TURN ? 1 : Ns;
-#pragma unroll
-      for (int r = 0; r < R; ++r) o[r * ostep] = v[p][r];
-    }
-  }
-  __syncthreads();
-}
-
-// Circular convolution of the transforms in shared memory (element l of transform i at
-// i * SS + l) with the spectrum factor(i)(l), unnormalised: the stages of fwd, the turn, the
-// remaining stages of inv, whose radices are fwd's in reverse.
-template <class Factor>
-__device__ __forceinline__ void convolve_smem(const StageDesc& fwd, const StageDesc& inv, float2* sm,
-                                              Factor factor) {
-  for (int s = 0; s + 1 < fwd.nst; ++s) {
-    switch (fwd.radix[s]) {
-#define FDR_STAGE(R) case R: stage_smem<R, -1, false>(fwd, s, sm, factor); break;
-      FDR_FOR_RADIX(FDR_STAGE)
-#undef FDR_STAGE
-    }
-  }
-  switch (fwd.radix[fwd.nst - 1]) {
-#define FDR_STAGE(R) case R: stage_smem<R, -1, true>(fwd, fwd.nst - 1, sm, factor); break;
+  switch (d.radix[d.nst - 1]) {
+#define FDR_STAGE(R) case R: stage_last<R, SIGN>(d, last_lane_i, sm, put); break;
     FDR_FOR_RADIX(FDR_STAGE)
 #undef FDR_STAGE
   }
-  for (int s = 1; s < inv.nst; ++s) {
-    switch (inv.radix[s]) {
-#define FDR_STAGE(R) case R: stage_smem<R, +1, false>(inv, s, sm, factor); break;
+}
+
+// Place of element l of a transform in shared memory.
+__device__ __forceinline__ int stage_place(const StageDesc& d, int l) {
+  const int m0 = div_magic(l, d.nbf_magic[0] /* n_1 = L / R_0 */);
+  return l + m0 * (d.pitch - d.nbf[0]);
+}
+
+// Circular convolution of the transforms in shared memory (element l of transform i at
+// i * SS + stage_place(l)) with the spectrum factor(i)(l), unnormalised.
+template <class Factor>
+__device__ __forceinline__ void convolve_smem(const StageDesc& d, float2* sm, Factor factor) {
+  for (int s = 0; s + 1 < d.nst; ++s) {
+    switch (d.radix[s]) {
+#define FDR_STAGE(R) case R: stage_mid<R, -1, false>(d, s, sm); break;
       FDR_FOR_RADIX(FDR_STAGE)
 #undef FDR_STAGE
     }
+    __syncthreads();
+  }
+  switch (d.radix[d.nst - 1]) {
+#define FDR_STAGE(R) case R: stage_turn<R>(d, sm, factor); break;
+    FDR_FOR_RADIX(FDR_STAGE)
+#undef FDR_STAGE
+  }
+  __syncthreads();
+  for (int s = d.nst - 2; s >= 0; --s) {
+    switch (d.radix[s]) {
+#define FDR_STAGE(R) case R: stage_mid<R, +1, true>(d, s, sm); break;
+      FDR_FOR_RADIX(FDR_STAGE)
+#undef FDR_STAGE
+    }
+    __syncthreads();
   }
 }
 
@@ -310,8 +319,6 @@ __device__ __forceinline__ void convolve_smem(const StageDesc& fwd, const StageD
 // neighbouring addresses (rows: CTAs then take at least 8 of them, 64 bytes a row); false if L
 // has a prime factor above 13 or exceeds kStageElems.
 bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, StageDesc* d);
-// The plan whose stages run in the reverse order.
-StageDesc stage_reversed(const StageDesc& d);
 size_t stage_smem_bytes(const StageDesc& d);
 int stage_threads(const StageDesc& d);
 

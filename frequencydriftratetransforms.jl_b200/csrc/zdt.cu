@@ -123,7 +123,7 @@ __global__ void zdt_postprocess_kernel(float2* __restrict__ Y, long long K, long
 // zdt_preprocess_kernel, the convolution's two transforms and zdt_postprocess_kernel; columns
 // past Nr receive what convolve! leaves there.
 struct ConvArgs {
-  StageDesc fwd, inv;
+  StageDesc d;
   const float2* F;
   const float2* V;
   float2* Y;
@@ -133,9 +133,9 @@ struct ConvArgs {
   float r0, dr;
 };
 
-__global__ void __launch_bounds__(kStageThreads, 2) zdt_conv_kernel(const __grid_constant__ ConvArgs a) {
+__global__ void __launch_bounds__(kStageThreads, kStageCtas) zdt_conv_kernel(const __grid_constant__ ConvArgs a) {
   extern __shared__ float2 sm[];
-  const StageDesc& d = a.fwd;
+  const StageDesc& d = a.d;
   const int bpc = d.bpc, lg = d.bpc_log2, SS = d.SS;
   const long long k0 = (long long)blockIdx.x << lg, K = a.K;
   const int nb = (int)min((long long)bpc, K - k0);
@@ -147,12 +147,12 @@ __global__ void __launch_bounds__(kStageThreads, 2) zdt_conv_kernel(const __grid
     const long long k = k0 + min(i, nb - 1);
     const float2 ph = a.exact ? prephase_exact(k, l, a.r0, a.dr, (double)a.Nf)
                               : prephase_ref(k, l, a.r0, a.dr, Nf_f);
-    sm[i * SS + l] = cmul_rn(__ldg(a.F + k + l * K), ph);
+    sm[i * SS + stage_place(d, l)] = cmul_rn(__ldg(a.F + k + l * K), ph);
   }
   for (int e = (a.Nt << lg) + threadIdx.x; e < a.Nl << lg; e += blockDim.x)
-    sm[(e & (bpc - 1)) * SS + (e >> lg)] = make_float2(0.f, 0.f);
+    sm[(e & (bpc - 1)) * SS + stage_place(d, e >> lg)] = make_float2(0.f, 0.f);
   __syncthreads();
-  convolve_smem(a.fwd, a.inv, sm, [&](int i) {
+  convolve_smem(d, sm, [&](int i) {
     const float2* const v = a.V + k0 + min(i, nb - 1);
     return [=](int l) { return __ldg(v + l * K); };
   });
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kStageThreads, 2) zdt_conv_kernel(const __grid
   for (int e = threadIdx.x; e < a.Nl << lg; e += blockDim.x) {
     const int i = e & (bpc - 1), l = e >> lg;
     const long long k = k0 + i;
-    float2 y = cscale(sm[i * SS + l], scale);
+    float2 y = cscale(sm[i * SS + stage_place(d, l)], scale);
     if (l < a.Nr) {
       const float2 ph = a.exact ? postphase_exact(k, l, a.dr, (double)a.Nf) : postphase_ref(k, l, a.dr, Nf_f);
       y = postprocess_value(y, ph, i < nb ? k : 0, a.Nf, a.window, a.wk);
@@ -286,11 +286,10 @@ static int zdt_conv(fdr_zdt* ws, float r0, int window, const double* wk, cudaStr
   *done = false;
   ConvArgs a;
   memset(&a, 0, sizeof(a));
-  if (!stage_plan(ws->Nl, ws->K, 1, true, &a.fwd)) return FDR_OK;
+  if (!stage_plan(ws->Nl, ws->K, 1, true, &a.d)) return FDR_OK;
   FDR_TRY(zdt_ensure_staged(ws, s));
   FDR_TRY(zdt_ensure_F(ws, s));
-  FDR_TRY(get_roots(ws->Nl, &a.fwd.roots));
-  a.inv = stage_reversed(a.fwd);
+  FDR_TRY(get_roots(ws->Nl, &a.d.roots));
   a.F = ws->F; a.V = ws->V; a.Y = ws->Y; a.wk = wk;
   a.K = ws->K; a.Nf = ws->Nf;
   a.Nt = (int)ws->Nt; a.Nr = (int)ws->Nr; a.Nl = (int)ws->Nl;
@@ -304,7 +303,7 @@ static int zdt_conv(fdr_zdt* ws, float r0, int window, const double* wk, cudaStr
     FDR_CUDA(cudaFuncSetAttribute(zdt_conv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
     if (dev < 64) attr_set[dev] = true;
   }
-  zdt_conv_kernel<<<(unsigned)cdiv(ws->K, a.fwd.bpc), stage_threads(a.fwd), stage_smem_bytes(a.fwd), s>>>(a);
+  zdt_conv_kernel<<<(unsigned)cdiv(ws->K, a.d.bpc), stage_threads(a.d), stage_smem_bytes(a.d), s>>>(a);
   FDR_LAUNCH_CHECK("zdt_conv_kernel");
   *done = true;
   return FDR_OK;
