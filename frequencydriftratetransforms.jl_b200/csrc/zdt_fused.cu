@@ -6,15 +6,15 @@
 // and drift rate r_j = r0 + j*dr,
 //     S_j[k] = sum_t F[k, t] * exp(2*pi*i * k * t * r_j / Nf)
 // (the fftfdr.jl phasor form; Bluestein's convolution computes exactly this).  For the
-// small Nt of this path the direct evaluation per bin (Horner's rule in t) costs about
-// the same arithmetic as three length-Nl FFTs and needs neither V nor Y, so this path
-// keeps F on chip and never writes the K x Nl intermediates:
+// small Nt of this path the direct evaluation per bin costs less arithmetic than three
+// length-Nl FFTs (two rates and two steps at a time, see the sums below) and needs neither
+// V nor Y, so this path keeps F on chip and never writes the K x Nl intermediates:
 //
 //   kernel A (zdtf_input):  four-step pass 1 of the forward FFT of two real columns packed
 //                           as one complex column (t pairs): DFT_P over n_b, twiddle.
 //   kernel B (zdtf_czt):    per pair of bin residues {k1, P-k1}: forward DFT_Q (pass 2) and
 //                           two-for-one unpack into F[k, t] held in registers; then, per
-//                           block of drift rates, S_j[k] by Horner's rule with exact
+//                           block of drift rates, S_j[k] by folded sums with exact
 //                           integer phase reduction, the window, two-for-one packing of
 //                           rate pairs, inverse DFT_Q (pass 1 of the output FFT) and the
 //                           inter-pass twiddle (with the 1/Nf scale).
@@ -47,7 +47,6 @@ constexpr int kFusedMaxLog2 = 22;
 constexpr int kFusedMaxNt = 16;      // F in registers
 constexpr int kFusedMaxNtSmem = 64;  // F in shared memory
 constexpr int kRatesPerBlock = 8;  // 4 rate pairs (8 sequences) per inverse-FFT block in kernel B
-constexpr int kHorner = 4;         // rates evaluated together by one thread (a half block)
 
 // Shared-memory stride of one FFT sequence of kernels A and C (TILE sequences per CTA):
 // padded length plus an offset that spreads the TILE sequences over distinct banks.
@@ -56,10 +55,11 @@ __host__ __device__ constexpr int ac_stride() { return padlen(P) + 16 / TILE; }
 template <int Q>
 __host__ __device__ constexpr int b_stride() { return padlen(Q) + 1; }
 
+// Phases as 64-bit fractions of a turn, per bin: rate j of bin k turns k * (R0 + 2 j Rh) per time
+// step.  Multiplication and addition wrap modulo one turn, so every phase is exact.
 struct PhaseInt {
-  unsigned long long R0, Rd, mask;
-  int bits;
-  float scale;  // 2^(1-bits): converts a signed residue to half-turns
+  unsigned long long R0;  // r0 / Nf
+  unsigned long long Rh;  // dr / (2 Nf)
 };
 
 struct FusedTables {
@@ -76,11 +76,50 @@ __device__ __forceinline__ float2 tw_fwd(const FusedTables& t, long long m) {
   return cmul(__ldg(t.tw_hi + (m >> t.B)), __ldg(t.tw_lo + (m & ((1LL << t.B) - 1))));
 }
 
-// exp(2 pi i ph / 2^bits) for a residue 0 <= ph < 2^bits.
-__device__ __forceinline__ float2 cis_phase(unsigned long long ph, const PhaseInt& p) {
-  long long sp = (long long)ph;
-  if ((ph >> (p.bits - 1)) & 1ULL) sp -= (long long)(1ULL << p.bits);
-  return cispif(__ll2float_rn(sp) * p.scale);
+// Packed-FP32 helpers (sm_100 FFMA2 / FMUL2 / FADD2): lane 0 and lane 1 carry two independent
+// evaluations, each lane performing exactly the scalar operation sequence.
+__device__ __forceinline__ float2 pk_fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 pk_mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 pk_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 pk_set(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 pk_neg(float2 a) { return __fmul2_rn(a, make_float2(-1.f, -1.f)); }
+// (ax + i ay) (bx + i by)
+__device__ __forceinline__ void pk_cmul(float2 ax, float2 ay, float2 bx, float2 by, float2& x, float2& y) {
+  x = pk_fma(ax, bx, pk_mul(pk_neg(ay), by));
+  y = pk_fma(ax, by, pk_mul(ay, bx));
+}
+
+// exp(2 pi i ph / 2^64) for the phases of two bins: the nearest quarter turn is taken off in
+// integers and sin and cos of the rest, x quarter turns with |x| <= 1/2, come from polynomials in
+// x^2 fitted on Chebyshev nodes (degrees 7 and 8; the leading sine coefficient pi/2 is held in two
+// parts).  Errors over all 32-bit phases: 1.4e-8 (sin) and 1.9e-8 (cos) rms, 7.1e-8 at most,
+// against 1.4e-8 and 1.8e-8 rms for correctly rounded values of the rounded argument.  The two
+// bins share packed operations: about 33 instructions for both, where two sincospif with their
+// 64-bit conversions took about 80.
+__device__ __forceinline__ void cis_turn_pk(unsigned long long ph0, unsigned long long ph1, float2& c, float2& s) {
+  const int h0 = (int)((ph0 + 0x80000000ull) >> 32), h1 = (int)((ph1 + 0x80000000ull) >> 32);
+  const unsigned q0 = ((unsigned)h0 + (1u << 29)) >> 30, q1 = ((unsigned)h1 + (1u << 29)) >> 30;
+  const float2 x = pk_mul(make_float2(__int2float_rn(h0 - (int)(q0 << 30)), __int2float_rn(h1 - (int)(q1 << 30))),
+                          pk_set(9.31322574615478515625e-10f));  // 2^-30
+  const float2 y = pk_mul(x, x);
+  float2 p = pk_fma(y, pk_set(-4.602149128913879e-3f), pk_set(7.968021929264069e-2f));
+  p = pk_fma(p, y, pk_set(-6.459634900093079e-1f));
+  p = pk_fma(p, y, pk_set(-4.8553051357203e-8f));
+  const float2 sn = pk_fma(x, pk_set(1.5707963705062866f), pk_mul(x, p));
+  float2 e = pk_fma(y, pk_set(9.036280680447817e-4f), pk_set(-2.086007036268711e-2f));
+  e = pk_fma(e, y, pk_set(2.5366920232772827e-1f));
+  e = pk_fma(e, y, pk_set(-1.2337005138397217f));
+  const float2 cs = pk_fma(e, y, pk_set(1.f));
+  auto sign = [](float v, unsigned bit) { return __uint_as_float(__float_as_uint(v) ^ (bit << 30)); };
+  c.x = sign((q0 & 1) ? sn.x : cs.x, (q0 + 1) & 2);
+  s.x = sign((q0 & 1) ? cs.x : sn.x, q0 & 2);
+  c.y = sign((q1 & 1) ? sn.y : cs.y, (q1 + 1) & 2);
+  s.y = sign((q1 & 1) ? cs.y : sn.y, q1 & 2);
+}
+__device__ __forceinline__ float2 cis_turn(unsigned long long ph) {
+  float2 c, s;
+  cis_turn_pk(ph, ph, c, s);
+  return make_float2(c.x, s.x);
 }
 
 // ------------------------------------------------------------------------------------
@@ -241,11 +280,15 @@ struct CztArgs {
   float2* W;          // [pair][k1][na] for pairs [0, npairs)
   float2* F;          // A->F mode output (K x Nt) or NULL
   const double* wk;   // custom window values (K) or NULL
-  const int* blk_base;  // rate index (on the r0 + j*dr grid) of each 8-rate block's first
-                        // rate, or NULL for 8*block (the contiguous rates 0..Nr-1)
+  const int* blk_base;  // SUBSET kernels: rate index (on the r0 + j*dr grid) of each 8-rate
+                        // block's first rate, a multiple of 8
   long long N;
-  int P, Nt, NP, Nr, npairs, pairs_per_group, window;
+  int P, Nt, NP, Nr, npairs, window;
+  int half;             // h: super pairs of the whole grid (rates 2h + m and 2h - 1 - m)
+  int nblk, blocks_per_group;  // 8-rate blocks in all and per grid.y group
+  int pshift;           // F in registers: time pairs are held this many pairs up
   PhaseInt ph;
+  unsigned long long center;  // the grid centre's rate over Nf: R0 + (4h - 1) Rh
   FusedTables tab;
 };
 
@@ -256,9 +299,9 @@ __device__ __forceinline__ void mirror_of(int c, int side, int k2, int Q, int* m
   else { *ms = 1 - side; *mk2 = Q - 1 - k2; }
 }
 
-// Forward pass 2 + two-for-one unpack: G[b][t] = F[k_b, t] for the two bases of this
+// Forward pass 2 + two-for-one unpack: G[b][t + 2 pshift] = F[k_b, t] for the two bases of this
 // thread (b = side, k2 = threadIdx.x); CTA 0's thread 0 also stores the Nyquist bin's
-// F[N/2, t] into gnyq (shared memory).  buf holds 8 sequences of stride b_stride<Q>().
+// F[N/2, t] into gnyq[t] (shared memory).  buf holds 8 sequences of stride b_stride<Q>().
 template <int Q, int NTR>
 __device__ __forceinline__ void czt_forward(const CztArgs& a, int c, const int* k1s, float2* buf,
                                             const float2* twt, float2* gnyq,
@@ -276,7 +319,7 @@ __device__ __forceinline__ void czt_forward(const CztArgs& a, int c, const int* 
     for (int t = 0; t < NTR; ++t) gnyq[t] = make_float2(0.f, 0.f);
 #pragma unroll
   for (int p0 = 0; p0 < NTR / 2; p0 += PC) {
-    if (p0 < a.NP) {
+    if (p0 < a.NP + a.pshift && p0 + PC > a.pshift) {
       __syncthreads();
       {
         constexpr int NL = 2 * PC * Q / T;  // loads per thread, issued before any is stored
@@ -285,8 +328,8 @@ __device__ __forceinline__ void czt_forward(const CztArgs& a, int c, const int* 
         for (int i = 0; i < NL; ++i) {
           const int e = tid + i * T;
           const int seq = e / Q, na = e - seq * Q;
-          const int pp = p0 + (seq >> 1), side = seq & 1;
-          v[i] = (pp < a.NP && FDR_DBG_OK(((long long)pp * a.P + k1s[side]) * Q + na < (long long)a.NP * a.P * Q))
+          const int pp = p0 + (seq >> 1) - a.pshift, side = seq & 1;
+          v[i] = ((unsigned)pp < (unsigned)a.NP && FDR_DBG_OK(((long long)pp * a.P + k1s[side]) * Q + na < (long long)a.NP * a.P * Q))
                      ? __ldcs(a.A + ((long long)pp * a.P + k1s[side]) * Q + na)
                              : make_float2(0.f, 0.f);
         }
@@ -317,10 +360,11 @@ __device__ __forceinline__ void czt_forward(const CztArgs& a, int c, const int* 
       if (c == 0 && tid == 0) {
 #pragma unroll
         for (int u = 0; u < PC; ++u) {
-          if (2 * (p0 + u) + 1 < NTR) {
+          const int pp = p0 + u - a.pshift;
+          if ((unsigned)pp < (unsigned)a.NP) {
             const float2 z = buf[(2 * u) * SS + pidx(Q / 2)];
-            gnyq[2 * (p0 + u)] = make_float2(z.x, 0.f);
-            gnyq[2 * (p0 + u) + 1] = make_float2(z.y, 0.f);
+            gnyq[2 * pp] = make_float2(z.x, 0.f);
+            gnyq[2 * pp + 1] = make_float2(z.y, 0.f);
           }
         }
       }
@@ -329,50 +373,273 @@ __device__ __forceinline__ void czt_forward(const CztArgs& a, int c, const int* 
   __syncthreads();
 }
 
-template <int NTR>
-__device__ __forceinline__ float2 horner(const float2 (&G)[NTR], float2 w) {
-  float2 s = G[NTR - 1];
-#pragma unroll
-  for (int t = NTR - 2; t >= 0; --t) {
-    s = make_float2(fmaf(s.x, w.x, fmaf(-s.y, w.y, G[t].x)), fmaf(s.x, w.y, fmaf(s.y, w.x, G[t].y)));
-  }
-  return s;
-}
-
-// Packed-FP32 helpers (sm_100 FFMA2 / FMUL2): lane 0 and lane 1 carry two independent
-// evaluations, each lane performing exactly the scalar operation sequence.
-__device__ __forceinline__ float2 pk_fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 pk_mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 pk_neg(float2 a) { return __fmul2_rn(a, make_float2(-1.f, -1.f)); }
-
-// horner() for the two bins of a thread at once: (Gx[t], Gy[t]) hold the real and imaginary
-// parts of F[k_b, t] for b = 0, 1 in the two lanes; (wx, wy) the two multipliers.
-template <int NTR>
-__device__ __forceinline__ void horner_pk(const float2 (&Gx)[NTR], const float2 (&Gy)[NTR], float2 wx,
-                                          float2 wy, float2& sx, float2& sy) {
-  const float2 nwy = pk_neg(wy);
-  sx = Gx[NTR - 1];
-  sy = Gy[NTR - 1];
-#pragma unroll
-  for (int t = NTR - 2; t >= 0; --t) {
-    const float2 tx = pk_fma(sx, wx, pk_fma(sy, nwy, Gx[t]));
-    const float2 ty = pk_fma(sx, wy, pk_fma(sy, wx, Gy[t]));
-    sx = tx;
-    sy = ty;
-  }
-}
-
 __device__ __forceinline__ float window_value(const CztArgs& a, long long k) {
   if (a.window == FDR_WINDOW_HAMMING) return (float)(0.53836 + 0.46164 * cospi(2.0 * (double)k / (double)a.N));
   if (a.window == FDR_WINDOW_CUSTOM) return (float)a.wk[k];
   return 1.f;
 }
 
+// Horner's rule over the Nyquist bin's steps; the real part is its value.
+__device__ __forceinline__ float nyquist_value(const CztArgs& a, const float2* gnyq, long long j) {
+  const unsigned long long kny = (unsigned long long)(a.N / 2);
+  const float2 w = cis_turn(kny * a.ph.R0 + 2ull * (unsigned long long)j * (kny * a.ph.Rh));
+  float2 s = gnyq[a.Nt - 1];
+  for (int t = a.Nt - 2; t >= 0; --t)
+    s = make_float2(fmaf(s.x, w.x, fmaf(-s.y, w.y, gnyq[t].x)), fmaf(s.x, w.y, fmaf(s.y, w.x, gnyq[t].y)));
+  return s.x;
+}
+
+// First rate pair of W and rate of its sequence pair u (0..3) of an 8-rate block: the upper and
+// lower rate pairs of super pairs 2 blk and 2 blk + 1, or four consecutive pairs of a subset.
+template <bool SUBSET>
+__device__ __forceinline__ int block_pair(const CztArgs& a, int blk, int u) {
+  if (SUBSET) return 4 * blk + u;
+  const int i = 2 * blk + (u >> 1);
+  const int p = (u & 1) ? a.half - 1 - i : a.half + i;
+  return i < a.half && p < a.npairs ? p : -1;
+}
+
+// The real-only Nyquist bin of a block's 8 rates, one lane each (tid < 8), as floats of the
+// packed sequences: value(u, hh, v).
+template <bool SUBSET, class Put>
+__device__ __forceinline__ void nyquist_block(const CztArgs& a, const float2* gnyq, int blk, int lane, Put put) {
+  const int u = lane >> 1, hh = lane & 1;
+  const int p = block_pair<SUBSET>(a, blk, u);
+  if (p < 0) return;
+  const long long j = SUBSET ? (long long)__ldg(a.blk_base + blk) + 2 * u + hh : 2LL * p + hh;
+  const float v = nyquist_value(a, gnyq, j) * window_value(a, a.N / 2);
+  put(u, hh, 2 * p + hh < a.Nr ? v : 0.f);
+}
+
+// ------------------------------------------------------------------------------------
+// Sums over the time steps at pairs of rates about the grid's centre.
+//
+// Rates 2H + m and 2H - 1 - m of a grid padded to 4h rates (H = 2h; h "super pairs" of two rate
+// pairs) lie at +-phi, phi = (2m + 1) k dr / (2 Nf) turns, about its centre.  With the centre's
+// phase theta and a middle step c taken out of F,
+//     F'_t = F_t exp(2 pi i t theta),  G_u = F'_{c+u} + F'_{c-u},  H_u = F'_{c+u} - F'_{c-u},
+// both sums share two real-weighted ones:
+//     S(+-phi) = exp(+-2 pi i c phi) (C +- i D),
+//     C = F'_c + sum_u G_u cos(2 pi u phi),  D = sum_u H_u sin(2 pi u phi).
+// That is 4 multiply-adds a step for the weights' recurrence and 4 a step for C and D, for two
+// rates, where Horner's rule takes 4 for each step and rate (the steps come in pairs: 16 steps are
+// 8 terms).  It also rounds less: the recurrence's start enters with powers up to c, not 2c, and
+// the factor exp(2 pi i c phi) is exact.  Simulated relative error against float64, Horner's rule
+// -> this form: 3.8e-7 -> 1.8e-7 at 16 steps, 7.5e-7 -> 3.3e-7 at 32, 1.6e-6 -> 5.8e-7 at 64.
+// A rate's value does not depend on which other rates are computed: m fixes its arithmetic
+// (start value exact at m & ~3, times exact factors for m & 3), so that rate subsets agree bit for
+// bit with the whole grid.
+// ------------------------------------------------------------------------------------
+// One rate's value from C, D and the rotation (rx, ry) = exp(2 pi i c phi).
+__device__ __forceinline__ void fold_plus(float2 cx, float2 cy, float2 dx, float2 dy, float2 rx, float2 ry,
+                                          float2 nry, float2& x, float2& y) {
+  const float2 px = pk_fma(dy, pk_set(-1.f), cx), py = pk_add(cy, dx);
+  x = pk_fma(px, rx, pk_mul(py, nry));
+  y = pk_fma(px, ry, pk_mul(py, rx));
+}
+__device__ __forceinline__ void fold_minus(float2 cx, float2 cy, float2 dx, float2 dy, float2 rx, float2 ry,
+                                           float2 nry, float2& x, float2& y) {
+  const float2 px = pk_add(cx, dy), py = pk_fma(dx, pk_set(-1.f), cy);
+  x = pk_fma(px, rx, pk_mul(py, ry));
+  y = pk_fma(py, rx, pk_mul(px, nry));
+}
+
+// C and D of two bins (lanes) with F in registers: slot c = NTR/2 holds F'_c, c + u and c - u
+// hold H_u and G_u, slot 0 holds F'_0 (G_c = F'_0, H_c = -F'_0), whose weight is the rotation: in
+// slots c - u = 0 only where the middle step is c.  (zx, zy) = exp(2 pi i phi).
+template <int NTR>
+__device__ __forceinline__ void fold_sums(const float2 (&Gx)[NTR], const float2 (&Gy)[NTR], float2 zx, float2 zy,
+                                          float2 rx, float2 nry, float2& cx, float2& cy, float2& dx, float2& dy) {
+  constexpr int c = NTR / 2;
+  const float2 nzy = pk_neg(zy);
+  float2 wx = zx, wy = zy;
+  cx = pk_fma(Gx[c - 1], wx, Gx[c]);
+  cy = pk_fma(Gy[c - 1], wx, Gy[c]);
+  dx = pk_mul(Gx[c + 1], wy);
+  dy = pk_mul(Gy[c + 1], wy);
+#pragma unroll
+  for (int u = 2; u < c; ++u) {
+    const float2 tx = pk_fma(wx, zx, pk_mul(wy, nzy));
+    wy = pk_fma(wx, zy, pk_mul(wy, zx));
+    wx = tx;
+    cx = pk_fma(Gx[c - u], wx, cx);
+    cy = pk_fma(Gy[c - u], wx, cy);
+    dx = pk_fma(Gx[c + u], wy, dx);
+    dy = pk_fma(Gy[c + u], wy, dy);
+  }
+  cx = pk_fma(Gx[0], rx, cx);
+  cy = pk_fma(Gy[0], rx, cy);
+  dx = pk_fma(Gx[0], nry, dx);
+  dy = pk_fma(Gy[0], nry, dy);
+}
+
+// The same with the folded F of a bin pair in shared memory: g[t * stride] = {x0, x1, y0, y1} of
+// time step t (F'_c at t = c = Nt / 2, H_u at c + u, G_u at c - u), without F'_0's term for even
+// Nt.  M values of m at a time share the loads: two 16-byte loads for 8 M packed multiply-adds.
+template <int M>
+__device__ __forceinline__ void fold_sums_smem(const float4* g, int stride, int Nt, const float2 (&zx)[M],
+                                               const float2 (&zy)[M], float2 (&cx)[M], float2 (&cy)[M],
+                                               float2 (&dx)[M], float2 (&dy)[M]) {
+  const int c = Nt >> 1;
+  const int n = (Nt & 1) ? c : c - 1;
+  float2 wx[M], wy[M], nzy[M];
+  const float4 gc = g[c * stride];
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    cx[i] = make_float2(gc.x, gc.y);
+    cy[i] = make_float2(gc.z, gc.w);
+    dx[i] = dy[i] = make_float2(0.f, 0.f);
+    nzy[i] = pk_neg(zy[i]);
+    wx[i] = zx[i];
+    wy[i] = zy[i];
+  }
+  const float4* lo = g + (c - 1) * stride;
+  const float4* hi = g + (c + 1) * stride;
+#pragma unroll 2
+  for (int u = 1; u <= n; ++u, lo -= stride, hi += stride) {
+    const float4 a = *lo, b = *hi;
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      cx[i] = pk_fma(make_float2(a.x, a.y), wx[i], cx[i]);
+      cy[i] = pk_fma(make_float2(a.z, a.w), wx[i], cy[i]);
+      dx[i] = pk_fma(make_float2(b.x, b.y), wy[i], dx[i]);
+      dy[i] = pk_fma(make_float2(b.z, b.w), wy[i], dy[i]);
+      const float2 tx = pk_fma(wx[i], zx[i], pk_mul(wy[i], nzy[i]));
+      wy[i] = pk_fma(wx[i], zy[i], pk_mul(wy[i], zx[i]));
+      wx[i] = tx;
+    }
+  }
+}
+// F'_0's term of even Nt (G_c = F'_0, H_c = -F'_0; its weight is the rotation).
+__device__ __forceinline__ void fold_first_step(const float4* g, int Nt, float2 rx, float2 nry, float2& cx, float2& cy,
+                                                float2& dx, float2& dy) {
+  if (Nt & 1) return;
+  const float4 a = g[0];
+  cx = pk_fma(make_float2(a.x, a.y), rx, cx);
+  cy = pk_fma(make_float2(a.z, a.w), rx, cy);
+  dx = pk_fma(make_float2(a.x, a.y), nry, dx);
+  dy = pk_fma(make_float2(a.z, a.w), nry, dy);
+}
+
+// exp(2 pi i phi) and exp(2 pi i c phi) of the values of m in one group m & ~3 of a bin pair.
+struct FoldPhase {
+  unsigned long long rh0, rh1;  // k Rh of the two bins
+  int c;
+  float2 zx, zy, rx, ry;        // at m = 4 * group
+  __device__ __forceinline__ void start(int group) {
+    const unsigned long long n = 8ull * (unsigned)group + 1ull;
+    const unsigned long long p0 = n * rh0, p1 = n * rh1;
+    cis_turn_pk(p0, p1, zx, zy);
+    cis_turn_pk((unsigned)c * p0, (unsigned)c * p1, rx, ry);
+  }
+};
+// The factors of m & 3 = q > 0: exp(2 pi i 2 q k Rh) and its c-th power.
+__device__ __forceinline__ void fold_factor(const FoldPhase& f, int q, float2& zx, float2& zy, float2& rx, float2& ry) {
+  const unsigned long long p0 = 2ull * q * f.rh0, p1 = 2ull * q * f.rh1;
+  cis_turn_pk(p0, p1, zx, zy);
+  cis_turn_pk((unsigned)f.c * p0, (unsigned)f.c * p1, rx, ry);
+}
+
+// The phases of a thread of the kernels with F in shared memory: the factors stay in registers.
+struct FoldPhases : FoldPhase {
+  float2 fzx[3], fzy[3], frx[3], fry[3];
+  __device__ __forceinline__ void setup(unsigned long long k0, unsigned long long k1, unsigned long long Rh, int middle) {
+    rh0 = k0 * Rh;
+    rh1 = k1 * Rh;
+    c = middle;
+#pragma unroll
+    for (int q = 1; q < 4; ++q) fold_factor(*this, q, fzx[q - 1], fzy[q - 1], frx[q - 1], fry[q - 1]);
+  }
+  // z at m = 4 group + q (start(group) first); q uniform over the warp
+  __device__ __forceinline__ void z_of(int q, float2& x, float2& y) const {
+    if (q == 0) { x = zx; y = zy; }
+    else if (q == 1) pk_cmul(zx, zy, fzx[0], fzy[0], x, y);
+    else if (q == 2) pk_cmul(zx, zy, fzx[1], fzy[1], x, y);
+    else pk_cmul(zx, zy, fzx[2], fzy[2], x, y);
+  }
+  __device__ __forceinline__ void r_of(int q, float2& x, float2& y) const {
+    if (q == 0) { x = rx; y = ry; }
+    else if (q == 1) pk_cmul(rx, ry, frx[0], fry[0], x, y);
+    else if (q == 2) pk_cmul(rx, ry, frx[1], fry[1], x, y);
+    else pk_cmul(rx, ry, frx[2], fry[2], x, y);
+  }
+};
+
+// Both rates of the M values m = 4 group + q0 + i of a bin pair (start(group) first).
+template <int M>
+__device__ __forceinline__ void fold_pairs_smem(const FoldPhases& f, const float4* g, int stride, int Nt, int q0,
+                                                float2 (&px)[M], float2 (&py)[M], float2 (&mx)[M], float2 (&my)[M]) {
+  float2 zx[M], zy[M], cx[M], cy[M], dx[M], dy[M];
+#pragma unroll
+  for (int i = 0; i < M; ++i) f.z_of(q0 + i, zx[i], zy[i]);
+  fold_sums_smem<M>(g, stride, Nt, zx, zy, cx, cy, dx, dy);
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    float2 rx, ry;
+    f.r_of(q0 + i, rx, ry);
+    const float2 nry = pk_neg(ry);
+    fold_first_step(g, Nt, rx, nry, cx[i], cy[i], dx[i], dy[i]);
+    fold_plus(cx[i], cy[i], dx[i], dy[i], rx, ry, nry, px[i], py[i]);
+    fold_minus(cx[i], cy[i], dx[i], dy[i], rx, ry, nry, mx[i], my[i]);
+  }
+}
+// One rate j of the grid (SUBSET kernels).
+__device__ __forceinline__ void fold_rate_smem(FoldPhases& f, const float4* g, int stride, int Nt, int j, int half,
+                                               float2& x, float2& y) {
+  const int d = j - 2 * half;
+  const int m = d >= 0 ? d : -1 - d;
+  f.start(m >> 2);
+  float2 px[1], py[1], mx[1], my[1];
+  fold_pairs_smem<1>(f, g, stride, Nt, m & 3, px, py, mx, my);
+  x = d >= 0 ? px[0] : mx[0];
+  y = d >= 0 ? py[0] : my[0];
+}
+
+// F'_t = F_t exp(2 pi i t theta) in place, then G_u and H_u in the places of F'_{c-u} and F'_{c+u},
+// for nbp bin pairs in shared memory by all T threads of the block (T a multiple of nbp; F visible
+// before, G and H after).  k0(bp): the pair's first bin, its second is P further.
+template <int T, class Bin>
+__device__ __forceinline__ void fold_smem(const CztArgs& a, float4* gs4, int nbp, Bin k0) {
+  const int bp = threadIdx.x % nbp, part = threadIdx.x / nbp, parts = T / nbp;
+  const unsigned long long th0 = k0(bp) * a.center, th1 = (k0(bp) + (unsigned long long)a.P) * a.center;
+  float4* const g = gs4 + bp;
+  {
+    float2 bx[7], by[7];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) cis_turn_pk((unsigned)i * th0, (unsigned)i * th1, bx[i - 1], by[i - 1]);
+    for (int t0 = 8 * part; t0 < a.Nt; t0 += 8 * parts) {
+      float2 ax, ay;
+      cis_turn_pk((unsigned)t0 * th0, (unsigned)t0 * th1, ax, ay);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (t0 + i < a.Nt) {
+          float2 wx = ax, wy = ay, x, y;
+          if (i > 0) pk_cmul(ax, ay, bx[i - 1], by[i - 1], wx, wy);
+          const float4 v = g[(t0 + i) * nbp];
+          pk_cmul(make_float2(v.x, v.y), make_float2(v.z, v.w), wx, wy, x, y);
+          g[(t0 + i) * nbp] = make_float4(x.x, x.y, y.x, y.y);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  const int c = a.Nt >> 1;
+  for (int u = 1 + part; c + u < a.Nt; u += parts) {
+    const float4 h = g[(c + u) * nbp], l = g[(c - u) * nbp];
+    g[(c + u) * nbp] = make_float4(h.x - l.x, h.y - l.y, h.z - l.z, h.w - l.w);
+    g[(c - u) * nbp] = make_float4(h.x + l.x, h.y + l.y, h.z + l.z, h.w + l.w);
+  }
+  __syncthreads();
+}
+
 // ------------------------------------------------------------------------------------
 // Kernel B: grid (P/2, rate groups), Q/2 threads.
 // ------------------------------------------------------------------------------------
 // WINDOWED = false: the rectangular window (weights 1, skipped: the same FDR bit for bit).
-template <int Q, int NTR, bool WINDOWED>
+// SUBSET: the 8-rate blocks at a.blk_base instead of the whole grid.
+// Per CTA and 8-rate block: the sums of 4 values of m, two rates each, two rates packed per
+// complex sequence (Hermitian halves at k and its mirror), inverse DFT_Q, W.
+template <int Q, int NTR, bool WINDOWED, bool SUBSET>
 __global__ void __launch_bounds__(Q / 2, (Q <= 512 ? 2 : 1)) zdtf_czt_kernel(CztArgs a) {
   constexpr int T = Q / 2;
   constexpr int SS = b_stride<Q>();
@@ -382,8 +649,10 @@ __global__ void __launch_bounds__(Q / 2, (Q <= 512 ? 2 : 1)) zdtf_czt_kernel(Czt
   float2* twr = twt + tw_size(Q);             // 2 * Q
   float2* gnyq = twr + 2 * Q;                 // NTR
   float2* buf2 = gnyq + NTR;                  // kRatesPerBlock * SS
-  // the thread's phase residues alpha_b, beta_b (kept in shared memory, not registers)
-  unsigned long long* phs = reinterpret_cast<unsigned long long*>(buf2 + kRatesPerBlock * SS);
+  // per thread, kept in shared memory instead of registers: the phase steps k Rh of its bins and
+  // the factors of m & 3 = 1..3 (real and imaginary parts of exp(2 pi i phi) and of the rotation)
+  float2* const pw = buf2 + kRatesPerBlock * SS + threadIdx.x;                     // [3][4][T]
+  unsigned long long* const rhs = reinterpret_cast<unsigned long long*>(pw + 12 * T);  // [2][T]
   const int tid = threadIdx.x;
   const int c = blockIdx.x;
   const int P = a.P;
@@ -404,134 +673,157 @@ __global__ void __launch_bounds__(Q / 2, (Q <= 512 ? 2 : 1)) zdtf_czt_kernel(Czt
       Gy[t] = make_float2(G[0][t].y, G[1][t].y);
     }
   }
-
-  // Per-base phase state: w_{k,j} = exp(2 pi i (alpha + j*beta) / 2^bits); rates are taken
-  // kHorner at a time, w = w(first rate of the group, exact) * pw[jr] (exact).
-  const unsigned long long mask = a.ph.mask;
-  // PWx/PWy[i - 1] = exact w(k_b, i*dr) for i = 1..kHorner (lanes = b; w(k_b, 0) = 1)
-  float2 PWx[kHorner], PWy[kHorner];
-  float2 WIN;
+  const unsigned long long kb0 = (unsigned long long)k1s[0] + (unsigned long long)P * tid;
+  const unsigned long long kb1 = (unsigned long long)k1s[1] + (unsigned long long)P * tid;
+  FoldPhase fp;
+  fp.c = NTR / 2 - 2 * a.pshift;
+  {
+    // F'_t = F_t exp(2 pi i t theta), t = slot - 2 pshift, from exact factors for slot & ~3 and
+    // slot & 3; then G_u and H_u in the slots c - u and c + u
+    const unsigned long long th0 = kb0 * a.center, th1 = kb1 * a.center;
+    float2 bx[3], by[3];
 #pragma unroll
-  for (int b = 0; b < 2; ++b) {
-    const unsigned long long k = (unsigned long long)k1s[b] + (unsigned long long)P * tid;
-    const unsigned long long beta = (k * a.ph.Rd) & mask;
-    phs[(2 * b) * T + tid] = (k * a.ph.R0) & mask;
-    phs[(2 * b + 1) * T + tid] = beta;
+    for (int i = 1; i < 4; ++i) cis_turn_pk((unsigned)i * th0, (unsigned)i * th1, bx[i - 1], by[i - 1]);
 #pragma unroll
-    for (int i = 1; i <= kHorner; ++i) {
-      const float2 p = cis_phase(((unsigned long long)i * beta) & mask, a.ph);
-      if (b == 0) { PWx[i - 1].x = p.x; PWy[i - 1].x = p.y; } else { PWx[i - 1].y = p.x; PWy[i - 1].y = p.y; }
+    for (int g = 0; g < NTR / 4; ++g) {
+      const unsigned long long t0 = (unsigned long long)(long long)(4 * g - 2 * a.pshift);
+      float2 ax, ay;
+      cis_turn_pk(t0 * th0, t0 * th1, ax, ay);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float2 wx = ax, wy = ay;
+        if (i > 0) pk_cmul(ax, ay, bx[i - 1], by[i - 1], wx, wy);
+        const float2 fx = Gx[4 * g + i], fy = Gy[4 * g + i];
+        pk_cmul(fx, fy, wx, wy, Gx[4 * g + i], Gy[4 * g + i]);
+      }
     }
-    const float wv = window_value(a, (long long)k);
-    if (b == 0) WIN.x = wv; else WIN.y = wv;
+#pragma unroll
+    for (int u = 1; u < NTR / 2; ++u) {
+      const int lo = NTR / 2 - u, hi = NTR / 2 + u;
+      const float2 lx = Gx[lo], ly = Gy[lo];
+      Gx[lo] = pk_add(Gx[hi], lx);
+      Gy[lo] = pk_add(Gy[hi], ly);
+      Gx[hi] = pk_fma(lx, pk_set(-1.f), Gx[hi]);
+      Gy[hi] = pk_fma(ly, pk_set(-1.f), Gy[hi]);
+    }
+    fp.rh0 = kb0 * a.ph.Rh;
+    fp.rh1 = kb1 * a.ph.Rh;
+    rhs[0] = fp.rh0;
+    rhs[T] = fp.rh1;
+#pragma unroll
+    for (int q = 1; q < 4; ++q) {
+      float2 zx, zy, rx, ry;
+      fold_factor(fp, q, zx, zy, rx, ry);
+      float2* const o = pw + (q - 1) * 4 * T;
+      o[0] = zx;
+      o[T] = zy;
+      o[2 * T] = rx;
+      o[3 * T] = ry;
+    }
   }
-  // Nyquist bin (CTA 0, thread 0)
-  const unsigned long long kny = (unsigned long long)(a.N / 2);
-
+  const float2 win = make_float2(window_value(a, (long long)kb0), window_value(a, (long long)kb1));
   int ms[2], mk2[2];
 #pragma unroll
   for (int b = 0; b < 2; ++b) mirror_of(c, b, tid, Q, &ms[b], &mk2[b]);
   const bool dc = (c == 0 && tid == 0);
 
+  // z and rotation of m = 4 group + q
+  auto phase = [&](int q, float2& zx, float2& zy, float2& rx, float2& ry) {
+    if (q == 0) {
+      zx = fp.zx; zy = fp.zy; rx = fp.rx; ry = fp.ry;
+    } else {
+      const float2* const o = pw + (q - 1) * 4 * T;
+      pk_cmul(fp.zx, fp.zy, o[0], o[T], zx, zy);
+      pk_cmul(fp.rx, fp.ry, o[2 * T], o[3 * T], rx, ry);
+    }
+  };
   // Rate blocks alternate between buf2 and buf (the forward pass used buf): the inverse
-  // DFT_Q ping-pongs between the two, and the buffer a block's Horner sums go to was last
-  // read before the previous block's final barrier, so no barrier precedes the writes.
+  // DFT_Q ping-pongs between the two, and the buffer a block's sums go to was last read
+  // before the previous block's final barrier, so no barrier precedes the writes.
   constexpr bool kFlip = (passes_before_emit(Q) % 2) == 0;
   float2* hb = buf2;
   float2* ob = buf;
-  const int q_begin = blockIdx.y * a.pairs_per_group;
-  const int q_end = min(a.npairs, q_begin + a.pairs_per_group);
-  for (int q0 = q_begin; q0 < q_end; q0 += kRatesPerBlock / 2) {
-    const int j0 = 2 * q0;
-    const long long jg = a.blk_base ? (long long)__ldg(a.blk_base + (q0 >> 2)) : (long long)j0;
-    // exact phase of the block's first rate; the second half starts at w0 * w(k, 4*dr)
-    float2 Wbx, Wby;
-    {
-      const float2 w0 = cis_phase((phs[tid] + (unsigned long long)jg * phs[T + tid]) & mask, a.ph);
-      const float2 w1 = cis_phase((phs[2 * T + tid] + (unsigned long long)jg * phs[3 * T + tid]) & mask, a.ph);
-      Wbx = make_float2(w0.x, w1.x);
-      Wby = make_float2(w0.y, w1.y);
+  // sequence pair u: rates a and b of both bins (lanes), b or both zero past the grid's last
+  auto put_pair = [&](int u, float2 ax, float2 ay, float2 bx, float2 by) {
+    if (WINDOWED) {
+      ax = pk_mul(ax, win); ay = pk_mul(ay, win);
+      bx = pk_mul(bx, win); by = pk_mul(by, win);
     }
 #pragma unroll
-    for (int h = 0; h < kRatesPerBlock / kHorner; ++h) {
-      const int jh = j0 + h * kHorner;
-      float2 S[2][kHorner];
-      float2 W0x = Wbx, W0y = Wby;
-      if (h > 0) {  // w(first rate of the half) = wb * w(k, kHorner*dr)
-        W0x = pk_fma(Wbx, PWx[kHorner - 1], pk_mul(pk_neg(Wby), PWy[kHorner - 1]));
-        W0y = pk_fma(Wbx, PWy[kHorner - 1], pk_mul(Wby, PWx[kHorner - 1]));
-      }
-      const float2 NW0y = pk_neg(W0y);
-      if (jh < a.Nr) {
-#pragma unroll
-        for (int jr = 0; jr < kHorner; ++jr) {
-          float2 wx = W0x, wy = W0y;  // jr = 0: w(k, 0) = 1
-          if (jr > 0) {
-            wx = pk_fma(W0x, PWx[jr - 1], pk_mul(NW0y, PWy[jr - 1]));
-            wy = pk_fma(W0x, PWy[jr - 1], pk_mul(W0y, PWx[jr - 1]));
-          }
-          float2 sx, sy;
-          horner_pk<NTR>(Gx, Gy, wx, wy, sx, sy);
-          if (WINDOWED) {
-            sx = pk_mul(sx, WIN);
-            sy = pk_mul(sy, WIN);
-          }
-          S[0][jr] = make_float2(sx.x, sy.x);
-          S[1][jr] = make_float2(sx.y, sy.y);
-        }
-        if (jh + kHorner > a.Nr) {  // rates past the grid's last (uniform over the CTA): zero
-#pragma unroll
-          for (int jr = 0; jr < kHorner; ++jr)
-            if (jh + jr >= a.Nr) S[0][jr] = S[1][jr] = make_float2(0.f, 0.f);
-        }
-      } else {  // a half block past the last rate (uniform over the CTA): no sums
-#pragma unroll
-        for (int jr = 0; jr < kHorner; ++jr) S[0][jr] = S[1][jr] = make_float2(0.f, 0.f);
-      }
-#pragma unroll
-      for (int b = 0; b < 2; ++b) {
-#pragma unroll
-        for (int u2 = 0; u2 < kHorner / 2; ++u2) {
-          const int u = h * (kHorner / 2) + u2;  // rate pair within the block
-          const float2 sa = S[b][2 * u2], sb = S[b][2 * u2 + 1];
-          if (dc && b == 0) {
-            hb[(2 * u) * SS + pidx(0)] = make_float2(sa.x, sb.x);  // real-only DC bin
-          } else {
-            hb[(2 * u + b) * SS + pidx(tid)] = make_float2(sa.x - sb.y, sa.y + sb.x);          // sa + i sb
-            hb[(2 * u + ms[b]) * SS + pidx(mk2[b])] = make_float2(sa.x + sb.y, sb.x - sa.y);  // conj(sa) + i conj(sb)
-          }
-        }
+    for (int b = 0; b < 2; ++b) {
+      const float2 sa = b ? make_float2(ax.y, ay.y) : make_float2(ax.x, ay.x);
+      const float2 sb = b ? make_float2(bx.y, by.y) : make_float2(bx.x, by.x);
+      if (dc && b == 0) {
+        hb[(2 * u) * SS + pidx(0)] = make_float2(sa.x, sb.x);  // real-only DC bin
+      } else {
+        hb[(2 * u + b) * SS + pidx(tid)] = make_float2(sa.x - sb.y, sa.y + sb.x);          // sa + i sb
+        hb[(2 * u + ms[b]) * SS + pidx(mk2[b])] = make_float2(sa.x + sb.y, sb.x - sa.y);  // conj(sa) + i conj(sb)
       }
     }
-    if (c == 0 && tid == 0) {
-      float2 Gn[NTR];
+  };
+  const float2 zero = make_float2(0.f, 0.f);
+  const int blk_end = min(a.nblk, (int)(blockIdx.y + 1) * a.blocks_per_group);
+  for (int blk = blockIdx.y * a.blocks_per_group; blk < blk_end; ++blk) {
+    fp.rh0 = rhs[0];
+    fp.rh1 = rhs[T];
+    if (!SUBSET) {
+      fp.start(blk);
 #pragma unroll
-      for (int t = 0; t < NTR; ++t) Gn[t] = gnyq[t];
-      const float wn = window_value(a, (long long)kny);
+      for (int i = 0; i < 2; ++i) {
+        const int sp = 2 * blk + i;
+        if (sp < a.half) {  // uniform; an odd last super pair leaves its sequences unused
+          float2 px[2], py[2], mx[2], my[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float2 zx, zy, rx, ry, cx, cy, dx, dy;
+            phase(2 * i + e, zx, zy, rx, ry);
+            const float2 nry = pk_neg(ry);
+            fold_sums<NTR>(Gx, Gy, zx, zy, rx, nry, cx, cy, dx, dy);
+            fold_plus(cx, cy, dx, dy, rx, ry, nry, px[e], py[e]);
+            fold_minus(cx, cy, dx, dy, rx, ry, nry, mx[e], my[e]);
+          }
+          const int ja = 2 * (a.half + sp);  // rates past the grid's last (uniform): zero
+          if (ja >= a.Nr) px[0] = py[0] = zero;
+          if (ja + 1 >= a.Nr) px[1] = py[1] = zero;
+          put_pair(2 * i, px[0], py[0], px[1], py[1]);
+          put_pair(2 * i + 1, mx[1], my[1], mx[0], my[0]);
+        }
+      }
+    } else {
+      const int jg = __ldg(a.blk_base + blk);
+      int group = -1;
+#pragma unroll
       for (int u = 0; u < kRatesPerBlock / 2; ++u) {
-        float v[2];
+        float2 vx[2], vy[2];
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          const int j = j0 + 2 * u + hh;
-          const unsigned long long alpha_n = (kny * a.ph.R0) & mask, beta_n = (kny * a.ph.Rd) & mask;
-          const float2 w = cis_phase((alpha_n + (unsigned long long)(jg + 2 * u + hh) * beta_n) & mask, a.ph);
-          const float2 sv = horner<NTR>(Gn, w);
-          v[hh] = (j < a.Nr) ? sv.x * wn : 0.f;  // real-only Nyquist bin
+        for (int e = 0; e < 2; ++e) {
+          const int d = jg + 2 * u + e - 2 * a.half;
+          const int m = d >= 0 ? d : -1 - d;
+          if ((m >> 2) != group) {  // uniform over the CTA
+            group = m >> 2;
+            fp.start(group);
+          }
+          float2 zx, zy, rx, ry, cx, cy, dx, dy;
+          phase(m & 3, zx, zy, rx, ry);
+          const float2 nry = pk_neg(ry);
+          fold_sums<NTR>(Gx, Gy, zx, zy, rx, nry, cx, cy, dx, dy);
+          if (d >= 0) fold_plus(cx, cy, dx, dy, rx, ry, nry, vx[e], vy[e]);
+          else fold_minus(cx, cy, dx, dy, rx, ry, nry, vx[e], vy[e]);
         }
-        hb[(2 * u) * SS + pidx(Q / 2)] = make_float2(v[0], v[1]);
+        put_pair(u, vx[0], vy[0], vx[1], vy[1]);
       }
     }
+    if (c == 0 && tid < kRatesPerBlock)
+      nyquist_block<SUBSET>(a, gnyq, blk, tid, [&](int u, int hh, float v) {
+        reinterpret_cast<float*>(hb + (2 * u) * SS + pidx(Q / 2))[hh] = v;
+      });
     __syncthreads();
-    // inverse DFT_Q; its last pass writes W (with the inter-pass twiddle and 1/Nf) directly.
-    // Row (q0 + p, k1) of W starts at Wq + (p*P + k1)*Q: a 32-bit offset (p < 4; the fused
-    // path has P*Q = Nf <= 2^22).
-    float2* const Wq = a.W + (long long)q0 * P * Q;
+    // inverse DFT_Q; its last pass writes W (with the inter-pass twiddle and 1/Nf) directly
     const int k1a = k1s[0], k1b = k1s[1];
     stockham_passes_emit_pp<Q, kRatesPerBlock, SS, T, +1, 1>(hb, ob, twt, [&](int seq, int na, float2 v) {
-      const int p = seq >> 1, side = seq & 1;
-      const unsigned off = (unsigned)((p * P + (side ? k1b : k1a)) * Q + na);
-      if (q0 + p < q_end && FDR_DBG_OK((long long)q0 * P * Q + off < (long long)a.npairs * P * Q))
-        Wq[off] = cmul(v, twr[side * Q + na]);
+      const int p = block_pair<SUBSET>(a, blk, seq >> 1), side = seq & 1;
+      const long long at = ((long long)p * P + (side ? k1b : k1a)) * Q + na;
+      if (p >= 0 && FDR_DBG_OK(at < (long long)a.npairs * P * Q)) a.W[at] = cmul(v, twr[side * Q + na]);
     });
     if (kFlip) {
       float2* t = hb;
@@ -546,15 +838,14 @@ __global__ void __launch_bounds__(Q / 2, (Q <= 512 ? 2 : 1)) zdtf_czt_kernel(Czt
 // memory, t-major with the bases in adjacent pairs interleaved by component: float4
 // gs4[t*(Q/2) + b/2] = {Re F[b0], Re F[b1], Im F[b0], Im F[b1]} for b0 = b & ~1, b1 = b0 + 1,
 // so one 16-byte load gives the packed-FP32 operands (Re, Re) and (Im, Im) of a base pair.
-// T = Q*G threads, G = threads per base pair and rate half; each thread evaluates RT = 4/G
-// rates of every 8-rate block for its two bases, lanes = bases.  Base b (0 <= b < Q) is side
-// b/(Q/2), k2 = b % (Q/2) (a pair never straddles the sides: Q/2 is even).
+// T = Q*G threads; a thread evaluates one super pair (4 rates) of every 8-rate block for its two
+// bases, lanes = bases (with G = 2 half of the threads only transform).  Base b (0 <= b < Q) is
+// side b/(Q/2), k2 = b % (Q/2) (a pair never straddles the sides: Q/2 is even).
 // ------------------------------------------------------------------------------------
 template <int Q>
 struct CztSmemShape {
   static constexpr int G = Q >= 512 ? 1 : 2;
   static constexpr int T = Q * G;
-  static constexpr int RT = 4 / G;
   // gs starts on a 16-byte boundary (an even float2 offset)
   static constexpr int GS_OFF = (kRatesPerBlock * b_stride<Q>() + tw_size(Q) + 2 * Q + 1) & ~1;
   template <int NT>
@@ -644,10 +935,30 @@ __device__ __forceinline__ void czt_forward_smem(const CztArgs& a, int c, const 
   __syncthreads();
 }
 
-template <int Q, int NT>
+// Packs rates a and b of a base pair (lanes; bases k20 and k20 + 1 of `side`) into the two
+// sequences at `seq`: sa + i sb at the base, conj(sa) + i conj(sb) at its mirror.
+template <int SS>
+__device__ __forceinline__ void put_rate_pair(float2* seq, int side, int k20, const int (&ms)[2], const int (&mk2)[2],
+                                              bool dc, float2 win, float2 ax, float2 ay, float2 bx, float2 by) {
+  ax = pk_mul(ax, win); ay = pk_mul(ay, win);
+  bx = pk_mul(bx, win); by = pk_mul(by, win);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const float2 sa = h ? make_float2(ax.y, ay.y) : make_float2(ax.x, ay.x);
+    const float2 sb = h ? make_float2(bx.y, by.y) : make_float2(bx.x, by.x);
+    if (dc && h == 0) {
+      seq[pidx(0)] = make_float2(sa.x, sb.x);
+    } else {
+      seq[side * SS + pidx(k20 + h)] = make_float2(sa.x - sb.y, sa.y + sb.x);
+      seq[ms[h] * SS + pidx(mk2[h])] = make_float2(sa.x + sb.y, sb.x - sa.y);
+    }
+  }
+}
+
+template <int Q, int NT, bool SUBSET>
 __global__ void __launch_bounds__(CztSmemShape<Q>::T, 1) zdtf_czt_smem_kernel(CztArgs a) {
   using SH = CztSmemShape<Q>;
-  constexpr int T = SH::T, RT = SH::RT;
+  constexpr int T = SH::T;
   constexpr int SS = b_stride<Q>();
   extern __shared__ float2 sm[];
   float2* buf = sm;
@@ -667,8 +978,14 @@ __global__ void __launch_bounds__(CztSmemShape<Q>::T, 1) zdtf_czt_smem_kernel(Cz
   }
   czt_forward_smem<Q, NT>(a, c, k1s, buf, twt, gs, gnyq);
 
-  // thread -> (base pair bp, rate group rg): bases b0 = 2 bp and b0 + 1 (the two lanes of
-  // every packed operation), rates rg*RT .. rg*RT + RT - 1 of each 8-rate block
+  auto bin0 = [&](int bp) {
+    const int b0 = 2 * bp, side = b0 / (Q / 2);
+    return (unsigned long long)k1s[side] + (unsigned long long)P * (b0 - side * (Q / 2));
+  };
+  fold_smem<T>(a, reinterpret_cast<float4*>(gs), Q / 2, bin0);
+
+  // thread -> (base pair bp, super pair rg of every block): bases b0 = 2 bp and b0 + 1 (the two
+  // lanes of every packed operation); threads past the second super pair only transform
   const int bp = tid % (Q / 2), rg = tid / (Q / 2);
   const int b0 = 2 * bp;
   const int side = b0 / (Q / 2), k20 = b0 - side * (Q / 2);
@@ -676,144 +993,71 @@ __global__ void __launch_bounds__(CztSmemShape<Q>::T, 1) zdtf_czt_smem_kernel(Cz
   mirror_of(c, side, k20, Q, &ms[0], &mk2[0]);
   mirror_of(c, side, k20 + 1, Q, &ms[1], &mk2[1]);
   const bool dc = (c == 0 && side == 0 && k20 == 0);  // lane 0 is the DC bin
-  const unsigned long long mask = a.ph.mask;
-  unsigned long long alpha[2], beta[2];
-  float2 pwx[RT], pwy[RT];  // pw[i] = exact w(k_lane, i*dr), lanes = the two bases
-  float2 win;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const unsigned long long k = (unsigned long long)k1s[side] + (unsigned long long)P * (k20 + h);
-    alpha[h] = (k * a.ph.R0) & mask;
-    beta[h] = (k * a.ph.Rd) & mask;
-#pragma unroll
-    for (int i = 0; i < RT; ++i) {
-      const float2 p = cis_phase(((unsigned long long)i * beta[h]) & mask, a.ph);
-      if (h == 0) { pwx[i].x = p.x; pwy[i].x = p.y; } else { pwx[i].y = p.x; pwy[i].y = p.y; }
-    }
-    const float wv = window_value(a, (long long)k);
-    if (h == 0) win.x = wv; else win.y = wv;
-  }
-  const unsigned long long kny = (unsigned long long)(a.N / 2);
-  const unsigned long long alpha_n = (kny * a.ph.R0) & mask, beta_n = (kny * a.ph.Rd) & mask;
+  const float2 win = make_float2(window_value(a, (long long)bin0(bp)), window_value(a, (long long)bin0(bp) + P));
   const int Nt = a.Nt;
-  const float4* gs4 = reinterpret_cast<const float4*>(gs);
+  FoldPhases fp;
+  fp.setup(bin0(bp), bin0(bp) + (unsigned long long)P, a.ph.Rh, Nt >> 1);
+  const float4* const g = reinterpret_cast<const float4*>(gs) + bp;
+  const float2 zero = make_float2(0.f, 0.f);
 
-  const int q_begin = blockIdx.y * a.pairs_per_group;
-  const int q_end = min(a.npairs, q_begin + a.pairs_per_group);
-  for (int q0 = q_begin; q0 < q_end; q0 += kRatesPerBlock / 2) {
-    const int j0 = 2 * q0 + rg * RT;  // this thread's first rate of the block
-    const long long jb = a.blk_base ? (long long)__ldg(a.blk_base + (q0 >> 2)) : (long long)(2 * q0);
-    // w(k_lane, first rate) exact; the thread's other rates = that * pw[i] (exact pw)
-    float2 W0x, W0y;
-    {
-      const unsigned long long jj = (unsigned long long)(jb + rg * RT);
-      const float2 w0 = cis_phase((alpha[0] + jj * beta[0]) & mask, a.ph);
-      const float2 w1 = cis_phase((alpha[1] + jj * beta[1]) & mask, a.ph);
-      W0x = make_float2(w0.x, w1.x);
-      W0y = make_float2(w0.y, w1.y);
-    }
-    float2 Wx[RT], Wy[RT], NWy[RT], Sx[RT], Sy[RT];
-    {
-      const float2 NW0y = pk_neg(W0y);
-      const float4 gl = gs4[(Nt - 1) * (Q / 2) + bp];
-#pragma unroll
-      for (int r = 0; r < RT; ++r) {
-        if (r == 0) {
-          Wx[r] = W0x;
-          Wy[r] = W0y;
-        } else {
-          Wx[r] = pk_fma(W0x, pwx[r], pk_mul(NW0y, pwy[r]));
-          Wy[r] = pk_fma(W0x, pwy[r], pk_mul(W0y, pwx[r]));
-        }
-        NWy[r] = pk_neg(Wy[r]);
-        Sx[r] = make_float2(gl.x, gl.y);
-        Sy[r] = make_float2(gl.z, gl.w);
+  const int blk_end = min(a.nblk, (int)(blockIdx.y + 1) * a.blocks_per_group);
+  for (int blk = blockIdx.y * a.blocks_per_group; blk < blk_end; ++blk) {
+    float2 px[2] = {zero, zero}, py[2] = {zero, zero}, mx[2] = {zero, zero}, my[2] = {zero, zero};
+    if (SUBSET) {
+      if (rg < 2) {
+        const int j = __ldg(a.blk_base + blk) + 4 * rg;  // pairs 2 rg (px) and 2 rg + 1 (mx, swapped)
+        fold_rate_smem(fp, g, Q / 2, Nt, j, a.half, px[0], py[0]);
+        fold_rate_smem(fp, g, Q / 2, Nt, j + 1, a.half, px[1], py[1]);
+        fold_rate_smem(fp, g, Q / 2, Nt, j + 2, a.half, mx[1], my[1]);
+        fold_rate_smem(fp, g, Q / 2, Nt, j + 3, a.half, mx[0], my[0]);
       }
-    }
-    // Horner's rule over t for the thread's RT rates, both bases in the packed lanes
-#pragma unroll 4
-    for (int t = Nt - 2; t >= 0; --t) {
-      const float4 gt = gs4[t * (Q / 2) + bp];
-      const float2 gx = make_float2(gt.x, gt.y), gy = make_float2(gt.z, gt.w);
-#pragma unroll
-      for (int r = 0; r < RT; ++r) {
-        const float2 tx = pk_fma(Sx[r], Wx[r], pk_fma(Sy[r], NWy[r], gx));
-        const float2 ty = pk_fma(Sx[r], Wy[r], pk_fma(Sy[r], Wx[r], gy));
-        Sx[r] = tx;
-        Sy[r] = ty;
-      }
+    } else if (rg < 2 && 2 * blk + rg < a.half) {
+      fp.start(blk);
+      fold_pairs_smem<2>(fp, g, Q / 2, Nt, 2 * rg, px, py, mx, my);
+      const int ja = 2 * (a.half + 2 * blk + rg);  // rates past the grid's last: zero
+      if (ja >= a.Nr) px[0] = py[0] = zero;
+      if (ja + 1 >= a.Nr) px[1] = py[1] = zero;
     }
     __syncthreads();  // buf is free
-#pragma unroll
-    for (int up = 0; up < RT / 2; ++up) {
-      const int u = rg * (RT / 2) + up;  // rate pair within the block
-      const bool ok_a = j0 + 2 * up < a.Nr, ok_b = j0 + 2 * up + 1 < a.Nr;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float wh = h ? win.y : win.x;
-        const float2 sa = ok_a ? cscale(make_float2(h ? Sx[2 * up].y : Sx[2 * up].x,
-                                                    h ? Sy[2 * up].y : Sy[2 * up].x), wh)
-                               : make_float2(0.f, 0.f);
-        const float2 sb = ok_b ? cscale(make_float2(h ? Sx[2 * up + 1].y : Sx[2 * up + 1].x,
-                                                    h ? Sy[2 * up + 1].y : Sy[2 * up + 1].x), wh)
-                               : make_float2(0.f, 0.f);
-        if (dc && h == 0) {
-          buf[(2 * u) * SS + pidx(0)] = make_float2(sa.x, sb.x);
-        } else {
-          buf[(2 * u + side) * SS + pidx(k20 + h)] = make_float2(sa.x - sb.y, sa.y + sb.x);
-          buf[(2 * u + ms[h]) * SS + pidx(mk2[h])] = make_float2(sa.x + sb.y, sb.x - sa.y);
-        }
-      }
+    if (rg < 2) {
+      put_rate_pair<SS>(buf + 4 * rg * SS, side, k20, ms, mk2, dc, win, px[0], py[0], px[1], py[1]);
+      put_rate_pair<SS>(buf + (4 * rg + 2) * SS, side, k20, ms, mk2, dc, win, mx[1], my[1], mx[0], my[0]);
     }
-    if (c == 0 && tid == 0) {
-      const float wn = window_value(a, (long long)kny);
-      for (int u = 0; u < kRatesPerBlock / 2; ++u) {
-        float v[2];
-        for (int hh = 0; hh < 2; ++hh) {
-          const int j = 2 * q0 + 2 * u + hh;
-          const float2 wv = cis_phase((alpha_n + (unsigned long long)(jb + 2 * u + hh) * beta_n) & mask, a.ph);
-          float2 sv = gnyq[Nt - 1];
-          for (int t = Nt - 2; t >= 0; --t)
-            sv = make_float2(fmaf(sv.x, wv.x, fmaf(-sv.y, wv.y, gnyq[t].x)),
-                             fmaf(sv.x, wv.y, fmaf(sv.y, wv.x, gnyq[t].y)));
-          v[hh] = (j < a.Nr) ? sv.x * wn : 0.f;
-        }
-        buf[(2 * u) * SS + pidx(Q / 2)] = make_float2(v[0], v[1]);
-      }
-    }
+    if (c == 0 && tid < kRatesPerBlock)
+      nyquist_block<SUBSET>(a, gnyq, blk, tid, [&](int u, int hh, float v) {
+        reinterpret_cast<float*>(buf + (2 * u) * SS + pidx(Q / 2))[hh] = v;
+      });
     __syncthreads();
-    float2* const W = a.W;
     const int k1a = k1s[0], k1b = k1s[1];
     smem_fft_emit<Q, kRatesPerBlock, SS, T, +1>(buf, twt, [&](int seq, int na, float2 v) {
-      const int q = q0 + (seq >> 1), sd = seq & 1;
-      if (q < q_end && FDR_DBG_OK(((long long)q * P + (sd ? k1b : k1a)) * Q + na < (long long)a.npairs * P * Q))
-        W[((long long)q * P + (sd ? k1b : k1a)) * Q + na] = cmul(v, twr[sd * Q + na]);
+      const int p = block_pair<SUBSET>(a, blk, seq >> 1), sd = seq & 1;
+      const long long at = ((long long)p * P + (sd ? k1b : k1a)) * Q + na;
+      if (p >= 0 && FDR_DBG_OK(at < (long long)a.npairs * P * Q)) a.W[at] = cmul(v, twr[sd * Q + na]);
     });
   }
 }
 
 // ------------------------------------------------------------------------------------
 // Kernel B, warp-specialised (Q = 256 or 512, Nt <= NT): F of the CTA's Q bases in shared
-// memory (pair-interleaved as for zdtf_czt_smem_kernel).  H = 256 Horner threads (one base
-// pair each, RT = 8 or 4 rates of every 8-rate block, two bases per packed-FP32 lane pair)
-// fill one of two rate-block buffers while the I = Q/2 FFT threads run the inverse DFT_Q of
-// the other and write W.  The hand-over uses hardware named barriers (bar.sync / bar.arrive
-// with thread counts, no polling):
-//   FULL(i mod 2):  the Horner threads arrive once block i is in buffer i mod 2; the FFT
+// memory (pair-interleaved as for zdtf_czt_smem_kernel).  256 sum threads fill one of two
+// rate-block buffers while the I = Q/2 FFT threads run the inverse DFT_Q of the other and write
+// W.  A sum thread takes a base pair (lanes) and all 4 values of m of a block, so that two
+// 16-byte loads of F feed 32 packed multiply-adds; with Q = 256 the two halves of the sum
+// threads take alternate blocks, each with its own buffer.  The hand-over uses hardware named
+// barriers (bar.sync / bar.arrive with thread counts, no polling) of the HG sum threads of a
+// block and the FFT threads:
+//   FULL(i mod 2):  the sum threads arrive once block i is in buffer i mod 2; the FFT
 //                   threads wait on it before transforming block i;
 //   EMPTY(i mod 2): the FFT threads arrive once they have read block i (when block i + 2
-//                   exists); the Horner threads wait on it before writing block i + 2.
-// The FFT phase (shared-memory latency and its own barriers) thus runs under the Horner phase
-// instead of after it: measured 6-9% faster than zdtf_czt_smem_kernel at Nt = 32 and 64.
-// (The Horner phase itself stays latency-bound; 512 Horner threads, or loads of F issued two
-// steps ahead, measured no faster.)
+//                   exists); the sum threads wait on it before writing block i + 2.
+// The FFT phase (shared-memory latency and its own barriers) thus runs under the sums instead
+// of after them.
 // ------------------------------------------------------------------------------------
 template <int Q>
 struct CztWsShape {
-  static constexpr int H = 256;                   // Horner threads
-  static constexpr int RG = 2 * H / Q;            // rate groups: 1 (Q = 512) or 2 (Q = 256)
-  static constexpr int RT = kRatesPerBlock / RG;  // rates of a block per Horner thread
-  static constexpr int C = RT < 4 ? RT : 4;       // rates evaluated together
+  static constexpr int H = 256;                   // sum threads
+  static constexpr int HG = Q / 2;                // of one block: one base pair each
+  static constexpr int RG = H / HG;               // blocks in progress: 1 (Q = 512) or 2 (Q = 256)
   static constexpr int I = Q / 2;                 // FFT threads
   static constexpr int T = H + I;
   static constexpr int SS = b_stride<Q>();
@@ -826,11 +1070,12 @@ struct CztWsShape {
 };
 constexpr int kBarFull = 1, kBarEmpty = 3, kBarFft = 5;
 
-template <int Q, int NT>
+template <int Q, int NT, bool SUBSET>
 __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArgs a) {
   using SH = CztWsShape<Q>;
-  constexpr int T = SH::T, H = SH::H, I = SH::I, RT = SH::RT, C = SH::C, SS = SH::SS;
-  static_assert(RT % C == 0 && C % 2 == 0 && (Q / 2) % 32 == 0, "rate pairs; warp-uniform rate groups");
+  constexpr int T = SH::T, H = SH::H, HG = SH::HG, RG = SH::RG, I = SH::I, SS = SH::SS;
+  constexpr int BT = HG + I;  // threads of a hand-over barrier
+  static_assert(HG * RG == H && (RG == 1 || RG == 2) && HG % 32 == 0, "whole warps, one buffer per group");
   extern __shared__ float2 sm[];
   float2* const buf0 = sm;
   float2* const buf1 = sm + SH::BUF1;
@@ -849,157 +1094,84 @@ __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArg
     twr[i] = cscale(cconj(tw_fwd(a.tab, (long long)k1s[side] * na)), invN);
   }
   czt_forward_smem<Q, NT, T>(a, c, k1s, buf0, twt, gs, gnyq);  // ends with a barrier
+  auto bin0 = [&](int bp) {
+    const int b0 = 2 * bp, side = b0 / (Q / 2);
+    return (unsigned long long)k1s[side] + (unsigned long long)P * (b0 - side * (Q / 2));
+  };
+  fold_smem<T>(a, reinterpret_cast<float4*>(gs), Q / 2, bin0);  // ends with a barrier
 
-  const int q_begin = blockIdx.y * a.pairs_per_group;
-  const int q_end = min(a.npairs, q_begin + a.pairs_per_group);
-  const int nblk = q_end > q_begin ? (q_end - q_begin + kRatesPerBlock / 2 - 1) / (kRatesPerBlock / 2) : 0;
+  const int blk0 = blockIdx.y * a.blocks_per_group;
+  const int nblk = min(a.nblk - blk0, a.blocks_per_group);
 
   if (tid < H) {
-    // ---------------- Horner threads ----------------
-    const int bp = tid % (Q / 2), rg = tid / (Q / 2);
+    // ---------------- sum threads ----------------
+    const int bp = tid % HG, rg = tid / HG;
     const int b0 = 2 * bp;
     const int side = b0 / (Q / 2), k20 = b0 - side * (Q / 2);
     int ms[2], mk2[2];
     mirror_of(c, side, k20, Q, &ms[0], &mk2[0]);
     mirror_of(c, side, k20 + 1, Q, &ms[1], &mk2[1]);
     const bool dc = (c == 0 && side == 0 && k20 == 0);  // lane 0 is the DC bin
-    const unsigned long long mask = a.ph.mask;
-    unsigned long long alpha[2], beta[2];
-    float2 pwx[C], pwy[C];  // exact w(k_lane, i*dr) for i = 1..C (lanes = the two bases)
-    float2 win;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const unsigned long long k = (unsigned long long)k1s[side] + (unsigned long long)P * (k20 + h);
-      alpha[h] = (k * a.ph.R0) & mask;
-      beta[h] = (k * a.ph.Rd) & mask;
-#pragma unroll
-      for (int i = 1; i <= C; ++i) {
-        const float2 p = cis_phase(((unsigned long long)i * beta[h]) & mask, a.ph);
-        if (h == 0) { pwx[i - 1].x = p.x; pwy[i - 1].x = p.y; } else { pwx[i - 1].y = p.x; pwy[i - 1].y = p.y; }
-      }
-      const float wv = window_value(a, (long long)k);
-      if (h == 0) win.x = wv; else win.y = wv;
-    }
-    const unsigned long long kny = (unsigned long long)(a.N / 2);
-    const unsigned long long alpha_n = (kny * a.ph.R0) & mask, beta_n = (kny * a.ph.Rd) & mask;
+    const float2 win = make_float2(window_value(a, (long long)bin0(bp)), window_value(a, (long long)bin0(bp) + P));
     const int Nt = a.Nt;
-    const float4* gs4 = reinterpret_cast<const float4*>(gs);
-    for (int ib = 0; ib < nblk; ++ib) {
-      const int q0 = q_begin + ib * (kRatesPerBlock / 2);
+    FoldPhases fp;
+    fp.setup(bin0(bp), bin0(bp) + (unsigned long long)P, a.ph.Rh, Nt >> 1);
+    const float4* const g = reinterpret_cast<const float4*>(gs) + bp;
+    const float2 zero = make_float2(0.f, 0.f);
+    for (int ib = rg; ib < nblk; ib += RG) {
+      const int blk = blk0 + ib;
       float2* const hb = (ib & 1) ? buf1 : buf0;
-      const int j0 = 2 * q0 + rg * RT;  // this thread's first rate of the block
-      const long long jb = a.blk_base ? (long long)__ldg(a.blk_base + (q0 >> 2)) : (long long)(2 * q0);
-      float2 Wbx, Wby;  // exact w(k_lane, first rate of the thread)
-      {
-        const unsigned long long jj = (unsigned long long)(jb + rg * RT);
-        const float2 w0 = cis_phase((alpha[0] + jj * beta[0]) & mask, a.ph);
-        const float2 w1 = cis_phase((alpha[1] + jj * beta[1]) & mask, a.ph);
-        Wbx = make_float2(w0.x, w1.x);
-        Wby = make_float2(w0.y, w1.y);
-      }
-#pragma unroll
-      for (int ch = 0; ch < RT / C; ++ch) {  // chunks of C rates
-        float2 Sx[C], Sy[C];
-        const bool live = j0 + C * ch < a.Nr;  // uniform over the warp (rg is)
-        if (live) {
-          float2 W0x = Wbx, W0y = Wby;
-          if (ch > 0) {  // w(first rate of the chunk) = wb * w(k, C*dr) (ch = 1 only: RT <= 2C)
-            W0x = pk_fma(Wbx, pwx[C - 1], pk_mul(pk_neg(Wby), pwy[C - 1]));
-            W0y = pk_fma(Wbx, pwy[C - 1], pk_mul(Wby, pwx[C - 1]));
-          }
-          const float2 NW0y = pk_neg(W0y);
-          float2 Wx[C], Wy[C], NWy[C];
-          const float4 gl = gs4[(Nt - 1) * (Q / 2) + bp];
-#pragma unroll
-          for (int r = 0; r < C; ++r) {
-            if (r == 0) {
-              Wx[r] = W0x;
-              Wy[r] = W0y;
-            } else {
-              Wx[r] = pk_fma(W0x, pwx[r - 1], pk_mul(NW0y, pwy[r - 1]));
-              Wy[r] = pk_fma(W0x, pwy[r - 1], pk_mul(W0y, pwx[r - 1]));
-            }
-            NWy[r] = pk_neg(Wy[r]);
-            Sx[r] = make_float2(gl.x, gl.y);
-            Sy[r] = make_float2(gl.z, gl.w);
-          }
-#pragma unroll 4
-          for (int t = Nt - 2; t >= 0; --t) {
-            const float4 gt = gs4[t * (Q / 2) + bp];
-            const float2 gx = make_float2(gt.x, gt.y), gy = make_float2(gt.z, gt.w);
-#pragma unroll
-            for (int r = 0; r < C; ++r) {
-              const float2 tx = pk_fma(Sx[r], Wx[r], pk_fma(Sy[r], NWy[r], gx));
-              const float2 ty = pk_fma(Sx[r], Wy[r], pk_fma(Sy[r], Wx[r], gy));
-              Sx[r] = tx;
-              Sy[r] = ty;
-            }
-          }
-        } else {
-#pragma unroll
-          for (int r = 0; r < C; ++r) Sx[r] = Sy[r] = make_float2(0.f, 0.f);
+      auto wait_empty = [&]() {  // the FFT threads have read this buffer's previous block
+        if (ib >= 2) {
+          if (ib & 1) named_sync<kBarEmpty + 1, BT>(); else named_sync<kBarEmpty, BT>();
         }
-        if (ch == 0 && ib >= 2) {  // the FFT threads have read this buffer's previous block
-          if (ib & 1) named_sync<kBarEmpty + 1, T>(); else named_sync<kBarEmpty, T>();
-        }
-#pragma unroll
-        for (int up = 0; up < C / 2; ++up) {
-          const int u = rg * (RT / 2) + ch * (C / 2) + up;  // rate pair within the block
-          const int ja = j0 + C * ch + 2 * up;
-          const bool ok_a = ja < a.Nr, ok_b = ja + 1 < a.Nr;
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const float wh = h ? win.y : win.x;
-            const float2 sa = ok_a ? cscale(make_float2(h ? Sx[2 * up].y : Sx[2 * up].x,
-                                                        h ? Sy[2 * up].y : Sy[2 * up].x), wh)
-                                   : make_float2(0.f, 0.f);
-            const float2 sb = ok_b ? cscale(make_float2(h ? Sx[2 * up + 1].y : Sx[2 * up + 1].x,
-                                                        h ? Sy[2 * up + 1].y : Sy[2 * up + 1].x), wh)
-                                   : make_float2(0.f, 0.f);
-            if (dc && h == 0) {
-              hb[(2 * u) * SS + pidx(0)] = make_float2(sa.x, sb.x);
-            } else {
-              hb[(2 * u + side) * SS + pidx(k20 + h)] = make_float2(sa.x - sb.y, sa.y + sb.x);
-              hb[(2 * u + ms[h]) * SS + pidx(mk2[h])] = make_float2(sa.x + sb.y, sb.x - sa.y);
-            }
-          }
-        }
-      }
-      if (c == 0 && tid == 0) {  // the real-only Nyquist bin of every rate of the block
-        const float wn = window_value(a, (long long)kny);
+      };
+      if (SUBSET) {
+        wait_empty();
+        const int j = __ldg(a.blk_base + blk);
+#pragma unroll 1
         for (int u = 0; u < kRatesPerBlock / 2; ++u) {
-          float v[2];
-          for (int hh = 0; hh < 2; ++hh) {
-            const int j = 2 * q0 + 2 * u + hh;
-            const float2 wv = cis_phase((alpha_n + (unsigned long long)(jb + 2 * u + hh) * beta_n) & mask, a.ph);
-            float2 sv = gnyq[Nt - 1];
-            for (int t = Nt - 2; t >= 0; --t)
-              sv = make_float2(fmaf(sv.x, wv.x, fmaf(-sv.y, wv.y, gnyq[t].x)),
-                               fmaf(sv.x, wv.y, fmaf(sv.y, wv.x, gnyq[t].y)));
-            v[hh] = (j < a.Nr) ? sv.x * wn : 0.f;
-          }
-          hb[(2 * u) * SS + pidx(Q / 2)] = make_float2(v[0], v[1]);
+          float2 ax, ay, bx, by;
+          fold_rate_smem(fp, g, Q / 2, Nt, j + 2 * u, a.half, ax, ay);
+          fold_rate_smem(fp, g, Q / 2, Nt, j + 2 * u + 1, a.half, bx, by);
+          put_rate_pair<SS>(hb + 2 * u * SS, side, k20, ms, mk2, dc, win, ax, ay, bx, by);
+        }
+      } else {
+        float2 px[4], py[4], mx[4], my[4];
+        fp.start(blk);
+        fold_pairs_smem<4>(fp, g, Q / 2, Nt, 0, px, py, mx, my);
+        wait_empty();
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {  // a super pair past the last one leaves unused sequences
+          const int ja = 2 * (a.half + 2 * blk + i);  // rates past the grid's last: zero
+          if (ja >= a.Nr) px[2 * i] = py[2 * i] = zero;
+          if (ja + 1 >= a.Nr) px[2 * i + 1] = py[2 * i + 1] = zero;
+          put_rate_pair<SS>(hb + 4 * i * SS, side, k20, ms, mk2, dc, win, px[2 * i], py[2 * i], px[2 * i + 1], py[2 * i + 1]);
+          put_rate_pair<SS>(hb + (4 * i + 2) * SS, side, k20, ms, mk2, dc, win, mx[2 * i + 1], my[2 * i + 1], mx[2 * i], my[2 * i]);
         }
       }
-      if (ib & 1) named_arrive<kBarFull + 1, T>(); else named_arrive<kBarFull, T>();
+      if (c == 0 && bp < kRatesPerBlock)
+        nyquist_block<SUBSET>(a, gnyq, blk, bp, [&](int u, int hh, float v) {
+          reinterpret_cast<float*>(hb + (2 * u) * SS + pidx(Q / 2))[hh] = v;
+        });
+      __syncwarp();
+      if (ib & 1) named_arrive<kBarFull + 1, BT>(); else named_arrive<kBarFull, BT>();
     }
   } else {
     // ---------------- FFT threads ----------------
     const int ltid = tid - H;
     const int k1a = k1s[0], k1b = k1s[1];
     for (int ib = 0; ib < nblk; ++ib) {
-      const int q0 = q_begin + ib * (kRatesPerBlock / 2);
+      const int blk = blk0 + ib;
       float2* const hb = (ib & 1) ? buf1 : buf0;
-      float2* const Wq = a.W + (long long)q0 * P * Q;  // 32-bit offsets below (Nf <= 2^22)
-      if (ib & 1) named_sync<kBarFull + 1, T>(); else named_sync<kBarFull, T>();
+      if (ib & 1) named_sync<kBarFull + 1, BT>(); else named_sync<kBarFull, BT>();
       group_fft_emit<Q, kRatesPerBlock, SS, I, +1, kBarFft, 1>(hb, twt, ltid, [&](int seq, int na, float2 v) {
-        const int p = seq >> 1, sd = seq & 1;
-        const unsigned off = (unsigned)((p * P + (sd ? k1b : k1a)) * Q + na);
-        if (q0 + p < q_end && FDR_DBG_OK((long long)q0 * P * Q + off < (long long)a.npairs * P * Q))
-          Wq[off] = cmul(v, twr[sd * Q + na]);
+        const int p = block_pair<SUBSET>(a, blk, seq >> 1), sd = seq & 1;
+        const long long at = ((long long)p * P + (sd ? k1b : k1a)) * Q + na;
+        if (p >= 0 && FDR_DBG_OK(at < (long long)a.npairs * P * Q)) a.W[at] = cmul(v, twr[sd * Q + na]);
       });
       if (ib + 2 < nblk) {
-        if (ib & 1) named_arrive<kBarEmpty + 1, T>(); else named_arrive<kBarEmpty, T>();
+        if (ib & 1) named_arrive<kBarEmpty + 1, BT>(); else named_arrive<kBarEmpty, BT>();
       }
     }
   }
@@ -1009,13 +1181,14 @@ __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArg
 // Kernel B for 32 < Nt <= 64 with 512 bins per residue pair (the split 2048 x 512 at Nf =
 // 2^20 and 4096 x 512 at 2^21, instead of 4096 x 256 / 8192 x 256): F of 64 steps for 512
 // bins (256 KB) does not fit one CTA, so a cluster of two CTAs shares the residue pair.  CTA
-// rank s keeps F of side s (residue k1 or P - k1: 256 bins, 128 KB) and evaluates Horner's
-// rule for them.  Each rate pair of a block has an owner (pairs 0 and 1: rank 0; 2 and 3:
-// rank 1); every CTA writes its sums, at the direct and the mirror positions, into the
-// owner's rate-block buffer through distributed shared memory.  One cluster barrier per
-// block makes them visible, then each CTA runs the inverse DFT_Q of its own two rate pairs
-// (4 sequences) and writes W.  The two rate-block buffers alternate, so a CTA may write into
-// its peer's buffer for block i + 1 while the peer still transforms block i.
+// rank s keeps F of side s (residue k1 or P - k1: 256 bins, 128 KB) and evaluates the sums for
+// them.  Of a super pair's two rate pairs the upper one belongs to rank 0 and the lower one to
+// rank 1 (of a rate subset, one block to each); every CTA writes its sums, at the direct and
+// the mirror positions, into the owner's rate-block buffer through distributed shared memory.
+// One cluster barrier per two blocks makes them visible, then each CTA runs the inverse DFT_Q
+// of its own four rate pairs (8 sequences) and writes W.  The two rate-block buffers alternate,
+// so a CTA may write into its peer's buffer for the next blocks while the peer still
+// transforms the current ones.
 // ------------------------------------------------------------------------------------
 // Forward DFT_Q for a two-CTA cluster (zdtf_czt_cl_kernel): CTA `rank` transforms only the A
 // rows of its own side (PC = 8 t pairs per chunk, 8 sequences in buf) and takes the mirror
@@ -1088,8 +1261,7 @@ __device__ __forceinline__ void czt_forward_cluster(const CztArgs& a, int c, con
 struct CztClShape {
   static constexpr int Q = 512, NT = 64, T = 512;
   static constexpr int QH = Q / 2;                    // bins of one side (one CTA)
-  static constexpr int RG = 2 * T / QH;               // rate groups: 4 (128 bin pairs)
-  static constexpr int RT = kRatesPerBlock / RG;      // 2 rates (one rate pair) per thread
+  static constexpr int RG = 2 * T / QH;               // super pairs at a time: 4 (128 bin pairs)
   static constexpr int SS = b_stride<Q>();
   static constexpr int TWT = 2 * kRatesPerBlock * SS;  // after two 8-sequence buffers
   static constexpr int TWR = TWT + tw_size(Q);
@@ -1097,11 +1269,12 @@ struct CztClShape {
   static constexpr size_t SMEM = sizeof(float2) * (GS_OFF + NT * QH + NT);
 };
 
+template <bool SUBSET>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CztClShape::T, 1)
 zdtf_czt_cl_kernel(CztArgs a) {
   using SH = CztClShape;
-  constexpr int Q = SH::Q, NT = SH::NT, T = SH::T, QH = SH::QH, RT = SH::RT, SS = SH::SS;
-  static_assert(RT == 2, "one rate pair per thread");
+  constexpr int Q = SH::Q, NT = SH::NT, T = SH::T, QH = SH::QH, SS = SH::SS;
+  static_assert(SH::RG == 4, "two blocks of two super pairs at a time");
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ float2 sm[];
   float2* const buf = sm;  // forward pass: 8 sequences; then two buffers of 8 (two rate blocks)
@@ -1121,136 +1294,74 @@ zdtf_czt_cl_kernel(CztArgs a) {
     twr[i] = cscale(cconj(tw_fwd(a.tab, (long long)k1s[sd] * na)), invN);
   }
   czt_forward_cluster<Q, NT, T>(a, c, k1s, buf, twt, gs, gnyq, rank, cluster);
+  auto bin0 = [&](int bp) { return (unsigned long long)k1s[rank] + (unsigned long long)P * (2 * bp); };
+  fold_smem<T>(a, reinterpret_cast<float4*>(gs), QH / 2, bin0);
 
-  // thread -> (bin pair bp of this side, rate pair rg of every block)
+  // thread -> (bin pair bp of this side, super pair rg of every two blocks)
   const int bp = tid % (QH / 2), rg = tid / (QH / 2);
   const int side = rank, k20 = 2 * bp;
   int ms[2], mk2[2];
   mirror_of(c, side, k20, Q, &ms[0], &mk2[0]);
   mirror_of(c, side, k20 + 1, Q, &ms[1], &mk2[1]);
   const bool dc = (c == 0 && side == 0 && k20 == 0);  // lane 0 is the DC bin
-  const unsigned long long mask = a.ph.mask;
-  unsigned long long alpha[2], beta[2];
-  float2 pwx, pwy;  // exact w(k_lane, dr) (lanes = the two bins)
-  float2 win;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const unsigned long long k = (unsigned long long)k1s[side] + (unsigned long long)P * (k20 + h);
-    alpha[h] = (k * a.ph.R0) & mask;
-    beta[h] = (k * a.ph.Rd) & mask;
-    const float2 p = cis_phase(beta[h] & mask, a.ph);
-    if (h == 0) { pwx.x = p.x; pwy.x = p.y; } else { pwx.y = p.x; pwy.y = p.y; }
-    const float wv = window_value(a, (long long)k);
-    if (h == 0) win.x = wv; else win.y = wv;
-  }
-  const unsigned long long kny = (unsigned long long)(a.N / 2);
-  const unsigned long long alpha_n = (kny * a.ph.R0) & mask, beta_n = (kny * a.ph.Rd) & mask;
+  const float2 win = make_float2(window_value(a, (long long)bin0(bp)), window_value(a, (long long)bin0(bp) + P));
   const int Nt = a.Nt;
-  const float4* gs4 = reinterpret_cast<const float4*>(gs);
-  const int owner = rg >> 1, ul = rg & 1;  // this thread's rate pair: owner CTA, pair there
+  FoldPhases fp;
+  fp.setup(bin0(bp), bin0(bp) + (unsigned long long)P, a.ph.Rh, Nt >> 1);
+  const float4* const g = reinterpret_cast<const float4*>(gs) + bp;
+  const float2 zero = make_float2(0.f, 0.f);
   const int k1a = k1s[0], k1b = k1s[1];
 
-  const int q_begin = blockIdx.y * a.pairs_per_group;
-  const int q_end = min(a.npairs, q_begin + a.pairs_per_group);
-  const int nblk = q_end > q_begin ? (q_end - q_begin + kRatesPerBlock / 2 - 1) / (kRatesPerBlock / 2) : 0;
-  // two rate blocks per cluster barrier: 8 sequences per buffer ([block 0: 4][block 1: 4])
-  const int nsb = (nblk + 1) / 2;
-  for (int isb = 0; isb < nsb; ++isb) {
-    float2* const hb_local = buf + (isb & 1) * kRatesPerBlock * SS;  // 8 sequences
-    float2* const hb_owner = owner == rank ? hb_local : cluster.map_shared_rank(hb_local, owner);
+  const int blk0 = blockIdx.y * a.blocks_per_group;
+  const int blk_end = min(a.nblk, blk0 + a.blocks_per_group);
+  for (int b2 = blk0; b2 < blk_end; b2 += 2) {
+    float2* const hb_local = buf + (((b2 - blk0) >> 1) & 1) * kRatesPerBlock * SS;  // 8 sequences
+    float2* const hb_peer = cluster.map_shared_rank(hb_local, rank ^ 1);
+    float2* const hb0 = rank == 0 ? hb_local : hb_peer;
+    float2* const hb1 = rank == 1 ? hb_local : hb_peer;
+    const int blk = b2 + (rg >> 1);
+    if (SUBSET) {
+      if (blk < blk_end) {
+        const int j = __ldg(a.blk_base + blk) + 4 * (rg & 1);
+        float2* const hb = (rg >> 1) ? hb1 : hb0;
 #pragma unroll 1
-    for (int bb = 0; bb < 2; ++bb) {
-      const int ib = 2 * isb + bb;
-      const bool live = ib < nblk;  // an odd last block leaves the second half unused
-      const int q0 = q_begin + ib * (kRatesPerBlock / 2);
-      float2* const hb = hb_owner + bb * 4 * SS;
-      const int j0 = 2 * q0 + rg * RT;  // this thread's first rate of the block
-      const long long jb = !live ? 0 : a.blk_base ? (long long)__ldg(a.blk_base + (q0 >> 2)) : (long long)(2 * q0);
-      float2 Sx[2], Sy[2];
-      if (live && j0 < a.Nr) {  // uniform over the warp (rg is)
-        float2 W0x, W0y;
-        {
-          const unsigned long long jj = (unsigned long long)(jb + rg * RT);
-          const float2 w0 = cis_phase((alpha[0] + jj * beta[0]) & mask, a.ph);
-          const float2 w1 = cis_phase((alpha[1] + jj * beta[1]) & mask, a.ph);
-          W0x = make_float2(w0.x, w1.x);
-          W0y = make_float2(w0.y, w1.y);
-        }
-        const float2 NW0y = pk_neg(W0y);
-        float2 Wx[2], Wy[2], NWy[2];
-        Wx[0] = W0x;
-        Wy[0] = W0y;
-        Wx[1] = pk_fma(W0x, pwx, pk_mul(NW0y, pwy));
-        Wy[1] = pk_fma(W0x, pwy, pk_mul(W0y, pwx));
-        NWy[0] = NW0y;
-        NWy[1] = pk_neg(Wy[1]);
-        const float4 gl = gs4[(Nt - 1) * (QH / 2) + bp];
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          Sx[r] = make_float2(gl.x, gl.y);
-          Sy[r] = make_float2(gl.z, gl.w);
-        }
-#pragma unroll 4
-        for (int t = Nt - 2; t >= 0; --t) {
-          const float4 gt = gs4[t * (QH / 2) + bp];
-          const float2 gx = make_float2(gt.x, gt.y), gy = make_float2(gt.z, gt.w);
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const float2 tx = pk_fma(Sx[r], Wx[r], pk_fma(Sy[r], NWy[r], gx));
-            const float2 ty = pk_fma(Sx[r], Wy[r], pk_fma(Sy[r], Wx[r], gy));
-            Sx[r] = tx;
-            Sy[r] = ty;
-          }
-        }
-      } else {
-        Sx[0] = Sx[1] = Sy[0] = Sy[1] = make_float2(0.f, 0.f);
-      }
-      const bool ok_a = live && j0 < a.Nr, ok_b = live && j0 + 1 < a.Nr;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float wh = h ? win.y : win.x;
-        const float2 sa = ok_a ? cscale(make_float2(h ? Sx[0].y : Sx[0].x, h ? Sy[0].y : Sy[0].x), wh)
-                               : make_float2(0.f, 0.f);
-        const float2 sb = ok_b ? cscale(make_float2(h ? Sx[1].y : Sx[1].x, h ? Sy[1].y : Sy[1].x), wh)
-                               : make_float2(0.f, 0.f);
-        if (dc && h == 0) {
-          hb[(2 * ul) * SS + pidx(0)] = make_float2(sa.x, sb.x);
-        } else {
-          hb[(2 * ul + side) * SS + pidx(k20 + h)] = make_float2(sa.x - sb.y, sa.y + sb.x);
-          hb[(2 * ul + ms[h]) * SS + pidx(mk2[h])] = make_float2(sa.x + sb.y, sb.x - sa.y);
+        for (int e = 0; e < 2; ++e) {
+          float2 ax, ay, bx, by;
+          fold_rate_smem(fp, g, QH / 2, Nt, j + 2 * e, a.half, ax, ay);
+          fold_rate_smem(fp, g, QH / 2, Nt, j + 2 * e + 1, a.half, bx, by);
+          put_rate_pair<SS>(hb + 2 * (2 * (rg & 1) + e) * SS, side, k20, ms, mk2, dc, win, ax, ay, bx, by);
         }
       }
-      if (c == 0 && rank == 0 && tid == 0) {  // the real-only Nyquist bin of every rate of the block
-        const float wn = window_value(a, (long long)kny);
-        for (int u = 0; u < kRatesPerBlock / 2; ++u) {
-          float v[2];
-          for (int hh = 0; hh < 2; ++hh) {
-            const int j = 2 * q0 + 2 * u + hh;
-            float2 sv = make_float2(0.f, 0.f);
-            if (live) {
-              const float2 wv = cis_phase((alpha_n + (unsigned long long)(jb + 2 * u + hh) * beta_n) & mask, a.ph);
-              sv = gnyq[Nt - 1];
-              for (int t = Nt - 2; t >= 0; --t)
-                sv = make_float2(fmaf(sv.x, wv.x, fmaf(-sv.y, wv.y, gnyq[t].x)),
-                                 fmaf(sv.x, wv.y, fmaf(sv.y, wv.x, gnyq[t].y)));
-            }
-            v[hh] = (live && j < a.Nr) ? sv.x * wn : 0.f;
-          }
-          float2* const hbo = ((u >> 1) == rank ? hb_local : cluster.map_shared_rank(hb_local, u >> 1)) + bb * 4 * SS;
-          hbo[(2 * (u & 1)) * SS + pidx(Q / 2)] = make_float2(v[0], v[1]);
-        }
+    } else {
+      const int sp = 2 * blk + (rg & 1);
+      if (blk < blk_end && sp < a.half) {  // uniform over the warp (rg is)
+        float2 px[2], py[2], mx[2], my[2];
+        fp.start(blk);
+        fold_pairs_smem<2>(fp, g, QH / 2, Nt, 2 * (rg & 1), px, py, mx, my);
+        const int ja = 2 * (a.half + sp);  // rates past the grid's last: zero
+        if (ja >= a.Nr) px[0] = py[0] = zero;
+        if (ja + 1 >= a.Nr) px[1] = py[1] = zero;
+        put_rate_pair<SS>(hb0 + 2 * rg * SS, side, k20, ms, mk2, dc, win, px[0], py[0], px[1], py[1]);
+        put_rate_pair<SS>(hb1 + 2 * rg * SS, side, k20, ms, mk2, dc, win, mx[1], my[1], mx[0], my[0]);
       }
     }
+    if (c == 0 && rank == 0 && tid < 2 * kRatesPerBlock) {
+      const int bb = tid / kRatesPerBlock;
+      if (b2 + bb < blk_end)
+        nyquist_block<SUBSET>(a, gnyq, b2 + bb, tid % kRatesPerBlock, [&](int u, int hh, float v) {
+          float2* const hb = (SUBSET ? bb : u & 1) ? hb1 : hb0;
+          const int slot = SUBSET ? u : 2 * bb + (u >> 1);
+          reinterpret_cast<float*>(hb + (2 * slot) * SS + pidx(Q / 2))[hh] = v;
+        });
+    }
     cluster.sync();  // both blocks' sums, local and remote, are in the owners' buffers
-    // the inverse DFT_Q of this CTA's rate pairs 2*rank, 2*rank + 1 of both blocks (8
-    // sequences); the last pass writes W
-    smem_fft_emit<Q, 2 * kRatesPerBlock / 2, SS, T, +1>(hb_local, twt, [&](int ls, int na, float2 v) {
-      const int bb = ls >> 2, lq = ls & 3;
-      const int q0 = q_begin + (2 * isb + bb) * (kRatesPerBlock / 2);
-      const int p = 2 * rank + (lq >> 1), sd = lq & 1;
-      const unsigned off = (unsigned)((p * P + (sd ? k1b : k1a)) * Q + na);
-      if (q0 + p < q_end && FDR_DBG_OK((long long)q0 * P * Q + off < (long long)a.npairs * P * Q))
-        a.W[(long long)q0 * P * Q + off] = cmul(v, twr[sd * Q + na]);
+    // the inverse DFT_Q of this CTA's four rate pairs; the last pass writes W
+    smem_fft_emit<Q, kRatesPerBlock, SS, T, +1>(hb_local, twt, [&](int ls, int na, float2 v) {
+      const int lp = ls >> 1, sd = ls & 1;
+      const int b = SUBSET ? b2 + rank : b2 + (lp >> 1);
+      const int p = b < blk_end ? block_pair<SUBSET>(a, b, SUBSET ? lp : 2 * (lp & 1) + rank) : -1;
+      const long long at = ((long long)p * P + (sd ? k1b : k1a)) * Q + na;
+      if (p >= 0 && FDR_DBG_OK(at < (long long)a.npairs * P * Q)) a.W[at] = cmul(v, twr[sd * Q + na]);
     });
   }
 }
@@ -2466,15 +2577,15 @@ struct AcShape {
 };
 
 template <int Q>
-struct CztShape {  // buf | twt | twr | gnyq | buf2 (the second rate-block buffer) | phase residues
+struct CztShape {  // buf | twt | twr | gnyq | buf2 (the second rate-block buffer) | phase factors, steps
   static constexpr size_t SMEM =
-      sizeof(float2) * (2 * kRatesPerBlock * b_stride<Q>() + tw_size(Q) + 2 * Q + kFusedMaxNt) +
-      sizeof(unsigned long long) * 4 * (Q / 2);
+      sizeof(float2) * (2 * kRatesPerBlock * b_stride<Q>() + tw_size(Q) + 2 * Q + kFusedMaxNt + 12 * (Q / 2)) +
+      sizeof(unsigned long long) * 2 * (Q / 2);
 };
 
 // log2 of the four-step factor Q for Nf = 2^L and Nt time steps.  With F in registers
 // (Nt <= 16): 512 bins per CTA up to Nf = 2^20 (256 threads, two CTAs per SM, so one CTA's
-// barriers overlap the other's Horner sums; P <= 2048 keeps the TMA output passes), 1024
+// barriers overlap the other's sums; P <= 2048 keeps the TMA output passes), 1024
 // above; with F in shared memory 512 (Nt <= 32) and 256 (Nt <= 64).  Mixed-precision
 // workspaces split the same way (their tensor-core output passes cover P = 1024 and 2048).
 static int fused_qlog(int L, int64_t Nt) {
@@ -2509,6 +2620,8 @@ static void float_parts(float x, long long* m, int* e) {
   *e = ee;
 }
 
+// Exact phase steps of Nf = 2^L channels; false for rates whose phases need more than 62 bits (a
+// half rate step then fits the 64 of PhaseInt).
 static bool make_phase(float r0, float dr, int L, PhaseInt* ph) {
   if (!isfinite(r0) || !isfinite(dr)) return false;
   long long m0, md;
@@ -2518,20 +2631,14 @@ static bool make_phase(float r0, float dr, int L, PhaseInt* ph) {
   int s = 0;
   if (m0 != 0 && -e0 > s) s = -e0;
   if (md != 0 && -ed > s) s = -ed;
-  const int bits = L + s;
-  if (bits > 62) return false;
-  const unsigned long long mask = (1ULL << bits) - 1ULL;
-  auto part = [&](long long m, int e) -> unsigned long long {
-    if (m == 0) return 0ULL;
-    const int sh = e + s;  // >= 0
-    if (sh >= bits) return 0ULL;
-    return (((unsigned long long)m) << sh) & mask;  // two's complement wrap is exact mod 2^bits
+  if (L + s > 62) return false;
+  // m 2^e turns in units of 2^-64 turn, modulo one turn (two's complement wrap is exact)
+  auto part = [](long long m, int e) -> unsigned long long {
+    const int sh = 64 + e;
+    return m == 0 || sh >= 64 ? 0ULL : ((unsigned long long)m) << sh;
   };
-  ph->R0 = part(m0, e0);
-  ph->Rd = part(md, ed);
-  ph->mask = mask;
-  ph->bits = bits;
-  ph->scale = ldexpf(1.0f, 1 - bits);
+  ph->R0 = part(m0, e0 - L);
+  ph->Rh = part(md, ed - 1 - L);
   return true;
 }
 
@@ -2543,6 +2650,7 @@ struct FusedPlan {
   float2* tables = nullptr;  // twP | twQ | tw_lo | tw_hi | rootsP
   FusedTables tab;
   int64_t NP = 0, npairs = 0;
+  int64_t half = 0;  // super pairs of the whole grid (kept by rate subsets)
 };
 
 static std::vector<float2> roots_table(long long n, long long N, long long count) {
@@ -2609,35 +2717,33 @@ static int set_smem_attrs() {
   // P = 2048 input: Nf = 2^20 or 2^21, table split B = 10 or 11
   FDR_CUDA(cudaFuncSetAttribute(zdtf_input64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)In64Shape::smem(11, 1LL << 21)));
+#define SET_ATTR(kernel, bytes) \
+  FDR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes)));
 #define SET_B(Q)                                                                               \
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_czt_kernel<Q, kFusedMaxNt, false>,                        \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CztShape<Q>::SMEM)); \
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_czt_kernel<Q, kFusedMaxNt, true>,                         \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CztShape<Q>::SMEM)); \
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_a2f_kernel<Q, kFusedMaxNt>,                               \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CztShape<Q>::SMEM));
+  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, false, false>), CztShape<Q>::SMEM)                 \
+  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, true, false>), CztShape<Q>::SMEM)                  \
+  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, true, true>), CztShape<Q>::SMEM)                   \
+  SET_ATTR((zdtf_a2f_kernel<Q, kFusedMaxNt>), CztShape<Q>::SMEM)
   FDR_FOR_Q(SET_B)
 #undef SET_B
 #define SET_BS(Q, NT)                                                                          \
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_czt_smem_kernel<Q, NT>,                                   \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                (int)CztSmemShape<Q>::template smem<NT>()));                   \
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_a2f_smem_kernel<Q, NT>,                                   \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                (int)CztSmemShape<Q>::template smem<NT>()));
-  SET_BS(64, 32) SET_BS(128, 32) SET_BS(256, 32) SET_BS(512, 32)
-  SET_BS(64, 64) SET_BS(128, 64) SET_BS(256, 64)
+  SET_ATTR((zdtf_czt_smem_kernel<Q, NT, false>), (CztSmemShape<Q>::template smem<NT>()))       \
+  SET_ATTR((zdtf_czt_smem_kernel<Q, NT, true>), (CztSmemShape<Q>::template smem<NT>()))
+  SET_BS(64, 32) SET_BS(128, 32) SET_BS(64, 64) SET_BS(128, 64)
 #undef SET_BS
+#define SET_AF(Q, NT) SET_ATTR((zdtf_a2f_smem_kernel<Q, NT>), (CztSmemShape<Q>::template smem<NT>()))
+  SET_AF(64, 32) SET_AF(128, 32) SET_AF(256, 32) SET_AF(512, 32)
+  SET_AF(64, 64) SET_AF(128, 64) SET_AF(256, 64)
+#undef SET_AF
 #define SET_WS(Q, NT)                                                                          \
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_czt_ws_kernel<Q, NT>,                                     \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                (int)CztWsShape<Q>::template smem<NT>()));
+  SET_ATTR((zdtf_czt_ws_kernel<Q, NT, false>), (CztWsShape<Q>::template smem<NT>()))           \
+  SET_ATTR((zdtf_czt_ws_kernel<Q, NT, true>), (CztWsShape<Q>::template smem<NT>()))
   SET_WS(512, 32) SET_WS(256, 32) SET_WS(256, 64)
 #undef SET_WS
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_czt_cl_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)CztClShape::SMEM));
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_a2f_half_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)CztClShape::SMEM));
+  SET_ATTR(zdtf_czt_cl_kernel<false>, CztClShape::SMEM)
+  SET_ATTR(zdtf_czt_cl_kernel<true>, CztClShape::SMEM)
+  SET_ATTR(zdtf_a2f_half_kernel, CztClShape::SMEM)
+#undef SET_ATTR
   if (dev < 64) done[dev] = true;
   return FDR_OK;
 }
@@ -2659,6 +2765,7 @@ int fused_plan_create(FusedPlan** out, int64_t N, int64_t Nt, int64_t Nr) {
   st->B = (st->L + 1) / 2;
   st->NP = cdiv(Nt, 2);
   st->npairs = cdiv(Nr, 2);
+  st->half = cdiv(st->npairs, 2);
   const long long P = st->P, Q = st->Q;
   const long long nlo = 1LL << st->B, nhi = N >> st->B;
   const long long ntwP = tw_size((int)P), ntwQ = tw_size((int)Q);
@@ -2729,6 +2836,7 @@ static CztArgs czt_args(const FusedPlan* st, const float2* A, float2* W) {
   a.NP = (int)st->NP;
   a.Nr = (int)st->Nr;
   a.npairs = (int)st->npairs;
+  a.half = (int)st->half;
   a.tab = st->tab;
   return a;
 }
@@ -2799,14 +2907,16 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
   a.window = window;
   a.wk = wk;
   a.blk_base = blk_base;
+  a.center = ph.R0 + (unsigned long long)(4 * st->half - 1) * ph.Rh;
   const int Q = st->Q, ctas = st->P / 2;
+  a.nblk = (int)(blk_base ? st->npairs / 4 : cdiv(st->half, 2));
+  if (st->Nt <= kFusedMaxNt) a.pshift = (int)(kFusedMaxNt / 2 - st->Nt / 2) / 2;
   if (groups <= 0) groups = fused_default_groups(st);
-  int ppg = (int)cdiv(st->npairs, groups);
-  ppg = (int)cdiv(ppg, kRatesPerBlock / 2) * (kRatesPerBlock / 2);
-  groups = (int)cdiv(st->npairs, ppg);
-  a.pairs_per_group = ppg;
+  a.blocks_per_group = (int)cdiv(a.nblk, groups);
+  groups = (int)cdiv(a.nblk, a.blocks_per_group);
   if (st->Nt > 32 && Q == CztClShape::Q) {  // F of 64 steps for 512 bins: two-CTA cluster
-    zdtf_czt_cl_kernel<<<dim3(2 * ctas, groups), CztClShape::T, CztClShape::SMEM, s>>>(a);
+    if (blk_base) zdtf_czt_cl_kernel<true><<<dim3(2 * ctas, groups), CztClShape::T, CztClShape::SMEM, s>>>(a);
+    else zdtf_czt_cl_kernel<false><<<dim3(2 * ctas, groups), CztClShape::T, CztClShape::SMEM, s>>>(a);
     FDR_LAUNCH_CHECK("zdtf_czt_cl_kernel");
     return FDR_OK;
   }
@@ -2816,8 +2926,8 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
     const int NT = st->Nt <= 32 ? 32 : 64;
 #define LAUNCH_WS(QQ, NN)                                                                      \
     if (Q == QQ && NT == NN) {                                                                 \
-      zdtf_czt_ws_kernel<QQ, NN><<<dim3(ctas, groups), CztWsShape<QQ>::T,                      \
-                                   CztWsShape<QQ>::template smem<NN>(), s>>>(a);               \
+      auto kernel = blk_base ? zdtf_czt_ws_kernel<QQ, NN, true> : zdtf_czt_ws_kernel<QQ, NN, false>; \
+      kernel<<<dim3(ctas, groups), CztWsShape<QQ>::T, CztWsShape<QQ>::template smem<NN>(), s>>>(a); \
       FDR_LAUNCH_CHECK("zdtf_czt_ws_kernel");                                                  \
       return FDR_OK;                                                                           \
     }
@@ -2828,21 +2938,20 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
     const int NT = st->Nt <= 32 ? 32 : 64;
 #define LAUNCH_BS(QQ, NN)                                                                      \
     if (Q == QQ && NT == NN) {                                                                 \
-      zdtf_czt_smem_kernel<QQ, NN><<<dim3(ctas, groups), CztSmemShape<QQ>::T,                  \
-                                     CztSmemShape<QQ>::template smem<NN>(), s>>>(a);           \
+      auto kernel = blk_base ? zdtf_czt_smem_kernel<QQ, NN, true> : zdtf_czt_smem_kernel<QQ, NN, false>; \
+      kernel<<<dim3(ctas, groups), CztSmemShape<QQ>::T, CztSmemShape<QQ>::template smem<NN>(), s>>>(a); \
       FDR_LAUNCH_CHECK("zdtf_czt_smem_kernel");                                                \
       return FDR_OK;                                                                           \
     }
-    LAUNCH_BS(64, 32) LAUNCH_BS(128, 32) LAUNCH_BS(256, 32) LAUNCH_BS(512, 32)
-    LAUNCH_BS(64, 64) LAUNCH_BS(128, 64) LAUNCH_BS(256, 64)
+    LAUNCH_BS(64, 32) LAUNCH_BS(128, 32) LAUNCH_BS(64, 64) LAUNCH_BS(128, 64)
 #undef LAUNCH_BS
   } else {
 #define LAUNCH_B(QQ)                                                                           \
     if (Q == QQ) {                                                                             \
-      if (window == FDR_WINDOW_RECT)                                                           \
-        zdtf_czt_kernel<QQ, kFusedMaxNt, false><<<dim3(ctas, groups), QQ / 2, CztShape<QQ>::SMEM, s>>>(a); \
-      else                                                                                     \
-        zdtf_czt_kernel<QQ, kFusedMaxNt, true><<<dim3(ctas, groups), QQ / 2, CztShape<QQ>::SMEM, s>>>(a); \
+      auto kernel = blk_base ? zdtf_czt_kernel<QQ, kFusedMaxNt, true, true>                    \
+                    : window == FDR_WINDOW_RECT ? zdtf_czt_kernel<QQ, kFusedMaxNt, false, false> \
+                                                : zdtf_czt_kernel<QQ, kFusedMaxNt, true, false>; \
+      kernel<<<dim3(ctas, groups), QQ / 2, CztShape<QQ>::SMEM, s>>>(a);                        \
       FDR_LAUNCH_CHECK("zdtf_czt_kernel");                                                     \
       return FDR_OK;                                                                           \
     }
