@@ -2882,11 +2882,17 @@ bool fused_phase_ok(const FusedPlan* st, float r0, float dr) {
   return make_phase(r0, dr, st->L, &ph);
 }
 
-// Rate groups (grid.y of the czt kernel) by default: about four waves of one CTA per SM.
+// Rate groups (grid.y of the czt kernel) by default: as many as keep the grid within one wave of
+// two CTAs an SM (Nt <= 16; three at Q = 128 and four at Q = 64, whose CTAs are smaller) or one
+// (F in shared memory).  Every group repeats the forward transform and the phase set-up, so a
+// split that the SMs do not need costs more than it spreads: measured czt times in us for 1, 2, 3
+// and all groups of one block, Nf = 2^16 Nt = 16 33 rates 22.6, 20.5, 24.7, 30.4; 2^18 Nt = 16 129
+// rates 101, 113, 123, 152; 2^16 Nt = 64 65 rates 47, 61, 78, 111; 2^14 Nt = 16 33 rates 21.5,
+// 18.4, 16.4, 14.4; 2^15 22.6, 18.5, 17.5, 21.9.
 int fused_default_groups(const FusedPlan* st) {
   const int ctas = st->P / 2;
-  return std::max(1, std::min<int>((int)cdiv(4 * sm_count(), ctas),
-                                   (int)cdiv(st->npairs, kRatesPerBlock / 2)));
+  const int per_sm = st->Nt > kFusedMaxNt ? 1 : st->Q >= 256 ? 2 : st->Q == 128 ? 3 : 4;
+  return std::max(1, std::min(per_sm * sm_count() / ctas, (int)cdiv(st->half, 2)));
 }
 
 int fused_czt(const FusedPlan* st, const float2* A, float2* W, float r0, float dr, int window,
@@ -2912,6 +2918,7 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
   a.nblk = (int)(blk_base ? st->npairs / 4 : cdiv(st->half, 2));
   if (st->Nt <= kFusedMaxNt) a.pshift = (int)(kFusedMaxNt / 2 - st->Nt / 2) / 2;
   if (groups <= 0) groups = fused_default_groups(st);
+  groups = std::min(groups, a.nblk);
   a.blocks_per_group = (int)cdiv(a.nblk, groups);
   groups = (int)cdiv(a.nblk, a.blocks_per_group);
   if (st->Nt > 32 && Q == CztClShape::Q) {  // F of 64 steps for 512 bins: two-CTA cluster
