@@ -13,6 +13,7 @@
 // fixed order (per-block partial sums, then an ordered sum), so results are deterministic
 // and a resumed training run matches an uninterrupted one bit for bit.
 #include <cuda_fp16.h>
+#include <limits.h>
 #include <math.h>
 #include <string.h>
 
@@ -40,13 +41,15 @@ struct fdr_propose_net {
   float* grad = nullptr;
   int64_t step = 0;
   uint64_t seed = 0;
-  // activations for backward (allocated for max batch)
+  // for backward (allocated for max batch)
   int maxb = 0;
-  float* act[4] = {nullptr, nullptr, nullptr, nullptr};  // outputs of layers 1..4
+  float* act[3] = {nullptr, nullptr, nullptr};  // outputs of layers 1..3
+  float* tile_max = nullptr;                    // per (sample, tile, window): largest logit,
+  int* tile_arg = nullptr;                      //   its bin
   int* argmax = nullptr;
-  float* dact[2] = {nullptr, nullptr};                    // ping-pong gradient buffers
-  float* partial = nullptr;                               // per-block weight-grad partials
-  int64_t partial_elems = 0;
+  float* dlogit = nullptr;                      // gradient of the loss wrt the logits
+  float* gact = nullptr;                        // per sample: SparseGrad
+  float* partial = nullptr;                     // per sample: gradient of every parameter
   float* loss = nullptr;                                  // device scalar
 };
 
@@ -166,89 +169,175 @@ static int launch_input(const float* spec, int64_t Nf, int64_t Nt, int factor, i
 }
 
 // --------------------------------------------------------------------------------------
-// Convolution forward: y[b][co][x] = b[co] + sum_{ci,k} w[co][ci][k] * in[b][ci][x+k-pad]
-// grid (X/kConvTile, B), block kConvTile threads (one bin each, all output channels).
+// Convolution forward: y[b][co][x] = b[co] + sum_{ci,k} w[co][ci][k] * in[b][ci][x+k-pad], ReLU.
+// grid (X/kConvTile, B), kConvTile / 2 threads: a thread takes two bins and all 32 output
+// channels, two channels per packed multiply-add, so that a 16-byte broadcast load of weights
+// feeds four of them (one scalar weight load per multiply-add bound the scalar form: 190 us a
+// layer at 64 x 4096 bins, 33 channels).  Every output sums over (ci, k) in order from its bias.
+// HEAD: the last hidden layer also forms the 16 window logits of its bins (the 1x1 layer, same
+// order of sums) and their maximum over the tile's bins, the first bin on ties.
 // --------------------------------------------------------------------------------------
-template <int COUT, int KS>
-__global__ void __launch_bounds__(kConvTile)
+constexpr int kWidth = 32, kWin = 16, kTaps = 5, kPad = kTaps / 2;
+constexpr int kConvThreads = kConvTile / 2;
+
+template <bool HEAD>
+__global__ void __launch_bounds__(kConvThreads, 4)
 conv_fwd_kernel(const float* __restrict__ in, int cin, int X, const __half* __restrict__ w,
-                const float* __restrict__ bias, int relu, float* __restrict__ out) {
-  extern __shared__ float sm[];
-  const int pad = KS / 2;
-  const int TW = kConvTile + KS - 1;
-  float* xs = sm;                 // cin * TW
-  float* wsm = sm + cin * TW;     // COUT * cin * KS
-  const int b = blockIdx.y, x0 = blockIdx.x * kConvTile;
-  const float* inb = in + (long long)b * cin * X;
-  for (int i = threadIdx.x; i < cin * TW; i += blockDim.x) {
-    const int ci = i / TW, xx = x0 - pad + (i - ci * TW);
+                const float* __restrict__ bias, float* __restrict__ out, const __half* __restrict__ w3,
+                const float* __restrict__ bias3, float* __restrict__ tile_max, int* __restrict__ tile_arg) {
+  extern __shared__ float4 sm4[];
+  constexpr int TW = kConvTile + kTaps - 1;
+  float* const wsm = reinterpret_cast<float*>(sm4);  // [ci][k][co]
+  float* const w3sm = wsm + cin * kTaps * kWidth;     // HEAD: [ci][window]
+  float* const xs = w3sm + (HEAD ? kWidth * kWin : 0);  // [ci][TW]
+  const int b = blockIdx.y, x0 = blockIdx.x * kConvTile, tid = threadIdx.x;
+  const float* const inb = in + (long long)b * cin * X;
+  for (int i = tid; i < cin * TW; i += kConvThreads) {
+    const int ci = i / TW, xx = x0 - kPad + (i - ci * TW);
     xs[i] = (xx >= 0 && xx < X) ? inb[(long long)ci * X + xx] : 0.f;
   }
-  for (int i = threadIdx.x; i < COUT * cin * KS; i += blockDim.x) wsm[i] = __half2float(w[i]);
+  for (int i = tid; i < cin * kTaps * kWidth; i += kConvThreads) {
+    const int co = i / (cin * kTaps), r = i - co * cin * kTaps;
+    wsm[r * kWidth + co] = __half2float(w[i]);
+  }
+  if (HEAD)
+    for (int i = tid; i < kWidth * kWin; i += kConvThreads)
+      w3sm[(i % kWidth) * kWin + i / kWidth] = __half2float(w3[i]);
   __syncthreads();
-  const int x = x0 + threadIdx.x;
-  if (x >= X) return;
-  float acc[COUT];
+  float2 acc[2][kWidth / 2];
 #pragma unroll
-  for (int co = 0; co < COUT; ++co) acc[co] = bias[co];
+  for (int p = 0; p < kWidth / 2; ++p) acc[0][p] = acc[1][p] = make_float2(bias[2 * p], bias[2 * p + 1]);
   for (int ci = 0; ci < cin; ++ci) {
+    const float* const xr = xs + ci * TW + tid;
 #pragma unroll
-    for (int k = 0; k < KS; ++k) {
-      const float v = xs[ci * TW + threadIdx.x + k];
+    for (int k = 0; k < kTaps; ++k) {
+      const float v0 = xr[k], v1 = xr[kConvThreads + k];
+      const float2 a0 = make_float2(v0, v0), a1 = make_float2(v1, v1);
+      const float4* const wr = sm4 + (ci * kTaps + k) * (kWidth / 4);
 #pragma unroll
-      for (int co = 0; co < COUT; ++co) acc[co] = fmaf(wsm[(co * cin + ci) * KS + k], v, acc[co]);
+      for (int q = 0; q < kWidth / 4; ++q) {
+        const float4 wv = wr[q];
+        acc[0][2 * q] = __ffma2_rn(make_float2(wv.x, wv.y), a0, acc[0][2 * q]);
+        acc[0][2 * q + 1] = __ffma2_rn(make_float2(wv.z, wv.w), a0, acc[0][2 * q + 1]);
+        acc[1][2 * q] = __ffma2_rn(make_float2(wv.x, wv.y), a1, acc[1][2 * q]);
+        acc[1][2 * q + 1] = __ffma2_rn(make_float2(wv.z, wv.w), a1, acc[1][2 * q + 1]);
+      }
     }
   }
-  float* ob = out + (long long)b * COUT * X;
+  float* const ob = out + (long long)b * kWidth * X;
 #pragma unroll
-  for (int co = 0; co < COUT; ++co) ob[(long long)co * X + x] = relu ? fmaxf(acc[co], 0.f) : acc[co];
-}
-
-// logits[b][w] = max_x y[b][w][x] (first maximum), argmax kept for the backward pass.
-__global__ void maxpool_kernel(const float* __restrict__ y, int nw, int X, float* __restrict__ logits,
-                               int* __restrict__ argmax) {
-  const int b = blockIdx.y, w = blockIdx.x;
-  const float* r = y + ((long long)b * nw + w) * X;
-  float best = -INFINITY;
-  int bi = 0;
-  for (int x = threadIdx.x; x < X; x += blockDim.x) {
-    const float v = r[x];
-    if (v > best) { best = v; bi = x; }
+  for (int h = 0; h < 2; ++h) {
+    const int x = x0 + tid + h * kConvThreads;
+#pragma unroll
+    for (int p = 0; p < kWidth / 2; ++p) {
+      acc[h][p] = make_float2(fmaxf(acc[h][p].x, 0.f), fmaxf(acc[h][p].y, 0.f));
+      if (x < X) {
+        ob[(long long)(2 * p) * X + x] = acc[h][p].x;
+        ob[(long long)(2 * p + 1) * X + x] = acc[h][p].y;
+      }
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_down_sync(0xffffffffu, best, o);
-    const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-    if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
+  if (!HEAD) return;
+  __shared__ float rv[kConvThreads / 32][kWin];
+  __shared__ int ri[kConvThreads / 32][kWin];
+  const int lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {  // 8 windows at a time
+    float best[kWin / 2];
+    int at[kWin / 2];
+#pragma unroll
+    for (int j = 0; j < kWin / 2; ++j) {
+      best[j] = -INFINITY;
+      at[j] = 0;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float2 z[kWin / 4];
+#pragma unroll
+      for (int p = 0; p < kWin / 4; ++p)
+        z[p] = make_float2(bias3[8 * half + 2 * p], bias3[8 * half + 2 * p + 1]);
+#pragma unroll
+      for (int ci = 0; ci < kWidth; ++ci) {
+        const float v = ci & 1 ? acc[h][ci / 2].y : acc[h][ci / 2].x;
+        const float2 vv = make_float2(v, v);
+        const float4* const wr = reinterpret_cast<const float4*>(w3sm + ci * kWin + 8 * half);
+        const float4 wa = wr[0], wb = wr[1];
+        z[0] = __ffma2_rn(make_float2(wa.x, wa.y), vv, z[0]);
+        z[1] = __ffma2_rn(make_float2(wa.z, wa.w), vv, z[1]);
+        z[2] = __ffma2_rn(make_float2(wb.x, wb.y), vv, z[2]);
+        z[3] = __ffma2_rn(make_float2(wb.z, wb.w), vv, z[3]);
+      }
+      const int x = x0 + tid + h * kConvThreads;
+#pragma unroll
+      for (int j = 0; j < kWin / 2; ++j) {
+        const float v = j & 1 ? z[j / 2].y : z[j / 2].x;
+        if (x < X && v > best[j]) {
+          best[j] = v;
+          at[j] = x;
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kWin / 2; ++j) {
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_down_sync(0xffffffffu, best[j], o);
+        const int oi = __shfl_down_sync(0xffffffffu, at[j], o);
+        if (ov > best[j] || (ov == best[j] && oi < at[j])) {
+          best[j] = ov;
+          at[j] = oi;
+        }
+      }
+      if (lane == 0) {
+        rv[warp][8 * half + j] = best[j];
+        ri[warp][8 * half + j] = at[j];
+      }
+    }
   }
-  __shared__ float sv[32];
-  __shared__ int si[32];
-  if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = best; si[threadIdx.x >> 5] = bi; }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float bv = sv[0];
-    int bix = si[0];
-    for (int i = 1; i < (int)(blockDim.x + 31) / 32; ++i)
-      if (sv[i] > bv || (sv[i] == bv && si[i] < bix)) { bv = sv[i]; bix = si[i]; }
-    logits[(long long)b * nw + w] = bv;
-    argmax[(long long)b * nw + w] = bix;
+  if (tid < kWin) {
+    float v = rv[0][tid];
+    int i = ri[0][tid];
+    for (int q = 1; q < kConvThreads / 32; ++q)
+      if (rv[q][tid] > v || (rv[q][tid] == v && ri[q][tid] < i)) {
+        v = rv[q][tid];
+        i = ri[q][tid];
+      }
+    const long long o = ((long long)b * gridDim.x + blockIdx.x) * kWin + tid;
+    tile_max[o] = v;
+    tile_arg[o] = i;
   }
 }
 
-// Mean BCE with logits (single block, fixed order) and its gradient scattered to the
-// argmax bins of dy (dy must be zero on entry).
-__global__ void bce_kernel(const float* __restrict__ logits, const float* __restrict__ labels,
-                           const int* __restrict__ argmax, int n, int nw, int X,
-                           float* __restrict__ dy, float* __restrict__ loss) {
+// logits[b][w] = the largest logit over the tiles (first bin on ties), argmax its bin.
+__global__ void maxpool_kernel(const float* __restrict__ tile_max, const int* __restrict__ tile_arg, int tiles, int n,
+                               float* __restrict__ logits, int* __restrict__ argmax) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const long long at = (long long)(i / kWin) * tiles * kWin + i % kWin;
+  float v = tile_max[at];
+  int bi = tile_arg[at];
+  for (int t = 1; t < tiles; ++t) {
+    const float tv = tile_max[at + (long long)t * kWin];
+    const int ti = tile_arg[at + (long long)t * kWin];
+    if (tv > v || (tv == v && ti < bi)) {
+      v = tv;
+      bi = ti;
+    }
+  }
+  logits[i] = v;
+  argmax[i] = bi;
+}
+
+// Mean BCE with logits (single block, fixed order) and its gradient wrt the logits.
+__global__ void bce_kernel(const float* __restrict__ logits, const float* __restrict__ labels, int n,
+                           float* __restrict__ dlogit, float* __restrict__ loss) {
   __shared__ float part[256];
   float s = 0.f;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const float z = logits[i], y = labels[i];
     s += fmaxf(z, 0.f) - z * y + log1pf(expf(-fabsf(z)));
-    if (dy) {
-      const float p = 1.f / (1.f + expf(-z));
-      const int b = i / nw, w = i - b * nw;
-      dy[((long long)b * nw + w) * X + argmax[i]] = (p - y) / (float)n;
-    }
+    const float p = 1.f / (1.f + expf(-z));
+    dlogit[i] = (p - y) / (float)n;
   }
   part[threadIdx.x] = s;
   __syncthreads();
@@ -259,91 +348,213 @@ __global__ void bce_kernel(const float* __restrict__ logits, const float* __rest
   }
 }
 
-// d_in[b][ci][x] = sum_{co,k} w[co][ci][k] * g[b][co][x-k+pad],
-// g = d_out masked by the ReLU of the layer output (when relu_out != NULL).
-__global__ void __launch_bounds__(kConvTile)
-conv_bwd_data_kernel(const float* __restrict__ dout, const float* __restrict__ relu_out, int cout,
-                     int cin, int ks, int X, const __half* __restrict__ w, float* __restrict__ din) {
-  extern __shared__ float sm[];
-  const int pad = ks / 2;
-  const int TW = kConvTile + ks - 1;
-  float* gs = sm;                  // cout * TW
-  float* wsm = sm + cout * TW;     // cout * cin * ks
-  const int b = blockIdx.y, x0 = blockIdx.x * kConvTile;
-  for (int i = threadIdx.x; i < cout * TW; i += blockDim.x) {
-    const int co = i / TW, xx = x0 + pad - (ks - 1) + (i - co * TW);  // covers x - k + pad
-    float g = 0.f;
-    if (xx >= 0 && xx < X) {
-      const long long idx = ((long long)b * cout + co) * X + xx;
-      g = dout[idx];
-      if (relu_out && relu_out[idx] <= 0.f) g = 0.f;
+// --------------------------------------------------------------------------------------
+// Backward.  The maximum over bins passes a window's gradient to one bin, so at most 16 bins of
+// a sample's last hidden layer have one, 5 bins around each of them in the layer below and 9 in
+// the first: 16, 80 and 144 of the (4096) bins.  Everything else is zero and is not touched (the
+// dense form multiplied it out: 3.4 of a training step's 4.1 ms).  The bins of a layer are listed
+// in ascending order, those around the selected ones merged; bins outside [0, X) stay in the list
+// with zero gradient so that five neighbouring bins are neighbours in the list below.
+// --------------------------------------------------------------------------------------
+constexpr int kMaxBins = kWin * 9;       // listed bins of the first layer
+constexpr int kMaxInBins = kWin * 13;    // and of its input
+
+struct SparseGrad {                 // of one sample
+  int n[3];                         // listed bins of layers 1, 2, 3 (index 0, 1, 2)
+  int bins[3][kMaxBins];
+  float g[3][kMaxBins * kWidth];    // [bin][channel], masked by the layer's ReLU
+};
+
+// The bins within `radius` of the sorted distinct bins sel[0..n), ascending, without repeats.
+__device__ __forceinline__ int list_bins(const int* sel, int n, int radius, int* out) {
+  int m = 0, next = INT_MIN;
+  for (int i = 0; i < n; ++i)
+    for (int x = max(next, sel[i] - radius); x <= sel[i] + radius; ++x) {
+      out[m++] = x;
+      next = x + 1;
     }
-    gs[i] = g;
+  return m;
+}
+// Index in the ascending list of bin x (which is in it).
+__device__ __forceinline__ int find_bin(const int* list, int n, int x) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (list[mid] < x) lo = mid + 1; else hi = mid;
   }
-  for (int i = threadIdx.x; i < cout * cin * ks; i += blockDim.x) wsm[i] = __half2float(w[i]);
+  return lo;
+}
+
+// Gradients of a sample's hidden layers at the listed bins.  grid B, kSparseThreads threads.
+constexpr int kSparseThreads = 512;
+
+__global__ void __launch_bounds__(kSparseThreads)
+sparse_grad_kernel(const float* __restrict__ dlogit, const int* __restrict__ argmax,
+                   const float* __restrict__ act0, const float* __restrict__ act1, const float* __restrict__ act2,
+                   int X, const __half* __restrict__ w1, const __half* __restrict__ w2, const __half* __restrict__ w3,
+                   SparseGrad* __restrict__ out) {
+  extern __shared__ float sm[];
+  float* const wsm = sm;                                     // [k][co][ci] of a 32 x 32 layer
+  float* const ga = wsm + kTaps * kWidth * kWidth;           // [bin + 4][channel]: the layer above
+  float* const gb = ga + (kMaxBins + 4) * kWidth;
+  __shared__ int sel[kWin], nsel, bins[3][kMaxBins], nb[3];
+  const int b = blockIdx.x, tid = threadIdx.x;
+  SparseGrad& o = out[b];
+  if (tid == 0) {
+    int n = 0;
+    for (int w = 0; w < kWin; ++w) {  // insertion into the sorted distinct bins
+      const int x = argmax[b * kWin + w];
+      int i = n;
+      while (i > 0 && sel[i - 1] > x) --i;
+      if (i > 0 && sel[i - 1] == x) continue;
+      for (int j = n; j > i; --j) sel[j] = sel[j - 1];
+      sel[i] = x;
+      ++n;
+    }
+    nsel = n;
+  }
   __syncthreads();
-  const int x = x0 + threadIdx.x;
-  if (x >= X) return;
-  for (int ci = 0; ci < cin; ++ci) {
-    float acc = 0.f;
-    for (int co = 0; co < cout; ++co)
-      for (int k = 0; k < ks; ++k)
-        acc = fmaf(wsm[(co * cin + ci) * ks + k], gs[co * TW + threadIdx.x + (ks - 1) - k], acc);
-    din[((long long)b * cin + ci) * X + x] = acc;
+  if (tid < 3) {
+    nb[tid] = list_bins(sel, nsel, 4 - 2 * tid, bins[tid]);
+    o.n[tid] = nb[tid];
+  }
+  __syncthreads();
+  for (int l = 0; l < 3; ++l)
+    for (int i = tid; i < nb[l]; i += kSparseThreads) o.bins[l][i] = bins[l][i];
+  // last hidden layer: the 1x1 layer's weights of the windows whose bin this is, in window order
+  for (int i = tid; i < nb[2] * kWidth; i += kSparseThreads) {
+    const int x = bins[2][i / kWidth], c = i % kWidth;
+    float g = 0.f;
+    for (int w = 0; w < kWin; ++w)
+      if (argmax[b * kWin + w] == x) g = fmaf(__half2float(w3[w * kWidth + c]), dlogit[b * kWin + w], g);
+    if (act2[((long long)b * kWidth + c) * X + x] <= 0.f) g = 0.f;
+    ga[i] = g;
+    o.g[2][i] = g;
+  }
+  float* from = ga;
+  float* to = gb;
+  for (int l = 1; l >= 0; --l) {  // layer l + 1 from the layer above it
+    const __half* const w = l == 1 ? w2 : w1;
+    const float* const act = l == 1 ? act1 : act0;
+    for (int i = tid; i < kTaps * kWidth * kWidth; i += kSparseThreads) {
+      const int co = i / (kWidth * kTaps), r = i - co * kWidth * kTaps, ci = r / kTaps, k = r - ci * kTaps;
+      wsm[(k * kWidth + co) * kWidth + ci] = __half2float(w[i]);
+    }
+    __syncthreads();
+    for (int i = tid; i < nb[l] * kWidth; i += kSparseThreads) {
+      const int x = bins[l][i / kWidth], ci = i % kWidth;
+      float g = 0.f;
+      if (x >= 0 && x < X) {
+        for (int k = 0; k < kTaps; ++k) {  // d_in[x] += w[.][ci][k] g[x + pad - k]
+          const int xo = x + kPad - k;
+          const int s = find_bin(bins[l + 1], nb[l + 1], xo);
+          if (bins[l + 1][s] != xo) continue;  // uniform over the warp (32 channels of a bin)
+          const float* const gr = from + s * kWidth;
+          const float* const wr = wsm + k * kWidth * kWidth + ci;
+#pragma unroll 8
+          for (int co = 0; co < kWidth; ++co) g = fmaf(wr[co * kWidth], gr[co], g);
+        }
+        if (act[((long long)b * kWidth + ci) * X + x] <= 0.f) g = 0.f;
+      }
+      to[i] = g;
+      o.g[l][i] = g;
+    }
+    __syncthreads();
+    float* const t = from;
+    from = to;
+    to = t;
   }
 }
 
-// Per-block partial weight / bias gradients: partial[blk][co][ci][k] and [blk][bias co],
-// blk = (b, x-tile).  grid (X/kConvTile, B), block kConvTile.
-__global__ void __launch_bounds__(kConvTile)
-conv_bwd_weight_kernel(const float* __restrict__ dout, const float* __restrict__ relu_out,
-                       const float* __restrict__ in, int cout, int cin, int ks, int X,
-                       float* __restrict__ partial) {
-  extern __shared__ float sm[];
-  const int pad = ks / 2;
-  const int TW = kConvTile + ks - 1;
-  float* xs = sm;                       // cin * TW
-  float* gs = sm + cin * TW;            // cout * kConvTile
-  const int b = blockIdx.y, x0 = blockIdx.x * kConvTile;
-  for (int i = threadIdx.x; i < cin * TW; i += blockDim.x) {
-    const int ci = i / TW, xx = x0 - pad + (i - ci * TW);
-    xs[i] = (xx >= 0 && xx < X) ? in[((long long)b * cin + ci) * X + xx] : 0.f;
-  }
-  for (int i = threadIdx.x; i < cout * kConvTile; i += blockDim.x) {
-    const int co = i / kConvTile, xx = x0 + (i - co * kConvTile);
-    float g = 0.f;
-    if (xx < X) {
-      const long long idx = ((long long)b * cout + co) * X + xx;
-      g = dout[idx];
-      if (relu_out && relu_out[idx] <= 0.f) g = 0.f;
+// A sample's gradient of one layer's parameters: grid (4 layers, B).  Layers 1 to 3: a thread
+// takes four output channels, an input channel and the five taps; the layer's input at the listed
+// bins and two either side sits in shared memory in list order.  Layer 4 (1x1): its selected bins.
+__global__ void __launch_bounds__(kSparseThreads)
+sparse_weight_grad_kernel(const SparseGrad* __restrict__ sg, const float* __restrict__ x0,
+                          const float* __restrict__ act0, const float* __restrict__ act1,
+                          const float* __restrict__ act2, const float* __restrict__ dlogit,
+                          const int* __restrict__ argmax, int cin0, int X, Layer L0, Layer L1, Layer L2, Layer L3,
+                          float* __restrict__ partial, long long nparams) {
+  extern __shared__ float4 sm4[];
+  const int l = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
+  float* const pb = partial + b * nparams;
+  if (l == 3) {
+    for (int i = tid; i < kWin * kWidth; i += kSparseThreads) {
+      const int w = i / kWidth, c = i % kWidth;
+      pb[L3.woff + i] = dlogit[b * kWin + w] * act2[((long long)b * kWidth + c) * X + argmax[b * kWin + w]];
     }
-    gs[i] = g;
+    for (int w = tid; w < kWin; w += kSparseThreads) pb[L3.boff + w] = dlogit[b * kWin + w];
+    return;
+  }
+  const Layer& L = l == 0 ? L0 : l == 1 ? L1 : L2;
+  const int cin = l == 0 ? cin0 : kWidth;
+  const float* const in = (l == 0 ? x0 : l == 1 ? act0 : act1) + (long long)b * cin * X;
+  const SparseGrad& s = sg[b];
+  const int n = s.n[l];
+  float* const gsm = reinterpret_cast<float*>(sm4);          // [bin][channel]
+  float* const xsm = gsm + kMaxBins * kWidth;             // [ci][kMaxInBins]: bins within two of the list
+  __shared__ int bins[kMaxBins], first[kMaxBins], ext[kMaxInBins], next_n;
+  for (int i = tid; i < n; i += kSparseThreads) bins[i] = s.bins[l][i];
+  for (int i = tid; i < n * kWidth; i += kSparseThreads) gsm[i] = s.g[l][i];
+  __syncthreads();
+  if (tid == 0) {
+    int m = 0, next = INT_MIN;
+    for (int i = 0; i < n; ++i) {
+      for (int x = max(next, bins[i] - kPad); x <= bins[i] + kPad; ++x) {
+        ext[m++] = x;
+        next = x + 1;
+      }
+      first[i] = m - kTaps;  // bin bins[i] - 2: the list holds all five
+    }
+    next_n = m;
   }
   __syncthreads();
-  const int nw = cout * cin * ks;
-  const long long blk = (long long)blockIdx.y * gridDim.x + blockIdx.x;
-  float* pb = partial + blk * (nw + cout);
-  for (int i = threadIdx.x; i < nw + cout; i += blockDim.x) {
-    float acc = 0.f;
-    if (i < nw) {
-      const int co = i / (cin * ks), r = i - co * cin * ks, ci = r / ks, k = r - ci * ks;
-      for (int x = 0; x < kConvTile; ++x) acc = fmaf(gs[co * kConvTile + x], xs[ci * TW + x + k], acc);
-    } else {
-      const int co = i - nw;
-      for (int x = 0; x < kConvTile; ++x) acc += gs[co * kConvTile + x];
+  const int ne = next_n;
+  for (int i = tid; i < cin * ne; i += kSparseThreads) {
+    const int ci = i / ne, e = i - ci * ne, x = ext[e];
+    xsm[ci * kMaxInBins + e] = (x >= 0 && x < X) ? in[(long long)ci * X + x] : 0.f;
+  }
+  __syncthreads();
+  for (int u = tid; u < (kWidth / 4) * cin; u += kSparseThreads) {
+    const int cg = u % (kWidth / 4), ci = u / (kWidth / 4);
+    const float* const xr = xsm + ci * kMaxInBins;
+    float a[4][kTaps];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int k = 0; k < kTaps; ++k) a[q][k] = 0.f;
+    for (int i = 0; i < n; ++i) {
+      const float4 g = sm4[i * (kWidth / 4) + cg];
+      const float* const xe = xr + first[i];
+#pragma unroll
+      for (int k = 0; k < kTaps; ++k) {
+        const float v = xe[k];
+        a[0][k] = fmaf(g.x, v, a[0][k]);
+        a[1][k] = fmaf(g.y, v, a[1][k]);
+        a[2][k] = fmaf(g.z, v, a[2][k]);
+        a[3][k] = fmaf(g.w, v, a[3][k]);
+      }
     }
-    pb[i] = acc;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int k = 0; k < kTaps; ++k) pb[L.woff + ((long long)(4 * cg + q) * cin + ci) * kTaps + k] = a[q][k];
+  }
+  for (int c = tid; c < kWidth; c += kSparseThreads) {
+    float a = 0.f;
+    for (int i = 0; i < n; ++i) a += gsm[i * kWidth + c];
+    pb[L.boff + c] = a;
   }
 }
 
-// grad[off + i] = sum over blocks (in order) of partial[blk][i]
-__global__ void reduce_partials_kernel(const float* __restrict__ partial, int nblk, int n,
-                                       float* __restrict__ gw, float* __restrict__ gb, int nw) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// grad[i] = sum over samples (in order) of partial[b][i]
+__global__ void reduce_partials_kernel(const float* __restrict__ partial, int B, long long n, float* __restrict__ grad) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   float s = 0.f;
-  for (int k = 0; k < nblk; ++k) s += partial[(long long)k * n + i];
-  if (i < nw) gw[i] = s; else gb[i - nw] = s;
+#pragma unroll 8
+  for (int k = 0; k < B; ++k) s += partial[k * n + i];
+  grad[i] = s;
 }
 
 __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
@@ -379,45 +590,32 @@ static int set_attrs() {
   int dev = 0;
   FDR_CUDA(cudaGetDevice(&dev));
   if (dev < 64 && done[dev]) return FDR_OK;
-  const int big = 160 * 1024;  // conv layers with up to 64 input channels need <= 107 KB
-  FDR_CUDA(cudaFuncSetAttribute(conv_fwd_kernel<32, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FDR_CUDA(cudaFuncSetAttribute(conv_fwd_kernel<16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FDR_CUDA(cudaFuncSetAttribute(conv_bwd_data_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  FDR_CUDA(cudaFuncSetAttribute(conv_bwd_weight_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  const int big = 160 * 1024;  // conv layers with up to 64 input channels need <= 110 KB
+  FDR_CUDA(cudaFuncSetAttribute(conv_fwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  FDR_CUDA(cudaFuncSetAttribute(conv_fwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  FDR_CUDA(cudaFuncSetAttribute(sparse_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  FDR_CUDA(cudaFuncSetAttribute(sparse_weight_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   if (dev < 64) done[dev] = true;
-  return FDR_OK;
-}
-
-static int conv_forward(const fdr_propose_net* n, int li, const float* in, int B, float* out,
-                        cudaStream_t s) {
-  const Layer& L = n->L[li];
-  const int X = n->nbins;
-  const int TW = kConvTile + L.k - 1;
-  const size_t sm = sizeof(float) * (L.cin * TW + L.cout * L.cin * L.k);
-  dim3 grid((unsigned)cdiv(X, kConvTile), (unsigned)B);
-  const int relu = li < 3;
-  const __half* w = n->wh + L.woff;
-  const float* bias = n->params + L.boff;
-  if (L.cout == 32 && L.k == 5) {
-    conv_fwd_kernel<32, 5><<<grid, kConvTile, sm, s>>>(in, L.cin, X, w, bias, relu, out);
-  } else if (L.cout == 16 && L.k == 1) {
-    conv_fwd_kernel<16, 1><<<grid, kConvTile, sm, s>>>(in, L.cin, X, w, bias, relu, out);
-  } else {
-    set_error(FDR_ERR_INVALID_ARGUMENT, "proposal net: unsupported layer shape");
-    return FDR_ERR_INVALID_ARGUMENT;
-  }
-  FDR_LAUNCH_CHECK("conv_fwd_kernel");
   return FDR_OK;
 }
 
 static int net_forward(fdr_propose_net* n, const float* x, int B, float* logits, cudaStream_t s) {
   FDR_CHECK_ARG(B >= 1 && B <= n->maxb, "proposal net: batch %d exceeds the maximum %d", B, n->maxb);
   const float* in = x;
-  for (int li = 0; li < 4; ++li) {
-    FDR_TRY(conv_forward(n, li, in, B, n->act[li], s));
+  const int X = n->nbins, tiles = (int)cdiv(X, kConvTile);
+  const dim3 grid((unsigned)tiles, (unsigned)B);
+  for (int li = 0; li < 3; ++li) {
+    const Layer& L = n->L[li];
+    const size_t sm = sizeof(float) * (L.cin * (kConvTile + kTaps - 1) + kWidth * L.cin * kTaps +
+                                       (li == 2 ? kWidth * kWin : 0));
+    auto kernel = li == 2 ? conv_fwd_kernel<true> : conv_fwd_kernel<false>;
+    kernel<<<grid, kConvThreads, sm, s>>>(in, L.cin, X, n->wh + L.woff, n->params + L.boff, n->act[li],
+                                          n->wh + n->L[3].woff, n->params + n->L[3].boff, n->tile_max, n->tile_arg);
+    FDR_LAUNCH_CHECK("conv_fwd_kernel");
     in = n->act[li];
   }
-  maxpool_kernel<<<dim3(n->nwin, B), 256, 0, s>>>(n->act[3], n->nwin, n->nbins, logits, n->argmax);
+  maxpool_kernel<<<(unsigned)cdiv(B * n->nwin, 64), 64, 0, s>>>(n->tile_max, n->tile_arg, tiles, B * n->nwin, logits,
+                                                               n->argmax);
   FDR_LAUNCH_CHECK("maxpool_kernel");
   return FDR_OK;
 }
@@ -427,34 +625,21 @@ static int net_grad(fdr_propose_net* n, const float* x, const float* labels, int
                     cudaStream_t s) {
   FDR_TRY(net_forward(n, x, B, logits, s));
   const int X = n->nbins;
-  float* dy = n->dact[0];
-  FDR_CUDA(cudaMemsetAsync(dy, 0, sizeof(float) * (size_t)B * n->nwin * X, s));
-  bce_kernel<<<1, 256, 0, s>>>(logits, labels, n->argmax, B * n->nwin, n->nwin, X, dy, n->loss);
+  bce_kernel<<<1, 256, 0, s>>>(logits, labels, B * n->nwin, n->dlogit, n->loss);
   FDR_LAUNCH_CHECK("bce_kernel");
-  for (int li = 3; li >= 0; --li) {
-    const Layer& L = n->L[li];
-    const float* layer_in = li == 0 ? x : n->act[li - 1];
-    const float* relu_out = li < 3 ? n->act[li] : nullptr;
-    const int TW = kConvTile + L.k - 1;
-    dim3 grid((unsigned)cdiv(X, kConvTile), (unsigned)B);
-    const int nblk = grid.x * grid.y;
-    const int nwp = L.cout * L.cin * L.k + L.cout;
-    size_t smw = sizeof(float) * (L.cin * TW + L.cout * kConvTile);
-    conv_bwd_weight_kernel<<<grid, kConvTile, smw, s>>>(dy, relu_out, layer_in, L.cout, L.cin, L.k,
-                                                        X, n->partial);
-    FDR_LAUNCH_CHECK("conv_bwd_weight_kernel");
-    reduce_partials_kernel<<<(unsigned)cdiv(nwp, 256), 256, 0, s>>>(
-        n->partial, nblk, nwp, n->grad + L.woff, n->grad + L.boff, L.cout * L.cin * L.k);
-    FDR_LAUNCH_CHECK("reduce_partials_kernel");
-    if (li > 0) {
-      float* din = (dy == n->dact[0]) ? n->dact[1] : n->dact[0];
-      size_t smd = sizeof(float) * (L.cout * TW + L.cout * L.cin * L.k);
-      conv_bwd_data_kernel<<<grid, kConvTile, smd, s>>>(dy, relu_out, L.cout, L.cin, L.k, X,
-                                                        n->wh + L.woff, din);
-      FDR_LAUNCH_CHECK("conv_bwd_data_kernel");
-      dy = din;
-    }
-  }
+  SparseGrad* const sg = reinterpret_cast<SparseGrad*>(n->gact);
+  const size_t sm1 = sizeof(float) * (kTaps * kWidth * kWidth + 2 * (kMaxBins + 4) * kWidth);
+  sparse_grad_kernel<<<B, kSparseThreads, sm1, s>>>(n->dlogit, n->argmax, n->act[0], n->act[1], n->act[2], X,
+                                                    n->wh + n->L[1].woff, n->wh + n->L[2].woff,
+                                                    n->wh + n->L[3].woff, sg);
+  FDR_LAUNCH_CHECK("sparse_grad_kernel");
+  const size_t sm2 = sizeof(float) * (kMaxBins * kWidth + std::max(n->nt, kWidth) * kMaxInBins);
+  sparse_weight_grad_kernel<<<dim3(4, B), kSparseThreads, sm2, s>>>(
+      sg, x, n->act[0], n->act[1], n->act[2], n->dlogit, n->argmax, n->nt, X, n->L[0], n->L[1], n->L[2], n->L[3],
+      n->partial, n->nparams);
+  FDR_LAUNCH_CHECK("sparse_weight_grad_kernel");
+  reduce_partials_kernel<<<(unsigned)cdiv(n->nparams, 128), 128, 0, s>>>(n->partial, B, n->nparams, n->grad);
+  FDR_LAUNCH_CHECK("reduce_partials_kernel");
   return FDR_OK;
 }
 
@@ -466,8 +651,11 @@ static void net_release(fdr_propose_net* n) {
   cudaFree(n->v);
   cudaFree(n->grad);
   for (auto* a : n->act) cudaFree(a);
+  cudaFree(n->tile_max);
+  cudaFree(n->tile_arg);
   cudaFree(n->argmax);
-  for (auto* a : n->dact) cudaFree(a);
+  cudaFree(n->dlogit);
+  cudaFree(n->gact);
   cudaFree(n->partial);
   cudaFree(n->loss);
   delete n;
@@ -511,19 +699,20 @@ int fdr_propose_create(fdr_propose_net** out, int nbins, int nt, int width, int 
     }
   }
   const size_t act_elems = (size_t)max_batch * width * nbins;
-  int64_t maxblk = cdiv(nbins, kConvTile) * max_batch, maxw = 0;
-  for (int i = 0; i < 4; ++i) maxw = std::max<int64_t>(maxw, (int64_t)couts[i] * cins[i] * ks[i] + couts[i]);
-  n->partial_elems = maxblk * maxw;
+  const size_t tile_elems = (size_t)cdiv(nbins, kConvTile) * max_batch * nwin;
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = cudaMalloc(&n->params, sizeof(float) * off);
   if (e == cudaSuccess) e = cudaMalloc(&n->wh, sizeof(__half) * off);
   if (e == cudaSuccess) e = cudaMalloc(&n->m, sizeof(float) * off);
   if (e == cudaSuccess) e = cudaMalloc(&n->v, sizeof(float) * off);
   if (e == cudaSuccess) e = cudaMalloc(&n->grad, sizeof(float) * off);
-  for (int i = 0; i < 4 && e == cudaSuccess; ++i) e = cudaMalloc(&n->act[i], sizeof(float) * act_elems);
-  for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMalloc(&n->dact[i], sizeof(float) * act_elems);
+  for (int i = 0; i < 3 && e == cudaSuccess; ++i) e = cudaMalloc(&n->act[i], sizeof(float) * act_elems);
+  if (e == cudaSuccess) e = cudaMalloc(&n->tile_max, sizeof(float) * tile_elems);
+  if (e == cudaSuccess) e = cudaMalloc(&n->tile_arg, sizeof(int) * tile_elems);
+  if (e == cudaSuccess) e = cudaMalloc(&n->dlogit, sizeof(float) * (size_t)max_batch * nwin);
+  if (e == cudaSuccess) e = cudaMalloc(&n->gact, sizeof(SparseGrad) * (size_t)max_batch);
   if (e == cudaSuccess) e = cudaMalloc(&n->argmax, sizeof(int) * (size_t)max_batch * nwin);
-  if (e == cudaSuccess) e = cudaMalloc(&n->partial, sizeof(float) * n->partial_elems);
+  if (e == cudaSuccess) e = cudaMalloc(&n->partial, sizeof(float) * (size_t)max_batch * off);
   if (e == cudaSuccess) e = cudaMalloc(&n->loss, sizeof(float));
   if (e == cudaSuccess) e = cudaMemcpy(n->params, h.data(), sizeof(float) * off, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(n->m, 0, sizeof(float) * off);
