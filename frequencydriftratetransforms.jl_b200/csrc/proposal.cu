@@ -35,7 +35,8 @@ struct fdr_propose_net {
   fdr::Layer L[4];
   int64_t nparams = 0;
   float* params = nullptr;   // float32 master weights (w then b per layer)
-  __half* wh = nullptr;      // float16 copy used by the forward pass
+  __half* wh = nullptr;      // float16 copy used by both passes
+  float* wt = nullptr;       // its values, each layer as [input channel][tap][output channel]
   float* m = nullptr;        // Adam moments
   float* v = nullptr;
   float* grad = nullptr;
@@ -182,8 +183,8 @@ constexpr int kConvThreads = kConvTile / 2;
 
 template <bool HEAD>
 __global__ void __launch_bounds__(kConvThreads, 4)
-conv_fwd_kernel(const float* __restrict__ in, int cin, int X, const __half* __restrict__ w,
-                const float* __restrict__ bias, float* __restrict__ out, const __half* __restrict__ w3,
+conv_fwd_kernel(const float* __restrict__ in, int cin, int X, const float* __restrict__ wt,
+                const float* __restrict__ bias, float* __restrict__ out, const float* __restrict__ wt3,
                 const float* __restrict__ bias3, float* __restrict__ tile_max, int* __restrict__ tile_arg) {
   extern __shared__ float4 sm4[];
   constexpr int TW = kConvTile + kTaps - 1;
@@ -192,17 +193,20 @@ conv_fwd_kernel(const float* __restrict__ in, int cin, int X, const __half* __re
   float* const xs = w3sm + (HEAD ? kWidth * kWin : 0);  // [ci][TW]
   const int b = blockIdx.y, x0 = blockIdx.x * kConvTile, tid = threadIdx.x;
   const float* const inb = in + (long long)b * cin * X;
-  for (int i = tid; i < cin * TW; i += kConvThreads) {
-    const int ci = i / TW, xx = x0 - kPad + (i - ci * TW);
-    xs[i] = (xx >= 0 && xx < X) ? inb[(long long)ci * X + xx] : 0.f;
+  const int lane = tid & 31, warp = tid >> 5;
+#pragma unroll 2
+  for (int ci = warp; ci < cin; ci += kConvThreads / 32) {  // a warp per row: loads in flight together
+    const float* const row = inb + (long long)ci * X;
+#pragma unroll
+    for (int j = 0; j < (TW + 31) / 32; ++j) {
+      const int i = lane + 32 * j, xx = x0 - kPad + i;
+      if (i < TW) xs[ci * TW + i] = (xx >= 0 && xx < X) ? __ldg(row + xx) : 0.f;
+    }
   }
-  for (int i = tid; i < cin * kTaps * kWidth; i += kConvThreads) {
-    const int co = i / (cin * kTaps), r = i - co * cin * kTaps;
-    wsm[r * kWidth + co] = __half2float(w[i]);
-  }
+#pragma unroll 4
+  for (int i = tid; i < cin * kTaps * kWidth; i += kConvThreads) wsm[i] = __ldg(wt + i);
   if (HEAD)
-    for (int i = tid; i < kWidth * kWin; i += kConvThreads)
-      w3sm[(i % kWidth) * kWin + i / kWidth] = __half2float(w3[i]);
+    for (int i = tid; i < kWidth * kWin; i += kConvThreads) w3sm[i] = __ldg(wt3 + i);
   __syncthreads();
   float2 acc[2][kWidth / 2];
 #pragma unroll
@@ -240,7 +244,6 @@ conv_fwd_kernel(const float* __restrict__ in, int cin, int X, const __half* __re
   if (!HEAD) return;
   __shared__ float rv[kConvThreads / 32][kWin];
   __shared__ int ri[kConvThreads / 32][kWin];
-  const int lane = tid & 31, warp = tid >> 5;
 #pragma unroll
   for (int half = 0; half < 2; ++half) {  // 8 windows at a time
     float best[kWin / 2];
@@ -365,24 +368,53 @@ struct SparseGrad {                 // of one sample
   float g[3][kMaxBins * kWidth];    // [bin][channel], masked by the layer's ReLU
 };
 
-// The bins within `radius` of the sorted distinct bins sel[0..n), ascending, without repeats.
-__device__ __forceinline__ int list_bins(const int* sel, int n, int radius, int* out) {
-  int m = 0, next = INT_MIN;
-  for (int i = 0; i < n; ++i)
-    for (int x = max(next, sel[i] - radius); x <= sel[i] + radius; ++x) {
-      out[m++] = x;
-      next = x + 1;
+// The selected bins of a sample, sorted and distinct, and lists of the bins around them.
+struct BinSet {
+  int sel[kWin], n;
+  int start[kWin + 1];
+  // by all threads of the block, from the 16 bins in `raw` (shared memory, visible)
+  __device__ __forceinline__ void sort(const int* raw) {
+    const int t = threadIdx.x;
+    if (t < kWin) {
+      int rank = 0, distinct = 0;
+      bool repeat = false;
+      for (int w = 0; w < kWin; ++w) {
+        bool seen = false;  // raw[w] occurs before w
+        for (int v = 0; v < w; ++v) seen |= raw[v] == raw[w];
+        repeat |= w < t && raw[w] == raw[t];
+        if (!seen) {
+          ++distinct;
+          rank += raw[w] < raw[t];
+        }
+      }
+      if (!repeat) sel[rank] = raw[t];
+      if (t == 0) n = distinct;
     }
-  return m;
-}
-// Index in the ascending list of bin x (which is in it).
-__device__ __forceinline__ int find_bin(const int* list, int n, int x) {
+    __syncthreads();
+  }
+  // the bins within `radius` of a selected one, ascending, without repeats; their number
+  __device__ __forceinline__ int list(int radius, int* out) {
+    const int t = threadIdx.x, w = 2 * radius + 1;
+    if (t <= kWin) {
+      int s = 0;
+      for (int i = 0; i < n && i < t; ++i) s += i == 0 ? w : min(w, sel[i] - sel[i - 1]);
+      start[t] = s;
+    }
+    __syncthreads();
+    const int i = t / 16, j = t % 16;  // w <= 13
+    if (i < n && j < start[i + 1] - start[i]) out[start[i] + j] = sel[i] + radius + 1 - (start[i + 1] - start[i]) + j;
+    __syncthreads();
+    return start[n];
+  }
+};
+// Index in the ascending list of bin x, or `none` if it is not there.
+__device__ __forceinline__ int find_bin(const int* list, int n, int x, int none) {
   int lo = 0, hi = n - 1;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
     if (list[mid] < x) lo = mid + 1; else hi = mid;
   }
-  return lo;
+  return list[lo] == x ? lo : none;
 }
 
 // Gradients of a sample's hidden layers at the listed bins.  grid B, kSparseThreads threads.
@@ -391,73 +423,85 @@ constexpr int kSparseThreads = 512;
 __global__ void __launch_bounds__(kSparseThreads)
 sparse_grad_kernel(const float* __restrict__ dlogit, const int* __restrict__ argmax,
                    const float* __restrict__ act0, const float* __restrict__ act1, const float* __restrict__ act2,
-                   int X, const __half* __restrict__ w1, const __half* __restrict__ w2, const __half* __restrict__ w3,
+                   int X, const float* __restrict__ wt1, const float* __restrict__ wt2, const __half* __restrict__ w3,
                    SparseGrad* __restrict__ out) {
-  extern __shared__ float sm[];
-  float* const wsm = sm;                                     // [k][co][ci] of a 32 x 32 layer
-  float* const ga = wsm + kTaps * kWidth * kWidth;           // [bin + 4][channel]: the layer above
-  float* const gb = ga + (kMaxBins + 4) * kWidth;
-  __shared__ int sel[kWin], nsel, bins[3][kMaxBins], nb[3];
+  extern __shared__ float4 sm4[];
+  float* const wsm = reinterpret_cast<float*>(sm4);          // [k][co][ci] of a 32 x 32 layer
+  float* const ga = wsm + kTaps * kWidth * kWidth;           // [bin][channel]; a row of zeros after the last
+  float* const gb = ga + (kMaxBins + 1) * kWidth;
+  __shared__ BinSet set;
+  __shared__ int raw[kWin], bins[3][kMaxBins], slot[kMaxBins][kTaps];
   const int b = blockIdx.x, tid = threadIdx.x;
   SparseGrad& o = out[b];
-  if (tid == 0) {
-    int n = 0;
-    for (int w = 0; w < kWin; ++w) {  // insertion into the sorted distinct bins
-      const int x = argmax[b * kWin + w];
-      int i = n;
-      while (i > 0 && sel[i - 1] > x) --i;
-      if (i > 0 && sel[i - 1] == x) continue;
-      for (int j = n; j > i; --j) sel[j] = sel[j - 1];
-      sel[i] = x;
-      ++n;
-    }
-    nsel = n;
-  }
+  if (tid < kWin) raw[tid] = argmax[b * kWin + tid];
   __syncthreads();
-  if (tid < 3) {
-    nb[tid] = list_bins(sel, nsel, 4 - 2 * tid, bins[tid]);
-    o.n[tid] = nb[tid];
+  set.sort(raw);
+  int nb[3];
+  for (int l = 0; l < 3; ++l) {
+    nb[l] = set.list(4 - 2 * l, bins[l]);
+    if (tid == 0) o.n[l] = nb[l];
+    if (tid < nb[l]) o.bins[l][tid] = bins[l][tid];
   }
-  __syncthreads();
-  for (int l = 0; l < 3; ++l)
-    for (int i = tid; i < nb[l]; i += kSparseThreads) o.bins[l][i] = bins[l][i];
   // last hidden layer: the 1x1 layer's weights of the windows whose bin this is, in window order
   for (int i = tid; i < nb[2] * kWidth; i += kSparseThreads) {
     const int x = bins[2][i / kWidth], c = i % kWidth;
+    const float relu = act2[((long long)b * kWidth + c) * X + x];
     float g = 0.f;
     for (int w = 0; w < kWin; ++w)
-      if (argmax[b * kWin + w] == x) g = fmaf(__half2float(w3[w * kWidth + c]), dlogit[b * kWin + w], g);
-    if (act2[((long long)b * kWidth + c) * X + x] <= 0.f) g = 0.f;
+      if (raw[w] == x) g = fmaf(__half2float(w3[w * kWidth + c]), dlogit[b * kWin + w], g);
+    if (relu <= 0.f) g = 0.f;
     ga[i] = g;
     o.g[2][i] = g;
   }
   float* from = ga;
   float* to = gb;
   for (int l = 1; l >= 0; --l) {  // layer l + 1 from the layer above it
-    const __half* const w = l == 1 ? w2 : w1;
+    const float* const w = l == 1 ? wt2 : wt1;  // [ci][k][co]
     const float* const act = l == 1 ? act1 : act0;
     for (int i = tid; i < kTaps * kWidth * kWidth; i += kSparseThreads) {
-      const int co = i / (kWidth * kTaps), r = i - co * kWidth * kTaps, ci = r / kTaps, k = r - ci * kTaps;
-      wsm[(k * kWidth + co) * kWidth + ci] = __half2float(w[i]);
+      const int co = i / (kWidth * kTaps), r = i - co * kWidth * kTaps, k = r / kWidth, ci = r - k * kWidth;
+      wsm[(k * kWidth + co) * kWidth + ci] = __ldg(w + (ci * kTaps + k) * kWidth + co);
     }
+    for (int i = tid; i < nb[l] * kTaps; i += kSparseThreads) {
+      const int s = i / kTaps, k = i - s * kTaps;
+      slot[s][k] = find_bin(bins[l + 1], nb[l + 1], bins[l][s] + kPad - k, nb[l + 1]);
+    }
+    if (tid < kWidth) from[nb[l + 1] * kWidth + tid] = 0.f;
     __syncthreads();
-    for (int i = tid; i < nb[l] * kWidth; i += kSparseThreads) {
-      const int x = bins[l][i / kWidth], ci = i % kWidth;
-      float g = 0.f;
-      if (x >= 0 && x < X) {
-        for (int k = 0; k < kTaps; ++k) {  // d_in[x] += w[.][ci][k] g[x + pad - k]
-          const int xo = x + kPad - k;
-          const int s = find_bin(bins[l + 1], nb[l + 1], xo);
-          if (bins[l + 1][s] != xo) continue;  // uniform over the warp (32 channels of a bin)
-          const float* const gr = from + s * kWidth;
-          const float* const wr = wsm + k * kWidth * kWidth + ci;
-#pragma unroll 8
-          for (int co = 0; co < kWidth; ++co) g = fmaf(wr[co * kWidth], gr[co], g);
-        }
-        if (act[((long long)b * kWidth + ci) * X + x] <= 0.f) g = 0.f;
+    // d_in[x] = sum over k, co of w[co][ci][k] g[x + pad - k]: a thread takes channel ci of four
+    // bins, so that its four weights feed 16 multiply-adds
+    const int ci = tid % kWidth;
+    for (int s0 = 4 * (tid / kWidth); s0 < nb[l]; s0 += 4 * (kSparseThreads / kWidth)) {
+      float g[4] = {0.f, 0.f, 0.f, 0.f}, relu[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int x = bins[l][min(s0 + q, nb[l] - 1)];
+        relu[q] = x >= 0 && x < X ? act[((long long)b * kWidth + ci) * X + x] : 0.f;
       }
-      to[i] = g;
-      o.g[l][i] = g;
+      for (int k = 0; k < kTaps; ++k) {
+        const float4* gr[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          gr[q] = reinterpret_cast<const float4*>(from + slot[min(s0 + q, nb[l] - 1)][k] * kWidth);
+        const float* const wr = wsm + k * kWidth * kWidth + ci;
+#pragma unroll
+        for (int c4 = 0; c4 < kWidth / 4; ++c4) {
+          const float w0 = wr[(4 * c4) * kWidth], w1 = wr[(4 * c4 + 1) * kWidth], w2 = wr[(4 * c4 + 2) * kWidth],
+                      w3v = wr[(4 * c4 + 3) * kWidth];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float4 v = gr[q][c4];
+            g[q] = fmaf(w3v, v.w, fmaf(w2, v.z, fmaf(w1, v.y, fmaf(w0, v.x, g[q]))));
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (s0 + q < nb[l]) {
+          if (relu[q] <= 0.f) g[q] = 0.f;
+          to[(s0 + q) * kWidth + ci] = g[q];
+          o.g[l][(s0 + q) * kWidth + ci] = g[q];
+        }
     }
     __syncthreads();
     float* const t = from;
@@ -493,23 +537,14 @@ sparse_weight_grad_kernel(const SparseGrad* __restrict__ sg, const float* __rest
   const int n = s.n[l];
   float* const gsm = reinterpret_cast<float*>(sm4);          // [bin][channel]
   float* const xsm = gsm + kMaxBins * kWidth;             // [ci][kMaxInBins]: bins within two of the list
-  __shared__ int bins[kMaxBins], first[kMaxBins], ext[kMaxInBins], next_n;
-  for (int i = tid; i < n; i += kSparseThreads) bins[i] = s.bins[l][i];
+  __shared__ BinSet set;
+  __shared__ int raw[kWin], first[kMaxBins], ext[kMaxInBins];
+  if (tid < kWin) raw[tid] = argmax[b * kWin + tid];
   for (int i = tid; i < n * kWidth; i += kSparseThreads) gsm[i] = s.g[l][i];
   __syncthreads();
-  if (tid == 0) {
-    int m = 0, next = INT_MIN;
-    for (int i = 0; i < n; ++i) {
-      for (int x = max(next, bins[i] - kPad); x <= bins[i] + kPad; ++x) {
-        ext[m++] = x;
-        next = x + 1;
-      }
-      first[i] = m - kTaps;  // bin bins[i] - 2: the list holds all five
-    }
-    next_n = m;
-  }
-  __syncthreads();
-  const int ne = next_n;
+  set.sort(raw);
+  const int ne = set.list(6 - 2 * l, ext);  // the input's bins: two either side of the layer's
+  for (int i = tid; i < n; i += kSparseThreads) first[i] = find_bin(ext, ne, s.bins[l][i] - kPad, 0);
   for (int i = tid; i < cin * ne; i += kSparseThreads) {
     const int ci = i / ne, e = i - ci * ne, x = ext[e];
     xsm[ci * kMaxInBins + e] = (x >= 0 && x < X) ? in[(long long)ci * X + x] : 0.f;
@@ -557,9 +592,25 @@ __global__ void reduce_partials_kernel(const float* __restrict__ partial, int B,
   grad[i] = s;
 }
 
+// Where weight i of the layers goes in their [ci][k][co] order (biases keep their place).
+struct LayerOrder {
+  Layer L[4];
+};
+__device__ __forceinline__ long long transposed_place(const LayerOrder& o, long long i) {
+#pragma unroll
+  for (int l = 0; l < 4; ++l) {
+    const Layer& L = o.L[l];
+    if (i >= L.woff && i < L.boff) {
+      const int r = (int)(i - L.woff), per = L.cin * L.k;
+      return L.woff + (long long)(r % per) * L.cout + r / per;
+    }
+  }
+  return i;
+}
+
 __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                            float* __restrict__ v, __half* __restrict__ wh, long long n, float lr,
-                            float b1, float b2, float eps, float c1, float c2) {
+                            float* __restrict__ v, __half* __restrict__ wh, float* __restrict__ wt, LayerOrder order,
+                            long long n, float lr, float b1, float b2, float eps, float c1, float c2) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float gi = g[i];
@@ -569,15 +620,27 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, 
   v[i] = vi;
   const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
   p[i] = pi;
-  wh[i] = __float2half_rn(pi);
+  const __half h = __float2half_rn(pi);
+  wh[i] = h;
+  wt[transposed_place(order, i)] = __half2float(h);
 }
 
-__global__ void to_half_kernel(const float* __restrict__ p, __half* __restrict__ wh, long long n) {
+__global__ void to_half_kernel(const float* __restrict__ p, __half* __restrict__ wh, float* __restrict__ wt,
+                               LayerOrder order, long long n) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i < n) wh[i] = __float2half_rn(p[i]);
+  if (i >= n) return;
+  const __half h = __float2half_rn(p[i]);
+  wh[i] = h;
+  wt[transposed_place(order, i)] = __half2float(h);
 }
 
 // ---- host helpers ---------------------------------------------------------------------
+static LayerOrder layer_order(const fdr_propose_net* n) {
+  LayerOrder o;
+  for (int i = 0; i < 4; ++i) o.L[i] = n->L[i];
+  return o;
+}
+
 static uint64_t splitmix(uint64_t& s) {
   uint64_t z = (s += 0x9E3779B97F4A7C15ULL);
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
@@ -609,8 +672,8 @@ static int net_forward(fdr_propose_net* n, const float* x, int B, float* logits,
     const size_t sm = sizeof(float) * (L.cin * (kConvTile + kTaps - 1) + kWidth * L.cin * kTaps +
                                        (li == 2 ? kWidth * kWin : 0));
     auto kernel = li == 2 ? conv_fwd_kernel<true> : conv_fwd_kernel<false>;
-    kernel<<<grid, kConvThreads, sm, s>>>(in, L.cin, X, n->wh + L.woff, n->params + L.boff, n->act[li],
-                                          n->wh + n->L[3].woff, n->params + n->L[3].boff, n->tile_max, n->tile_arg);
+    kernel<<<grid, kConvThreads, sm, s>>>(in, L.cin, X, n->wt + L.woff, n->params + L.boff, n->act[li],
+                                          n->wt + n->L[3].woff, n->params + n->L[3].boff, n->tile_max, n->tile_arg);
     FDR_LAUNCH_CHECK("conv_fwd_kernel");
     in = n->act[li];
   }
@@ -628,9 +691,9 @@ static int net_grad(fdr_propose_net* n, const float* x, const float* labels, int
   bce_kernel<<<1, 256, 0, s>>>(logits, labels, B * n->nwin, n->dlogit, n->loss);
   FDR_LAUNCH_CHECK("bce_kernel");
   SparseGrad* const sg = reinterpret_cast<SparseGrad*>(n->gact);
-  const size_t sm1 = sizeof(float) * (kTaps * kWidth * kWidth + 2 * (kMaxBins + 4) * kWidth);
+  const size_t sm1 = sizeof(float) * (kTaps * kWidth * kWidth + 2 * (kMaxBins + 1) * kWidth);
   sparse_grad_kernel<<<B, kSparseThreads, sm1, s>>>(n->dlogit, n->argmax, n->act[0], n->act[1], n->act[2], X,
-                                                    n->wh + n->L[1].woff, n->wh + n->L[2].woff,
+                                                    n->wt + n->L[1].woff, n->wt + n->L[2].woff,
                                                     n->wh + n->L[3].woff, sg);
   FDR_LAUNCH_CHECK("sparse_grad_kernel");
   const size_t sm2 = sizeof(float) * (kMaxBins * kWidth + std::max(n->nt, kWidth) * kMaxInBins);
@@ -647,6 +710,7 @@ static void net_release(fdr_propose_net* n) {
   if (!n) return;
   cudaFree(n->params);
   cudaFree(n->wh);
+  cudaFree(n->wt);
   cudaFree(n->m);
   cudaFree(n->v);
   cudaFree(n->grad);
@@ -703,6 +767,7 @@ int fdr_propose_create(fdr_propose_net** out, int nbins, int nt, int width, int 
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = cudaMalloc(&n->params, sizeof(float) * off);
   if (e == cudaSuccess) e = cudaMalloc(&n->wh, sizeof(__half) * off);
+  if (e == cudaSuccess) e = cudaMalloc(&n->wt, sizeof(float) * off);
   if (e == cudaSuccess) e = cudaMalloc(&n->m, sizeof(float) * off);
   if (e == cudaSuccess) e = cudaMalloc(&n->v, sizeof(float) * off);
   if (e == cudaSuccess) e = cudaMalloc(&n->grad, sizeof(float) * off);
@@ -722,7 +787,7 @@ int fdr_propose_create(fdr_propose_net** out, int nbins, int nt, int width, int 
     net_release(n);
     return st2;
   }
-  to_half_kernel<<<(unsigned)cdiv(off, 256), 256>>>(n->params, n->wh, off);
+  to_half_kernel<<<(unsigned)cdiv(off, 256), 256>>>(n->params, n->wh, n->wt, layer_order(n), off);
   e = cudaDeviceSynchronize();
   if (e != cudaSuccess) { int st2 = cuda_status(e, "fdr_propose_create"); net_release(n); return st2; }
   count_launch();
@@ -784,8 +849,8 @@ int fdr_propose_train_step(fdr_propose_net* n, const float* x, const float* labe
   n->step += 1;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   const float c1 = 1.f - powf(b1, (float)n->step), c2 = 1.f - powf(b2, (float)n->step);
-  adam_kernel<<<(unsigned)cdiv(n->nparams, 256), 256, 0, s>>>(n->params, n->grad, n->m, n->v, n->wh,
-                                                               n->nparams, lr, b1, b2, eps, c1, c2);
+  adam_kernel<<<(unsigned)cdiv(n->nparams, 256), 256, 0, s>>>(n->params, n->grad, n->m, n->v, n->wh, n->wt,
+                                                               layer_order(n), n->nparams, lr, b1, b2, eps, c1, c2);
   FDR_LAUNCH_CHECK("adam_kernel");
   if (loss_out) FDR_CUDA(cudaMemcpyAsync(loss_out, n->loss, sizeof(float), cudaMemcpyDeviceToDevice, s));
   return FDR_OK;
@@ -810,7 +875,7 @@ int fdr_propose_set_state(fdr_propose_net* n, const float* params, const float* 
   if (m) FDR_CUDA(cudaMemcpy(n->m, m, sizeof(float) * n->nparams, cudaMemcpyHostToDevice));
   if (v) FDR_CUDA(cudaMemcpy(n->v, v, sizeof(float) * n->nparams, cudaMemcpyHostToDevice));
   n->step = step;
-  to_half_kernel<<<(unsigned)cdiv(n->nparams, 256), 256>>>(n->params, n->wh, n->nparams);
+  to_half_kernel<<<(unsigned)cdiv(n->nparams, 256), 256>>>(n->params, n->wh, n->wt, layer_order(n), n->nparams);
   FDR_LAUNCH_CHECK("to_half_kernel");
   FDR_CUDA(cudaDeviceSynchronize());
   return FDR_OK;
