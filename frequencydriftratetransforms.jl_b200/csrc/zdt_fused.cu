@@ -178,98 +178,113 @@ zdtf_input_kernel(const float* __restrict__ spec, long long N, int Nt, int Q,
 //   X[k1b + 32 k1a] = sum_nb1 w64^(k1a nb1) [w^(k1b nb1) sum_nb2 x[nb1 + 64 nb2] w32^(k1b nb2)]
 // with w = exp(-2 pi i / P).  Thread (seq, nb1) loads its 32 values of the two packed time
 // steps straight from the spectrogram and transforms them over nb2; lanes h and h + 16 then
-// share the 64-point DFT over nb1 (decimation in time: lane h takes nb1 = 2k + h, lane 1
-// applies w64^n, one shuffle exchange), and A is stored with the inter-pass twiddle
-// exp(-2 pi i k1 n_a / Nf) from a two-level table in shared memory.  Shared-memory strides
-// as in the output kernel (S1 = 33, SSEQ = 2 mod 16): conflict-free transposes.
+// share the 64-point DFT over nb1 (decimation in time: lane h takes nb1 = 2k + h, the O values
+// take w64^n, one shuffle exchange), and A is stored with the inter-pass twiddle
+// exp(-2 pi i k1 n_a / Nf) = exp(-2 pi i k1b n_a / Nf) exp(-2 pi i 32 k1a n_a / Nf): the first
+// factor once per thread, the second from a table of the tile (8 residues x 64), both from exact
+// phases (a two-level table by k1 n_a took 64-bit products and scattered shared-memory loads for
+// every element).  Persistent CTAs walk the (residues, time pair) tiles.  At Nf = 2^20, Nt = 16:
+// 64 -> 48 us (134 MB read and written, 2.8 TB/s); an L2 prefetch of the next tile (50 us) and its
+// first column by cp.async into shared memory (55 us) were slower: the loads and stores of 32-
+// and 64-byte rows keep the load/store queue full, not their latency.
+// Shared-memory strides as in the output kernel (S1 = 33, SSEQ = 2 mod 16): conflict-free
+// transposes.
 struct In64Shape {
   static constexpr int P1 = 64, P2 = 32, P = P1 * P2, TS = 8, T = 64 * TS;
   static constexpr int S1 = P2 + 1;
   static constexpr int SSEQ = ((P1 * S1 + 15) / 16) * 16 + 16 / TS;
-  static constexpr size_t REGION = sizeof(float2) * TS * SSEQ;
   static constexpr int TW1 = P1 * S1;  // tw1[nb1][k] = w^(nb1 k), rows S1 apart
-  static constexpr size_t smem(int B, long long N) {
-    return REGION + sizeof(float2) * (TW1 + P1 / 2 + (1LL << B) + (N >> B));
-  }
+  static constexpr size_t SMEM = sizeof(float2) * (TS * SSEQ + TW1 + P1 / 2 + P1 * TS);
 };
 
+template <int Q>
 __global__ void __launch_bounds__(In64Shape::T, 1)
-zdtf_input64_kernel(const float* __restrict__ spec, long long N, int Nt, int Q,
-                    float2* __restrict__ A, FusedTables tab) {
+zdtf_input64_kernel(const float* __restrict__ spec, long long N, int Nt, int NP, float2* __restrict__ A,
+                    const float2* __restrict__ rootsP) {
   using SH = In64Shape;
   constexpr int P = SH::P, P1 = SH::P1, P2 = SH::P2, TS = SH::TS, S1 = SH::S1, SSEQ = SH::SSEQ;
   extern __shared__ float2 sm[];
   float2* region = sm;           // TS * SSEQ: the transpose
-  float2* tw1 = sm + TS * SSEQ;  // w^(nb1 k): P1 rows of S1
+  float2* tw1 = sm + TS * SSEQ;  // w^(nb1 k): P1 rows of S1; rows 3 (mod 4) negated, see pass 2
   float2* tw2 = tw1 + SH::TW1;   // w64^n, n < P1 / 2
-  const int nlo = 1 << tab.B, nhi = (int)(N >> tab.B);
-  float2* tlo = tw2 + P1 / 2;  // exp(-2 pi i m / N), m < 2^B
-  float2* thi = tlo + nlo;     // exp(-2 pi i m 2^B / N), m < N / 2^B
+  float2* ta = tw2 + P1 / 2;     // exp(-2 pi i 32 k1a n_a / Nf): [k1a][seq]
   const int tid = threadIdx.x;
-  for (int i = tid; i < P; i += SH::T)
-    tw1[(i / P2) * S1 + i % P2] = __ldg(tab.rootsP + (((i / P2) * (i % P2)) & (P - 1)));
-  for (int i = tid; i < P1 / 2; i += SH::T) tw2[i] = __ldg(tab.rootsP + i * (P / P1));
-  for (int i = tid; i < nlo; i += SH::T) tlo[i] = __ldg(tab.tw_lo + i);
-  for (int i = tid; i < nhi; i += SH::T) thi[i] = __ldg(tab.tw_hi + i);
-  const int na0 = blockIdx.x * TS;
-  const int p = blockIdx.y;
-  const float* c0 = spec + (long long)(2 * p) * N;
-  const bool has1 = (2 * p + 1) < Nt;
-  const float* c1 = spec + (long long)(2 * p + 1) * N;
-  // pass 1: thread (seq, nb1), all 32 loads of each column issued before any is used
+  for (int i = tid; i < P; i += SH::T) {
+    const float2 w = __ldg(rootsP + (((i / P2) * (i % P2)) & (P - 1)));
+    tw1[(i / P2) * S1 + i % P2] = (i / P2) % 4 == 3 ? make_float2(-w.x, -w.y) : w;
+  }
+  for (int i = tid; i < P1 / 2; i += SH::T) tw2[i] = __ldg(rootsP + i * (P / P1));
+  constexpr unsigned long long kTurn = ~0ull / ((unsigned long long)P * Q) + 1;  // 2^64 / Nf
+  constexpr int ntna = Q / TS;
+  const int ntiles = ntna * NP;
+  // pass 1: thread (seq, nb1); pass 2: lane = seq + TS * (k1b mod (16 / TS)) + 16 * h
   const int seq1 = tid % TS, nb1 = tid / TS;
-  float2 v[P2];
-  {
-    const long long n0 = (long long)(na0 + seq1) + (long long)Q * nb1;
-    const long long st = (long long)Q * P1;
-#pragma unroll
-    for (int m = 0; m < P2; ++m) v[m].x = FDR_DBG_OK(n0 + st * m < N) ? __ldcs(c0 + n0 + st * m) : 0.f;
-#pragma unroll
-    for (int m = 0; m < P2; ++m) v[m].y = (has1 && FDR_DBG_OK(n0 + st * m < N)) ? __ldcs(c1 + n0 + st * m) : 0.f;
-  }
-  __syncthreads();  // the tables are in shared memory
-  Dft<P2>::run(v, -1);
-  {
-    float2* b = region + seq1 * SSEQ + nb1 * S1;
-    const float2* t1 = tw1 + nb1 * S1;
-#pragma unroll
-    for (int k = 0; k < P2; ++k) b[k] = cmul(v[k], t1[k]);
-  }
-  __syncthreads();
-  // pass 2: lane = seq + TS * (k1b mod (16 / TS)) + 16 * h
   const int lane = tid & 31;
   const int seq2 = lane % TS, h = lane >> 4;
   const int k1b = ((lane / TS) % (16 / TS)) + (16 / TS) * (tid >> 5);
-  {
-    const float2* b = region + seq2 * SSEQ + h * S1 + k1b;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int na0 = (tile % ntna) * TS, p = tile / ntna;
+    const bool has1 = (2 * p + 1) < Nt;
+    float2 v[P2];
+    {
+      // all 32 loads of each column issued before any is used
+      const float* const c0 = spec + (long long)(2 * p) * N + na0 + seq1 + Q * nb1;
+      const float* const c1 = has1 ? c0 + N : c0;
 #pragma unroll
-    for (int k = 0; k < P1 / 2; ++k) v[k] = b[2 * k * S1];
-  }
-  Dft<P1 / 2>::run(v, -1);  // E (h = 0) or O (h = 1) at n mod 32
-  // lane 0-half keeps E[0..15] and receives O[0..15]; lane 1-half keeps O[16..31] and
-  // receives E[16..31]; each applies w64^n to its 16 O values:
-  // X[n] = E[n] + w64^n O[n], X[n + 32] = E[n] - w64^n O[n]
+      for (int m = 0; m < P2; ++m)
+        v[m].x = FDR_DBG_OK(na0 + seq1 + Q * (nb1 + P1 * m) < N) ? __ldcs(c0 + Q * P1 * m) : 0.f;
 #pragma unroll
-  for (int i = 0; i < P1 / 4; ++i) {
-    const float2 s = h ? v[i] : v[i + P1 / 4];
-    float2 o;
-    o.x = __shfl_xor_sync(0xffffffffu, s.x, 16);
-    o.y = __shfl_xor_sync(0xffffffffu, s.y, 16);
-    const float2 e = h ? o : v[i];
-    const float2 w = cmul(h ? v[i + P1 / 4] : o, tw2[i + (P1 / 4) * h]);
-    v[i] = cadd(e, w);           // k1a = i + 16h
-    v[i + P1 / 4] = csub(e, w);  // k1a = i + 16h + 32
-  }
-  const int na = na0 + seq2;
-  float2* a0 = A + (long long)p * P * Q + na;
+      for (int m = 0; m < P2; ++m)
+        v[m].y = FDR_DBG_OK(na0 + seq1 + Q * (nb1 + P1 * m) < N) ? __ldcs(c1 + Q * P1 * m) : 0.f;
+    }
+    {
+      const unsigned long long na = (unsigned)(na0 + seq1);
+      ta[nb1 * TS + seq1] = cconj(cis_turn(na * (unsigned)(P2 * nb1) * kTurn));  // here nb1 stands for k1a
+    }
+    const float2 tb = cconj(cis_turn((unsigned long long)(unsigned)(na0 + seq2) * (unsigned)k1b * kTurn));
+    if (!has1) {
 #pragma unroll
-  for (int i = 0; i < P1 / 2; ++i) {
-    const int k1a = (i & (P1 / 4 - 1)) + 16 * h + (i >= P1 / 4 ? P1 / 2 : 0);
-    const int k1 = k1b + P2 * k1a;
-    const long long m = (long long)k1 * na;
-    const float2 t = cmul(thi[m >> tab.B], tlo[m & (nlo - 1)]);
-    if (FDR_DBG_OK((long long)p * P * Q + na + (long long)k1 * Q < (long long)gridDim.y * P * Q))
-      a0[(long long)k1 * Q] = cmul(v[i], t);
+      for (int m = 0; m < P2; ++m) v[m].y = 0.f;
+    }
+    __syncthreads();  // the tables are in shared memory; the last tile's transpose is read
+    Dft<P2>::run(v, -1);
+    {
+      float2* b = region + seq1 * SSEQ + nb1 * S1;
+      const float2* t1 = tw1 + nb1 * S1;
+#pragma unroll
+      for (int k = 0; k < P2; ++k) b[k] = cmul(v[k], t1[k]);
+    }
+    __syncthreads();
+    {
+      const float2* b = region + seq2 * SSEQ + h * S1 + k1b;
+#pragma unroll
+      for (int k = 0; k < P1 / 2; ++k) v[k] = b[2 * k * S1];
+    }
+    Dft<P1 / 2>::run(v, -1);  // E at n (h = 0) or O at n + 16 mod 32 (h = 1: its odd inputs are negated)
+    // Both lanes keep v[0..15] and send v[16..31]: lane 0 holds E[0..15] and receives O[0..15],
+    // lane 1 holds O[16..31] and receives E[16..31]; each applies w64^n to its 16 O values:
+    // X[n] = E[n] + w64^n O[n], X[n + 32] = E[n] - w64^n O[n]
+#pragma unroll
+    for (int i = 0; i < P1 / 4; ++i) {
+      float2 o;
+      o.x = __shfl_xor_sync(0xffffffffu, v[i + P1 / 4].x, 16);
+      o.y = __shfl_xor_sync(0xffffffffu, v[i + P1 / 4].y, 16);
+      const float2 e = h ? o : v[i];
+      const float2 w = cmul(h ? v[i] : o, tw2[i + (P1 / 4) * h]);
+      v[i] = cadd(e, w);           // k1a = i + 16h
+      v[i + P1 / 4] = csub(e, w);  // k1a = i + 16h + 32
+    }
+    const int na = na0 + seq2;
+    float2* const a0 = A + (long long)p * P * Q + na + Q * (k1b + P2 * 16 * h);
+    const float2* const t0 = ta + 16 * h * TS + seq2;
+#pragma unroll
+    for (int i = 0; i < P1 / 2; ++i) {
+      const int k1a = (i & (P1 / 4 - 1)) + (i >= P1 / 4 ? P1 / 2 : 0);  // and 16h in the bases
+      const float2 t = cmul(tb, t0[k1a * TS]);
+      if (FDR_DBG_OK((long long)p * P * Q + na + (long long)Q * (k1b + P2 * (16 * h + k1a)) < (long long)NP * P * Q))
+        a0[Q * P2 * k1a] = cmul(v[i], t);
+    }
+    __syncthreads();  // ta and the transpose are read
   }
 }
 // ------------------------------------------------------------------------------------
@@ -1669,16 +1684,12 @@ __global__ void bounded_wait_selftest_kernel(unsigned long long limit_ns) {
 // FDR store of one row of a rate pair through lane pairs: v = (rate j, rate j + 1) values of
 // this lane's channel; lanes 2s and 2s + 1 hold adjacent channels, so the even lane writes
 // both channels of rate j and the odd lane both of rate j + 1 as one 8-byte streaming store
-// each (half the store instructions of per-lane scalar stores).  Every lane of the warp
-// must call it; d0 is this lane's element of rate j, d1 = d0 + Nf.
-__device__ __forceinline__ void store_rate_pair(float* d0, float* d1, float2 v, bool odd, bool has1,
-                                                const float* dlo, const float* dhi) {
+// each.  Every lane of the warp must call it; p is the even lane's element of rate j or the
+// element before the odd lane's of rate j + 1, live: that rate exists.
+__device__ __forceinline__ void store_rate_pair(float* p, float2 v, bool odd, bool live, const float* dlo, const float* dhi) {
   const float recv = __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
-  if (!odd) {
-    if (FDR_DBG_OK(d0 >= dlo && d0 + 2 <= dhi)) __stcs(reinterpret_cast<float2*>(d0), make_float2(v.x, recv));
-  } else if (has1) {
-    if (FDR_DBG_OK(d1 - 1 >= dlo && d1 + 1 <= dhi)) __stcs(reinterpret_cast<float2*>(d1 - 1), make_float2(recv, v.y));
-  }
+  if (live && FDR_DBG_OK(p >= dlo && p + 2 <= dhi))
+    __stcs(reinterpret_cast<float2*>(p), make_float2(odd ? recv : v.x, odd ? v.y : recv));
 }
 
 // 2-D tiled TMA load (no multicast) of box {x .. x+15 floats, y .. y+255 rows} into dst.
@@ -1717,10 +1728,13 @@ struct OutTmaShape {
   static constexpr int MINB = 2;  // CTAs per SM
 };
 
-template <int P1, int P2, int TS>
+// Q is a template parameter: tile numbers split by shifts and a thread's FDR rows lie at constant
+// distances.  (With the 64-bit division, row addresses and a store for each lane parity the P =
+// 2048 kernel below executed 135 M warp instructions at Nf = 2^20, 129 rates, now 82 M: 238 ->
+// 222 us, 1.09 GB read and written, 4.9 TB/s.)
+template <int P1, int P2, int TS, int Q>
 __global__ void __launch_bounds__(OutTmaShape<P1, P2, TS>::T, OutTmaShape<P1, P2, TS>::MINB)
-zdtf_output_tma_kernel(const __grid_constant__ CUtensorMap wmap, long long N, int Q, int Nr,
-                        int npairs, float* __restrict__ dest, const float2* __restrict__ rootsP,
+zdtf_output_tma_kernel(const __grid_constant__ CUtensorMap wmap, long long N, int Nr, int npairs, float* __restrict__ dest, const float2* __restrict__ rootsP,
                         double* __restrict__ acc) {
   using SH = OutTmaShape<P1, P2, TS>;
   constexpr int P = SH::P, S1 = SH::S1, SSEQ = SH::SSEQ;
@@ -1730,33 +1744,33 @@ zdtf_output_tma_kernel(const __grid_constant__ CUtensorMap wmap, long long N, in
   float2* roots = (float2*)(base + ((SH::REGION + 127) / 128) * 128);
   unsigned long long* bar = (unsigned long long*)(roots + P);
   const int tid = threadIdx.x;
-  const int ntna = Q / TS;
-  const long long ntiles = (long long)ntna * npairs;
+  constexpr int ntna = Q / TS;
+  const int ntiles = ntna * npairs;
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (int i = tid; i < P; i += SH::T) roots[i] = __ldg(rootsP + i);
   __syncthreads();
-  auto issue = [&](long long tile) {  // thread 0 only
-    const int q = (int)(tile / ntna), nat = (int)(tile - (long long)q * ntna);
+  auto issue = [&](int tile) {  // thread 0 only
+    const int q = tile / ntna, nat = tile % ntna;
     mbar_expect_tx(&bar[0], SH::TILEB);
 #pragma unroll
     for (int b = 0; b < SH::NBOX; ++b)
       tma_load_2d(region + b * SH::BOXR * TS, &wmap, 2 * TS * nat, q * P + b * SH::BOXR, &bar[0]);
   };
-  const long long first = blockIdx.x, stride = gridDim.x;
+  const int first = blockIdx.x, stride = gridDim.x;
   if (tid == 0 && first < ntiles) issue(first);
   const int seq = tid % TS;
   const int r = tid / TS;
   int it = 0;
-  for (long long tile = first; tile < ntiles; tile += stride, ++it) {
+  for (int tile = first; tile < ntiles; tile += stride, ++it) {
     const bool ok = mbar_wait_bounded(&bar[0], (unsigned)(it & 1));
     if (__syncthreads_or(!ok)) {
       if (tid == 0) atomicOr(&g_fused_fault, 1);
       return;
     }
-    const int q = (int)(tile / ntna), nat = (int)(tile - (long long)q * ntna);
+    const int q = tile / ntna, nat = tile % ntna;
     const int na0 = nat * TS;
     float2 v[P2];
     if (r < P1) {
@@ -1791,13 +1805,11 @@ zdtf_output_tma_kernel(const __grid_constant__ CUtensorMap wmap, long long N, in
     static_assert(SH::T == TS * P2 && TS % 2 == 0, "every lane stores, channel pairs in lane pairs");
     if (r < P2) {
       Dft<P1>::run(w, +1);
-      float* d0 = dest + (long long)j * N + na0 + seq + (long long)Q * r;
-      float* d1 = d0 + N;
+      const bool odd = seq & 1;
+      float* const d = dest + (long long)(j + odd) * N + na0 + (seq & ~1) + Q * r;
 #pragma unroll
-      for (int nba = 0; nba < P1; ++nba) {
-        const long long off = (long long)Q * P2 * nba;
-        store_rate_pair(d0 + off, d1 + off, w[nba], seq & 1, has1, dest, dest + N * (long long)Nr);
-      }
+      for (int nba = 0; nba < P1; ++nba)
+        store_rate_pair(d + Q * P2 * nba, w[nba], odd, !odd || has1, dest, dest + N * (long long)Nr);
       if (acc) {
 #pragma unroll
         for (int nba = 0; nba < P1; ++nba) {
@@ -1831,9 +1843,12 @@ zdtf_output_tma_kernel(const __grid_constant__ CUtensorMap wmap, long long N, in
 // 64 B = 128 KB, one CTA of 512 threads per SM; tiles of 4 residues, 32-byte rows, two
 // CTAs per SM, measured 4x slower).  Pass 1: thread (seq, k1a < 64) transforms its 32
 // values over k1b.  Pass 2 (the 64-point DFT over k1a) is split between lanes h = 0, 1 of a
-// warp (decimation in time): lane h transforms the 32 values k1a = 2k + h, lane 1 applies
+// warp (decimation in time): lane h transforms the 32 values k1a = 2k + h, the O values take
 // w_64^n, and the two exchange half of their results by shuffles, so every lane ends with
 // 32 of the 64 outputs.
+// (Fetching the tile as two halves, the first into a buffer of its own while the tile before is
+// still transformed, measured the same, 225 against 222 us at Nf = 2^20, 129 rates: the fetch is
+// not what bounds the pass.)
 // Shared-memory strides: S1 = 33 (odd) and SSEQ = 16/TS (mod 16) keep the transposed
 // writes of pass 1 (TS seq x 16/TS k1a per half-warp) and the reads of pass 2 (TS seq x
 // 16/TS nb_b per half-warp, h fixed) on distinct bank pairs.
@@ -1854,10 +1869,9 @@ struct OutTma64Shape {
   static constexpr int MINB = TS <= 4 ? 2 : 1;
 };
 
-template <int TS_>
+template <int TS_, int Q>
 __global__ void __launch_bounds__(OutTma64Shape<TS_>::T, OutTma64Shape<TS_>::MINB)
-zdtf_output_tma64_kernel(const __grid_constant__ CUtensorMap wmap, long long N, int Q, int Nr,
-                         int npairs, float* __restrict__ dest, const float2* __restrict__ rootsP,
+zdtf_output_tma64_kernel(const __grid_constant__ CUtensorMap wmap, long long N, int Nr, int npairs, float* __restrict__ dest, const float2* __restrict__ rootsP,
                          double* __restrict__ acc) {
   using SH = OutTma64Shape<TS_>;
   constexpr int P = SH::P, P1 = SH::P1, P2 = SH::P2, TS = SH::TS, S1 = SH::S1, SSEQ = SH::SSEQ;
@@ -1868,24 +1882,28 @@ zdtf_output_tma64_kernel(const __grid_constant__ CUtensorMap wmap, long long N, 
   float2* tw2 = tw1 + SH::TW1;                                          // P1 / 2
   unsigned long long* bar = (unsigned long long*)(tw2 + P1 / 2);
   const int tid = threadIdx.x;
-  const int ntna = Q / TS;
-  const long long ntiles = (long long)ntna * npairs;
+  constexpr int ntna = Q / TS;
+  const int ntiles = ntna * npairs;
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int i = tid; i < P; i += SH::T)
-    tw1[(i / P2) * S1 + i % P2] = cconj(__ldg(rootsP + (((i / P2) * (i % P2)) & (P - 1))));
+  for (int i = tid; i < P; i += SH::T) {
+    const float2 w = cconj(__ldg(rootsP + (((i / P2) * (i % P2)) & (P - 1))));
+    // rows k1a = 3 (mod 4) negated: lane h = 1's odd inputs in pass 2, whose DFT then comes out
+    // rotated by half its length
+    tw1[(i / P2) * S1 + i % P2] = (i / P2) % 4 == 3 ? make_float2(-w.x, -w.y) : w;
+  }
   for (int i = tid; i < P1 / 2; i += SH::T) tw2[i] = cconj(__ldg(rootsP + i * (P / P1)));
   __syncthreads();
-  auto issue = [&](long long tile) {  // thread 0 only
-    const int q = (int)(tile / ntna), nat = (int)(tile - (long long)q * ntna);
+  auto issue = [&](int tile) {  // thread 0 only
+    const int q = tile / ntna, nat = tile % ntna;
     mbar_expect_tx(&bar[0], SH::TILEB);
 #pragma unroll
     for (int b = 0; b < SH::NBOX; ++b)
       tma_load_2d(region + b * SH::BOXR * TS, &wmap, 2 * TS * nat, q * P + b * SH::BOXR, &bar[0]);
   };
-  const long long first = blockIdx.x, stride = gridDim.x;
+  const int first = blockIdx.x, stride = gridDim.x;
   if (tid == 0 && first < ntiles) issue(first);
   // pass 1 roles
   const int seq1 = tid % TS, r = tid / TS;  // r = k1a < 64
@@ -1894,13 +1912,13 @@ zdtf_output_tma64_kernel(const __grid_constant__ CUtensorMap wmap, long long N, 
   const int seq2 = lane % TS, h = lane >> 4;
   const int nbb = ((lane / TS) % (16 / TS)) + (16 / TS) * (tid >> 5);
   int it = 0;
-  for (long long tile = first; tile < ntiles; tile += stride, ++it) {
+  for (int tile = first; tile < ntiles; tile += stride, ++it) {
     const bool ok = mbar_wait_bounded(&bar[0], (unsigned)(it & 1));
     if (__syncthreads_or(!ok)) {
       if (tid == 0) atomicOr(&g_fused_fault, 1);
       return;
     }
-    const int q = (int)(tile / ntna), nat = (int)(tile - (long long)q * ntna);
+    const int q = tile / ntna, nat = tile % ntna;
     const int na0 = nat * TS;
     float2 v[P2];
 #pragma unroll
@@ -1924,18 +1942,17 @@ zdtf_output_tma64_kernel(const __grid_constant__ CUtensorMap wmap, long long N, 
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       issue(tile + stride);
     }
-    Dft<P1 / 2>::run(v, +1);  // E (h = 0) or O (h = 1) at n mod 32
-    // lane 0-half keeps E[0..15] and receives O[0..15]; lane 1-half keeps O[16..31] and
-    // receives E[16..31]; each applies w^n to its 16 O values:
+    Dft<P1 / 2>::run(v, +1);  // E at n (h = 0) or O at n + 16 mod 32 (h = 1)
+    // Both lanes keep v[0..15] and send v[16..31]: lane 0 holds E[0..15] and receives O[0..15],
+    // lane 1 holds O[16..31] and receives E[16..31]; each applies w^n to its 16 O values:
     // z[n] = E[n] + w^n O[n], z[n + 32] = E[n] - w^n O[n]
 #pragma unroll
     for (int i = 0; i < P1 / 4; ++i) {
-      const float2 s = h ? v[i] : v[i + P1 / 4];
       float2 o;
-      o.x = __shfl_xor_sync(0xffffffffu, s.x, 16);
-      o.y = __shfl_xor_sync(0xffffffffu, s.y, 16);
+      o.x = __shfl_xor_sync(0xffffffffu, v[i + P1 / 4].x, 16);
+      o.y = __shfl_xor_sync(0xffffffffu, v[i + P1 / 4].y, 16);
       const float2 e = h ? o : v[i];
-      const float2 w = cmul(h ? v[i + P1 / 4] : o, tw2[i + (P1 / 4) * h]);
+      const float2 w = cmul(h ? v[i] : o, tw2[i + (P1 / 4) * h]);
       v[i] = cadd(e, w);             // z[i + 16h]
       v[i + P1 / 4] = csub(e, w);    // z[i + 16h + 32]
     }
@@ -1943,14 +1960,12 @@ zdtf_output_tma64_kernel(const __grid_constant__ CUtensorMap wmap, long long N, 
     const bool has1 = (j + 1) < Nr;
     double m[4] = {0.0, 0.0, 0.0, 0.0};
     {
-      float* d0 = dest + (long long)j * N + na0 + seq2 + (long long)Q * nbb;
-      float* d1 = d0 + N;
+      const bool odd = seq2 & 1;
+      float* const d = dest + (long long)(j + odd) * N + na0 + (seq2 & ~1) + Q * (nbb + P2 * 16 * h);
 #pragma unroll
-      for (int i = 0; i < P1 / 2; ++i) {
-        const int nba = (i & (P1 / 4 - 1)) + 16 * h + (i >= P1 / 4 ? P1 / 2 : 0);
-        const long long off = (long long)Q * P2 * nba;
-        store_rate_pair(d0 + off, d1 + off, v[i], seq2 & 1, has1, dest, dest + N * (long long)Nr);
-      }
+      for (int i = 0; i < P1 / 2; ++i)
+        store_rate_pair(d + Q * P2 * ((i & (P1 / 4 - 1)) + (i >= P1 / 4 ? P1 / 2 : 0)), v[i], odd, !odd || has1,
+                        dest, dest + N * (long long)Nr);
       if (acc) {
 #pragma unroll
         for (int i = 0; i < P1 / 2; ++i) {
@@ -2709,14 +2724,20 @@ static int set_smem_attrs() {
                                 (int)OutMmaShape::SMEM));
   FDR_CUDA(cudaFuncSetAttribute(zdtf_output_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)OutUmmaShape::SMEM));
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_output_tma_kernel<32, 32, 8>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)OutTmaShape<32, 32, 8>::SMEM));
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_output_tma64_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+#define SET_OUT(Q)                                                                             \
+  FDR_CUDA(cudaFuncSetAttribute(zdtf_output_tma_kernel<32, 32, 8, Q>,                          \
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
+                                (int)OutTmaShape<32, 32, 8>::SMEM));                           \
+  FDR_CUDA(cudaFuncSetAttribute(zdtf_output_tma64_kernel<8, Q>,                                \
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
                                 (int)OutTma64Shape<8>::SMEM));
-  // P = 2048 input: Nf = 2^20 or 2^21, table split B = 10 or 11
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_input64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)In64Shape::smem(11, 1LL << 21)));
+  SET_OUT(256) SET_OUT(512) SET_OUT(1024)
+#undef SET_OUT
+#define SET_IN(Q)                                                                              \
+  FDR_CUDA(cudaFuncSetAttribute(zdtf_input64_kernel<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                (int)In64Shape::SMEM));
+  SET_IN(256) SET_IN(512) SET_IN(1024)
+#undef SET_IN
 #define SET_ATTR(kernel, bytes) \
   FDR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes)));
 #define SET_B(Q)                                                                               \
@@ -2805,12 +2826,16 @@ int64_t fused_W_elems(const FusedPlan* st) { return st->N * st->npairs; }
 
 int fused_input(const FusedPlan* st, const float* spec, float2* A, cudaStream_t s) {
   const int P = st->P, Q = st->Q;
-  if (P == 2048 && Q >= In64Shape::TS) {
-    zdtf_input64_kernel<<<dim3(Q / In64Shape::TS, (unsigned)st->NP), In64Shape::T,
-                          In64Shape::smem(st->B, st->N), s>>>(spec, st->N, (int)st->Nt, Q, A, st->tab);
-    FDR_LAUNCH_CHECK("zdtf_input64_kernel");
-    return FDR_OK;
+#define LAUNCH_IN(QQ)                                                                          \
+  if (P == 2048 && Q == QQ) {                                                                  \
+    const int grid = (int)std::min<int64_t>(Q / In64Shape::TS * st->NP, sm_count());           \
+    zdtf_input64_kernel<QQ><<<grid, In64Shape::T, In64Shape::SMEM, s>>>(                       \
+        spec, st->N, (int)st->Nt, (int)st->NP, A, st->tab.rootsP);                             \
+    FDR_LAUNCH_CHECK("zdtf_input64_kernel");                                                   \
+    return FDR_OK;                                                                             \
   }
+  LAUNCH_IN(256) LAUNCH_IN(512) LAUNCH_IN(1024)  // the Q of P = 2048 (fused_qlog)
+#undef LAUNCH_IN
 #define LAUNCH_A(PP)                                                                           \
   if (P == PP) {                                                                               \
     constexpr int TA = AcShape<PP>::TILE, T = AcShape<PP>::T;                                  \
@@ -3073,28 +3098,28 @@ int fused_output_mixed(const FusedPlan* st, const float2* W, float* dest, double
 
 int fused_output(const FusedPlan* st, const float2* W, float* dest, double* acc, cudaStream_t s) {
   const int P = st->P, Q = st->Q;
-  if (P == 1024 && Q >= 8 && tma_output_enabled()) {
+  // P = 1024 or 2048: Q is 256 to 1024 (fused_qlog)
+  if ((P == 1024 || P == 2048) && tma_output_enabled()) {
     CUtensorMap map;
     if (w_tensor_map(&map, W, Q, st->npairs * (int64_t)P, 8)) {
       const long long ntiles = (long long)(Q / 8) * st->npairs;
-      using SH = OutTmaShape<32, 32, 8>;
-      const int grid = (int)std::min<long long>(ntiles, (long long)SH::MINB * sm_count());
-      zdtf_output_tma_kernel<32, 32, 8><<<grid, SH::T, SH::SMEM, s>>>(
-          map, st->N, Q, (int)st->Nr, (int)st->npairs, dest, st->tab.rootsP, acc);
-      FDR_LAUNCH_CHECK("zdtf_output_tma_kernel");
-      return FDR_OK;
-    }
-  }
-  if (P == 2048 && Q >= 8 && tma_output_enabled()) {
-    CUtensorMap map;
-    using SH = OutTma64Shape<8>;
-    if (w_tensor_map(&map, W, Q, st->npairs * (int64_t)P, SH::TS)) {
-      const long long ntiles = (long long)(Q / SH::TS) * st->npairs;
-      const int grid = (int)std::min<long long>(ntiles, (long long)SH::MINB * sm_count());
-      zdtf_output_tma64_kernel<8><<<grid, SH::T, SH::SMEM, s>>>(
-          map, st->N, Q, (int)st->Nr, (int)st->npairs, dest, st->tab.rootsP, acc);
-      FDR_LAUNCH_CHECK("zdtf_output_tma64_kernel");
-      return FDR_OK;
+#define LAUNCH_OUT(PP, QQ, SH, KERNEL)                                                         \
+      if (P == PP && Q == QQ) {                                                                \
+        const int grid = (int)std::min<long long>(ntiles, (long long)SH::MINB * sm_count());   \
+        KERNEL<<<grid, SH::T, SH::SMEM, s>>>(map, st->N, (int)st->Nr, (int)st->npairs, dest,   \
+                                             st->tab.rootsP, acc);                             \
+        FDR_LAUNCH_CHECK(#KERNEL);                                                             \
+        return FDR_OK;                                                                         \
+      }
+      using S1024 = OutTmaShape<32, 32, 8>;
+      using S2048 = OutTma64Shape<8>;
+      LAUNCH_OUT(1024, 256, S1024, (zdtf_output_tma_kernel<32, 32, 8, 256>))
+      LAUNCH_OUT(1024, 512, S1024, (zdtf_output_tma_kernel<32, 32, 8, 512>))
+      LAUNCH_OUT(1024, 1024, S1024, (zdtf_output_tma_kernel<32, 32, 8, 1024>))
+      LAUNCH_OUT(2048, 256, S2048, (zdtf_output_tma64_kernel<8, 256>))
+      LAUNCH_OUT(2048, 512, S2048, (zdtf_output_tma64_kernel<8, 512>))
+      LAUNCH_OUT(2048, 1024, S2048, (zdtf_output_tma64_kernel<8, 1024>))
+#undef LAUNCH_OUT
     }
   }
 #define LAUNCH_C2(PP, P1, P2)                                                                  \
