@@ -1200,10 +1200,11 @@ __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArg
 // them.  Of a super pair's two rate pairs the upper one belongs to rank 0 and the lower one to
 // rank 1 (of a rate subset, one block to each); every CTA writes its sums, at the direct and
 // the mirror positions, into the owner's rate-block buffer through distributed shared memory.
-// One cluster barrier per two blocks makes them visible, then each CTA runs the inverse DFT_Q
-// of its own four rate pairs (8 sequences) and writes W.  The two rate-block buffers alternate,
-// so a CTA may write into its peer's buffer for the next blocks while the peer still
-// transforms the current ones.
+// 256 sum threads take a bin pair and the 4 values of m of one of two blocks; the other 256
+// threads meanwhile run the inverse DFT_Q of the two blocks before (this CTA's four rate pairs,
+// 8 sequences) and write W.  One cluster barrier per two blocks makes the sums visible and frees
+// the other buffer: the two rate-block buffers alternate, and a buffer is written, locally and by
+// the peer, only after the barrier that follows its transform.
 // ------------------------------------------------------------------------------------
 // Forward DFT_Q for a two-CTA cluster (zdtf_czt_cl_kernel): CTA `rank` transforms only the A
 // rows of its own side (PC = 8 t pairs per chunk, 8 sequences in buf) and takes the mirror
@@ -1276,7 +1277,8 @@ __device__ __forceinline__ void czt_forward_cluster(const CztArgs& a, int c, con
 struct CztClShape {
   static constexpr int Q = 512, NT = 64, T = 512;
   static constexpr int QH = Q / 2;                    // bins of one side (one CTA)
-  static constexpr int RG = 2 * T / QH;               // super pairs at a time: 4 (128 bin pairs)
+  static constexpr int H = 256;                       // sum threads: two blocks of 128 bin pairs
+  static constexpr int I = T - H;                     // FFT threads
   static constexpr int SS = b_stride<Q>();
   static constexpr int TWT = 2 * kRatesPerBlock * SS;  // after two 8-sequence buffers
   static constexpr int TWR = TWT + tw_size(Q);
@@ -1289,7 +1291,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CztClShape::T, 1)
 zdtf_czt_cl_kernel(CztArgs a) {
   using SH = CztClShape;
   constexpr int Q = SH::Q, NT = SH::NT, T = SH::T, QH = SH::QH, SS = SH::SS;
-  static_assert(SH::RG == 4, "two blocks of two super pairs at a time");
+  static_assert(SH::H == QH, "two blocks at a time, a bin pair per thread");
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ float2 sm[];
   float2* const buf = sm;  // forward pass: 8 sequences; then two buffers of 8 (two rate blocks)
@@ -1312,72 +1314,80 @@ zdtf_czt_cl_kernel(CztArgs a) {
   auto bin0 = [&](int bp) { return (unsigned long long)k1s[rank] + (unsigned long long)P * (2 * bp); };
   fold_smem<T>(a, reinterpret_cast<float4*>(gs), QH / 2, bin0);
 
-  // thread -> (bin pair bp of this side, super pair rg of every two blocks)
-  const int bp = tid % (QH / 2), rg = tid / (QH / 2);
-  const int side = rank, k20 = 2 * bp;
-  int ms[2], mk2[2];
-  mirror_of(c, side, k20, Q, &ms[0], &mk2[0]);
-  mirror_of(c, side, k20 + 1, Q, &ms[1], &mk2[1]);
-  const bool dc = (c == 0 && side == 0 && k20 == 0);  // lane 0 is the DC bin
-  const float2 win = make_float2(window_value(a, (long long)bin0(bp)), window_value(a, (long long)bin0(bp) + P));
-  const int Nt = a.Nt;
-  FoldPhases fp;
-  fp.setup(bin0(bp), bin0(bp) + (unsigned long long)P, a.ph.Rh, Nt >> 1);
-  const float4* const g = reinterpret_cast<const float4*>(gs) + bp;
-  const float2 zero = make_float2(0.f, 0.f);
-  const int k1a = k1s[0], k1b = k1s[1];
-
   const int blk0 = blockIdx.y * a.blocks_per_group;
   const int blk_end = min(a.nblk, blk0 + a.blocks_per_group);
-  for (int b2 = blk0; b2 < blk_end; b2 += 2) {
-    float2* const hb_local = buf + (((b2 - blk0) >> 1) & 1) * kRatesPerBlock * SS;  // 8 sequences
-    float2* const hb_peer = cluster.map_shared_rank(hb_local, rank ^ 1);
-    float2* const hb0 = rank == 0 ? hb_local : hb_peer;
-    float2* const hb1 = rank == 1 ? hb_local : hb_peer;
-    const int blk = b2 + (rg >> 1);
-    if (SUBSET) {
-      if (blk < blk_end) {
-        const int j = __ldg(a.blk_base + blk) + 4 * (rg & 1);
-        float2* const hb = (rg >> 1) ? hb1 : hb0;
+  const int steps = (blk_end - blk0 + 1) / 2;  // the same in both CTAs: they meet `steps` times below
+
+  if (tid < SH::H) {
+    // ---------------- sum threads: bin pair bp of this side, block bb of every two ----------------
+    const int bp = tid % (QH / 2), bb = tid / (QH / 2);
+    const int side = rank, k20 = 2 * bp;
+    int ms[2], mk2[2];
+    mirror_of(c, side, k20, Q, &ms[0], &mk2[0]);
+    mirror_of(c, side, k20 + 1, Q, &ms[1], &mk2[1]);
+    const bool dc = (c == 0 && side == 0 && k20 == 0);  // lane 0 is the DC bin
+    const float2 win = make_float2(window_value(a, (long long)bin0(bp)), window_value(a, (long long)bin0(bp) + P));
+    const int Nt = a.Nt;
+    FoldPhases fp;
+    fp.setup(bin0(bp), bin0(bp) + (unsigned long long)P, a.ph.Rh, Nt >> 1);
+    const float4* const g = reinterpret_cast<const float4*>(gs) + bp;
+    const float2 zero = make_float2(0.f, 0.f);
+    for (int st = 0; st < steps; ++st) {
+      float2* const hb_local = buf + (st & 1) * kRatesPerBlock * SS;  // 8 sequences
+      float2* const hb_peer = cluster.map_shared_rank(hb_local, rank ^ 1);
+      float2* const hb0 = rank == 0 ? hb_local : hb_peer;
+      float2* const hb1 = rank == 1 ? hb_local : hb_peer;
+      const int blk = blk0 + 2 * st + bb;
+      if (blk < blk_end) {  // uniform over the warp
+        if (SUBSET) {  // block bb belongs to rank bb
+          const int j = __ldg(a.blk_base + blk);
 #pragma unroll 1
-        for (int e = 0; e < 2; ++e) {
-          float2 ax, ay, bx, by;
-          fold_rate_smem(fp, g, QH / 2, Nt, j + 2 * e, a.half, ax, ay);
-          fold_rate_smem(fp, g, QH / 2, Nt, j + 2 * e + 1, a.half, bx, by);
-          put_rate_pair<SS>(hb + 2 * (2 * (rg & 1) + e) * SS, side, k20, ms, mk2, dc, win, ax, ay, bx, by);
+          for (int u = 0; u < kRatesPerBlock / 2; ++u) {
+            float2 ax, ay, bx, by;
+            fold_rate_smem(fp, g, QH / 2, Nt, j + 2 * u, a.half, ax, ay);
+            fold_rate_smem(fp, g, QH / 2, Nt, j + 2 * u + 1, a.half, bx, by);
+            put_rate_pair<SS>((bb ? hb1 : hb0) + 2 * u * SS, side, k20, ms, mk2, dc, win, ax, ay, bx, by);
+          }
+        } else {
+          float2 px[4], py[4], mx[4], my[4];
+          fp.start(blk);
+          fold_pairs_smem<4>(fp, g, QH / 2, Nt, 0, px, py, mx, my);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {  // a super pair past the last one leaves unused sequences
+            const int ja = 2 * (a.half + 2 * blk + i);  // rates past the grid's last: zero
+            if (ja >= a.Nr) px[2 * i] = py[2 * i] = zero;
+            if (ja + 1 >= a.Nr) px[2 * i + 1] = py[2 * i + 1] = zero;
+            const int slot = 2 * (2 * bb + i);
+            put_rate_pair<SS>(hb0 + slot * SS, side, k20, ms, mk2, dc, win, px[2 * i], py[2 * i], px[2 * i + 1], py[2 * i + 1]);
+            put_rate_pair<SS>(hb1 + slot * SS, side, k20, ms, mk2, dc, win, mx[2 * i + 1], my[2 * i + 1], mx[2 * i], my[2 * i]);
+          }
         }
+        if (c == 0 && rank == 0 && bp < kRatesPerBlock)
+          nyquist_block<SUBSET>(a, gnyq, blk, bp, [&](int u, int hh, float v) {
+            float2* const hb = (SUBSET ? bb : u & 1) ? hb1 : hb0;
+            const int slot = SUBSET ? u : 2 * bb + (u >> 1);
+            reinterpret_cast<float*>(hb + (2 * slot) * SS + pidx(Q / 2))[hh] = v;
+          });
       }
-    } else {
-      const int sp = 2 * blk + (rg & 1);
-      if (blk < blk_end && sp < a.half) {  // uniform over the warp (rg is)
-        float2 px[2], py[2], mx[2], my[2];
-        fp.start(blk);
-        fold_pairs_smem<2>(fp, g, QH / 2, Nt, 2 * (rg & 1), px, py, mx, my);
-        const int ja = 2 * (a.half + sp);  // rates past the grid's last: zero
-        if (ja >= a.Nr) px[0] = py[0] = zero;
-        if (ja + 1 >= a.Nr) px[1] = py[1] = zero;
-        put_rate_pair<SS>(hb0 + 2 * rg * SS, side, k20, ms, mk2, dc, win, px[0], py[0], px[1], py[1]);
-        put_rate_pair<SS>(hb1 + 2 * rg * SS, side, k20, ms, mk2, dc, win, mx[1], my[1], mx[0], my[0]);
-      }
+      __syncwarp();
+      cluster.sync();  // both blocks' sums, local and remote, are in the owners' buffers
     }
-    if (c == 0 && rank == 0 && tid < 2 * kRatesPerBlock) {
-      const int bb = tid / kRatesPerBlock;
-      if (b2 + bb < blk_end)
-        nyquist_block<SUBSET>(a, gnyq, b2 + bb, tid % kRatesPerBlock, [&](int u, int hh, float v) {
-          float2* const hb = (SUBSET ? bb : u & 1) ? hb1 : hb0;
-          const int slot = SUBSET ? u : 2 * bb + (u >> 1);
-          reinterpret_cast<float*>(hb + (2 * slot) * SS + pidx(Q / 2))[hh] = v;
-        });
+  } else {
+    // ---------------- FFT threads ----------------
+    const int ltid = tid - SH::H;
+    const int k1a = k1s[0], k1b = k1s[1];
+    for (int st = 0; st < steps; ++st) {
+      cluster.sync();  // the sums of step st are complete (this group's transform of st - 1 is, too)
+      const int b2 = blk0 + 2 * st;
+      group_fft_emit<Q, kRatesPerBlock, SS, SH::I, +1, kBarFft, 1>(
+          buf + (st & 1) * kRatesPerBlock * SS, twt, ltid, [&](int ls, int na, float2 v) {
+            const int lp = ls >> 1, sd = ls & 1;
+            const int b = SUBSET ? b2 + rank : b2 + (lp >> 1);
+            const int p = b < blk_end ? block_pair<SUBSET>(a, b, SUBSET ? lp : 2 * (lp & 1) + rank) : -1;
+            const long long at = ((long long)p * P + (sd ? k1b : k1a)) * Q + na;
+            if (p >= 0 && FDR_DBG_OK(at < (long long)a.npairs * P * Q)) a.W[at] = cmul(v, twr[sd * Q + na]);
+          });
     }
-    cluster.sync();  // both blocks' sums, local and remote, are in the owners' buffers
-    // the inverse DFT_Q of this CTA's four rate pairs; the last pass writes W
-    smem_fft_emit<Q, kRatesPerBlock, SS, T, +1>(hb_local, twt, [&](int ls, int na, float2 v) {
-      const int lp = ls >> 1, sd = ls & 1;
-      const int b = SUBSET ? b2 + rank : b2 + (lp >> 1);
-      const int p = b < blk_end ? block_pair<SUBSET>(a, b, SUBSET ? lp : 2 * (lp & 1) + rank) : -1;
-      const long long at = ((long long)p * P + (sd ? k1b : k1a)) * Q + na;
-      if (p >= 0 && FDR_DBG_OK(at < (long long)a.npairs * P * Q)) a.W[at] = cmul(v, twr[sd * Q + na]);
-    });
   }
 }
 
