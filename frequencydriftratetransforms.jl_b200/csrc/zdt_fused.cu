@@ -883,15 +883,15 @@ __device__ __forceinline__ float2 gs_get(const float2* gs, int Q, int t, int b) 
 // Forward DFT_Q of the CTA's A rows for all t into gs (pair-interleaved F), by all T
 // threads of the block.  HALF: keep only the bins of side own_side (Q/2 bins per row of gs;
 // the DFTs of both sides are still computed, the two-for-one unpacking needs both).
-template <int Q, int NT, int T = CztSmemShape<Q>::T, bool HALF = false>
+// PC time pairs (2 PC sequences in buf) at a time: the more, the fewer barriers and idle threads
+// (at Q = 512 a pass over 8 sequences has half a butterfly of radix 16 per thread).
+template <int Q, int NT, int T = CztSmemShape<Q>::T, bool HALF = false, int PC = 4>
 __device__ __forceinline__ void czt_forward_smem(const CztArgs& a, int c, const int* k1s,
                                                  float2* buf, const float2* twt, float2* gs,
                                                  float2* gnyq, int own_side = 0) {
   constexpr int SS = b_stride<Q>();
-  constexpr int PC = 4;
   constexpr int QROW = HALF ? Q / 2 : Q;  // bins per row of gs
   const int tid = threadIdx.x;
-  for (int i = tid; i < NT * QROW; i += T) gs[i] = make_float2(0.f, 0.f);
   if (c == 0 && tid == 0)
     for (int t = 0; t < NT; ++t) gnyq[t] = make_float2(0.f, 0.f);
   // A rows of chunk p0 (PC t pairs x 2 sides) into registers; the next chunk's loads are
@@ -1108,7 +1108,7 @@ __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArg
     const int side = i / Q, na = i - side * Q;
     twr[i] = cscale(cconj(tw_fwd(a.tab, (long long)k1s[side] * na)), invN);
   }
-  czt_forward_smem<Q, NT, T>(a, c, k1s, buf0, twt, gs, gnyq);  // ends with a barrier
+  czt_forward_smem<Q, NT, T, false, 8>(a, c, k1s, buf0, twt, gs, gnyq);  // ends with a barrier
   auto bin0 = [&](int bp) {
     const int b0 = 2 * bp, side = b0 / (Q / 2);
     return (unsigned long long)k1s[side] + (unsigned long long)P * (b0 - side * (Q / 2));
@@ -1207,7 +1207,7 @@ __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArg
 // the peer, only after the barrier that follows its transform.
 // ------------------------------------------------------------------------------------
 // Forward DFT_Q for a two-CTA cluster (zdtf_czt_cl_kernel): CTA `rank` transforms only the A
-// rows of its own side (PC = 8 t pairs per chunk, 8 sequences in buf) and takes the mirror
+// rows of its own side (PC = 16 t pairs per chunk, in both rate-block buffers) and takes the mirror
 // values of the two-for-one unpacking from the CTA that holds the mirror side (itself for
 // residue pair 0), through distributed shared memory.  Two cluster barriers per chunk: the
 // peer's transforms are complete before they are read, and read before they are replaced.
@@ -1216,10 +1216,9 @@ __device__ __forceinline__ void czt_forward_cluster(const CztArgs& a, int c, con
                                                     const float2* twt, float2* gs, float2* gnyq,
                                                     int rank, cg::cluster_group& cluster) {
   constexpr int SS = b_stride<Q>();
-  constexpr int PC = 8, QH = Q / 2;
+  constexpr int PC = 16, QH = Q / 2;
   constexpr int NE = PC * Q, NL = (NE + T - 1) / T;
   const int tid = threadIdx.x;
-  for (int i = tid; i < NT * QH; i += T) gs[i] = make_float2(0.f, 0.f);
   if (c == 0 && rank == 0 && tid == 0)
     for (int t = 0; t < NT; ++t) gnyq[t] = make_float2(0.f, 0.f);
   const long long k1 = k1s[rank];
