@@ -145,6 +145,34 @@ __device__ __forceinline__ float2 cispi_d(double h) {
 }
 
 // ------------------------------------------------------------------------------------
+// Programmatic dependent launch: a kernel launched by launch_dependent may start while the kernel
+// before it in the stream still runs (once all of that one's CTAs have called let_dependents_start
+// or ended), so that its launch and its prologue overlap that kernel's end.  It calls
+// wait_for_predecessor in every thread before its first access to memory that an earlier kernel
+// writes or reads; that waits for the predecessor to complete with its writes visible, and, as the
+// predecessor did the same or was launched plainly, for everything before it.  Kernels launched
+// plainly pass both calls at once.
+// ------------------------------------------------------------------------------------
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_dependents_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+inline cudaError_t launch_dependent(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                                    cudaStream_t s, A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// ------------------------------------------------------------------------------------
 // Small host utilities
 // ------------------------------------------------------------------------------------
 int64_t nextprod(const int64_t* factors, int nfactors, int64_t n);

@@ -132,6 +132,7 @@ zdtf_input_kernel(const float* __restrict__ spec, long long N, int Nt, int Q,
   constexpr int SS = ac_stride<P, TA>();
   constexpr int TP = TA / 2;  // sequence pairs: each thread moves two adjacent channels
   extern __shared__ float2 sm[];
+  let_dependents_start();
   float2* buf = sm;
   float2* twt = sm + TA * SS;
   const int na0 = blockIdx.x * TA;
@@ -204,6 +205,7 @@ zdtf_input64_kernel(const float* __restrict__ spec, long long N, int Nt, int NP,
   using SH = In64Shape;
   constexpr int P = SH::P, P1 = SH::P1, P2 = SH::P2, TS = SH::TS, S1 = SH::S1, SSEQ = SH::SSEQ;
   extern __shared__ float2 sm[];
+  let_dependents_start();
   float2* region = sm;           // TS * SSEQ: the transpose
   float2* tw1 = sm + TS * SSEQ;  // w^(nb1 k): P1 rows of S1; rows 3 (mod 4) negated, see pass 2
   float2* tw2 = tw1 + SH::TW1;   // w64^n, n < P1 / 2
@@ -668,6 +670,7 @@ __global__ void __launch_bounds__(Q / 2, (Q <= 512 ? 2 : 1)) zdtf_czt_kernel(Czt
   // the factors of m & 3 = 1..3 (real and imaginary parts of exp(2 pi i phi) and of the rotation)
   float2* const pw = buf2 + kRatesPerBlock * SS + threadIdx.x;                     // [3][4][T]
   unsigned long long* const rhs = reinterpret_cast<unsigned long long*>(pw + 12 * T);  // [2][T]
+  let_dependents_start();
   const int tid = threadIdx.x;
   const int c = blockIdx.x;
   const int P = a.P;
@@ -681,6 +684,7 @@ __global__ void __launch_bounds__(Q / 2, (Q <= 512 ? 2 : 1)) zdtf_czt_kernel(Czt
   float2 Gx[NTR], Gy[NTR];  // lanes = the thread's two bins
   {
     float2 G[2][NTR];
+    wait_for_predecessor();
     czt_forward<Q, NTR>(a, c, k1s, buf, twt, gnyq, G);
 #pragma unroll
     for (int t = 0; t < NTR; ++t) {
@@ -981,6 +985,7 @@ __global__ void __launch_bounds__(CztSmemShape<Q>::T, 1) zdtf_czt_smem_kernel(Cz
   float2* twr = twt + tw_size(Q);
   float2* gs = sm + SH::GS_OFF;
   float2* gnyq = gs + NT * Q;
+  let_dependents_start();
   const int tid = threadIdx.x;
   const int c = blockIdx.x;
   const int P = a.P;
@@ -991,6 +996,7 @@ __global__ void __launch_bounds__(CztSmemShape<Q>::T, 1) zdtf_czt_smem_kernel(Cz
     const int side = i / Q, na = i - side * Q;
     twr[i] = cscale(cconj(tw_fwd(a.tab, (long long)k1s[side] * na)), invN);
   }
+  wait_for_predecessor();
   czt_forward_smem<Q, NT>(a, c, k1s, buf, twt, gs, gnyq);
 
   auto bin0 = [&](int bp) {
@@ -1098,6 +1104,7 @@ __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArg
   float2* const twr = sm + SH::TWR;
   float2* const gs = sm + SH::GS_OFF;
   float2* const gnyq = gs + NT * Q;
+  let_dependents_start();
   const int tid = threadIdx.x;
   const int c = blockIdx.x;
   const int P = a.P;
@@ -1108,6 +1115,7 @@ __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArg
     const int side = i / Q, na = i - side * Q;
     twr[i] = cscale(cconj(tw_fwd(a.tab, (long long)k1s[side] * na)), invN);
   }
+  wait_for_predecessor();
   czt_forward_smem<Q, NT, T, false, 8>(a, c, k1s, buf0, twt, gs, gnyq);  // ends with a barrier
   auto bin0 = [&](int bp) {
     const int b0 = 2 * bp, side = b0 / (Q / 2);
@@ -1298,6 +1306,7 @@ zdtf_czt_cl_kernel(CztArgs a) {
   float2* const twr = sm + SH::TWR;
   float2* const gs = sm + SH::GS_OFF;
   float2* const gnyq = gs + NT * QH;
+  let_dependents_start();
   const int tid = threadIdx.x;
   const int rank = (int)cluster.block_rank();  // the side this CTA holds
   const int c = blockIdx.x >> 1;                // residue pair
@@ -1309,6 +1318,7 @@ zdtf_czt_cl_kernel(CztArgs a) {
     const int sd = i / Q, na = i - sd * Q;
     twr[i] = cscale(cconj(tw_fwd(a.tab, (long long)k1s[sd] * na)), invN);
   }
+  wait_for_predecessor();
   czt_forward_cluster<Q, NT, T>(a, c, k1s, buf, twt, gs, gnyq, rank, cluster);
   auto bin0 = [&](int bp) { return (unsigned long long)k1s[rank] + (unsigned long long)P * (2 * bp); };
   fold_smem<T>(a, reinterpret_cast<float4*>(gs), QH / 2, bin0);
@@ -1490,6 +1500,7 @@ zdtf_output_kernel(const float2* __restrict__ W, long long N, int Q, int Nr, flo
   const int q = blockIdx.y;
   for (int i = threadIdx.x; i < tw_size(P); i += T) twt[i] = __ldg(tab.twP + i);
   const float2* w = W + (long long)q * P * Q;
+  wait_for_predecessor();
   static_assert((TP * P) % T == 0, "tile must divide evenly");
   constexpr int NL = TP * P / T;  // loads per thread: all issued before any is consumed
   {
@@ -1579,6 +1590,7 @@ zdtf_output2_kernel(const float2* __restrict__ W, long long N, int Q, int Nr,
   const int seq = threadIdx.x % TS;
   const int r = threadIdx.x / TS;  // k1a in pass 1, nb_b in pass 2
   const float2* w = W + (long long)q * P * Q + na0 + seq;
+  wait_for_predecessor();
   __syncthreads();
   if (r < P1) {
     float2 v[P2];
@@ -1760,6 +1772,7 @@ zdtf_output_tma_kernel(const __grid_constant__ CUtensorMap wmap, long long N, in
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (int i = tid; i < P; i += SH::T) roots[i] = __ldg(rootsP + i);
+  wait_for_predecessor();
   __syncthreads();
   auto issue = [&](int tile) {  // thread 0 only
     const int q = tile / ntna, nat = tile % ntna;
@@ -1904,6 +1917,7 @@ zdtf_output_tma64_kernel(const __grid_constant__ CUtensorMap wmap, long long N, 
     tw1[(i / P2) * S1 + i % P2] = (i / P2) % 4 == 3 ? make_float2(-w.x, -w.y) : w;
   }
   for (int i = tid; i < P1 / 2; i += SH::T) tw2[i] = cconj(__ldg(rootsP + i * (P / P1)));
+  wait_for_predecessor();
   __syncthreads();
   auto issue = [&](int tile) {  // thread 0 only
     const int q = tile / ntna, nat = tile % ntna;
@@ -2833,6 +2847,12 @@ int64_t fused_plan_table_bytes(const FusedPlan* st) {
 int64_t fused_A_elems(const FusedPlan* st) { return st->N * st->NP; }
 int64_t fused_W_elems(const FusedPlan* st) { return st->N * st->npairs; }
 
+// Whether the czt and output kernels may start before the kernel in front has ended: where launches
+// are a good part of the call (Nf = 2^12, 17 rates 20.5 -> 18.6 us; 2^16, 33 rates 31.5 -> 30.7).
+// Larger grids end in partial waves whose SMs the waiting CTAs would hold (2^18, Nt = 32, 257 rates
+// 409 -> 431 us; a batch of 8 channels on four streams 5.21 -> 5.27 ms).
+static bool early_launch(const FusedPlan* st) { return st->N <= (1 << 17); }
+
 int fused_input(const FusedPlan* st, const float* spec, float2* A, cudaStream_t s) {
   const int P = st->P, Q = st->Q;
 #define LAUNCH_IN(QQ)                                                                          \
@@ -2956,8 +2976,8 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
   a.blocks_per_group = (int)cdiv(a.nblk, groups);
   groups = (int)cdiv(a.nblk, a.blocks_per_group);
   if (st->Nt > 32 && Q == CztClShape::Q) {  // F of 64 steps for 512 bins: two-CTA cluster
-    if (blk_base) zdtf_czt_cl_kernel<true><<<dim3(2 * ctas, groups), CztClShape::T, CztClShape::SMEM, s>>>(a);
-    else zdtf_czt_cl_kernel<false><<<dim3(2 * ctas, groups), CztClShape::T, CztClShape::SMEM, s>>>(a);
+    auto kernel = blk_base ? zdtf_czt_cl_kernel<true> : zdtf_czt_cl_kernel<false>;
+    FDR_CUDA(launch_dependent(early_launch(st), kernel, dim3(2 * ctas, groups), CztClShape::T, CztClShape::SMEM, s, a));
     FDR_LAUNCH_CHECK("zdtf_czt_cl_kernel");
     return FDR_OK;
   }
@@ -2968,7 +2988,7 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
 #define LAUNCH_WS(QQ, NN)                                                                      \
     if (Q == QQ && NT == NN) {                                                                 \
       auto kernel = blk_base ? zdtf_czt_ws_kernel<QQ, NN, true> : zdtf_czt_ws_kernel<QQ, NN, false>; \
-      kernel<<<dim3(ctas, groups), CztWsShape<QQ>::T, CztWsShape<QQ>::template smem<NN>(), s>>>(a); \
+      FDR_CUDA(launch_dependent(early_launch(st), kernel, dim3(ctas, groups), CztWsShape<QQ>::T, CztWsShape<QQ>::template smem<NN>(), s, a)); \
       FDR_LAUNCH_CHECK("zdtf_czt_ws_kernel");                                                  \
       return FDR_OK;                                                                           \
     }
@@ -2980,7 +3000,7 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
 #define LAUNCH_BS(QQ, NN)                                                                      \
     if (Q == QQ && NT == NN) {                                                                 \
       auto kernel = blk_base ? zdtf_czt_smem_kernel<QQ, NN, true> : zdtf_czt_smem_kernel<QQ, NN, false>; \
-      kernel<<<dim3(ctas, groups), CztSmemShape<QQ>::T, CztSmemShape<QQ>::template smem<NN>(), s>>>(a); \
+      FDR_CUDA(launch_dependent(early_launch(st), kernel, dim3(ctas, groups), CztSmemShape<QQ>::T, CztSmemShape<QQ>::template smem<NN>(), s, a)); \
       FDR_LAUNCH_CHECK("zdtf_czt_smem_kernel");                                                \
       return FDR_OK;                                                                           \
     }
@@ -2992,7 +3012,7 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
       auto kernel = blk_base ? zdtf_czt_kernel<QQ, kFusedMaxNt, true, true>                    \
                     : window == FDR_WINDOW_RECT ? zdtf_czt_kernel<QQ, kFusedMaxNt, false, false> \
                                                 : zdtf_czt_kernel<QQ, kFusedMaxNt, true, false>; \
-      kernel<<<dim3(ctas, groups), QQ / 2, CztShape<QQ>::SMEM, s>>>(a);                        \
+      FDR_CUDA(launch_dependent(early_launch(st), kernel, dim3(ctas, groups), QQ / 2, CztShape<QQ>::SMEM, s, a));  \
       FDR_LAUNCH_CHECK("zdtf_czt_kernel");                                                     \
       return FDR_OK;                                                                           \
     }
@@ -3115,8 +3135,8 @@ int fused_output(const FusedPlan* st, const float2* W, float* dest, double* acc,
 #define LAUNCH_OUT(PP, QQ, SH, KERNEL)                                                         \
       if (P == PP && Q == QQ) {                                                                \
         const int grid = (int)std::min<long long>(ntiles, (long long)SH::MINB * sm_count());   \
-        KERNEL<<<grid, SH::T, SH::SMEM, s>>>(map, st->N, (int)st->Nr, (int)st->npairs, dest,   \
-                                             st->tab.rootsP, acc);                             \
+        FDR_CUDA(launch_dependent(early_launch(st), KERNEL, grid, SH::T, SH::SMEM, s, map, st->N, (int)st->Nr,   \
+                                  (int)st->npairs, dest, st->tab.rootsP, acc));                \
         FDR_LAUNCH_CHECK(#KERNEL);                                                             \
         return FDR_OK;                                                                         \
       }
@@ -3134,8 +3154,8 @@ int fused_output(const FusedPlan* st, const float2* W, float* dest, double* acc,
 #define LAUNCH_C2(PP, P1, P2)                                                                  \
   if (P == PP) {                                                                               \
     using SH = Out2Shape<P1, P2, 8>;                                                           \
-    zdtf_output2_kernel<P1, P2, 8><<<dim3(Q / 8, (unsigned)st->npairs), SH::T, SH::SMEM, s>>>( \
-        W, st->N, Q, (int)st->Nr, dest, st->tab.rootsP, acc);                                  \
+    FDR_CUDA(launch_dependent(early_launch(st), zdtf_output2_kernel<P1, P2, 8>, dim3(Q / 8, (unsigned)st->npairs), \
+                              SH::T, SH::SMEM, s, W, st->N, Q, (int)st->Nr, dest, st->tab.rootsP, acc)); \
     FDR_LAUNCH_CHECK("zdtf_output2_kernel");                                                   \
     return FDR_OK;                                                                             \
   }
@@ -3148,8 +3168,8 @@ int fused_output(const FusedPlan* st, const float2* W, float* dest, double* acc,
 #define LAUNCH_C(PP)                                                                           \
   if (P == PP) {                                                                               \
     constexpr int TC = AcShape<PP>::TILE, T = AcShape<PP>::T;                                  \
-    zdtf_output_kernel<PP, TC, T><<<dim3(Q / TC, (unsigned)st->npairs), T, AcShape<PP>::SMEM, s>>>( \
-        W, st->N, Q, (int)st->Nr, dest, st->tab, acc);                                         \
+    FDR_CUDA(launch_dependent(early_launch(st), zdtf_output_kernel<PP, TC, T>, dim3(Q / TC, (unsigned)st->npairs), T, \
+                              AcShape<PP>::SMEM, s, W, st->N, Q, (int)st->Nr, dest, st->tab, acc)); \
     FDR_LAUNCH_CHECK("zdtf_output_kernel");                                                    \
     return FDR_OK;                                                                             \
   }
