@@ -76,45 +76,15 @@ __device__ __forceinline__ float2 tw_fwd(const FusedTables& t, long long m) {
   return cmul(__ldg(t.tw_hi + (m >> t.B)), __ldg(t.tw_lo + (m & ((1LL << t.B) - 1))));
 }
 
-// Packed-FP32 helpers (sm_100 FFMA2 / FMUL2 / FADD2): lane 0 and lane 1 carry two independent
-// evaluations, each lane performing exactly the scalar operation sequence.
-__device__ __forceinline__ float2 pk_fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 pk_mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 pk_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 pk_set(float x) { return make_float2(x, x); }
-__device__ __forceinline__ float2 pk_neg(float2 a) { return __fmul2_rn(a, make_float2(-1.f, -1.f)); }
-// (ax + i ay) (bx + i by)
-__device__ __forceinline__ void pk_cmul(float2 ax, float2 ay, float2 bx, float2 by, float2& x, float2& y) {
-  x = pk_fma(ax, bx, pk_mul(pk_neg(ay), by));
-  y = pk_fma(ax, by, pk_mul(ay, bx));
-}
-
 // exp(2 pi i ph / 2^64) for the phases of two bins: the nearest quarter turn is taken off in
-// integers and sin and cos of the rest, x quarter turns with |x| <= 1/2, come from polynomials in
-// x^2 fitted on Chebyshev nodes (degrees 7 and 8; the leading sine coefficient pi/2 is held in two
-// parts).  Errors over all 32-bit phases: 1.4e-8 (sin) and 1.9e-8 (cos) rms, 7.1e-8 at most,
-// against 1.4e-8 and 1.8e-8 rms for correctly rounded values of the rounded argument.  The two
-// bins share packed operations: about 33 instructions for both, where two sincospif with their
-// 64-bit conversions took about 80.
+// integers.  The two bins share packed operations: about 33 instructions for both, where two
+// sincospif with their 64-bit conversions took about 80.
 __device__ __forceinline__ void cis_turn_pk(unsigned long long ph0, unsigned long long ph1, float2& c, float2& s) {
   const int h0 = (int)((ph0 + 0x80000000ull) >> 32), h1 = (int)((ph1 + 0x80000000ull) >> 32);
   const unsigned q0 = ((unsigned)h0 + (1u << 29)) >> 30, q1 = ((unsigned)h1 + (1u << 29)) >> 30;
   const float2 x = pk_mul(make_float2(__int2float_rn(h0 - (int)(q0 << 30)), __int2float_rn(h1 - (int)(q1 << 30))),
                           pk_set(9.31322574615478515625e-10f));  // 2^-30
-  const float2 y = pk_mul(x, x);
-  float2 p = pk_fma(y, pk_set(-4.602149128913879e-3f), pk_set(7.968021929264069e-2f));
-  p = pk_fma(p, y, pk_set(-6.459634900093079e-1f));
-  p = pk_fma(p, y, pk_set(-4.8553051357203e-8f));
-  const float2 sn = pk_fma(x, pk_set(1.5707963705062866f), pk_mul(x, p));
-  float2 e = pk_fma(y, pk_set(9.036280680447817e-4f), pk_set(-2.086007036268711e-2f));
-  e = pk_fma(e, y, pk_set(2.5366920232772827e-1f));
-  e = pk_fma(e, y, pk_set(-1.2337005138397217f));
-  const float2 cs = pk_fma(e, y, pk_set(1.f));
-  auto sign = [](float v, unsigned bit) { return __uint_as_float(__float_as_uint(v) ^ (bit << 30)); };
-  c.x = sign((q0 & 1) ? sn.x : cs.x, (q0 + 1) & 2);
-  s.x = sign((q0 & 1) ? cs.x : sn.x, q0 & 2);
-  c.y = sign((q1 & 1) ? sn.y : cs.y, (q1 + 1) & 2);
-  s.y = sign((q1 & 1) ? cs.y : sn.y, q1 & 2);
+  cis_quarter_pk(x, q0, q1, c, s);
 }
 __device__ __forceinline__ float2 cis_turn(unsigned long long ph) {
   float2 c, s;
