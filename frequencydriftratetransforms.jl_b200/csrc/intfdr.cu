@@ -55,50 +55,77 @@ intfdr_kernel(const float* __restrict__ spec, long long Nf, int Nt, int nrates,
 // window of each column): a CTA stages, per time step t, the spectrogram channels
 // [n0 + lo_t, n0 + TN + hi_t] (modulo Nf) in shared memory and forms its TN output channels
 // of every rate from there, with the same sequence of float32 additions.  Each spectrogram
-// element is then read from HBM about once per CTA instead of once per rate.
+// element is then read from HBM about once per CTA instead of once per rate.  Bound by the one
+// shared-memory word per addition: 520 M of them at Nf = 2^20, Nt = 16, 31 rates take 56 us at 32 a
+// cycle and SM; 117 us with two indexed constant loads and the address per step, 86 us with the
+// positions of four steps in one constant load and the windows filled by asynchronous copies.  (A
+// form with 4 rates and 8 neighbouring channels per thread, which loads a quarter of the words and
+// branches on each rate's offset, took 190 us.)
 constexpr int kTiledMaxNt = 64;
 constexpr int kTiledMaxWords = 24576;  // shared-memory window floats (96 KB)
 
 struct TiledTable {
-  int32_t rel[kShiftParamWords];  // shift of rate jj at time t, minus lo_t: rel[jj*Nt + t]
+  // rel[jj*Ntp + t], Ntp = Nt rounded up to 4: shift of rate jj at time t, minus lo_t (host); word of
+  // win where the rate's channel n0 is at time t (in the launch)
+  int32_t rel[kShiftParamWords];
   int32_t lo[kTiledMaxNt];        // smallest signed shift at time t (in (-Nf/2, Nf/2])
   int32_t off[kTiledMaxNt + 1];   // start of time step t's window in shared memory
 };
 
-template <int TNV>  // TN = TNV * kIntfdrThreads output channels per CTA
-__global__ void __launch_bounds__(kIntfdrThreads)
+// T threads with TNV channels each, T apart: TN = TNV * T output channels per CTA.
+template <int TNV, int T>
+__global__ void __launch_bounds__(T)
 intfdr_tiled_kernel(const float* __restrict__ spec, long long Nf, int Nt, int nrates,
                     float* __restrict__ fdr, const __grid_constant__ TiledTable tab) {
-  constexpr int TN = TNV * kIntfdrThreads;
+  constexpr int TN = TNV * T;
   extern __shared__ float win[];
   const long long n0 = (long long)blockIdx.x * TN;
+  // asynchronous copies: every word of the windows is in flight at once
   for (int t = 0; t < Nt; ++t) {
     const float* col = spec + (long long)t * Nf;
-    const int len = tab.off[t + 1] - tab.off[t];
+    const int off = tab.off[t], len = tab.off[t + 1] - off;
     long long idx = (n0 + tab.lo[t]) % Nf;
     if (idx < 0) idx += Nf;
-    for (int i = threadIdx.x; i < len; i += kIntfdrThreads) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(win + off);
+    for (int i = threadIdx.x; i < len; i += T) {
       long long g = idx + i;
       if (g >= Nf) g -= Nf;  // len <= TN + Nf/4 < Nf: one wrap at most
-      if (FDR_DBG_OK(g >= 0 && g < Nf && tab.off[t] + i < kTiledMaxWords)) win[tab.off[t] + i] = __ldg(col + g);
+      if (FDR_DBG_OK(g >= 0 && g < Nf && off + i < kTiledMaxWords))
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4 * i), "l"(col + g) : "memory");
     }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   // the TNV channels of a thread are independent sums: interleaved, each in time order
+  const int Ntp = (Nt + 3) & ~3;
   for (int jj = 0; jj < nrates; ++jj) {
     float acc[TNV];
 #pragma unroll
     for (int v = 0; v < TNV; ++v) acc[v] = 0.0f;
-    for (int t = 0; t < Nt; ++t) {
-      const float* w = win + tab.off[t] + tab.rel[jj * Nt + t] + threadIdx.x;
+    const int4* const row = reinterpret_cast<const int4*>(tab.rel + jj * Ntp);
+    const float* const mine = win + threadIdx.x;
+    auto step = [&](int at, int t) {
 #pragma unroll
       for (int v = 0; v < TNV; ++v)
-        if (FDR_DBG_OK(tab.off[t] + tab.rel[jj * Nt + t] + (int)threadIdx.x + v * kIntfdrThreads < tab.off[t + 1]))
-          acc[v] = __fadd_rn(acc[v], w[v * kIntfdrThreads]);
+        if (FDR_DBG_OK(at + (int)threadIdx.x + v * T < tab.off[t + 1])) acc[v] = __fadd_rn(acc[v], mine[at + v * T]);
+    };
+#pragma unroll 2
+    for (int t0 = 0; t0 + 4 <= Nt; t0 += 4) {
+      const int4 p = row[t0 >> 2];
+      step(p.x, t0);
+      step(p.y, t0 + 1);
+      step(p.z, t0 + 2);
+      step(p.w, t0 + 3);
+    }
+    if (Nt & 3) {
+      const int4 p = row[Nt >> 2];
+      step(p.x, Nt & ~3);
+      if ((Nt & 3) > 1) step(p.y, (Nt & ~3) + 1);
+      if ((Nt & 3) > 2) step(p.z, (Nt & ~3) + 2);
     }
 #pragma unroll
     for (int v = 0; v < TNV; ++v) {
-      const long long n = n0 + threadIdx.x + v * kIntfdrThreads;
+      const long long n = n0 + threadIdx.x + v * T;
       if (n < Nf) fdr[(long long)jj * Nf + n] = acc[v];
     }
   }
@@ -139,8 +166,9 @@ static int32_t mod_nf(int64_t sh, int64_t Nf) {
 static bool run_intfdr_tiled(const float* spec, int64_t Nf, int64_t Nt, int64_t j0, int64_t nr,
                              float* fdr, const std::vector<int32_t>& sh, cudaStream_t s, int* status) {
   *status = FDR_OK;
-  if (Nt > kTiledMaxNt || nr * Nt > kShiftParamWords || Nf < 2 * kIntfdrThreads) return false;
-  TiledTable tab;
+  const int64_t Ntp = (Nt + 3) / 4 * 4;
+  if (Nt > kTiledMaxNt || nr * Ntp > kShiftParamWords || Nf < 2 * kIntfdrThreads) return false;
+  alignas(16) TiledTable tab;
   int64_t spans = 0;
   for (int64_t t = 0; t < Nt; ++t) {
     int64_t lo = 0, hi = 0;
@@ -156,7 +184,7 @@ static bool run_intfdr_tiled(const float* spec, int64_t Nf, int64_t Nt, int64_t 
     for (int64_t j = 0; j < nr; ++j) {
       int64_t v = sh[(j0 + j) * Nt + t];
       if (v > Nf / 2) v -= Nf;
-      tab.rel[j * Nt + t] = (int32_t)(v - lo);
+      tab.rel[j * Ntp + t] = (int32_t)(v - lo);
     }
   }
   int TN = 0;
@@ -166,20 +194,22 @@ static bool run_intfdr_tiled(const float* spec, int64_t Nf, int64_t Nt, int64_t 
   tab.off[0] = 0;
   for (int64_t t = 0; t < Nt; ++t) {
     int64_t hi = 0;
-    for (int64_t j = 0; j < nr; ++j) hi = std::max<int64_t>(hi, tab.rel[j * Nt + t]);
+    for (int64_t j = 0; j < nr; ++j) hi = std::max<int64_t>(hi, tab.rel[j * Ntp + t]);
     tab.off[t + 1] = tab.off[t] + (int32_t)(TN + hi);  // channels n0 + lo .. n0 + TN - 1 + hi
   }
+  for (int64_t j = 0; j < nr; ++j)
+    for (int64_t t = 0; t < Nt; ++t) tab.rel[j * Ntp + t] += tab.off[t];
   const size_t smem = sizeof(float) * (size_t)tab.off[Nt];
   cudaError_t ea = cudaSuccess;
-#define TILED(V)                                                                                \
-  if (TN == V * kIntfdrThreads) {                                                               \
-    ea = cudaFuncSetAttribute(intfdr_tiled_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+#define TILED(V, T)                                                                             \
+  if (TN == V * T) {                                                                            \
+    ea = cudaFuncSetAttribute(intfdr_tiled_kernel<V, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                               (int)(sizeof(float) * kTiledMaxWords));                           \
     if (ea == cudaSuccess)                                                                      \
-      intfdr_tiled_kernel<V><<<(unsigned)cdiv(Nf, TN), kIntfdrThreads, smem, s>>>(             \
+      intfdr_tiled_kernel<V, T><<<(unsigned)cdiv(Nf, TN), T, smem, s>>>(                        \
           spec, Nf, (int)Nt, (int)nr, fdr + j0 * Nf, tab);                                      \
   }
-  TILED(1) TILED(2) TILED(4)
+  TILED(1, 256) TILED(2, 256) TILED(4, 256)
 #undef TILED
   if (ea != cudaSuccess) { *status = cuda_status(ea, "intfdr tiled attribute"); return true; }
   cudaError_t e = cudaGetLastError();
@@ -191,7 +221,7 @@ static int run_intfdr(const float* spec, int64_t Nf, int64_t Nt, int64_t Nr, flo
                       const std::vector<int32_t>& sh, cudaStream_t s) {
   FDR_CHECK_ARG(Nt <= kShiftParamWords, "intfdr: Nt=%lld exceeds %d", (long long)Nt,
                 kShiftParamWords);
-  const int64_t chunk = std::max<int64_t>(1, kShiftParamWords / Nt);
+  const int64_t chunk = std::max<int64_t>(1, kShiftParamWords / (Nt + 3));  // the tiled kernel's rows are padded to 4
   const unsigned gx = (unsigned)cdiv(Nf, kIntfdrThreads * kIntfdrVec);
   ShiftTable tab;
   for (int64_t j0 = 0; j0 < Nr; j0 += chunk) {
