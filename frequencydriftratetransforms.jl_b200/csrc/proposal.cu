@@ -241,7 +241,7 @@ conv_fwd_kernel(const float* __restrict__ in, int cin, int X, const float* __res
       }
     }
   }
-  if (!HEAD) return;
+  if constexpr (!HEAD) return;
   __shared__ float rv[kConvThreads / 32][kWin];
   __shared__ int ri[kConvThreads / 32][kWin];
 #pragma unroll

@@ -66,15 +66,8 @@ struct FusedTables {
   const float2* rootsP;  // exp(-2 pi i m / P), m < P
   const float2* twP;     // Stockham pass twiddles of length P (tw_offset layout)
   const float2* twQ;     // Stockham pass twiddles of length Q
-  const float2* tw_lo;   // exp(-2 pi i m / N), m < 2^B
-  const float2* tw_hi;   // exp(-2 pi i m 2^B / N), m < N / 2^B
-  int B;
 };
 
-// exp(-2 pi i m / N) for 0 <= m < N (two-level table product).
-__device__ __forceinline__ float2 tw_fwd(const FusedTables& t, long long m) {
-  return cmul(__ldg(t.tw_hi + (m >> t.B)), __ldg(t.tw_lo + (m & ((1LL << t.B) - 1))));
-}
 
 // exp(2 pi i ph / 2^64) for the phases of two bins: the nearest quarter turn is taken off in
 // integers.  The two bins share packed operations: about 33 instructions for both, where two
@@ -98,7 +91,7 @@ __device__ __forceinline__ float2 cis_turn(unsigned long long ph) {
 template <int P, int TA, int T>
 __global__ void __launch_bounds__(T)
 zdtf_input_kernel(const float* __restrict__ spec, long long N, int Nt, int Q,
-                  float2* __restrict__ A, FusedTables tab) {
+                  float2* __restrict__ A, FusedTables tab, unsigned long long turn /* 2^64 / Nf */) {
   constexpr int SS = ac_stride<P, TA>();
   constexpr int TP = TA / 2;  // sequence pairs: each thread moves two adjacent channels
   extern __shared__ float2 sm[];
@@ -137,8 +130,12 @@ zdtf_input_kernel(const float* __restrict__ spec, long long N, int Nt, int Q,
   for (int e = threadIdx.x; e < TP * P; e += T) {
     const int sp = e % TP, k1 = e / TP;
     const int na = na0 + 2 * sp;
-    const float2 v0 = cmul(buf[(2 * sp) * SS + pidx(k1)], tw_fwd(tab, (long long)k1 * na));
-    const float2 v1 = cmul(buf[(2 * sp + 1) * SS + pidx(k1)], tw_fwd(tab, (long long)k1 * (na + 1)));
+    // exp(-2 pi i k1 n / Nf) of both channels from exact phases
+    const unsigned long long ph = (unsigned long long)k1 * (unsigned)na * turn;
+    float2 c, sn;
+    cis_turn_pk(ph, ph + (unsigned long long)k1 * turn, c, sn);
+    const float2 v0 = cmul(buf[(2 * sp) * SS + pidx(k1)], make_float2(c.x, -sn.x));
+    const float2 v1 = cmul(buf[(2 * sp + 1) * SS + pidx(k1)], make_float2(c.y, -sn.y));
     if (FDR_DBG_OK(((long long)p * P + k1) * Q + na + 2 <= (long long)gridDim.y * P * Q))
       *reinterpret_cast<float4*>(A + ((long long)p * P + k1) * Q + na) = make_float4(v0.x, v0.y, v1.x, v1.y);
   }
@@ -276,8 +273,23 @@ struct CztArgs {
   int pshift;           // F in registers: time pairs are held this many pairs up
   PhaseInt ph;
   unsigned long long center;  // the grid centre's rate over Nf: R0 + (4h - 1) Rh
+  unsigned long long turn;    // 2^64 / Nf
   FusedTables tab;
 };
+
+// twr[side * Q + n_a] = exp(2 pi i k1 n_a / Nf) / Nf, the inter-pass twiddle of the inverse
+// transform, from exact phases (both sides at once).
+template <int Q, int T>
+__device__ __forceinline__ void fill_output_twiddles(const CztArgs& a, const int* k1s, float2* twr) {
+  const float invN = 1.0f / (float)a.N;
+  const unsigned long long s0 = (unsigned)k1s[0] * a.turn, s1 = (unsigned)k1s[1] * a.turn;
+  for (int na = threadIdx.x; na < Q; na += T) {
+    float2 c, s;
+    cis_turn_pk((unsigned)na * s0, (unsigned)na * s1, c, s);
+    twr[na] = make_float2(c.x * invN, s.x * invN);
+    twr[Q + na] = make_float2(c.y * invN, s.y * invN);
+  }
+}
 
 // Position (side, k2) of the bin N - k for the base at (side, k2) of CTA c.
 __device__ __forceinline__ void mirror_of(int c, int side, int k2, int Q, int* ms, int* mk2) {
@@ -645,12 +657,8 @@ __global__ void __launch_bounds__(Q / 2, (Q <= 512 ? 2 : 1)) zdtf_czt_kernel(Czt
   const int c = blockIdx.x;
   const int P = a.P;
   const int k1s[2] = {c == 0 ? 0 : c, c == 0 ? P / 2 : P - c};
-  const float invN = 1.0f / (float)a.N;
   for (int i = tid; i < tw_size(Q); i += T) twt[i] = __ldg(a.tab.twQ + i);
-  for (int i = tid; i < 2 * Q; i += T) {
-    const int side = i / Q, na = i - side * Q;
-    twr[i] = cscale(cconj(tw_fwd(a.tab, (long long)k1s[side] * na)), invN);
-  }
+  fill_output_twiddles<Q, T>(a, k1s, twr);
   float2 Gx[NTR], Gy[NTR];  // lanes = the thread's two bins
   {
     float2 G[2][NTR];
@@ -960,12 +968,8 @@ __global__ void __launch_bounds__(CztSmemShape<Q>::T, 1) zdtf_czt_smem_kernel(Cz
   const int c = blockIdx.x;
   const int P = a.P;
   const int k1s[2] = {c == 0 ? 0 : c, c == 0 ? P / 2 : P - c};
-  const float invN = 1.0f / (float)a.N;
   for (int i = tid; i < tw_size(Q); i += T) twt[i] = __ldg(a.tab.twQ + i);
-  for (int i = tid; i < 2 * Q; i += T) {
-    const int side = i / Q, na = i - side * Q;
-    twr[i] = cscale(cconj(tw_fwd(a.tab, (long long)k1s[side] * na)), invN);
-  }
+  fill_output_twiddles<Q, T>(a, k1s, twr);
   wait_for_predecessor();
   czt_forward_smem<Q, NT>(a, c, k1s, buf, twt, gs, gnyq);
 
@@ -1079,12 +1083,8 @@ __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArg
   const int c = blockIdx.x;
   const int P = a.P;
   const int k1s[2] = {c == 0 ? 0 : c, c == 0 ? P / 2 : P - c};
-  const float invN = 1.0f / (float)a.N;
   for (int i = tid; i < tw_size(Q); i += T) twt[i] = __ldg(a.tab.twQ + i);
-  for (int i = tid; i < 2 * Q; i += T) {
-    const int side = i / Q, na = i - side * Q;
-    twr[i] = cscale(cconj(tw_fwd(a.tab, (long long)k1s[side] * na)), invN);
-  }
+  fill_output_twiddles<Q, T>(a, k1s, twr);
   wait_for_predecessor();
   czt_forward_smem<Q, NT, T, false, 8>(a, c, k1s, buf0, twt, gs, gnyq);  // ends with a barrier
   auto bin0 = [&](int bp) {
@@ -1282,12 +1282,8 @@ zdtf_czt_cl_kernel(CztArgs a) {
   const int c = blockIdx.x >> 1;                // residue pair
   const int P = a.P;
   const int k1s[2] = {c == 0 ? 0 : c, c == 0 ? P / 2 : P - c};
-  const float invN = 1.0f / (float)a.N;
   for (int i = tid; i < tw_size(Q); i += T) twt[i] = __ldg(a.tab.twQ + i);
-  for (int i = tid; i < 2 * Q; i += T) {
-    const int sd = i / Q, na = i - sd * Q;
-    twr[i] = cscale(cconj(tw_fwd(a.tab, (long long)k1s[sd] * na)), invN);
-  }
+  fill_output_twiddles<Q, T>(a, k1s, twr);
   wait_for_predecessor();
   czt_forward_cluster<Q, NT, T>(a, c, k1s, buf, twt, gs, gnyq, rank, cluster);
   auto bin0 = [&](int bp) { return (unsigned long long)k1s[rank] + (unsigned long long)P * (2 * bp); };
@@ -2580,7 +2576,7 @@ zdtf_output_umma_kernel(const __grid_constant__ CUtensorMap wmap, long long N, i
 template <int P>
 struct AcShape {
   static constexpr int TILE = P >= 4096 ? 4 : 8;
-  static constexpr int T = (TILE * P / 16 > 512) ? 512 : (TILE * P / 16 < 32 ? 32 : TILE * P / 16);
+  static constexpr int T = (TILE * P / 16 > 512) ? 512 : (TILE * P / 16 < 128 ? 128 : TILE * P / 16);
   static constexpr size_t SMEM = sizeof(float2) * (TILE * ac_stride<P, TILE>() + tw_size(P));
 };
 
@@ -2654,8 +2650,8 @@ static bool make_phase(float r0, float dr, int L, PhaseInt* ph) {
 // workspace and by batches of channels with the same shape.
 struct FusedPlan {
   int64_t N = 0, Nt = 0, Nr = 0;
-  int L = 0, B = 0, P = 0, Q = 0;
-  float2* tables = nullptr;  // twP | twQ | tw_lo | tw_hi | rootsP
+  int L = 0, P = 0, Q = 0;
+  float2* tables = nullptr;  // twP | twQ | rootsP
   FusedTables tab;
   int64_t NP = 0, npairs = 0;
   int64_t half = 0;  // super pairs of the whole grid (kept by rate subsets)
@@ -2776,31 +2772,24 @@ int fused_plan_create(FusedPlan** out, int64_t N, int64_t Nt, int64_t Nr) {
   const int Qlog = fused_qlog(st->L, Nt);
   st->Q = 1 << Qlog;
   st->P = (int)(N >> Qlog);
-  st->B = (st->L + 1) / 2;
   st->NP = cdiv(Nt, 2);
   st->npairs = cdiv(Nr, 2);
   st->half = cdiv(st->npairs, 2);
   const long long P = st->P, Q = st->Q;
-  const long long nlo = 1LL << st->B, nhi = N >> st->B;
   const long long ntwP = tw_size((int)P), ntwQ = tw_size((int)Q);
-  const long long ntab = ntwP + ntwQ + nlo + nhi + P;
+  const long long ntab = ntwP + ntwQ + P;
   cudaError_t e = cudaMalloc(&st->tables, sizeof(float2) * ntab);
   if (e != cudaSuccess) { delete st; return cuda_status(e, "cudaMalloc(fused tables)"); }
   std::vector<float2> h;
   auto append = [&](const std::vector<float2>& v) { h.insert(h.end(), v.begin(), v.end()); };
   append(pass_twiddles((int)P));
   append(pass_twiddles((int)Q));
-  append(roots_table(1, N, nlo));
-  append(roots_table(nlo, N, nhi));
   append(roots_table(1, P, P));
   e = cudaMemcpy(st->tables, h.data(), sizeof(float2) * ntab, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) { cudaFree(st->tables); delete st; return cuda_status(e, "upload fused tables"); }
   st->tab.twP = st->tables;
   st->tab.twQ = st->tables + ntwP;
-  st->tab.tw_lo = st->tables + ntwP + ntwQ;
-  st->tab.tw_hi = st->tables + ntwP + ntwQ + nlo;
-  st->tab.rootsP = st->tables + ntwP + ntwQ + nlo + nhi;
-  st->tab.B = st->B;
+  st->tab.rootsP = st->tables + ntwP + ntwQ;
   *out = st;
   return FDR_OK;
 }
@@ -2812,7 +2801,7 @@ void fused_plan_destroy(FusedPlan* st) {
 }
 
 int64_t fused_plan_table_bytes(const FusedPlan* st) {
-  return (int64_t)sizeof(float2) * (tw_size(st->P) + tw_size(st->Q) + (1LL << st->B) + (st->N >> st->B) + st->P);
+  return (int64_t)sizeof(float2) * (tw_size(st->P) + tw_size(st->Q) + st->P);
 }
 int64_t fused_A_elems(const FusedPlan* st) { return st->N * st->NP; }
 int64_t fused_W_elems(const FusedPlan* st) { return st->N * st->npairs; }
@@ -2839,7 +2828,7 @@ int fused_input(const FusedPlan* st, const float* spec, float2* A, cudaStream_t 
   if (P == PP) {                                                                               \
     constexpr int TA = AcShape<PP>::TILE, T = AcShape<PP>::T;                                  \
     zdtf_input_kernel<PP, TA, T><<<dim3(Q / TA, (unsigned)st->NP), T, AcShape<PP>::SMEM, s>>>( \
-        spec, st->N, (int)st->Nt, Q, A, st->tab);                                              \
+        spec, st->N, (int)st->Nt, Q, A, st->tab, 1ull << (64 - st->L));                        \
     FDR_LAUNCH_CHECK("zdtf_input_kernel");                                                     \
     return FDR_OK;                                                                             \
   }
@@ -2855,6 +2844,7 @@ static CztArgs czt_args(const FusedPlan* st, const float2* A, float2* W) {
   a.A = A;
   a.W = W;
   a.N = st->N;
+  a.turn = 1ull << (64 - st->L);
   a.P = st->P;
   a.Nt = (int)st->Nt;
   a.NP = (int)st->NP;
@@ -3097,7 +3087,8 @@ int fused_output_mixed(const FusedPlan* st, const float2* W, float* dest, double
 
 int fused_output(const FusedPlan* st, const float2* W, float* dest, double* acc, cudaStream_t s) {
   const int P = st->P, Q = st->Q;
-  // P = 1024 or 2048: Q is 256 to 1024 (fused_qlog)
+  // P = 1024 or 2048: Q is 256 to 1024 (fused_qlog).  (P = 512 through the TMA kernel, half of its
+  // threads idle in pass 1, took 130 us against zdtf_output2_kernel's 124 at Nf = 2^18, 257 rates.)
   if ((P == 1024 || P == 2048) && tma_output_enabled()) {
     CUtensorMap map;
     if (w_tensor_map(&map, W, Q, st->npairs * (int64_t)P, 8)) {
