@@ -85,8 +85,9 @@ def algorithmic_bytes():
 # zdtf_output_tma64<8>) from one ncu capture of this benchmark's plain leg.  ncu cannot run
 # inside the timed process, so the figure is carried here with the capture it came from.
 NCU_TRAFFIC = {
-    "bytes_per_call": 1_676_704_256,
-    "capture": "ncu --set full --clock-control none -k regex:zdtf_ -s 3 -c 3 python bench.py "
+    "bytes_per_call": 1_669_887_232,
+    "capture": "ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none "
+               "-k regex:zdtf_ -s 3 -c 3 python bench.py "
                "--steps 3 --warmup 1 --no-cpu-baseline --no-e2e --no-batched --no-proposal "
                "--no-fp32-peak --no-taylor --no-ingest --no-mixed",
 }

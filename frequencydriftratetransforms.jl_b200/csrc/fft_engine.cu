@@ -335,6 +335,12 @@ __device__ __forceinline__ float2 twiddle_at(const TwiddleTables& t, int i, int 
   return make_float2(h.x + fmaf(h.x, e.x, fmaf(-h.y, e.y, h.z)), h.y + fmaf(h.x, e.y, fmaf(h.y, e.x, h.w)));
 }
 
+// One pass: several transforms of length L per CTA in shared memory (64 KB, three CTAs per SM at 80
+// registers), the first stage reading and the last writing device memory.  Passes of Nf = 200,000,
+// 81 columns back: 59 and 51 us (99 and 80 with the butterflies of a thread in registers across the
+// stage, which spilled and ran into instruction fetches; the four Stockham kernels before both: over
+// 400).  Bound by instruction issue (55 to 62%), a good part of it integer addressing of the runtime
+// lengths, then by the latency of the loads.
 template <int SIGN, int IN, int OUT>
 __global__ void __launch_bounds__(kStageThreads, kStageCtas) fft_stage_kernel(const __grid_constant__ StageArgs a) {
   extern __shared__ float4 sm4[];

@@ -1,17 +1,19 @@
 // Generic batched FFT engine (any length whose prime factors are <= 64).
 //
-// This is the library's own FFT: mixed-radix Stockham stages in shared memory (radix 2, 3,
-// 4, 5, 8 specialised, other primes up to 64 by direct DFT), one pass per transform when
-// the length fits a CTA (<= kMaxCtaElems points) and the four-step split into two such
-// passes otherwise.  Real transforms use the two-for-one packing (two real columns in one
-// complex transform).  The reference gets these transforms from FFTW / cuFFT
+// This is the library's own FFT: one pass per transform when the length fits a CTA
+// (<= kMaxCtaElems points) and the four-step split into two such passes otherwise.  Lengths
+// whose prime factors are at most 13 take the in-place register-radix stages of
+// fft_stages.cuh, with the packing, twiddles and unpacking of a pass in its loads and stores;
+// the others mixed-radix Stockham stages in shared memory (radix 2, 3, 4, 5, 8 specialised,
+// other primes up to 64 by direct DFT).  Real transforms use the two-for-one packing (two
+// real columns in one complex transform).  The reference gets these transforms from FFTW / cuFFT
 // (zdtfdr.jl:119-123, ext/CUDAFrequencyDriftRateTransformsExt.jl:59-79).
 #pragma once
 #include "fdr_internal.cuh"
 
 namespace fdr {
 
-constexpr int kMaxCtaElems = 8192;   // complex points held by one CTA (double-buffered)
+constexpr int kMaxCtaElems = 8192;   // complex points held by one CTA (double-buffered by the Stockham stages)
 constexpr int kMaxRadixPrime = 64;   // largest prime factor handled by a direct-DFT stage
 constexpr int kMaxStages = 24;
 

@@ -1,4 +1,4 @@
-// Fused ZDT path for power-of-two Nf (2^12 .. 2^22) and Nt <= 16.
+// Fused ZDT path for power-of-two Nf (2^12 .. 2^22) and Nt <= 64.
 //
 // The reference computes zdtfdr! as rfft -> prephase -> FFT_l -> .*V -> IFFT_l ->
 // postphase -> irfft (zdtfdr.jl:349-362), materialising F, Y (K x Nl) and V (K x Nl) in
@@ -13,8 +13,8 @@
 //   kernel A (zdtf_input):  four-step pass 1 of the forward FFT of two real columns packed
 //                           as one complex column (t pairs): DFT_P over n_b, twiddle.
 //   kernel B (zdtf_czt):    per pair of bin residues {k1, P-k1}: forward DFT_Q (pass 2) and
-//                           two-for-one unpack into F[k, t] held in registers; then, per
-//                           block of drift rates, S_j[k] by folded sums with exact
+//                           two-for-one unpack into F[k, t] held in registers (Nt <= 16)
+//                           or shared memory; then, per block of drift rates, S_j[k] by folded sums with exact
 //                           integer phase reduction, the window, two-for-one packing of
 //                           rate pairs, inverse DFT_Q (pass 1 of the output FFT) and the
 //                           inter-pass twiddle (with the 1/Nf scale).
@@ -22,9 +22,9 @@
 //                           output columns of each rate pair.
 //
 // Nf = P*Q; bin k = k1 + P*k2, channel n = na + Q*nb.  Phases: r0 and dr are float32,
-// hence dyadic, so k*r_j/Nf is an exact fraction m / 2^bits with m computed in 64-bit
-// integer arithmetic modulo 2^bits; only the final conversion to a float in [-1, 1)
-// half-turns rounds.
+// hence dyadic, so k*r_j/Nf modulo one turn is an exact 64-bit fraction of a turn (integer
+// arithmetic that wraps); only the conversion of the rest after the nearest quarter turn to
+// float rounds.
 #define FDR_TU_ID 1  // index violations of the debug build report this file as unit 1
 #include <cuda.h>  // CUtensorMap (the encode entry point is fetched from the runtime)
 #include <cooperative_groups.h>
@@ -67,7 +67,6 @@ struct FusedTables {
   const float2* twP;     // Stockham pass twiddles of length P (tw_offset layout)
   const float2* twQ;     // Stockham pass twiddles of length Q
 };
-
 
 // exp(2 pi i ph / 2^64) for the phases of two bins: the nearest quarter turn is taken off in
 // integers.  The two bins share packed operations: about 33 instructions for both, where two
@@ -637,7 +636,11 @@ __device__ __forceinline__ void fold_smem(const CztArgs& a, float4* gs4, int nbp
 // WINDOWED = false: the rectangular window (weights 1, skipped: the same FDR bit for bit).
 // SUBSET: the 8-rate blocks at a.blk_base instead of the whole grid.
 // Per CTA and 8-rate block: the sums of 4 values of m, two rates each, two rates packed per
-// complex sequence (Hermitian halves at k and its mirror), inverse DFT_Q, W.
+// complex sequence (Hermitian halves at k and its mirror), inverse DFT_Q, W.  One bin of each
+// residue per thread, so that their F (4 floats a step) stays in registers; 128 of them allow 16
+// warps per SM.  At Nf = 2^20, Nt = 16, 129 rates (Q = 512): 381 -> 325 us in the call against
+// Horner's rule per rate, 239 -> 213 M warp instructions; bound by their issue (58% of the cycles,
+// FMA pipe 50%) between the block barriers, not by the 555 MB moved (24% of the copy rate).
 template <int Q, int NTR, bool WINDOWED, bool SUBSET>
 __global__ void __launch_bounds__(Q / 2, (Q <= 512 ? 2 : 1)) zdtf_czt_kernel(CztArgs a) {
   constexpr int T = Q / 2;
@@ -1046,7 +1049,8 @@ __global__ void __launch_bounds__(CztSmemShape<Q>::T, 1) zdtf_czt_smem_kernel(Cz
 //   EMPTY(i mod 2): the FFT threads arrive once they have read block i (when block i + 2
 //                   exists); the sum threads wait on it before writing block i + 2.
 // The FFT phase (shared-memory latency and its own barriers) thus runs under the sums instead
-// of after them.
+// of after them.  Bound by the FMA pipe (53%) and the hand-over barriers; with the pair sums
+// 323 -> 267 us at Nf = 2^18, Nt = 32, 257 rates.
 // ------------------------------------------------------------------------------------
 template <int Q>
 struct CztWsShape {
@@ -1263,6 +1267,12 @@ struct CztClShape {
   static constexpr size_t SMEM = sizeof(float2) * (GS_OFF + NT * QH + NT);
 };
 
+// Sums and inverse transforms side by side as in zdtf_czt_ws_kernel, handed over at the one
+// cluster barrier per two blocks that exchanging the mirrored halves needs.  At Nf = 2^20, Nt = 64,
+// 129 rates: 1.43 ms with Horner's rule, 1.19 with the pair sums by all threads in turn, 1.12 in
+// this form (510 M warp instructions, FMA pipe 40%).  Bound by the sum threads: two warps per
+// scheduler at 128 registers wait for shared-memory loads and for each other at the barrier; 512 of
+// them at 80 registers spilled (1.35 ms).
 template <bool SUBSET>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CztClShape::T, 1)
 zdtf_czt_cl_kernel(CztArgs a) {
