@@ -47,6 +47,7 @@ struct fdr_propose_net {
   float* act[3] = {nullptr, nullptr, nullptr};  // outputs of layers 1..3
   float* tile_max = nullptr;                    // per (sample, tile, window): largest logit,
   int* tile_arg = nullptr;                      //   its bin
+  int* odd = nullptr;                           // taps that meet a non-finite input, see conv_fwd_kernel
   int* argmax = nullptr;
   float* dlogit = nullptr;                      // gradient of the loss wrt the logits
   float* gact = nullptr;                        // per sample: SparseGrad
@@ -177,6 +178,10 @@ static int launch_input(const float* spec, int64_t Nf, int64_t Nt, int factor, i
 // layer at 64 x 4096 bins, 33 channels; now 83 us, FMA pipe 57%, the weights' loads behind it).  Every output sums over (ci, k) in order from its bias.
 // HEAD: the last hidden layer also forms the 16 window logits of its bins (the 1x1 layer, same
 // order of sums) and their maximum over the tile's bins, the first bin on ties.
+// odd: per (sample, tile, input channel) the taps that meet an infinity or NaN (bit k), for HEAD
+// also per (sample, tile) the output channels that hold an infinity: the gradient's sums over all
+// bins multiply these by zeros, which the sparse kernels below leave out, so that they turn the
+// sums that these would meet into NaN.
 // --------------------------------------------------------------------------------------
 constexpr int kWidth = 32, kWin = 16, kTaps = 5, kPad = kTaps / 2;
 constexpr int kConvThreads = kConvTile / 2;
@@ -185,7 +190,8 @@ template <bool HEAD>
 __global__ void __launch_bounds__(kConvThreads, 4)
 conv_fwd_kernel(const float* __restrict__ in, int cin, int X, const float* __restrict__ wt,
                 const float* __restrict__ bias, float* __restrict__ out, const float* __restrict__ wt3,
-                const float* __restrict__ bias3, float* __restrict__ tile_max, int* __restrict__ tile_arg) {
+                const float* __restrict__ bias3, float* __restrict__ tile_max, int* __restrict__ tile_arg,
+                int* __restrict__ odd, int* __restrict__ odd_head) {
   extern __shared__ float4 sm4[];
   constexpr int TW = kConvTile + kTaps - 1;
   float* const wsm = reinterpret_cast<float*>(sm4);  // [ci][k][co]
@@ -197,11 +203,25 @@ conv_fwd_kernel(const float* __restrict__ in, int cin, int X, const float* __res
 #pragma unroll 2
   for (int ci = warp; ci < cin; ci += kConvThreads / 32) {  // a warp per row: loads in flight together
     const float* const row = inb + (long long)ci * X;
+    bool any = false;
 #pragma unroll
     for (int j = 0; j < (TW + 31) / 32; ++j) {
       const int i = lane + 32 * j, xx = x0 - kPad + i;
-      if (i < TW) xs[ci * TW + i] = (xx >= 0 && xx < X) ? __ldg(row + xx) : 0.f;
+      if (i < TW) {
+        const float v = (xx >= 0 && xx < X) ? __ldg(row + xx) : 0.f;
+        xs[ci * TW + i] = v;
+        any |= !(fabsf(v) < INFINITY);
+      }
     }
+    int taps = 0;
+    if (__any_sync(0xffffffffu, any)) {
+      for (int i = lane; i < TW; i += 32)
+        if (!(fabsf(xs[ci * TW + i]) < INFINITY))
+          for (int k = 0; k < kTaps; ++k)
+            if (i >= k && i - k < kConvTile) taps |= 1 << k;  // tap k takes it to bin i - k of the tile
+      taps = __reduce_or_sync(0xffffffffu, taps);
+    }
+    if (lane == 0) odd[((long long)b * gridDim.x + blockIdx.x) * cin + ci] = taps;
   }
 #pragma unroll 4
   for (int i = tid; i < cin * kTaps * kWidth; i += kConvThreads) wsm[i] = __ldg(wt + i);
@@ -242,6 +262,24 @@ conv_fwd_kernel(const float* __restrict__ in, int cin, int X, const float* __res
     }
   }
   if constexpr (!HEAD) return;
+  __shared__ int inf_channels[kConvThreads / 32];
+  {
+    float top = 0.f;
+#pragma unroll
+    for (int p = 0; p < kWidth / 2; ++p)
+      top = fmaxf(top, fmaxf(fmaxf(acc[0][p].x, acc[0][p].y), fmaxf(acc[1][p].x, acc[1][p].y)));
+    int m = 0;
+    if (__any_sync(0xffffffffu, top == INFINITY)) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int p = 0; p < kWidth / 2; ++p)
+          if (x0 + tid + h * kConvThreads < X)
+            m |= ((acc[h][p].x == INFINITY) << (2 * p)) | ((int)((unsigned)(acc[h][p].y == INFINITY) << (2 * p + 1)));
+      m = __reduce_or_sync(0xffffffffu, m);
+    }
+    if (lane == 0) inf_channels[warp] = m;
+  }
   __shared__ float rv[kConvThreads / 32][kWin];
   __shared__ int ri[kConvThreads / 32][kWin];
 #pragma unroll
@@ -308,6 +346,11 @@ conv_fwd_kernel(const float* __restrict__ in, int cin, int X, const float* __res
     const long long o = ((long long)b * gridDim.x + blockIdx.x) * kWin + tid;
     tile_max[o] = v;
     tile_arg[o] = i;
+    if (tid == 0) {
+      int m = 0;
+      for (int q = 0; q < kConvThreads / 32; ++q) m |= inf_channels[q];
+      odd_head[(long long)b * gridDim.x + blockIdx.x] = m;
+    }
   }
 }
 
@@ -513,6 +556,12 @@ sparse_grad_kernel(const float* __restrict__ dlogit, const int* __restrict__ arg
   }
 }
 
+// Flags of conv_fwd_kernel for the inputs of the four layers.
+struct OddInputs {
+  const int* at[4];
+  int tiles;
+};
+
 // A sample's gradient of one layer's parameters: grid (4 layers, B).  Layers 1 to 3: a thread
 // takes four output channels, an input channel and the five taps; the layer's input at the listed
 // bins and two either side sits in shared memory in list order.  Layer 4 (1x1): its selected bins.
@@ -522,14 +571,17 @@ sparse_weight_grad_kernel(const SparseGrad* __restrict__ sg, const float* __rest
                           const float* __restrict__ act0, const float* __restrict__ act1,
                           const float* __restrict__ act2, const float* __restrict__ dlogit,
                           const int* __restrict__ argmax, int cin0, int X, Layer L0, Layer L1, Layer L2, Layer L3,
-                          float* __restrict__ partial, long long nparams) {
+                          float* __restrict__ partial, long long nparams, OddInputs odd) {
   extern __shared__ float4 sm4[];
   const int l = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   float* const pb = partial + b * nparams;
   if (l == 3) {
+    int inf = 0;
+    for (int t = 0; t < odd.tiles; ++t) inf |= odd.at[3][(long long)b * odd.tiles + t];
     for (int i = tid; i < kWin * kWidth; i += kSparseThreads) {
       const int w = i / kWidth, c = i % kWidth;
-      pb[L3.woff + i] = dlogit[b * kWin + w] * act2[((long long)b * kWidth + c) * X + argmax[b * kWin + w]];
+      const float v = dlogit[b * kWin + w] * act2[((long long)b * kWidth + c) * X + argmax[b * kWin + w]];
+      pb[L3.woff + i] = (inf >> c & 1) && fabsf(v) < INFINITY ? NAN : v;
     }
     for (int w = tid; w < kWin; w += kSparseThreads) pb[L3.boff + w] = dlogit[b * kWin + w];
     return;
@@ -574,10 +626,13 @@ sparse_weight_grad_kernel(const SparseGrad* __restrict__ sg, const float* __rest
         a[3][k] = fmaf(g.w, v, a[3][k]);
       }
     }
+    int taps = 0;
+    for (int t = 0; t < odd.tiles; ++t) taps |= __ldg(odd.at[l] + ((long long)b * odd.tiles + t) * cin + ci);
 #pragma unroll
     for (int q = 0; q < 4; ++q)
 #pragma unroll
-      for (int k = 0; k < kTaps; ++k) pb[L.woff + ((long long)(4 * cg + q) * cin + ci) * kTaps + k] = a[q][k];
+      for (int k = 0; k < kTaps; ++k)
+        pb[L.woff + ((long long)(4 * cg + q) * cin + ci) * kTaps + k] = (taps >> k & 1) && fabsf(a[q][k]) < INFINITY ? NAN : a[q][k];
   }
   for (int c = tid; c < kWidth; c += kSparseThreads) {
     float a = 0.f;
@@ -666,18 +721,33 @@ static int set_attrs() {
   return FDR_OK;
 }
 
+static OddInputs odd_inputs(const fdr_propose_net* n) {
+  OddInputs o;
+  o.tiles = (int)cdiv(n->nbins, kConvTile);
+  const int cin[3] = {n->nt, kWidth, kWidth};
+  const int* p = n->odd;
+  for (int l = 0; l < 3; ++l) {
+    o.at[l] = p;
+    p += (size_t)n->maxb * o.tiles * cin[l];
+  }
+  o.at[3] = p;
+  return o;
+}
+
 static int net_forward(fdr_propose_net* n, const float* x, int B, float* logits, cudaStream_t s) {
   FDR_CHECK_ARG(B >= 1 && B <= n->maxb, "proposal net: batch %d exceeds the maximum %d", B, n->maxb);
   const float* in = x;
   const int X = n->nbins, tiles = (int)cdiv(X, kConvTile);
   const dim3 grid((unsigned)tiles, (unsigned)B);
+  const OddInputs odd = odd_inputs(n);
   for (int li = 0; li < 3; ++li) {
     const Layer& L = n->L[li];
     const size_t sm = sizeof(float) * (L.cin * (kConvTile + kTaps - 1) + kWidth * L.cin * kTaps +
                                        (li == 2 ? kWidth * kWin : 0));
     auto kernel = li == 2 ? conv_fwd_kernel<true> : conv_fwd_kernel<false>;
     kernel<<<grid, kConvThreads, sm, s>>>(in, L.cin, X, n->wt + L.woff, n->params + L.boff, n->act[li],
-                                          n->wt + n->L[3].woff, n->params + n->L[3].boff, n->tile_max, n->tile_arg);
+                                          n->wt + n->L[3].woff, n->params + n->L[3].boff, n->tile_max, n->tile_arg,
+                                          const_cast<int*>(odd.at[li]), const_cast<int*>(odd.at[3]));
     FDR_LAUNCH_CHECK("conv_fwd_kernel");
     in = n->act[li];
   }
@@ -703,7 +773,7 @@ static int net_grad(fdr_propose_net* n, const float* x, const float* labels, int
   const size_t sm2 = sizeof(float) * (kMaxBins * kWidth + std::max(n->nt, kWidth) * kMaxInBins);
   sparse_weight_grad_kernel<<<dim3(4, B), kSparseThreads, sm2, s>>>(
       sg, x, n->act[0], n->act[1], n->act[2], n->dlogit, n->argmax, n->nt, X, n->L[0], n->L[1], n->L[2], n->L[3],
-      n->partial, n->nparams);
+      n->partial, n->nparams, odd_inputs(n));
   FDR_LAUNCH_CHECK("sparse_weight_grad_kernel");
   reduce_partials_kernel<<<(unsigned)cdiv(n->nparams, 128), 128, 0, s>>>(n->partial, B, n->nparams, n->grad);
   FDR_LAUNCH_CHECK("reduce_partials_kernel");
@@ -721,6 +791,7 @@ static void net_release(fdr_propose_net* n) {
   for (auto* a : n->act) cudaFree(a);
   cudaFree(n->tile_max);
   cudaFree(n->tile_arg);
+  cudaFree(n->odd);
   cudaFree(n->argmax);
   cudaFree(n->dlogit);
   cudaFree(n->gact);
@@ -778,6 +849,8 @@ int fdr_propose_create(fdr_propose_net** out, int nbins, int nt, int width, int 
   for (int i = 0; i < 3 && e == cudaSuccess; ++i) e = cudaMalloc(&n->act[i], sizeof(float) * act_elems);
   if (e == cudaSuccess) e = cudaMalloc(&n->tile_max, sizeof(float) * tile_elems);
   if (e == cudaSuccess) e = cudaMalloc(&n->tile_arg, sizeof(int) * tile_elems);
+  if (e == cudaSuccess)
+    e = cudaMalloc(&n->odd, sizeof(int) * tile_elems / kWin * ((size_t)n->nt + 2 * kWidth + 1));
   if (e == cudaSuccess) e = cudaMalloc(&n->dlogit, sizeof(float) * (size_t)max_batch * nwin);
   if (e == cudaSuccess) e = cudaMalloc(&n->gact, sizeof(SparseGrad) * (size_t)max_batch);
   if (e == cudaSuccess) e = cudaMalloc(&n->argmax, sizeof(int) * (size_t)max_batch * nwin);

@@ -41,3 +41,21 @@ def test_one_bin_for_all_windows(fdr, oracle):
     g, _ = net.gradients(torch.from_numpy(x).cuda(), torch.from_numpy(lab).cuda())
     _, ref = oracle.propose_loss_and_grad(net.get_state()["params"], x, lab, cin, half_weights=True)
     assert np.linalg.norm(g.cpu().numpy() - ref) <= TOL * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("X,at", [(300, 0), (300, 1), (300, 150), (300, 255), (300, 257), (300, 299), (256, 255)])
+def test_nan_outside_the_selected_bins(fdr, X, at):
+    """A NaN input makes every sum over the bins that it enters NaN (zero gradients included, up to
+    the end of the last tile of 256 bins), and no other: the hidden layers' ReLU takes it to 0."""
+    cin, ci = 16, 5
+    rng = np.random.default_rng(X + at)
+    net = fdr.proposal.ProposalNet(nbins=X, cin=cin, max_batch=2, seed=3)
+    x = rng.normal(0, 1, (2, cin, X)).astype(np.float32)
+    x[1, ci, at] = np.nan
+    lab = (rng.random((2, 16)) < 0.5).astype(np.float32)
+    g, _ = net.gradients(torch.from_numpy(x).cuda(), torch.from_numpy(lab).cuda())
+    bad = np.isnan(g.cpu().numpy())
+    want = np.zeros((32, cin, 5), bool)
+    for k in range(5):
+        want[:, ci, k] = 0 <= at + 2 - k < -(-X // 256) * 256
+    assert (bad[:want.size] == want.ravel()).all() and not bad[want.size:].any()
