@@ -64,7 +64,7 @@ intfdr_kernel(const float* __restrict__ spec, long long Nf, int Nt, int nrates,
 constexpr int kTiledMaxNt = 64;
 constexpr int kTiledMaxWords = 24576;  // shared-memory window floats (96 KB)
 
-struct TiledTable {
+struct alignas(16) TiledTable {  // rel is read four words at a time
   // rel[jj*Ntp + t], Ntp = Nt rounded up to 4: shift of rate jj at time t, minus lo_t (host); word of
   // win where the rate's channel n0 is at time t (in the launch)
   int32_t rel[kShiftParamWords];
