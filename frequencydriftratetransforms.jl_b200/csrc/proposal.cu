@@ -445,9 +445,10 @@ struct BinSet {
     }
     __syncthreads();
     const int i = t / 16, j = t % 16;  // w <= 13
+    const int total = start[n];        // before the barrier: the next call overwrites start after it
     if (i < n && j < start[i + 1] - start[i]) out[start[i] + j] = sel[i] + radius + 1 - (start[i + 1] - start[i]) + j;
     __syncthreads();
-    return start[n];
+    return total;
   }
 };
 // Index in the ascending list of bin x, or `none` if it is not there.
