@@ -242,7 +242,7 @@ unsigned magic_of(int d) { return d == 1 ? 0u : (unsigned)(((1ULL << 32) + d - 1
 
 }  // namespace
 
-bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, StageDesc* d) {
+bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, bool twiddles, StageDesc* d) {
   static const StagePlans plans;
   if (L < 2 || L > kStageElems || plans.count[L] == 0xff || plans.count[L] > kStageMax) return false;
   memset(d, 0, sizeof(*d));
@@ -265,10 +265,15 @@ bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, StageDesc* d) 
   int lg = 0;
   while ((L << (lg + 1)) <= kStageElems && lg < 8 && (int64_t(1) << lg) < nb) ++lg;
   while (lg > (rows ? 3 : 0) && cdiv(nb, int64_t(1) << lg) * groups < 2LL * sm_count()) --lg;
-  d->bpc_log2 = lg;
-  d->bpc = 1 << lg;
-  d->SS = (d->radix[0] * d->pitch + 15) / 16 * 16 + (d->bpc >= 16 ? 1 : 16 / d->bpc);
-  return true;
+  // (the padding and the twiddle tables can take more than the elements do: L = 52, 128 transforms)
+  for (;; --lg) {
+    d->bpc_log2 = lg;
+    d->bpc = 1 << lg;
+    d->SS = (d->radix[0] * d->pitch + 15) / 16 * 16 + (d->bpc >= 16 ? 1 : 16 / d->bpc);
+    const size_t bytes = stage_smem_bytes(*d) + (twiddles ? tw_bytes(d->L, d->bpc) : 0);
+    if (bytes <= kStageSmem) return true;
+    if (lg == 0) return false;
+  }
 }
 
 // Threads of a CTA: two rounds of butterflies of the widest stage, up to kStageThreads.
@@ -307,10 +312,6 @@ struct TwiddleTables {
   float2* lo;
   int nh;
 };
-__host__ __device__ constexpr int tw_rows(int L) { return ((L + 31) / 32) | 1; }
-__host__ __device__ inline size_t tw_bytes(int L, int bpc) {
-  return 16 + (size_t)bpc * (sizeof(float4) * tw_rows(L) + sizeof(float2) * 33);
-}
 
 template <int SIGN>
 __device__ __forceinline__ void fill_twiddles(const TwiddleTables& t, int bpc, int L, long long b1_0, double inv2N) {
@@ -428,7 +429,7 @@ int launch_stages(StageArgs& a, cudaStream_t s) {
   FDR_CUDA(cudaGetDevice(&dev));
   if (dev >= 64 || !attr_set[dev]) {
     FDR_CUDA(cudaFuncSetAttribute(fft_stage_kernel<SIGN, IN, OUT>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageSmem));
     if (dev < 64) attr_set[dev] = true;
   }
   const size_t smem = stage_smem_bytes(a.d) + (OUT == kOutTwiddle ? tw_bytes(a.d.L, a.d.bpc) : 0);
@@ -455,7 +456,7 @@ int fft_strided_inplace(float2* buf, long long L, long long sl, long long nb, lo
     return FDR_ERR_UNSUPPORTED_SIZE;
   }
   StageArgs a = blank_stages();
-  if (stage_plan(L, nb, 1, true, &a.d)) {
+  if (stage_plan(L, nb, 1, true, false, &a.d)) {
     a.in = a.out = buf;
     a.mul = mul;
     a.nb1 = nb;
@@ -629,7 +630,7 @@ static int real_stages(bool forward, const void* in, long long ldin, void* out, 
   a.ldi = ldin;
   a.ldo = ldout;
   if (N <= kMaxCtaElems) {
-    if (!stage_plan(N, np, 1, false, &a.d)) return FDR_OK;
+    if (!stage_plan(N, np, 1, false, false, &a.d)) return FDR_OK;
     a.nb1 = np;
     a.isl = a.osl = 1;
     a.pair_b1 = 1;
@@ -645,7 +646,8 @@ static int real_stages(bool forward, const void* in, long long ldin, void* out, 
   long long L1, L2;
   split_len(N, &L1, &L2);
   StageArgs b = a;
-  if (L1 == 0 || !stage_plan(L1, L2, np, true, &a.d) || !stage_plan(L2, L1, np, true, &b.d)) return FDR_OK;
+  if (L1 == 0 || !stage_plan(L1, L2, np, true, true, &a.d) || !stage_plan(L2, L1, np, true, false, &b.d))
+    return FDR_OK;
   *done = true;
   // Pass 1: n = n2 + L2*n1, DFT over n1 for each n2, twiddle, tmp[k1*L2 + n2]
   a.out = tmp;

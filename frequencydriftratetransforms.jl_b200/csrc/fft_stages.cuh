@@ -315,10 +315,18 @@ __device__ __forceinline__ void convolve_smem(const StageDesc& d, float2* sm, Fa
   }
 }
 
+// Tables of the four-step twiddles of a first pass (see TwiddleTables in fft_engine.cu), rows and bytes.
+__host__ __device__ constexpr int tw_rows(int L) { return ((L + 31) / 32) | 1; }
+__host__ __device__ inline size_t tw_bytes(int L, int bpc) {
+  return 16 + (size_t)bpc * (sizeof(float4) * tw_rows(L) + sizeof(float2) * 33);
+}
+
 // Fills d for `groups` sets of `nb` transforms of length L, neighbouring transforms of a set at
 // neighbouring addresses (rows: CTAs then take at least 8 of them, 64 bytes a row); false if L
-// has a prime factor above 13 or exceeds kStageElems.
-bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, StageDesc* d);
+// has a prime factor above 13 or exceeds kStageElems.  `twiddles`: the pass keeps twiddle tables
+// beside its transforms; both stay within kStageSmem.
+constexpr size_t kStageSmem = 112 * 1024;  // two CTAs per SM
+bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, bool twiddles, StageDesc* d);
 size_t stage_smem_bytes(const StageDesc& d);
 int stage_threads(const StageDesc& d);
 

@@ -288,7 +288,7 @@ static int zdt_conv(fdr_zdt* ws, float r0, int window, const double* wk, cudaStr
   *done = false;
   ConvArgs a;
   memset(&a, 0, sizeof(a));
-  if (!stage_plan(ws->Nl, ws->K, 1, true, &a.d)) return FDR_OK;
+  if (!stage_plan(ws->Nl, ws->K, 1, true, false, &a.d)) return FDR_OK;
   FDR_TRY(zdt_ensure_staged(ws, s));
   FDR_TRY(zdt_ensure_F(ws, s));
   FDR_TRY(get_roots(ws->Nl, &a.d.roots));
@@ -302,7 +302,7 @@ static int zdt_conv(fdr_zdt* ws, float r0, int window, const double* wk, cudaStr
   int dev = 0;
   FDR_CUDA(cudaGetDevice(&dev));
   if (dev >= 64 || !attr_set[dev]) {
-    FDR_CUDA(cudaFuncSetAttribute(zdt_conv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
+    FDR_CUDA(cudaFuncSetAttribute(zdt_conv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageSmem));
     if (dev < 64) attr_set[dev] = true;
   }
   zdt_conv_kernel<<<(unsigned)cdiv(ws->K, a.d.bpc), stage_threads(a.d), stage_smem_bytes(a.d), s>>>(a);
