@@ -38,15 +38,18 @@ __device__ __forceinline__ float2 phasor_ref(long long k, long long t, float r, 
 // one for each (k, t, r).  Their arguments are formed by the same rounded operations as in
 // phasor_ref, with cheaper instructions where they give the same value: for MULT (2k and t exact in
 // Float32) the rounded product Float32(2k) * Float32(t) is Float32(2kt), and for a power-of-two Nf
-// the quotient is the product with 1 / Nf.  For SMALL (every |argument| < 2^20 half-turns) the
+// the quotient is the product with 1 / Nf.  For a small rate (every |argument| < 2^19 half-turns) the
 // nearest quarter turn is the sum with 1.5 * 2^23 rounded, its low bits the quadrant, and the rest
-// is exact.  At Nf = 2^20, Nt = 16, 21 rates: 440 us with a thread per sum and sincospif, 246 us with
-// 8 rates per thread, 179 us with packed polynomials (70% of the FMA pipe).
+// is exact; the other rates, if any (LARGE: the bits of `large`), take cispif.  Each rate is decided
+// by itself, so that a column does not depend on the rates beside it.  At Nf = 2^20, Nt = 16, 21
+// rates: 440 us with a thread per sum and sincospif, 246 us with 8 rates per thread, 179 us with
+// packed polynomials (70% of the FMA pipe).
 constexpr int kRatesPerThread = 8;
 
-template <bool MULT, bool POW2, bool SMALL>
+template <bool MULT, bool POW2, bool LARGE>
 __global__ void __launch_bounds__(256) phasor_sum_kernel(const float2* __restrict__ F, long long K, int Nt,
-                                                         long long Nf, int nr, float2* __restrict__ S,
+                                                         long long Nf, int nr, unsigned large,
+                                                         float2* __restrict__ S,
                                                          const __grid_constant__ RateParams rp) {
   const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (k >= K) return;
@@ -64,16 +67,23 @@ __global__ void __launch_bounds__(256) phasor_sum_kernel(const float2* __restric
       if (j0 + 2 * q < nr) {  // uniform; rates past the last are zero
         const float2 x = pk_mul(pk_set(kt), make_float2(rp.r[j0 + 2 * q], rp.r[j0 + 2 * q + 1]));
         const float2 h = POW2 ? pk_mul(x, pk_set(inv)) : make_float2(__fdiv_rn(x.x, Nf_f), __fdiv_rn(x.y, Nf_f));
+        const float2 h2 = pk_add(h, h);
+        const float2 m = pk_add(h2, pk_set(12582912.f));
+        const float2 rest = csub(h2, pk_add(m, pk_set(-12582912.f)));
         float2 c, s;
-        if (SMALL) {
-          const float2 h2 = pk_add(h, h);
-          const float2 m = pk_add(h2, pk_set(12582912.f));
-          const float2 rest = csub(h2, pk_add(m, pk_set(-12582912.f)));
-          cis_quarter_pk(rest, __float_as_uint(m.x), __float_as_uint(m.y), c, s);
-        } else {
-          const float2 p0 = cispif(h.x), p1 = cispif(h.y);
-          c = make_float2(p0.x, p1.x);
-          s = make_float2(p0.y, p1.y);
+        cis_quarter_pk(rest, __float_as_uint(m.x), __float_as_uint(m.y), c, s);
+        if (LARGE) {
+          const unsigned two = large >> (j0 + 2 * q);  // uniform
+          if (two & 1) {
+            const float2 p = cispif(h.x);
+            c.x = p.x;
+            s.x = p.y;
+          }
+          if (two & 2) {
+            const float2 p = cispif(h.y);
+            c.y = p.x;
+            s.y = p.y;
+          }
         }
         // cmul_rn and a rounded sum, for both rates
         ax[q] = pk_add(ax[q], csub(pk_mul(fx, c), pk_mul(fy, s)));
@@ -196,15 +206,16 @@ int fdr_fftfdr(fdr_fft_ws* ws, const float* rates, int64_t Nr, float* fdr, fdr_s
     memset(&rp, 0, sizeof(rp));
     for (int i = 0; i < nr; ++i) rp.r[i] = rates[j0 + i];
     const bool mult = 2 * ws->K < (1LL << 24) && ws->Nt < (1LL << 24), pow2 = is_pow2(ws->Nf);
-    float most = 0.f;  // not a number: not small
-    for (int i = 0; i < nr; ++i) most = fabsf(rp.r[i]) <= most ? most : fabsf(rp.r[i]);
-    const bool small = (double)most * (double)ws->Nt < (double)(1 << 19);  // k / Nf <= 1/2
+    unsigned large = 0;  // rates with |argument| = 2 k t |r| / Nf possibly 2^19 or more, NaN among them
+    static_assert(kRateChunk == 32, "one bit per rate");
+    for (int i = 0; i < nr; ++i)
+      if (!((double)fabsf(rp.r[i]) * (double)ws->Nt < (double)(1 << 19))) large |= 1u << i;
     const dim3 grid((unsigned)cdiv(ws->K, 256), (unsigned)cdiv(nr, kRatesPerThread));
-    auto kernel = !small ? (mult ? (pow2 ? phasor_sum_kernel<true, true, false> : phasor_sum_kernel<true, false, false>)
-                                 : (pow2 ? phasor_sum_kernel<false, true, false> : phasor_sum_kernel<false, false, false>))
-                         : (mult ? (pow2 ? phasor_sum_kernel<true, true, true> : phasor_sum_kernel<true, false, true>)
-                                 : (pow2 ? phasor_sum_kernel<false, true, true> : phasor_sum_kernel<false, false, true>));
-    kernel<<<grid, 256, 0, s>>>(ws->F, ws->K, (int)ws->Nt, ws->Nf, nr, ws->S, rp);
+    auto kernel = large ? (mult ? (pow2 ? phasor_sum_kernel<true, true, true> : phasor_sum_kernel<true, false, true>)
+                                : (pow2 ? phasor_sum_kernel<false, true, true> : phasor_sum_kernel<false, false, true>))
+                        : (mult ? (pow2 ? phasor_sum_kernel<true, true, false> : phasor_sum_kernel<true, false, false>)
+                                : (pow2 ? phasor_sum_kernel<false, true, false> : phasor_sum_kernel<false, false, false>));
+    kernel<<<grid, 256, 0, s>>>(ws->F, ws->K, (int)ws->Nt, ws->Nf, nr, large, ws->S, rp);
     FDR_LAUNCH_CHECK("phasor_sum_kernel");
     FDR_TRY(irfft_columns(ws->S, ws->K, nr, ws->Nf, fdr + j0 * ws->Nf, ws->Nf, ws->rscratch,
                           ws->rscratch_pairs, s));
