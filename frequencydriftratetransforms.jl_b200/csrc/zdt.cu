@@ -311,17 +311,20 @@ static int zdt_conv(fdr_zdt* ws, float r0, int window, const double* wk, cudaStr
   return FDR_OK;
 }
 
-// One staged ZDT (zdtfdr.jl:355-358) for a given r0 into dest.
+// One staged ZDT (zdtfdr.jl:355-358) for a given r0 into dest.  With stage timing on, the three
+// functions run one by one, so that each has a time of its own.
 int zdt_staged_run(fdr_zdt* ws, float r0, float* dest, int window, const double* wk, double* acc,
                    cudaStream_t s) {
-  bool done;
-  FDR_TRY(zdt_conv(ws, r0, window, wk, s, &done));
-  if (!done) FDR_TRY(zdt_preprocess(ws, r0, s));
-  zdt_mark(ws, "preprocess", s);  // with convolve! and postprocess! where one kernel runs all
-  if (!done) FDR_TRY(zdt_convolve(ws, s));
-  zdt_mark(ws, "convolve", s);
-  if (!done) FDR_TRY(zdt_postprocess(ws, window, wk, s));
-  zdt_mark(ws, "postprocess", s);
+  bool done = false;
+  if (!ws->timing) FDR_TRY(zdt_conv(ws, r0, window, wk, s, &done));
+  if (!done) {
+    FDR_TRY(zdt_preprocess(ws, r0, s));
+    zdt_mark(ws, "preprocess", s);
+    FDR_TRY(zdt_convolve(ws, s));
+    zdt_mark(ws, "convolve", s);
+    FDR_TRY(zdt_postprocess(ws, window, wk, s));
+    zdt_mark(ws, "postprocess", s);
+  }
   FDR_TRY(zdt_output(ws, dest, s));
   if (acc) FDR_TRY(moments_accumulate(dest, ws->Nf, ws->Nr, acc, s));
   zdt_mark(ws, "output", s);

@@ -215,7 +215,9 @@ int fdr_zdtfdr_blocks_protohits(fdr_zdt* ws, const float* spectrogram, const int
                                 double threshold, int snr, int64_t* hits, int64_t capacity,
                                 int64_t* count, double* threshold_used, fdr_stream_t stream);
 /* Per-stage device time of the last fdr_zdt_execute call (enable with
-   fdr_zdt_set_timing(ws, 1)); times[i] in milliseconds, names via stage_names. */
+   fdr_zdt_set_timing(ws, 1)); times[i] in milliseconds, names via stage_names.  Staged calls
+   with timing enabled run preprocess!, convolve! and postprocess! one by one instead of in one
+   kernel: each stage has its own time, their sum is more than an untimed call takes. */
 int fdr_zdt_set_timing(fdr_zdt* ws, int enable);
 int fdr_zdt_stage_times(fdr_zdt* ws, float* times_ms, int max_stages, int* nstages,
                         const char** stage_names);
