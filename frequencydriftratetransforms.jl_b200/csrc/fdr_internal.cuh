@@ -132,6 +132,13 @@ __device__ __forceinline__ void pk_cmul(float2 ax, float2 ay, float2 bx, float2 
   y = pk_fma(ax, by, pk_mul(ay, bx));
 }
 
+// h = 2^-32 turns to the nearest quarter turn *q (0 to 3) and the rest, -2^29 <= rest < 2^29.  The
+// subtraction wraps: h from 0x60000000 on is nearest to half a turn, whose 2^31 is no int.
+__host__ __device__ __forceinline__ int quarter_rest(int h, unsigned* q) {
+  *q = ((unsigned)h + (1u << 29)) >> 30;
+  return (int)((unsigned)h - (*q << 30));
+}
+
 // cos and sin of x + q quarter turns for two values, |x| <= 1/2: polynomials in x^2 fitted on
 // Chebyshev nodes (degrees 7 and 8; the leading sine coefficient pi/2 is held in two parts).  Errors
 // over all 32-bit phases: 1.4e-8 (sin) and 1.9e-8 (cos) rms, 7.1e-8 at most, against 1.4e-8 and

@@ -73,8 +73,9 @@ struct FusedTables {
 // sincospif with their 64-bit conversions took about 80.
 __device__ __forceinline__ void cis_turn_pk(unsigned long long ph0, unsigned long long ph1, float2& c, float2& s) {
   const int h0 = (int)((ph0 + 0x80000000ull) >> 32), h1 = (int)((ph1 + 0x80000000ull) >> 32);
-  const unsigned q0 = ((unsigned)h0 + (1u << 29)) >> 30, q1 = ((unsigned)h1 + (1u << 29)) >> 30;
-  const float2 x = pk_mul(make_float2(__int2float_rn(h0 - (int)(q0 << 30)), __int2float_rn(h1 - (int)(q1 << 30))),
+  unsigned q0, q1;
+  const int r0 = quarter_rest(h0, &q0), r1 = quarter_rest(h1, &q1);
+  const float2 x = pk_mul(make_float2(__int2float_rn(r0), __int2float_rn(r1)),
                           pk_set(9.31322574615478515625e-10f));  // 2^-30
   cis_quarter_pk(x, q0, q1, c, s);
 }
