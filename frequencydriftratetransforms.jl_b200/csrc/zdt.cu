@@ -573,19 +573,17 @@ static int zdt_execute_blocks(fdr_zdt* ws, const float* spectrogram, const int32
   FDR_CHECK_ARG(4 * nblocks <= ws->W_pairs, "zdtfdr blocks: more than Nr/8 blocks");
   FDR_TRY(check_pair_aligned(dest, "zdtfdr blocks: dest"));
   if (spectrogram) FDR_TRY(check_pair_aligned(spectrogram, "zdtfdr blocks: spectrogram"));
-  // the kernels take the rate index of each block's first rate
-  std::vector<int> base((size_t)nblocks);
-  for (int64_t i = 0; i < nblocks; ++i) base[(size_t)i] = 8 * (int)blocks[i];
-  int* d_blk = nullptr;
-  FDR_TRY(scratch_alloc((void**)&d_blk, sizeof(int) * nblocks, s));
-  int st = upload_words(d_blk, base.data(), sizeof(int) * nblocks, s);
+  const RateRounds rounds = zdt_fused_rounds(ws, blocks, nblocks);
+  int* d_rounds = nullptr;
+  FDR_TRY(scratch_alloc((void**)&d_rounds, sizeof(int) * rounds.words.size(), s));
+  int st = upload_words(d_rounds, rounds.words.data(), sizeof(int) * rounds.words.size(), s);
   zdt_mark(ws, "start", s);
   if (st == FDR_OK && spectrogram) {
     st = fdr_zdt_input(ws, spectrogram, s);
     zdt_mark(ws, "input", s);
   }
-  if (st == FDR_OK) st = zdt_fused_run_blocks(ws, d_blk, nblocks, dest, window, custom_window, acc, s);
-  scratch_free(d_blk, s);
+  if (st == FDR_OK) st = zdt_fused_run_blocks(ws, d_rounds, rounds.both, nblocks, dest, window, custom_window, acc, s);
+  scratch_free(d_rounds, s);
   return st;
 }
 

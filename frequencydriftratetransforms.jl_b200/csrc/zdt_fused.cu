@@ -33,6 +33,8 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include "fft_device.cuh"
 #include "fft_engine.cuh"
 #include "umma.cuh"
@@ -264,8 +266,7 @@ struct CztArgs {
   float2* W;          // [pair][k1][na] for pairs [0, npairs)
   float2* F;          // A->F mode output (K x Nt) or NULL
   const double* wk;   // custom window values (K) or NULL
-  const int* blk_base;  // SUBSET kernels: rate index (on the r0 + j*dr grid) of each 8-rate
-                        // block's first rate, a multiple of 8
+  const int* rounds;  // SUBSET kernels: kRoundWords words for each round of 4 rate pairs, see fused_rounds
   long long N;
   int P, Nt, NP, Nr, npairs, window;
   int half;             // h: super pairs of the whole grid (rates 2h + m and 2h - 1 - m)
@@ -388,24 +389,49 @@ __device__ __forceinline__ float nyquist_value(const CztArgs& a, const float2* g
   return s.x;
 }
 
-// First rate pair of W and rate of its sequence pair u (0..3) of an 8-rate block: the upper and
-// lower rate pairs of super pairs 2 blk and 2 blk + 1, or four consecutive pairs of a subset.
-template <bool SUBSET>
+// A round of a rate subset (fused_rounds): words 4 to 7 are the rate pairs of W that its sequence
+// pairs 0 to 3 go to.  Words 0 to 3: four times 2 i + (1 for the lower rate pair of super pair i, 0
+// for the upper), or, with -1 in word 2, two super pairs whose upper and lower pairs are both wanted.
+constexpr int kRoundWords = 8;
+// What a czt kernel computes: the whole grid, rounds of single rate pairs only, or any rounds.
+// (The kernel for any rounds takes single pairs 4 to 6% slower than the one that has only them.)
+enum { kWhole, kSingles, kRounds };
+
+// Rate pair of W of the sequence pair u (0..3) of an 8-rate block: the upper and lower rate pairs
+// of super pairs 2 blk and 2 blk + 1, or what the round says.
+template <int SUBSET>
 __device__ __forceinline__ int block_pair(const CztArgs& a, int blk, int u) {
-  if (SUBSET) return 4 * blk + u;
+  if (SUBSET) return __ldg(a.rounds + kRoundWords * blk + 4 + u);
   const int i = 2 * blk + (u >> 1);
   const int p = (u & 1) ? a.half - 1 - i : a.half + i;
   return i < a.half && p < a.npairs ? p : -1;
 }
+// block_pair of all four sequence pairs, fetched before a transform whose emission asks for them many
+// times (looked up at each emission they took 3% of a subset call at Nf = 2^20, Nt = 16).
+template <int SUBSET>
+struct BlockPairs {
+  int p[4];
+  __device__ __forceinline__ BlockPairs(const CztArgs& a, int blk) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) p[u] = block_pair<SUBSET>(a, blk, u);
+  }
+  __device__ __forceinline__ int operator[](int u) const { return u < 2 ? (u ? p[1] : p[0]) : (u == 2 ? p[2] : p[3]); }
+};
+// Rate pair of the whole grid that sequence pair u of a round computes.
+__device__ __forceinline__ int round_grid_pair(const CztArgs& a, int blk, int u) {
+  const int* const r = a.rounds + kRoundWords * blk;
+  const int v = __ldg(r + 2) < 0 ? 2 * __ldg(r + (u >> 1)) + (u & 1) : __ldg(r + u);
+  return (v & 1) ? a.half - 1 - (v >> 1) : a.half + (v >> 1);
+}
 
 // The real-only Nyquist bin of a block's 8 rates, one lane each (tid < 8), as floats of the
 // packed sequences: value(u, hh, v).
-template <bool SUBSET, class Put>
+template <int SUBSET, class Put>
 __device__ __forceinline__ void nyquist_block(const CztArgs& a, const float2* gnyq, int blk, int lane, Put put) {
   const int u = lane >> 1, hh = lane & 1;
   const int p = block_pair<SUBSET>(a, blk, u);
   if (p < 0) return;
-  const long long j = SUBSET ? (long long)__ldg(a.blk_base + blk) + 2 * u + hh : 2LL * p + hh;
+  const long long j = 2LL * (SUBSET ? round_grid_pair(a, blk, u) : p) + hh;
   const float v = nyquist_value(a, gnyq, j) * window_value(a, a.N / 2);
   put(u, hh, 2 * p + hh < a.Nr ? v : 0.f);
 }
@@ -525,11 +551,17 @@ struct FoldPhase {
   unsigned long long rh0, rh1;  // k Rh of the two bins
   int c;
   float2 zx, zy, rx, ry;        // at m = 4 * group
-  __device__ __forceinline__ void start(int group) {
+  __device__ __forceinline__ void start_z(int group) {
     const unsigned long long n = 8ull * (unsigned)group + 1ull;
-    const unsigned long long p0 = n * rh0, p1 = n * rh1;
-    cis_turn_pk(p0, p1, zx, zy);
-    cis_turn_pk((unsigned)c * p0, (unsigned)c * p1, rx, ry);
+    cis_turn_pk(n * rh0, n * rh1, zx, zy);
+  }
+  __device__ __forceinline__ void start_r(int group) {
+    const unsigned long long n = (8ull * (unsigned)group + 1ull) * (unsigned)c;
+    cis_turn_pk(n * rh0, n * rh1, rx, ry);
+  }
+  __device__ __forceinline__ void start(int group) {
+    start_z(group);
+    start_r(group);
   }
 };
 // The factors of m & 3 = q > 0: exp(2 pi i 2 q k Rh) and its c-th power.
@@ -564,34 +596,85 @@ struct FoldPhases : FoldPhase {
   }
 };
 
+// C and D (with F'_0's term), rotations and their negated sines of M values of m.
+template <int M>
+struct FoldValues {
+  float2 cx[M], cy[M], dx[M], dy[M], rx[M], ry[M], nry[M];
+  __device__ __forceinline__ void finish(const float4* g, int Nt) {
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      nry[i] = pk_neg(ry[i]);
+      fold_first_step(g, Nt, rx[i], nry[i], cx[i], cy[i], dx[i], dy[i]);
+    }
+  }
+  __device__ __forceinline__ void plus(int i, float2& x, float2& y) const {
+    fold_plus(cx[i], cy[i], dx[i], dy[i], rx[i], ry[i], nry[i], x, y);
+  }
+  __device__ __forceinline__ void minus(int i, float2& x, float2& y) const {
+    fold_minus(cx[i], cy[i], dx[i], dy[i], rx[i], ry[i], nry[i], x, y);
+  }
+};
+// Those of m = 4 group + q0 + i (start(group) first).
+template <int M>
+__device__ __forceinline__ void fold_values_smem(const FoldPhases& f, const float4* g, int stride, int Nt, int q0,
+                                                 FoldValues<M>& o) {
+  float2 zx[M], zy[M];
+#pragma unroll
+  for (int i = 0; i < M; ++i) f.z_of(q0 + i, zx[i], zy[i]);
+  fold_sums_smem<M>(g, stride, Nt, zx, zy, o.cx, o.cy, o.dx, o.dy);
+#pragma unroll
+  for (int i = 0; i < M; ++i) f.r_of(q0 + i, o.rx[i], o.ry[i]);
+  o.finish(g, Nt);
+}
 // Both rates of the M values m = 4 group + q0 + i of a bin pair (start(group) first).
 template <int M>
 __device__ __forceinline__ void fold_pairs_smem(const FoldPhases& f, const float4* g, int stride, int Nt, int q0,
                                                 float2 (&px)[M], float2 (&py)[M], float2 (&mx)[M], float2 (&my)[M]) {
-  float2 zx[M], zy[M], cx[M], cy[M], dx[M], dy[M];
-#pragma unroll
-  for (int i = 0; i < M; ++i) f.z_of(q0 + i, zx[i], zy[i]);
-  fold_sums_smem<M>(g, stride, Nt, zx, zy, cx, cy, dx, dy);
+  FoldValues<M> o;
+  fold_values_smem<M>(f, g, stride, Nt, q0, o);
 #pragma unroll
   for (int i = 0; i < M; ++i) {
-    float2 rx, ry;
-    f.r_of(q0 + i, rx, ry);
-    const float2 nry = pk_neg(ry);
-    fold_first_step(g, Nt, rx, nry, cx[i], cy[i], dx[i], dy[i]);
-    fold_plus(cx[i], cy[i], dx[i], dy[i], rx, ry, nry, px[i], py[i]);
-    fold_minus(cx[i], cy[i], dx[i], dy[i], rx, ry, nry, mx[i], my[i]);
+    o.plus(i, px[i], py[i]);
+    o.minus(i, mx[i], my[i]);
   }
 }
-// One rate j of the grid (SUBSET kernels).
-__device__ __forceinline__ void fold_rate_smem(FoldPhases& f, const float4* g, int stride, int Nt, int j, int half,
-                                               float2& x, float2& y) {
-  const int d = j - 2 * half;
-  const int m = d >= 0 ? d : -1 - d;
-  f.start(m >> 2);
-  float2 px[1], py[1], mx[1], my[1];
-  fold_pairs_smem<1>(f, g, stride, Nt, m & 3, px, py, mx, my);
-  x = d >= 0 ? px[0] : mx[0];
-  y = d >= 0 ? py[0] : my[0];
+// The two values of m of each of super pairs i0 and i1 (SUBSET kernels).  Four values share the loads
+// of F; a rate at a time they bound the sums (two 16-byte loads for 8 packed multiply-adds).
+__device__ __forceinline__ void fold_super_smem(FoldPhases& f, const float4* g, int stride, int Nt, int i0, int i1,
+                                                FoldValues<4>& o) {
+  if (!(i0 & 1) && i1 == i0 + 1) {  // uniform, as all branches here: one group
+    f.start(i0 >> 1);
+    fold_values_smem<4>(f, g, stride, Nt, 0, o);
+    return;
+  }
+  float2 zx[4], zy[4];
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    const int i = p ? i1 : i0;
+    f.start_z(i >> 1);
+    f.z_of(2 * (i & 1), zx[2 * p], zy[2 * p]);
+    f.z_of(2 * (i & 1) + 1, zx[2 * p + 1], zy[2 * p + 1]);
+  }
+  fold_sums_smem<4>(g, stride, Nt, zx, zy, o.cx, o.cy, o.dx, o.dy);
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    const int i = p ? i1 : i0;
+    f.start_r(i >> 1);
+    f.r_of(2 * (i & 1), o.rx[2 * p], o.ry[2 * p]);
+    f.r_of(2 * (i & 1) + 1, o.rx[2 * p + 1], o.ry[2 * p + 1]);
+  }
+  o.finish(g, Nt);
+}
+// Super pair p (0 or 1) of o: the two rates of its upper or lower rate pair, in their order.
+__device__ __forceinline__ void rates_of(const FoldValues<4>& o, int p, bool lower, float2& ax, float2& ay, float2& bx,
+                                         float2& by) {
+  if (lower) {
+    o.minus(2 * p + 1, ax, ay);
+    o.minus(2 * p, bx, by);
+  } else {
+    o.plus(2 * p, ax, ay);
+    o.plus(2 * p + 1, bx, by);
+  }
 }
 
 // F'_t = F_t exp(2 pi i t theta) in place, then G_u and H_u in the places of F'_{c-u} and F'_{c+u},
@@ -635,14 +718,14 @@ __device__ __forceinline__ void fold_smem(const CztArgs& a, float4* gs4, int nbp
 // Kernel B: grid (P/2, rate groups), Q/2 threads.
 // ------------------------------------------------------------------------------------
 // WINDOWED = false: the rectangular window (weights 1, skipped: the same FDR bit for bit).
-// SUBSET: the 8-rate blocks at a.blk_base instead of the whole grid.
+// SUBSET: the rounds at a.rounds instead of the whole grid.
 // Per CTA and 8-rate block: the sums of 4 values of m, two rates each, two rates packed per
 // complex sequence (Hermitian halves at k and its mirror), inverse DFT_Q, W.  One bin of each
 // residue per thread, so that their F (4 floats a step) stays in registers; 128 of them allow 16
 // warps per SM.  At Nf = 2^20, Nt = 16, 129 rates (Q = 512): 381 -> 325 us in the call against
 // Horner's rule per rate, 239 -> 213 M warp instructions; bound by their issue (58% of the cycles,
 // FMA pipe 50%) between the block barriers, not by the 555 MB moved (24% of the copy rate).
-template <int Q, int NTR, bool WINDOWED, bool SUBSET>
+template <int Q, int NTR, bool WINDOWED, int SUBSET>
 __global__ void __launch_bounds__(Q / 2, (Q <= 512 ? 2 : 1)) zdtf_czt_kernel(CztArgs a) {
   constexpr int T = Q / 2;
   constexpr int SS = b_stride<Q>();
@@ -791,27 +874,44 @@ __global__ void __launch_bounds__(Q / 2, (Q <= 512 ? 2 : 1)) zdtf_czt_kernel(Czt
         }
       }
     } else {
-      const int jg = __ldg(a.blk_base + blk);
+      const int* const round = a.rounds + kRoundWords * blk;
       int group = -1;
-#pragma unroll
-      for (int u = 0; u < kRatesPerBlock / 2; ++u) {
-        float2 vx[2], vy[2];
+      if (SUBSET == kRounds && __ldg(round + 2) < 0) {  // all branches uniform
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const int d = jg + 2 * u + e - 2 * a.half;
-          const int m = d >= 0 ? d : -1 - d;
-          if ((m >> 2) != group) {  // uniform over the CTA
-            group = m >> 2;
-            fp.start(group);
+          const int i = __ldg(round + e);
+          if ((i >> 1) != group) fp.start(group = i >> 1);
+          float2 px[2], py[2], mx[2], my[2];
+#pragma unroll
+          for (int v = 0; v < 2; ++v) {
+            float2 zx, zy, rx, ry, cx, cy, dx, dy;
+            phase(2 * (i & 1) + v, zx, zy, rx, ry);
+            const float2 nry = pk_neg(ry);
+            fold_sums<NTR>(Gx, Gy, zx, zy, rx, nry, cx, cy, dx, dy);
+            fold_plus(cx, cy, dx, dy, rx, ry, nry, px[v], py[v]);
+            fold_minus(cx, cy, dx, dy, rx, ry, nry, mx[v], my[v]);
           }
-          float2 zx, zy, rx, ry, cx, cy, dx, dy;
-          phase(m & 3, zx, zy, rx, ry);
-          const float2 nry = pk_neg(ry);
-          fold_sums<NTR>(Gx, Gy, zx, zy, rx, nry, cx, cy, dx, dy);
-          if (d >= 0) fold_plus(cx, cy, dx, dy, rx, ry, nry, vx[e], vy[e]);
-          else fold_minus(cx, cy, dx, dy, rx, ry, nry, vx[e], vy[e]);
+          put_pair(2 * e, px[0], py[0], px[1], py[1]);
+          put_pair(2 * e + 1, mx[1], my[1], mx[0], my[0]);
         }
-        put_pair(u, vx[0], vy[0], vx[1], vy[1]);
+      } else {
+#pragma unroll
+        for (int u = 0; u < kRatesPerBlock / 2; ++u) {
+          const int word = __ldg(round + u), i = word >> 1;
+          if ((i >> 1) != group) fp.start(group = i >> 1);
+          float2 x[2], y[2];
+#pragma unroll
+          for (int v = 0; v < 2; ++v) {
+            float2 zx, zy, rx, ry, cx, cy, dx, dy;
+            phase(2 * (i & 1) + v, zx, zy, rx, ry);
+            const float2 nry = pk_neg(ry);
+            fold_sums<NTR>(Gx, Gy, zx, zy, rx, nry, cx, cy, dx, dy);
+            if (word & 1) fold_minus(cx, cy, dx, dy, rx, ry, nry, x[v], y[v]);
+            else fold_plus(cx, cy, dx, dy, rx, ry, nry, x[v], y[v]);
+          }
+          if (word & 1) put_pair(u, x[1], y[1], x[0], y[0]);
+          else put_pair(u, x[0], y[0], x[1], y[1]);
+        }
       }
     }
     if (c == 0 && tid < kRatesPerBlock)
@@ -821,8 +921,9 @@ __global__ void __launch_bounds__(Q / 2, (Q <= 512 ? 2 : 1)) zdtf_czt_kernel(Czt
     __syncthreads();
     // inverse DFT_Q; its last pass writes W (with the inter-pass twiddle and 1/Nf) directly
     const int k1a = k1s[0], k1b = k1s[1];
+    const BlockPairs<SUBSET> pairs(a, blk);
     stockham_passes_emit_pp<Q, kRatesPerBlock, SS, T, +1, 1>(hb, ob, twt, [&](int seq, int na, float2 v) {
-      const int p = block_pair<SUBSET>(a, blk, seq >> 1), side = seq & 1;
+      const int p = SUBSET ? pairs[seq >> 1] : block_pair<SUBSET>(a, blk, seq >> 1), side = seq & 1;
       const long long at = ((long long)p * P + (side ? k1b : k1a)) * Q + na;
       if (p >= 0 && FDR_DBG_OK(at < (long long)a.npairs * P * Q)) a.W[at] = cmul(v, twr[side * Q + na]);
     });
@@ -956,7 +1057,34 @@ __device__ __forceinline__ void put_rate_pair(float2* seq, int side, int k20, co
   }
 }
 
-template <int Q, int NT, bool SUBSET>
+// The sums of a round of a rate subset: put(u, ...) receives sequence pair u's two rates; ready() is
+// called before the first.
+template <int SUBSET, class Ready, class Put>
+__device__ __forceinline__ void round_sums(const CztArgs& a, int blk, FoldPhases& f, const float4* g, int stride,
+                                           Ready ready, Put put) {
+  const int* const round = a.rounds + kRoundWords * blk;
+  const bool both = SUBSET == kRounds && __ldg(round + 2) < 0;
+#pragma unroll 1
+  for (int e = 0; e < (both ? 1 : 2); ++e) {
+    const int w0 = __ldg(round + 2 * e), w1 = __ldg(round + 2 * e + 1);
+    FoldValues<4> o;
+    fold_super_smem(f, g, stride, a.Nt, both ? w0 : w0 >> 1, both ? w1 : w1 >> 1, o);
+    if (e == 0) ready();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const bool lower = !both && ((i ? w1 : w0) & 1);
+      float2 ax, ay, bx, by;
+      rates_of(o, i, lower, ax, ay, bx, by);
+      put(both ? 2 * i : 2 * e + i, ax, ay, bx, by);
+      if (both) {
+        rates_of(o, i, true, ax, ay, bx, by);
+        put(2 * i + 1, ax, ay, bx, by);
+      }
+    }
+  }
+}
+
+template <int Q, int NT, int SUBSET>
 __global__ void __launch_bounds__(CztSmemShape<Q>::T, 1) zdtf_czt_smem_kernel(CztArgs a) {
   using SH = CztSmemShape<Q>;
   constexpr int T = SH::T;
@@ -1004,11 +1132,18 @@ __global__ void __launch_bounds__(CztSmemShape<Q>::T, 1) zdtf_czt_smem_kernel(Cz
     float2 px[2] = {zero, zero}, py[2] = {zero, zero}, mx[2] = {zero, zero}, my[2] = {zero, zero};
     if (SUBSET) {
       if (rg < 2) {
-        const int j = __ldg(a.blk_base + blk) + 4 * rg;  // pairs 2 rg (px) and 2 rg + 1 (mx, swapped)
-        fold_rate_smem(fp, g, Q / 2, Nt, j, a.half, px[0], py[0]);
-        fold_rate_smem(fp, g, Q / 2, Nt, j + 1, a.half, px[1], py[1]);
-        fold_rate_smem(fp, g, Q / 2, Nt, j + 2, a.half, mx[1], my[1]);
-        fold_rate_smem(fp, g, Q / 2, Nt, j + 3, a.half, mx[0], my[0]);
+        const int* const round = a.rounds + kRoundWords * blk;
+        if (__ldg(round + 2) < 0) {
+          const int i = __ldg(round + rg);
+          fp.start(i >> 1);
+          fold_pairs_smem<2>(fp, g, Q / 2, Nt, 2 * (i & 1), px, py, mx, my);
+        } else {  // sequence pairs 2 rg (px) and 2 rg + 1 (mx, its rates the other way round)
+          const int w0 = __ldg(round + 2 * rg), w1 = __ldg(round + 2 * rg + 1);
+          FoldValues<4> o;
+          fold_super_smem(fp, g, Q / 2, Nt, w0 >> 1, w1 >> 1, o);
+          rates_of(o, 0, w0 & 1, px[0], py[0], px[1], py[1]);
+          rates_of(o, 1, w1 & 1, mx[1], my[1], mx[0], my[0]);
+        }
       }
     } else if (rg < 2 && 2 * blk + rg < a.half) {
       fp.start(blk);
@@ -1028,8 +1163,9 @@ __global__ void __launch_bounds__(CztSmemShape<Q>::T, 1) zdtf_czt_smem_kernel(Cz
       });
     __syncthreads();
     const int k1a = k1s[0], k1b = k1s[1];
+    const BlockPairs<SUBSET> pairs(a, blk);
     smem_fft_emit<Q, kRatesPerBlock, SS, T, +1>(buf, twt, [&](int seq, int na, float2 v) {
-      const int p = block_pair<SUBSET>(a, blk, seq >> 1), sd = seq & 1;
+      const int p = SUBSET ? pairs[seq >> 1] : block_pair<SUBSET>(a, blk, seq >> 1), sd = seq & 1;
       const long long at = ((long long)p * P + (sd ? k1b : k1a)) * Q + na;
       if (p >= 0 && FDR_DBG_OK(at < (long long)a.npairs * P * Q)) a.W[at] = cmul(v, twr[sd * Q + na]);
     });
@@ -1070,7 +1206,7 @@ struct CztWsShape {
 };
 constexpr int kBarFull = 1, kBarEmpty = 3, kBarFft = 5;
 
-template <int Q, int NT, bool SUBSET>
+template <int Q, int NT, int SUBSET>
 __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArgs a) {
   using SH = CztWsShape<Q>;
   constexpr int T = SH::T, H = SH::H, HG = SH::HG, RG = SH::RG, I = SH::I, SS = SH::SS;
@@ -1125,15 +1261,9 @@ __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArg
         }
       };
       if (SUBSET) {
-        wait_empty();
-        const int j = __ldg(a.blk_base + blk);
-#pragma unroll 1
-        for (int u = 0; u < kRatesPerBlock / 2; ++u) {
-          float2 ax, ay, bx, by;
-          fold_rate_smem(fp, g, Q / 2, Nt, j + 2 * u, a.half, ax, ay);
-          fold_rate_smem(fp, g, Q / 2, Nt, j + 2 * u + 1, a.half, bx, by);
+        round_sums<SUBSET>(a, blk, fp, g, Q / 2, wait_empty, [&](int u, float2 ax, float2 ay, float2 bx, float2 by) {
           put_rate_pair<SS>(hb + 2 * u * SS, side, k20, ms, mk2, dc, win, ax, ay, bx, by);
-        }
+        });
       } else {
         float2 px[4], py[4], mx[4], my[4];
         fp.start(blk);
@@ -1163,8 +1293,9 @@ __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArg
       const int blk = blk0 + ib;
       float2* const hb = (ib & 1) ? buf1 : buf0;
       if (ib & 1) named_sync<kBarFull + 1, BT>(); else named_sync<kBarFull, BT>();
+      const BlockPairs<SUBSET> pairs(a, blk);
       group_fft_emit<Q, kRatesPerBlock, SS, I, +1, kBarFft, 1>(hb, twt, ltid, [&](int seq, int na, float2 v) {
-        const int p = block_pair<SUBSET>(a, blk, seq >> 1), sd = seq & 1;
+        const int p = SUBSET ? pairs[seq >> 1] : block_pair<SUBSET>(a, blk, seq >> 1), sd = seq & 1;
         const long long at = ((long long)p * P + (sd ? k1b : k1a)) * Q + na;
         if (p >= 0 && FDR_DBG_OK(at < (long long)a.npairs * P * Q)) a.W[at] = cmul(v, twr[sd * Q + na]);
       });
@@ -1181,7 +1312,7 @@ __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArg
 // bins (256 KB) does not fit one CTA, so a cluster of two CTAs shares the residue pair.  CTA
 // rank s keeps F of side s (residue k1 or P - k1: 256 bins, 128 KB) and evaluates the sums for
 // them.  Of a super pair's two rate pairs the upper one belongs to rank 0 and the lower one to
-// rank 1 (of a rate subset, one block to each); every CTA writes its sums, at the direct and
+// rank 1 (of a rate subset, one round to each); every CTA writes its sums, at the direct and
 // the mirror positions, into the owner's rate-block buffer through distributed shared memory.
 // 256 sum threads take a bin pair and the 4 values of m of one of two blocks; the other 256
 // threads meanwhile run the inverse DFT_Q of the two blocks before (this CTA's four rate pairs,
@@ -1274,7 +1405,7 @@ struct CztClShape {
 // this form (510 M warp instructions, FMA pipe 40%).  Bound by the sum threads: two warps per
 // scheduler at 128 registers wait for shared-memory loads and for each other at the barrier; 512 of
 // them at 80 registers spilled (1.35 ms).
-template <bool SUBSET>
+template <int SUBSET>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CztClShape::T, 1)
 zdtf_czt_cl_kernel(CztArgs a) {
   using SH = CztClShape;
@@ -1325,15 +1456,10 @@ zdtf_czt_cl_kernel(CztArgs a) {
       float2* const hb1 = rank == 1 ? hb_local : hb_peer;
       const int blk = blk0 + 2 * st + bb;
       if (blk < blk_end) {  // uniform over the warp
-        if (SUBSET) {  // block bb belongs to rank bb
-          const int j = __ldg(a.blk_base + blk);
-#pragma unroll 1
-          for (int u = 0; u < kRatesPerBlock / 2; ++u) {
-            float2 ax, ay, bx, by;
-            fold_rate_smem(fp, g, QH / 2, Nt, j + 2 * u, a.half, ax, ay);
-            fold_rate_smem(fp, g, QH / 2, Nt, j + 2 * u + 1, a.half, bx, by);
+        if (SUBSET) {  // round bb belongs to rank bb
+          round_sums<SUBSET>(a, blk, fp, g, QH / 2, []() {}, [&](int u, float2 ax, float2 ay, float2 bx, float2 by) {
             put_rate_pair<SS>((bb ? hb1 : hb0) + 2 * u * SS, side, k20, ms, mk2, dc, win, ax, ay, bx, by);
-          }
+          });
         } else {
           float2 px[4], py[4], mx[4], my[4];
           fp.start(blk);
@@ -1365,11 +1491,12 @@ zdtf_czt_cl_kernel(CztArgs a) {
     for (int st = 0; st < steps; ++st) {
       cluster.sync();  // the sums of step st are complete (this group's transform of st - 1 is, too)
       const int b2 = blk0 + 2 * st;
+      const BlockPairs<SUBSET> pairs(a, min(b2 + rank, blk_end - 1));
       group_fft_emit<Q, kRatesPerBlock, SS, SH::I, +1, kBarFft, 1>(
           buf + (st & 1) * kRatesPerBlock * SS, twt, ltid, [&](int ls, int na, float2 v) {
             const int lp = ls >> 1, sd = ls & 1;
             const int b = SUBSET ? b2 + rank : b2 + (lp >> 1);
-            const int p = b < blk_end ? block_pair<SUBSET>(a, b, SUBSET ? lp : 2 * (lp & 1) + rank) : -1;
+            const int p = b >= blk_end ? -1 : SUBSET ? pairs[lp] : block_pair<SUBSET>(a, b, 2 * (lp & 1) + rank);
             const long long at = ((long long)p * P + (sd ? k1b : k1a)) * Q + na;
             if (p >= 0 && FDR_DBG_OK(at < (long long)a.npairs * P * Q)) a.W[at] = cmul(v, twr[sd * Q + na]);
           });
@@ -2741,15 +2868,17 @@ static int set_smem_attrs() {
 #define SET_ATTR(kernel, bytes) \
   FDR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes)));
 #define SET_B(Q)                                                                               \
-  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, false, false>), CztShape<Q>::SMEM)                 \
-  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, true, false>), CztShape<Q>::SMEM)                  \
-  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, true, true>), CztShape<Q>::SMEM)                   \
+  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, false, kWhole>), CztShape<Q>::SMEM)                \
+  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, true, kWhole>), CztShape<Q>::SMEM)                 \
+  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, false, kSingles>), CztShape<Q>::SMEM)              \
+  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, true, kSingles>), CztShape<Q>::SMEM)               \
+  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, true, kRounds>), CztShape<Q>::SMEM)                \
   SET_ATTR((zdtf_a2f_kernel<Q, kFusedMaxNt>), CztShape<Q>::SMEM)
   FDR_FOR_Q(SET_B)
 #undef SET_B
 #define SET_BS(Q, NT)                                                                          \
-  SET_ATTR((zdtf_czt_smem_kernel<Q, NT, false>), (CztSmemShape<Q>::template smem<NT>()))       \
-  SET_ATTR((zdtf_czt_smem_kernel<Q, NT, true>), (CztSmemShape<Q>::template smem<NT>()))
+  SET_ATTR((zdtf_czt_smem_kernel<Q, NT, kWhole>), (CztSmemShape<Q>::template smem<NT>()))       \
+  SET_ATTR((zdtf_czt_smem_kernel<Q, NT, kRounds>), (CztSmemShape<Q>::template smem<NT>()))
   SET_BS(64, 32) SET_BS(128, 32) SET_BS(64, 64) SET_BS(128, 64)
 #undef SET_BS
 #define SET_AF(Q, NT) SET_ATTR((zdtf_a2f_smem_kernel<Q, NT>), (CztSmemShape<Q>::template smem<NT>()))
@@ -2757,12 +2886,13 @@ static int set_smem_attrs() {
   SET_AF(64, 64) SET_AF(128, 64) SET_AF(256, 64)
 #undef SET_AF
 #define SET_WS(Q, NT)                                                                          \
-  SET_ATTR((zdtf_czt_ws_kernel<Q, NT, false>), (CztWsShape<Q>::template smem<NT>()))           \
-  SET_ATTR((zdtf_czt_ws_kernel<Q, NT, true>), (CztWsShape<Q>::template smem<NT>()))
+  SET_ATTR((zdtf_czt_ws_kernel<Q, NT, kWhole>), (CztWsShape<Q>::template smem<NT>()))           \
+  SET_ATTR((zdtf_czt_ws_kernel<Q, NT, kRounds>), (CztWsShape<Q>::template smem<NT>()))
   SET_WS(512, 32) SET_WS(256, 32) SET_WS(256, 64)
+  SET_ATTR((zdtf_czt_ws_kernel<512, 32, kSingles>), (CztWsShape<512>::smem<32>()))
 #undef SET_WS
-  SET_ATTR(zdtf_czt_cl_kernel<false>, CztClShape::SMEM)
-  SET_ATTR(zdtf_czt_cl_kernel<true>, CztClShape::SMEM)
+  SET_ATTR(zdtf_czt_cl_kernel<kWhole>, CztClShape::SMEM)
+  SET_ATTR(zdtf_czt_cl_kernel<kRounds>, CztClShape::SMEM)
   SET_ATTR(zdtf_a2f_half_kernel, CztClShape::SMEM)
 #undef SET_ATTR
   if (dev < 64) done[dev] = true;
@@ -2922,11 +3052,11 @@ int fused_default_groups(const FusedPlan* st) {
 
 int fused_czt(const FusedPlan* st, const float2* A, float2* W, float r0, float dr, int window,
               const double* wk, int groups, cudaStream_t s) {
-  return fused_czt_blocks(st, A, W, r0, dr, window, wk, nullptr, groups, s);
+  return fused_czt_blocks(st, A, W, r0, dr, window, wk, nullptr, false, groups, s);
 }
 
 int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, float dr,
-                     int window, const double* wk, const int* blk_base, int groups,
+                     int window, const double* wk, const int* rounds, bool both, int groups,
                      cudaStream_t s) {
   PhaseInt ph;
   if (!make_phase(r0, dr, st->L, &ph)) {
@@ -2937,17 +3067,17 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
   a.ph = ph;
   a.window = window;
   a.wk = wk;
-  a.blk_base = blk_base;
+  a.rounds = rounds;
   a.center = ph.R0 + (unsigned long long)(4 * st->half - 1) * ph.Rh;
   const int Q = st->Q, ctas = st->P / 2;
-  a.nblk = (int)(blk_base ? st->npairs / 4 : cdiv(st->half, 2));
+  a.nblk = (int)(rounds ? st->npairs / 4 : cdiv(st->half, 2));
   if (st->Nt <= kFusedMaxNt) a.pshift = (int)(kFusedMaxNt / 2 - st->Nt / 2) / 2;
   if (groups <= 0) groups = fused_default_groups(st);
   groups = std::min(groups, a.nblk);
   a.blocks_per_group = (int)cdiv(a.nblk, groups);
   groups = (int)cdiv(a.nblk, a.blocks_per_group);
   if (st->Nt > 32 && Q == CztClShape::Q) {  // F of 64 steps for 512 bins: two-CTA cluster
-    auto kernel = blk_base ? zdtf_czt_cl_kernel<true> : zdtf_czt_cl_kernel<false>;
+    auto kernel = rounds ? zdtf_czt_cl_kernel<kRounds> : zdtf_czt_cl_kernel<kWhole>;
     FDR_CUDA(launch_dependent(early_launch(st), kernel, dim3(2 * ctas, groups), CztClShape::T, CztClShape::SMEM, s, a));
     FDR_LAUNCH_CHECK("zdtf_czt_cl_kernel");
     return FDR_OK;
@@ -2958,7 +3088,8 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
     const int NT = st->Nt <= 32 ? 32 : 64;
 #define LAUNCH_WS(QQ, NN)                                                                      \
     if (Q == QQ && NT == NN) {                                                                 \
-      auto kernel = blk_base ? zdtf_czt_ws_kernel<QQ, NN, true> : zdtf_czt_ws_kernel<QQ, NN, false>; \
+      auto kernel = rounds ? zdtf_czt_ws_kernel<QQ, NN, kRounds> : zdtf_czt_ws_kernel<QQ, NN, kWhole>; \
+      if (rounds && !both && QQ == 512) kernel = zdtf_czt_ws_kernel<512, 32, kSingles>;        \
       FDR_CUDA(launch_dependent(early_launch(st), kernel, dim3(ctas, groups), CztWsShape<QQ>::T, CztWsShape<QQ>::template smem<NN>(), s, a)); \
       FDR_LAUNCH_CHECK("zdtf_czt_ws_kernel");                                                  \
       return FDR_OK;                                                                           \
@@ -2970,7 +3101,7 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
     const int NT = st->Nt <= 32 ? 32 : 64;
 #define LAUNCH_BS(QQ, NN)                                                                      \
     if (Q == QQ && NT == NN) {                                                                 \
-      auto kernel = blk_base ? zdtf_czt_smem_kernel<QQ, NN, true> : zdtf_czt_smem_kernel<QQ, NN, false>; \
+      auto kernel = rounds ? zdtf_czt_smem_kernel<QQ, NN, kRounds> : zdtf_czt_smem_kernel<QQ, NN, kWhole>; \
       FDR_CUDA(launch_dependent(early_launch(st), kernel, dim3(ctas, groups), CztSmemShape<QQ>::T, CztSmemShape<QQ>::template smem<NN>(), s, a)); \
       FDR_LAUNCH_CHECK("zdtf_czt_smem_kernel");                                                \
       return FDR_OK;                                                                           \
@@ -2980,9 +3111,13 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
   } else {
 #define LAUNCH_B(QQ)                                                                           \
     if (Q == QQ) {                                                                             \
-      auto kernel = blk_base ? zdtf_czt_kernel<QQ, kFusedMaxNt, true, true>                    \
-                    : window == FDR_WINDOW_RECT ? zdtf_czt_kernel<QQ, kFusedMaxNt, false, false> \
-                                                : zdtf_czt_kernel<QQ, kFusedMaxNt, true, false>; \
+      const bool rect = window == FDR_WINDOW_RECT;                                             \
+      auto kernel = rect ? zdtf_czt_kernel<QQ, kFusedMaxNt, false, kWhole>                     \
+                         : zdtf_czt_kernel<QQ, kFusedMaxNt, true, kWhole>;                     \
+      if (rounds)                                                                              \
+        kernel = both ? zdtf_czt_kernel<QQ, kFusedMaxNt, true, kRounds>                        \
+                      : rect ? zdtf_czt_kernel<QQ, kFusedMaxNt, false, kSingles>               \
+                             : zdtf_czt_kernel<QQ, kFusedMaxNt, true, kSingles>;               \
       FDR_CUDA(launch_dependent(early_launch(st), kernel, dim3(ctas, groups), QQ / 2, CztShape<QQ>::SMEM, s, a));  \
       FDR_LAUNCH_CHECK("zdtf_czt_kernel");                                                     \
       return FDR_OK;                                                                           \
@@ -3199,10 +3334,78 @@ int zdt_fused_run(fdr_zdt* ws, float r0, float* dest, int window, const double* 
   return FDR_OK;
 }
 
-// A subset of the workspace's rates: nblocks blocks of 8 consecutive rates, block i starting
-// at rate index blk_base[i] (device) of the r0 + j*dr grid; the FDR columns 8i..8i+7 of dest.
-// The plan's tables are shared; only the rate count differs.
-int zdt_fused_run_blocks(fdr_zdt* ws, const int* blk_base, int64_t nblocks, float* dest,
+// The rounds (kRoundWords words each, as many as blocks) in which the czt kernels compute the 8-rate
+// blocks `blocks` of the grid; block i goes to rate pairs 4 i .. 4 i + 3 of W.  Super pairs of which
+// both rate pairs are wanted are computed once for the two, two of them a round; the single pairs
+// come four to a round.  Neighbours i, i + 1 (i even) stay together where they can: they share a start.
+// Calls at Nf = 2^20 and 128 rates, all 16 blocks and every other one (which are all on one side or the
+// other): Nt = 32, 987 and 611 us with Horner's rule per rate, 1316 and 772 with pair sums of a rate at a
+// time, now 866 and 638 (one side alone takes the sums for two); Nt = 64, 1849 and 1168, 2117 and 1292,
+// now 1455 and 1143; Nt = 16, 672 and 401, 680 and 401, now 593 and 401.
+RateRounds fused_rounds(const FusedPlan* st, const int32_t* blocks, int64_t nblocks) {
+  struct Item {
+    int i, side, dest, other;  // other: W pair of the lower rate pair where both are wanted, or -1
+  };
+  const int half = (int)st->half;
+  std::vector<int> first(2 * (size_t)half, -1);  // by 2 i + side: where the pair goes
+  std::vector<Item> single, both;
+  for (int64_t b = 0; b < nblocks; ++b)
+    for (int u = 0; u < 4; ++u) {
+      const int p = 4 * (int)blocks[b] + u, dest = (int)(4 * b + u);
+      const int side = p < half, i = side ? half - 1 - p : p - half;
+      if (first[2 * (size_t)i + side] < 0) first[2 * (size_t)i + side] = dest;
+      else single.push_back({i, side, dest, -1});  // a block given twice
+    }
+  for (int i = 0; i < half; ++i) {
+    const int up = first[2 * (size_t)i], lo = first[2 * (size_t)i + 1];
+    if (up >= 0 && lo >= 0) both.push_back({i, 0, up, lo});
+    else if (up >= 0) single.push_back({i, 0, up, -1});
+    else if (lo >= 0) single.push_back({i, 1, lo, -1});
+  }
+  // an even number of them, or none where single pairs are more than three rounds in four
+  while (both.size() % 2 || (!both.empty() && 2 * (int64_t)both.size() < nblocks)) {
+    const Item t = both.back();
+    both.pop_back();
+    single.push_back({t.i, 0, t.dest, -1});
+    single.push_back({t.i, 1, t.other, -1});
+  }
+  auto neighbours_first = [](std::vector<Item>* v) {
+    std::stable_sort(v->begin(), v->end(), [](const Item& a, const Item& b) { return a.i < b.i; });
+    std::vector<Item> out, rest;
+    for (size_t k = 0; k < v->size();) {
+      if (k + 1 < v->size() && (*v)[k].i % 2 == 0 && (*v)[k + 1].i == (*v)[k].i + 1) {
+        out.push_back((*v)[k]);
+        out.push_back((*v)[k + 1]);
+        k += 2;
+      } else {
+        rest.push_back((*v)[k++]);
+      }
+    }
+    out.insert(out.end(), rest.begin(), rest.end());
+    v->swap(out);
+  };
+  neighbours_first(&single);
+  neighbours_first(&both);
+  RateRounds r;
+  std::vector<int>& words = r.words;
+  r.both = !both.empty();
+  words.reserve((size_t)nblocks * kRoundWords);
+  for (size_t k = 0; k < both.size(); k += 2)
+    words.insert(words.end(), {both[k].i, both[k + 1].i, -1, -1, both[k].dest, both[k].other, both[k + 1].dest,
+                               both[k + 1].other});
+  for (size_t k = 0; k + 3 < single.size(); k += 4) {
+    for (int e = 0; e < 4; ++e) words.push_back(2 * single[k + e].i + single[k + e].side);
+    for (int e = 0; e < 4; ++e) words.push_back(single[k + e].dest);
+  }
+  return r;  // whole rounds: 4 nblocks pairs, of which `both` holds a multiple of 4
+}
+
+// A subset of the workspace's rates in nblocks rounds (device words of zdt_fused_rounds), block i in
+// the FDR columns 8i..8i+7 of dest.  The plan's tables are shared; only the rate count differs.
+RateRounds zdt_fused_rounds(fdr_zdt* ws, const int32_t* blocks, int64_t nblocks) {
+  return fused_rounds(st_of(ws), blocks, nblocks);
+}
+int zdt_fused_run_blocks(fdr_zdt* ws, const int* rounds, bool both, int64_t nblocks, float* dest,
                          int window, const double* wk, double* acc, cudaStream_t s) {
   const FusedPlan* st = st_of(ws);
   FDR_CHECK_ARG(ws->A_valid, "zdtfdr blocks: the workspace holds no fused input stage");
@@ -3213,7 +3416,7 @@ int zdt_fused_run_blocks(fdr_zdt* ws, const int* blk_base, int64_t nblocks, floa
   FusedPlan sub = *st;
   sub.Nr = 8 * nblocks;
   sub.npairs = 4 * nblocks;
-  FDR_TRY(fused_czt_blocks(&sub, ws->A, ws->W, ws->r0, ws->dr, window, wk, blk_base, 0, s));
+  FDR_TRY(fused_czt_blocks(&sub, ws->A, ws->W, ws->r0, ws->dr, window, wk, rounds, both, 0, s));
   zdt_mark(ws, "czt", s);
   if (ws->flags & FDR_ZDT_MIXED_PRECISION) FDR_TRY(fused_output_mixed(&sub, ws->W, dest, acc, s));
   else FDR_TRY(fused_output(&sub, ws->W, dest, acc, s));

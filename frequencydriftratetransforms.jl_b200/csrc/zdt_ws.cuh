@@ -70,14 +70,20 @@ int fused_a2f(const FusedPlan* st, const float2* A, float2* F, cudaStream_t s);
 int fused_czt(const FusedPlan* st, const float2* A, float2* W, float r0, float dr, int window,
               const double* wk, int groups, cudaStream_t s);
 int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, float dr,
-                     int window, const double* wk, const int* blk_base, int groups,
+                     int window, const double* wk, const int* rounds, bool both, int groups,
                      cudaStream_t s);
 int fused_output(const FusedPlan* st, const float2* W, float* dest, double* acc, cudaStream_t s);
 int fused_output_mixed(const FusedPlan* st, const float2* W, float* dest, double* acc, cudaStream_t s);
 // Reads and clears the fused kernels' fault flag (a bounded TMA wait that ran out).
 int fused_take_fault();
 int bounded_wait_selftest(unsigned long long limit_ns, cudaStream_t s);
-int zdt_fused_run_blocks(fdr_zdt* ws, const int* blk_base, int64_t nblocks, float* dest,
+// What zdt_fused_run_blocks takes (its words on the device) for 8-rate blocks of the workspace's grid.
+struct RateRounds {
+  std::vector<int> words;
+  bool both = false;  // some rounds take both rate pairs of their super pairs
+};
+RateRounds zdt_fused_rounds(fdr_zdt* ws, const int32_t* blocks, int64_t nblocks);
+int zdt_fused_run_blocks(fdr_zdt* ws, const int* rounds, bool both, int64_t nblocks, float* dest,
                          int window, const double* wk, double* acc, cudaStream_t s);
 // timing helpers
 void zdt_mark(fdr_zdt* ws, const char* name, cudaStream_t s);
