@@ -9,6 +9,8 @@
 #include <math.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "fft_engine.cuh"
 
 struct fdr_fft_ws {
@@ -33,7 +35,7 @@ __device__ __forceinline__ float2 phasor_ref(long long k, long long t, float r, 
   return cispif(x);
 }
 
-// S[k + jj*K] = sum_t F[k, t] * phasor(k, t, r_jj).  A thread takes one bin and kRatesPerThread
+// S[k + jj*K] = sum_t F[k, t] * phasor(k, t, r_jj).  A thread takes one bin and RPT
 // rates, two per packed operation, so F is read once for all of them; the time goes to the phasors,
 // one for each (k, t, r).  Their arguments are formed by the same rounded operations as in
 // phasor_ref, with cheaper instructions where they give the same value: for MULT (2k and t exact in
@@ -44,26 +46,29 @@ __device__ __forceinline__ float2 phasor_ref(long long k, long long t, float r, 
 // by itself, so that a column does not depend on the rates beside it.  At Nf = 2^20, Nt = 16, 21
 // rates: 440 us with a thread per sum and sincospif, 246 us with 8 rates per thread, 179 us with
 // packed polynomials (70% of the FMA pipe).
+// RPT is 8 where that fills the GPU; a grid of less than one CTA an SM takes a pair per
+// thread, a quarter of the chain (calls of 16 rates at Nf = 10,200: 149 -> 132 us, 131 with a thread per
+// sum; 8 rates and 64 steps at Nf = 4096: 42 -> 27 us, 68 with a thread per sum).
 constexpr int kRatesPerThread = 8;
 
-template <bool MULT, bool POW2, bool LARGE>
+template <int RPT, bool MULT, bool POW2, bool LARGE>
 __global__ void __launch_bounds__(256) phasor_sum_kernel(const float2* __restrict__ F, long long K, int Nt,
                                                          long long Nf, int nr, unsigned large,
                                                          float2* __restrict__ S,
                                                          const __grid_constant__ RateParams rp) {
   const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (k >= K) return;
-  const int j0 = blockIdx.y * kRatesPerThread;
+  const int j0 = blockIdx.y * RPT;
   const float Nf_f = __ll2float_rn(Nf), inv = 1.f / Nf_f, k2 = __ll2float_rn(2 * k);
-  float2 ax[kRatesPerThread / 2], ay[kRatesPerThread / 2];  // lanes: rates 2q and 2q + 1
+  float2 ax[RPT / 2], ay[RPT / 2];  // lanes: rates 2q and 2q + 1
 #pragma unroll
-  for (int q = 0; q < kRatesPerThread / 2; ++q) ax[q] = ay[q] = make_float2(0.f, 0.f);
+  for (int q = 0; q < RPT / 2; ++q) ax[q] = ay[q] = make_float2(0.f, 0.f);
   for (int t = 0; t < Nt; ++t) {
     const float2 f = __ldg(F + k + t * K);
     const float2 fx = pk_set(f.x), fy = pk_set(f.y);
     const float kt = MULT ? __fmul_rn(k2, (float)t) : __ll2float_rn(2 * k * t);
 #pragma unroll
-    for (int q = 0; q < kRatesPerThread / 2; ++q) {
+    for (int q = 0; q < RPT / 2; ++q) {
       if (j0 + 2 * q < nr) {  // uniform; rates past the last are zero
         const float2 x = pk_mul(pk_set(kt), make_float2(rp.r[j0 + 2 * q], rp.r[j0 + 2 * q + 1]));
         const float2 h = POW2 ? pk_mul(x, pk_set(inv)) : make_float2(__fdiv_rn(x.x, Nf_f), __fdiv_rn(x.y, Nf_f));
@@ -92,7 +97,7 @@ __global__ void __launch_bounds__(256) phasor_sum_kernel(const float2* __restric
     }
   }
 #pragma unroll
-  for (int q = 0; q < kRatesPerThread / 2; ++q) {
+  for (int q = 0; q < RPT / 2; ++q) {
     if (j0 + 2 * q < nr) S[k + (j0 + 2 * q) * K] = make_float2(ax[q].x, ay[q].x);
     if (j0 + 2 * q + 1 < nr) S[k + (j0 + 2 * q + 1) * K] = make_float2(ax[q].y, ay[q].y);
   }
@@ -210,12 +215,17 @@ int fdr_fftfdr(fdr_fft_ws* ws, const float* rates, int64_t Nr, float* fdr, fdr_s
     static_assert(kRateChunk == 32, "one bit per rate");
     for (int i = 0; i < nr; ++i)
       if (!((double)fabsf(rp.r[i]) * (double)ws->Nt < (double)(1 << 19))) large |= 1u << i;
-    const dim3 grid((unsigned)cdiv(ws->K, 256), (unsigned)cdiv(nr, kRatesPerThread));
-    auto kernel = large ? (mult ? (pow2 ? phasor_sum_kernel<true, true, true> : phasor_sum_kernel<true, false, true>)
-                                : (pow2 ? phasor_sum_kernel<false, true, true> : phasor_sum_kernel<false, false, true>))
-                        : (mult ? (pow2 ? phasor_sum_kernel<true, true, false> : phasor_sum_kernel<true, false, false>)
-                                : (pow2 ? phasor_sum_kernel<false, true, false> : phasor_sum_kernel<false, false, false>));
-    kernel<<<grid, 256, 0, s>>>(ws->F, ws->K, (int)ws->Nt, ws->Nf, nr, large, ws->S, rp);
+    auto launch = [&](auto rpt) {
+      constexpr int RPT = decltype(rpt)::value;
+      auto kernel = large ? (mult ? (pow2 ? phasor_sum_kernel<RPT, true, true, true> : phasor_sum_kernel<RPT, true, false, true>)
+                                  : (pow2 ? phasor_sum_kernel<RPT, false, true, true> : phasor_sum_kernel<RPT, false, false, true>))
+                          : (mult ? (pow2 ? phasor_sum_kernel<RPT, true, true, false> : phasor_sum_kernel<RPT, true, false, false>)
+                                  : (pow2 ? phasor_sum_kernel<RPT, false, true, false> : phasor_sum_kernel<RPT, false, false, false>));
+      const dim3 grid((unsigned)cdiv(ws->K, 256), (unsigned)cdiv(nr, RPT));
+      kernel<<<grid, 256, 0, s>>>(ws->F, ws->K, (int)ws->Nt, ws->Nf, nr, large, ws->S, rp);
+    };
+    if (cdiv(ws->K, 256) * cdiv(nr, kRatesPerThread) >= sm_count()) launch(std::integral_constant<int, kRatesPerThread>());
+    else launch(std::integral_constant<int, 2>());
     FDR_LAUNCH_CHECK("phasor_sum_kernel");
     FDR_TRY(irfft_columns(ws->S, ws->K, nr, ws->Nf, fdr + j0 * ws->Nf, ws->Nf, ws->rscratch,
                           ws->rscratch_pairs, s));
