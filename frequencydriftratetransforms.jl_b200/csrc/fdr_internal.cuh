@@ -141,8 +141,12 @@ __host__ __device__ __forceinline__ int quarter_rest(int h, unsigned* q) {
 
 // cos and sin of x + q quarter turns for two values, |x| <= 1/2: polynomials in x^2 fitted on
 // Chebyshev nodes (degrees 7 and 8; the leading sine coefficient pi/2 is held in two parts).  Errors
-// over all 32-bit phases: 1.4e-8 (sin) and 1.9e-8 (cos) rms, 7.1e-8 at most, against 1.4e-8 and
-// 1.8e-8 rms for correctly rounded values of the rounded argument.
+// over random phases, rms and largest: 1.52e-8 and 5.9e-8 for a Float32 x (sincospif: 1.51e-8 and
+// 5.3e-8, rounded values: 1.46e-8 and 3.0e-8), 1.68e-8 and 7.4e-8 with the rounding of a 32-bit phase
+// to x (sincospif of the whole phase in Float32: 3.3e-8 and 1.2e-7).
+// EXACT, for phases given in Float32: the cosine's leading term has its rounding error returned (u lies
+// in [0.69, 1], so 1 - u is exact), 1.48e-8 and 4.5e-8.
+template <bool EXACT = false>
 __device__ __forceinline__ void cis_quarter_pk(float2 x, unsigned q0, unsigned q1, float2& c, float2& s) {
   const float2 y = pk_mul(x, x);
   float2 p = pk_fma(y, pk_set(-4.602149128913879e-3f), pk_set(7.968021929264069e-2f));
@@ -151,8 +155,16 @@ __device__ __forceinline__ void cis_quarter_pk(float2 x, unsigned q0, unsigned q
   const float2 sn = pk_fma(x, pk_set(1.5707963705062866f), pk_mul(x, p));
   float2 e = pk_fma(y, pk_set(9.036280680447817e-4f), pk_set(-2.086007036268711e-2f));
   e = pk_fma(e, y, pk_set(2.5366920232772827e-1f));
-  e = pk_fma(e, y, pk_set(-1.2337005138397217f));
-  const float2 cs = pk_fma(e, y, pk_set(1.f));
+  float2 cs;
+  if (EXACT) {  // 1 + y a + y (a' + y e), a + a' = -pi^2 / 8
+    const float2 a = pk_set(-1.2337005138397217f), one = pk_set(1.f);
+    const float2 u = pk_fma(y, a, one);
+    const float2 r = pk_fma(y, a, pk_fma(u, pk_set(-1.f), one));
+    cs = pk_add(u, pk_fma(y, pk_fma(e, y, pk_set(-3.629645e-8f)), r));
+  } else {
+    e = pk_fma(e, y, pk_set(-1.2337005138397217f));
+    cs = pk_fma(e, y, pk_set(1.f));
+  }
   auto sign = [](float v, unsigned bit) { return __uint_as_float(__float_as_uint(v) ^ (bit << 30)); };
   c.x = sign((q0 & 1) ? sn.x : cs.x, (q0 + 1) & 2);
   s.x = sign((q0 & 1) ? cs.x : sn.x, q0 & 2);

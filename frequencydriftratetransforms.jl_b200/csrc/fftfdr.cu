@@ -44,8 +44,8 @@ __device__ __forceinline__ float2 phasor_ref(long long k, long long t, float r, 
 // nearest quarter turn is the sum with 1.5 * 2^23 rounded, its low bits the quadrant, and the rest
 // is exact; the other rates, if any (LARGE: the bits of `large`), take cispif.  Each rate is decided
 // by itself, so that a column does not depend on the rates beside it.  At Nf = 2^20, Nt = 16, 21
-// rates: 440 us with a thread per sum and sincospif, 246 us with 8 rates per thread, 179 us with
-// packed polynomials (70% of the FMA pipe).
+// rates: 440 us with a thread per sum and sincospif, 246 us with 8 rates per thread, 201 us with
+// packed polynomials (179 us without EXACT, whose error was above that of sincospif).
 // RPT is 8 where that fills the GPU; a grid of less than one CTA an SM takes a pair per
 // thread, a quarter of the chain (calls of 16 rates at Nf = 10,200: 149 -> 132 us, 131 with a thread per
 // sum; 8 rates and 64 steps at Nf = 4096: 42 -> 27 us, 68 with a thread per sum).
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) phasor_sum_kernel(const float2* __restric
         const float2 m = pk_add(h2, pk_set(12582912.f));
         const float2 rest = csub(h2, pk_add(m, pk_set(-12582912.f)));
         float2 c, s;
-        cis_quarter_pk(rest, __float_as_uint(m.x), __float_as_uint(m.y), c, s);
+        cis_quarter_pk<true>(rest, __float_as_uint(m.x), __float_as_uint(m.y), c, s);
         if (LARGE) {
           const unsigned two = large >> (j0 + 2 * q);  // uniform
           if (two & 1) {
