@@ -290,6 +290,7 @@ enum { kOutComplex, kOutTwiddle, kOutRealPair };
 
 struct StageArgs {
   StageDesc d;
+  TwiddleTables tw;
   const void* in;
   void* out;
   const float2* mul;  // kOutComplex: pointwise factor addressed like the output, or NULL
@@ -302,39 +303,6 @@ struct StageArgs {
   int in_lane_i, out_lane_i;
   float scale;
 };
-
-// Four-step twiddle exp(SIGN 2 pi i l b / N) of the CTA's transforms b, as the product of a
-// factor for l / 32 (rounded value and its residue) and one for l mod 32 (its difference from
-// 1): within 0.2 ulp of the correctly rounded value for L >= 160, since the second factor's
-// angle is below 2 pi / 32 there.  All values come from float64, once per CTA.
-struct TwiddleTables {
-  float4* hi;
-  float2* lo;
-  int nh;
-};
-
-template <int SIGN>
-__device__ __forceinline__ void fill_twiddles(const TwiddleTables& t, int bpc, int L, long long b1_0, double inv2N) {
-  const int nh = (L + 31) / 32, per = nh + 32;
-  for (int e = threadIdx.x; e < bpc * per; e += blockDim.x) {
-    const int i = e / per, m = e - i * per;
-    const long long l = m < nh ? 32LL * m : m - nh;
-    double s, c;
-    sincospi((double)(l * (b1_0 + i)) * inv2N, &s, &c);
-    s *= SIGN;
-    if (m < nh) {
-      const float x = (float)c, y = (float)s;
-      t.hi[i * t.nh + m] = make_float4(x, y, (float)(c - x), (float)(s - y));
-    } else {
-      t.lo[i * 33 + m - nh] = make_float2((float)(c - 1.0), (float)s);
-    }
-  }
-}
-__device__ __forceinline__ float2 twiddle_at(const TwiddleTables& t, int i, int l) {
-  const float4 h = t.hi[i * t.nh + (l >> 5)];
-  const float2 e = t.lo[i * 33 + (l & 31)];
-  return make_float2(h.x + fmaf(h.x, e.x, fmaf(-h.y, e.y, h.z)), h.y + fmaf(h.x, e.y, fmaf(h.y, e.x, h.w)));
-}
 
 // One pass: several transforms of length L per CTA in shared memory (64 KB, three CTAs per SM at 80
 // registers), the first stage reading and the last writing device memory.  Passes of Nf = 200,000,
@@ -349,13 +317,8 @@ __global__ void __launch_bounds__(kStageThreads, kStageCtas) fft_stage_kernel(co
   const StageDesc& d = a.d;
   const long long b1_0 = (long long)blockIdx.x << d.bpc_log2;
   const int nb = (int)min((long long)d.bpc, a.nb1 - b1_0);
-  TwiddleTables tw;
-  if (OUT == kOutTwiddle) {
-    tw.hi = sm4 + (d.bpc * d.SS + 1) / 2;
-    tw.nh = tw_rows(d.L);
-    tw.lo = reinterpret_cast<float2*>(tw.hi + d.bpc * tw.nh);
-    fill_twiddles<SIGN>(tw, d.bpc, d.L, b1_0, 2.0 / (double)a.N);  // the first stage's barrier follows
-  }
+  if (OUT == kOutTwiddle)  // the first stage's barrier follows
+    fill_twiddles<SIGN>(a.tw, sm4, d.bpc, d.L, b1_0, 2.0 / (double)a.N);
   for (long long b0 = blockIdx.y; b0 < a.nb0; b0 += gridDim.y) {
     const float2* const in = static_cast<const float2*>(a.in) + b0 * a.is0 + b1_0 * a.is1;
     float2* const out = static_cast<float2*>(a.out) + b0 * a.os0 + b1_0 * a.os1;
@@ -398,7 +361,9 @@ __global__ void __launch_bounds__(kStageThreads, kStageCtas) fft_stage_kernel(co
       const float2* const mrow = mul ? mul + i * a.os1 : nullptr;
       float* const ra = static_cast<float*>(a.out) + c * a.ldo;
       const float scale = a.scale;
-      const TwiddleTables t = tw;
+      const float4* const hi = sm4 + a.tw.hi + i * a.tw.nh;
+      const float2* const lo = sm + a.tw.lo + (i << a.tw.lg) + i;
+      const int lg = a.tw.lg;
       return [=](int l, float2 v) {
         if (OUT == kOutRealPair) {
           v = cscale(v, scale);
@@ -407,7 +372,7 @@ __global__ void __launch_bounds__(kStageThreads, kStageCtas) fft_stage_kernel(co
           return;
         }
         if (OUT == kOutTwiddle) {
-          v = cmul(v, twiddle_at(t, i, l));
+          v = cmul(v, twiddle_at(hi, lo, lg, l));
         } else {
           if (mrow && live) v = cmul(v, __ldg(mrow + l * (long long)osl));
           v = cscale(v, scale);
@@ -432,6 +397,7 @@ int launch_stages(StageArgs& a, cudaStream_t s) {
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageSmem));
     if (dev < 64) attr_set[dev] = true;
   }
+  a.tw = twiddle_tables(a.d);
   const size_t smem = stage_smem_bytes(a.d) + (OUT == kOutTwiddle ? tw_bytes(a.d.L, a.d.bpc) : 0);
   const dim3 grid((unsigned)cdiv(a.nb1, a.d.bpc), (unsigned)std::min(a.nb0, 65535LL));
   fft_stage_kernel<SIGN, IN, OUT><<<grid, stage_threads(a.d), smem, s>>>(a);

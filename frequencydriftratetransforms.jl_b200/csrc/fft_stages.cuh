@@ -315,10 +315,16 @@ __device__ __forceinline__ void convolve_smem(const StageDesc& d, float2* sm, Fa
   }
 }
 
-// Tables of the four-step twiddles of a first pass (see TwiddleTables in fft_engine.cu), rows and bytes.
-__host__ __device__ constexpr int tw_rows(int L) { return ((L + 31) / 32) | 1; }
+// Tables of the four-step twiddles (TwiddleTables below): log2 of the outputs l that share a coarse
+// factor, rows of coarse factors and bytes.
+__host__ __device__ constexpr int tw_fine(int L) {
+  int lg = 0;
+  while ((32 << lg) <= L && lg < 5) ++lg;
+  return lg;
+}
+__host__ __device__ constexpr int tw_rows(int L) { return ((L + (1 << tw_fine(L)) - 1) >> tw_fine(L)) | 1; }
 __host__ __device__ inline size_t tw_bytes(int L, int bpc) {
-  return 16 + (size_t)bpc * (sizeof(float4) * tw_rows(L) + sizeof(float2) * 33);
+  return 16 + (size_t)bpc * (sizeof(float4) * tw_rows(L) + sizeof(float2) * ((1 << tw_fine(L)) + 1));
 }
 
 // Fills d for `groups` sets of `nb` transforms of length L, neighbouring transforms of a set at
@@ -329,5 +335,62 @@ constexpr size_t kStageSmem = 112 * 1024;  // two CTAs per SM
 bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, bool twiddles, StageDesc* d);
 size_t stage_smem_bytes(const StageDesc& d);
 int stage_threads(const StageDesc& d);
+
+// Four-step twiddle exp(SIGN 2 pi i l b / N) of the CTA's transforms b, as the product of a coarse
+// factor for l >> lg (rounded value and its residue) and a fine one for the rest of l (its difference
+// from 1), 2^lg of them, lg = tw_fine(L) with 2^lg <= L / 16: the fine angles stay below 2 pi / 16.
+// All values come from float64, once per CTA, eight of a table from one sincospi and the float64
+// powers of another.  Error in units of a rounded value's rms: 1.00 to 1.05 (1.05 to 1.5 for L < 512
+// with 32 fine factors whatever L; finer tables of L = 400 brought a CTA above 64 KB, and the pass from
+// 58 to 67 us).
+struct TwiddleTables {
+  int hi, lo;  // where they start in shared memory, in float4 and float2
+  int nh, lg;  // rows of coarse factors per transform; lg
+};
+
+inline TwiddleTables twiddle_tables(const StageDesc& d) {
+  TwiddleTables t;
+  t.nh = tw_rows(d.L);
+  t.lg = tw_fine(d.L);
+  t.hi = (d.bpc * d.SS + 1) / 2;
+  t.lo = 2 * (t.hi + d.bpc * t.nh);
+  return t;
+}
+
+template <int SIGN>
+__device__ __forceinline__ void fill_twiddles(const TwiddleTables& t, float4* sm4, int bpc, int L, long long b1_0,
+                                              double inv2N) {
+  const int nl = 1 << t.lg, nh = (L + nl - 1) >> t.lg, gh = (nh + 7) / 8, groups = gh + (nl + 7) / 8;
+  float4* const hi = sm4 + t.hi;
+  float2* const lo = reinterpret_cast<float2*>(sm4) + t.lo;
+  for (int e = threadIdx.x; e < bpc * groups; e += blockDim.x) {
+    const int i = e / groups, g = e - i * groups;
+    const bool fine = g >= gh;
+    const int m0 = 8 * (fine ? g - gh : g), n = min(8, (fine ? nl : nh) - m0);
+    const long long b = (b1_0 + i) << (fine ? 0 : t.lg);
+    double c, s, wc, ws;
+    sincospi((double)(m0 * b) * inv2N, &s, &c);
+    sincospi((double)b * inv2N, &ws, &wc);
+    for (int u = 0; u < n; ++u) {
+      const double ss = SIGN * s;
+      if (fine) {
+        lo[i * (nl + 1) + m0 + u] = make_float2((float)(c - 1.0), (float)ss);
+      } else {
+        const float x = (float)c, y = (float)ss;
+        hi[i * t.nh + m0 + u] = make_float4(x, y, (float)(c - x), (float)(ss - y));
+      }
+      const double cn = c * wc - s * ws;
+      s = c * ws + s * wc;
+      c = cn;
+    }
+  }
+}
+
+// Factor of output l from a transform's rows of the tables.
+__device__ __forceinline__ float2 twiddle_at(const float4* hi, const float2* lo, int lg, int l) {
+  const float4 h = hi[l >> lg];
+  const float2 e = lo[l & ((1 << lg) - 1)];
+  return make_float2(h.x + fmaf(h.x, e.x, fmaf(-h.y, e.y, h.z)), h.y + fmaf(h.x, e.y, fmaf(h.y, e.x, h.w)));
+}
 
 }  // namespace fdr
