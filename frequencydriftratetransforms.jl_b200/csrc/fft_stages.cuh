@@ -69,11 +69,32 @@ struct DftComposite {
   }
 };
 
-// cos and sin of 2 pi m / n
-struct CosSin6 {
-  float c[6] = {1.00000000000000000f, 0.50000000000000011f, -0.49999999999999978f, -1.00000000000000000f, -0.50000000000000044f, 0.50000000000000011f};
-  float s[6] = {0.00000000000000000f, 0.86602540378443860f, 0.86602540378443871f, 0.00000000000000012f, -0.86602540378443837f, -0.86602540378443860f};
+// DFT of R1 * R2 points, R1 and R2 coprime, without twiddles (Good's mapping): inputs R2 n1 + R1 n2,
+// outputs E1 k1 + E2 k2 (mod R1 R2) with E1 = 1 mod R1 and 0 mod R2, E2 = 0 mod R1 and 1 mod R2.
+template <int R1, int R2, int E1, int E2>
+struct DftCoprime {
+  static_assert(E1 % R1 == 1 && E1 % R2 == 0 && E2 % R1 == 0 && E2 % R2 == 1, "output mapping");
+  __device__ __forceinline__ static void run(float2* v, int sign) {
+    float2 y[R1][R2];
+#pragma unroll
+    for (int n1 = 0; n1 < R1; ++n1) {
+#pragma unroll
+      for (int n2 = 0; n2 < R2; ++n2) y[n1][n2] = v[(R2 * n1 + R1 * n2) % (R1 * R2)];
+      Dft<R2>::run(y[n1], sign);
+    }
+#pragma unroll
+    for (int k2 = 0; k2 < R2; ++k2) {
+      float2 t[R1];
+#pragma unroll
+      for (int n1 = 0; n1 < R1; ++n1) t[n1] = y[n1][k2];
+      Dft<R1>::run(t, sign);
+#pragma unroll
+      for (int k1 = 0; k1 < R1; ++k1) v[(E1 * k1 + E2 * k2) % (R1 * R2)] = t[k1];
+    }
+  }
 };
+
+// cos and sin of 2 pi m / n
 struct CosSin7 {
   float c[7] = {1.00000000000000000f, 0.62348980185873359f, -0.22252093395631434f, -0.90096886790241903f, -0.90096886790241915f, -0.22252093395631459f, 0.62348980185873337f};
   float s[7] = {0.00000000000000000f, 0.78183148246802980f, 0.97492791218182362f, 0.43388373911755823f, -0.43388373911755801f, -0.97492791218182362f, -0.78183148246802991f};
@@ -81,10 +102,6 @@ struct CosSin7 {
 struct CosSin9 {
   float c[9] = {1.00000000000000000f, 0.76604444311897801f, 0.17364817766693041f, -0.49999999999999978f, -0.93969262078590832f, -0.93969262078590843f, -0.50000000000000044f, 0.17364817766692997f, 0.76604444311897779f};
   float s[9] = {0.00000000000000000f, 0.64278760968653925f, 0.98480775301220802f, 0.86602540378443871f, 0.34202014332566888f, -0.34202014332566866f, -0.86602540378443837f, -0.98480775301220813f, -0.64278760968653958f};
-};
-struct CosSin10 {
-  float c[10] = {1.00000000000000000f, 0.80901699437494745f, 0.30901699437494745f, -0.30901699437494734f, -0.80901699437494734f, -1.00000000000000000f, -0.80901699437494756f, -0.30901699437494756f, 0.30901699437494723f, 0.80901699437494734f};
-  float s[10] = {0.00000000000000000f, 0.58778525229247314f, 0.95105651629515353f, 0.95105651629515364f, 0.58778525229247325f, 0.00000000000000012f, -0.58778525229247303f, -0.95105651629515353f, -0.95105651629515364f, -0.58778525229247336f};
 };
 struct CosSin11 {
   float c[11] = {1.00000000000000000f, 0.84125353283118121f, 0.41541501300188644f, -0.14231483827328500f, -0.65486073394528499f, -0.95949297361449737f, -0.95949297361449748f, -0.65486073394528521f, -0.14231483827328523f, 0.41541501300188605f, 0.84125353283118121f};
@@ -95,10 +112,10 @@ struct CosSin13 {
   float s[13] = {0.00000000000000000f, 0.46472317204376851f, 0.82298386589365635f, 0.99270887409805397f, 0.93501624268541483f, 0.66312265824079519f, 0.23931566428755768f, -0.23931566428755743f, -0.66312265824079497f, -0.93501624268541472f, -0.99270887409805397f, -0.82298386589365702f, -0.46472317204376840f};
 };
 
-template <> struct Dft<6> : DftComposite<2, 3, CosSin6> {};
+template <> struct Dft<6> : DftCoprime<2, 3, 3, 4> {};
 template <> struct Dft<7> : DftPrime<7, CosSin7> {};
 template <> struct Dft<9> : DftComposite<3, 3, CosSin9> {};
-template <> struct Dft<10> : DftComposite<2, 5, CosSin10> {};
+template <> struct Dft<10> : DftCoprime<2, 5, 5, 6> {};
 template <> struct Dft<11> : DftPrime<11, CosSin11> {};
 template <> struct Dft<13> : DftPrime<13, CosSin13> {};
 
