@@ -22,6 +22,8 @@ NVCC_FLAGS = [
     "-O3", "-lineinfo", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
     "--expt-relaxed-constexpr",
+    # decompressing the fused kernels' image took half of a process's first workspace (28 -> 13 ms)
+    "--compress-mode=none",
 ]
 
 

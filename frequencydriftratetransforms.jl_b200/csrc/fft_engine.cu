@@ -217,40 +217,44 @@ static PassDesc blank_pass() {
 // ------------------------------------------------------------------------------------
 namespace {
 
-// Fewest stages for every length up to kStageElems; of equal plans the one with the smaller
-// sum of radices.  first[n]: the radix to take from n, largest first.
-struct StagePlans {
-  std::vector<unsigned char> count, first;
-  std::vector<int> cost;
-  StagePlans() : count(kStageElems + 1, 0xff), first(kStageElems + 1, 0), cost(kStageElems + 1, 0) {
-    static const int radices[] = {16, 13, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
-    count[1] = 0;
-    for (int n = 2; n <= kStageElems; ++n)
-      for (int r : radices) {
-        if (n % r || count[n / r] == 0xff) continue;
-        const int c = count[n / r] + 1, w = cost[n / r] + r;
-        if (c < count[n] || (c == count[n] && w < cost[n])) {
-          count[n] = (unsigned char)c;
-          cost[n] = w;
-          first[n] = (unsigned char)r;
-        }
-      }
+// Radices of a plan of n with `left` stages, none above `top`, into r; the sum of the best (least; of
+// equal ones the larger first radix), or 0.
+int least_radices(int n, int left, int top, int* r) {
+  static const int radices[] = {16, 13, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+  int best = 0, rest[kStageMax];
+  for (int x : radices) {
+    int64_t most = 1;
+    for (int k = 0; k < left; ++k) most *= x;
+    if (most < n) break;  // nor do smaller radices reach n
+    if (x > top || n % x) continue;
+    int sum = left == 1 ? (x == n ? x : 0) : least_radices(n / x, left - 1, x, rest);
+    if (sum == 0) continue;
+    if (left > 1) sum += x;
+    if (best && sum >= best) continue;
+    best = sum;
+    r[0] = x;
+    for (int k = 1; k < left; ++k) r[k] = rest[k - 1];
   }
-};
+  return best;
+}
 
 unsigned magic_of(int d) { return d == 1 ? 0u : (unsigned)(((1ULL << 32) + d - 1) / d); }
 
 }  // namespace
 
 bool stage_plan(int64_t L, int64_t nb, int64_t groups, bool rows, bool twiddles, StageDesc* d) {
-  static const StagePlans plans;
-  if (L < 2 || L > kStageElems || plans.count[L] == 0xff || plans.count[L] > kStageMax) return false;
+  if (L < 2 || L > kStageElems) return false;
+  int64_t smooth = L;
+  for (int p : {2, 3, 5, 7, 11, 13})
+    while (smooth % p == 0) smooth /= p;
+  if (smooth > 1) return false;
   memset(d, 0, sizeof(*d));
   d->L = (int)L;
-  for (int n = (int)L; n > 1; n /= plans.first[n]) d->radix[d->nst++] = plans.first[n];
+  // fewest stages, then the least sum of radices
+  while (++d->nst <= kStageMax && least_radices((int)L, d->nst, 16, d->radix) == 0) {}
+  if (d->nst > kStageMax) return false;
   // the largest radix second: of the orders tried the least error at nearly every length (2^20: 0.99 of
   // that of radices 8, 8, 8, 2 in time order; largest first 1.01, and 3.7% less time)
-  std::sort(d->radix, d->radix + d->nst, [](int a, int b) { return a > b; });
   if (d->nst >= 3) std::swap(d->radix[0], d->radix[1]);
   int Ns = 1;
   for (int s = 0; s < d->nst; ++s) {

@@ -34,6 +34,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "fft_device.cuh"
 #include "fft_engine.cuh"
@@ -2829,73 +2830,79 @@ static std::vector<float2> pass_twiddles(int len) {
 #define FDR_FOR_P(X) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096)
 #define FDR_FOR_Q(X) X(64) X(128) X(256) X(512) X(1024)
 
-static int set_smem_attrs() {
-  static bool done[64] = {false};
+// Shared-memory limits of the kernels that a split P x Q and Nt steps can launch, once per device (setting
+// one loads its kernel, and a process uses a few of the 80).
+static int set_smem_attrs(int P, int Q, int64_t Nt) {
+  const int NT = Nt <= kFusedMaxNt ? kFusedMaxNt : Nt <= 32 ? 32 : 64;
+  static std::atomic<bool> done[64][kFusedMaxLog2 + 1][kFusedMaxLog2 + 1][3];
   int dev = 0;
   FDR_CUDA(cudaGetDevice(&dev));
-  if (dev < 64 && done[dev]) return FDR_OK;
-#define SET_AC(P)                                                                              \
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_input_kernel<P, AcShape<P>::TILE, AcShape<P>::T>,         \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AcShape<P>::SMEM)); \
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_output_kernel<P, AcShape<P>::TILE, AcShape<P>::T>,        \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AcShape<P>::SMEM));
-  FDR_FOR_P(SET_AC)
-#undef SET_AC
-#define SET_C2(P1, P2)                                                                         \
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_output2_kernel<P1, P2, 8>,                                \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                (int)Out2Shape<P1, P2, 8>::SMEM));
-  SET_C2(8, 8) SET_C2(8, 16) SET_C2(16, 16) SET_C2(16, 32) SET_C2(32, 32)
-#undef SET_C2
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_output_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)OutMmaShape::SMEM));
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_output_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)OutUmmaShape::SMEM));
-#define SET_OUT(Q)                                                                             \
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_output_tma_kernel<32, 32, 8, Q>,                          \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                (int)OutTmaShape<32, 32, 8>::SMEM));                           \
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_output_tma64_kernel<8, Q>,                                \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
-                                (int)OutTma64Shape<8>::SMEM));
-  SET_OUT(256) SET_OUT(512) SET_OUT(1024)
-#undef SET_OUT
-#define SET_IN(Q)                                                                              \
-  FDR_CUDA(cudaFuncSetAttribute(zdtf_input64_kernel<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                (int)In64Shape::SMEM));
-  SET_IN(256) SET_IN(512) SET_IN(1024)
-#undef SET_IN
+  std::atomic<bool>* const mark = dev < 64 ? &done[dev][ilog2(P)][ilog2(Q)][NT / 32] : nullptr;
+  if (mark && mark->load()) return FDR_OK;
 #define SET_ATTR(kernel, bytes) \
   FDR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes)));
-#define SET_B(Q)                                                                               \
-  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, false, kWhole>), CztShape<Q>::SMEM)                \
-  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, true, kWhole>), CztShape<Q>::SMEM)                 \
-  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, false, kSingles>), CztShape<Q>::SMEM)              \
-  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, true, kSingles>), CztShape<Q>::SMEM)               \
-  SET_ATTR((zdtf_czt_kernel<Q, kFusedMaxNt, true, kRounds>), CztShape<Q>::SMEM)                \
-  SET_ATTR((zdtf_a2f_kernel<Q, kFusedMaxNt>), CztShape<Q>::SMEM)
+#define SET_AC(PP)                                                                             \
+  if (P == PP) {                                                                               \
+    SET_ATTR((zdtf_input_kernel<PP, AcShape<PP>::TILE, AcShape<PP>::T>), AcShape<PP>::SMEM)    \
+    SET_ATTR((zdtf_output_kernel<PP, AcShape<PP>::TILE, AcShape<PP>::T>), AcShape<PP>::SMEM)   \
+  }
+  FDR_FOR_P(SET_AC)
+#undef SET_AC
+#define SET_C2(P1, P2) \
+  if (P == P1 * P2) SET_ATTR((zdtf_output2_kernel<P1, P2, 8>), (Out2Shape<P1, P2, 8>::SMEM))
+  SET_C2(8, 8) SET_C2(8, 16) SET_C2(16, 16) SET_C2(16, 32) SET_C2(32, 32)
+#undef SET_C2
+  if (P == 1024) SET_ATTR(zdtf_output_mma_kernel, OutMmaShape::SMEM)
+  if (P == 2048) SET_ATTR(zdtf_output_umma_kernel, OutUmmaShape::SMEM)
+#define SET_PQ(PP, QQ, kernel, bytes) \
+  if (P == PP && Q == QQ) SET_ATTR(kernel, bytes)
+  SET_PQ(1024, 256, (zdtf_output_tma_kernel<32, 32, 8, 256>), (OutTmaShape<32, 32, 8>::SMEM))
+  SET_PQ(1024, 512, (zdtf_output_tma_kernel<32, 32, 8, 512>), (OutTmaShape<32, 32, 8>::SMEM))
+  SET_PQ(1024, 1024, (zdtf_output_tma_kernel<32, 32, 8, 1024>), (OutTmaShape<32, 32, 8>::SMEM))
+#define SET_P2048(QQ)                                                                          \
+  SET_PQ(2048, QQ, (zdtf_output_tma64_kernel<8, QQ>), OutTma64Shape<8>::SMEM)                  \
+  SET_PQ(2048, QQ, zdtf_input64_kernel<QQ>, In64Shape::SMEM)
+  SET_P2048(256) SET_P2048(512) SET_P2048(1024)
+#undef SET_P2048
+#undef SET_PQ
+#define SET_B(QQ)                                                                              \
+  if (Q == QQ && NT == kFusedMaxNt) {                                                          \
+    SET_ATTR((zdtf_czt_kernel<QQ, kFusedMaxNt, false, kWhole>), CztShape<QQ>::SMEM)            \
+    SET_ATTR((zdtf_czt_kernel<QQ, kFusedMaxNt, true, kWhole>), CztShape<QQ>::SMEM)             \
+    SET_ATTR((zdtf_czt_kernel<QQ, kFusedMaxNt, false, kSingles>), CztShape<QQ>::SMEM)          \
+    SET_ATTR((zdtf_czt_kernel<QQ, kFusedMaxNt, true, kSingles>), CztShape<QQ>::SMEM)           \
+    SET_ATTR((zdtf_czt_kernel<QQ, kFusedMaxNt, true, kRounds>), CztShape<QQ>::SMEM)            \
+    SET_ATTR((zdtf_a2f_kernel<QQ, kFusedMaxNt>), CztShape<QQ>::SMEM)                           \
+  }
   FDR_FOR_Q(SET_B)
 #undef SET_B
-#define SET_BS(Q, NT)                                                                          \
-  SET_ATTR((zdtf_czt_smem_kernel<Q, NT, kWhole>), (CztSmemShape<Q>::template smem<NT>()))       \
-  SET_ATTR((zdtf_czt_smem_kernel<Q, NT, kRounds>), (CztSmemShape<Q>::template smem<NT>()))
+#define SET_BS(QQ, NN)                                                                         \
+  if (Q == QQ && NT == NN) {                                                                   \
+    SET_ATTR((zdtf_czt_smem_kernel<QQ, NN, kWhole>), (CztSmemShape<QQ>::template smem<NN>()))  \
+    SET_ATTR((zdtf_czt_smem_kernel<QQ, NN, kRounds>), (CztSmemShape<QQ>::template smem<NN>())) \
+  }
   SET_BS(64, 32) SET_BS(128, 32) SET_BS(64, 64) SET_BS(128, 64)
 #undef SET_BS
-#define SET_AF(Q, NT) SET_ATTR((zdtf_a2f_smem_kernel<Q, NT>), (CztSmemShape<Q>::template smem<NT>()))
+#define SET_AF(QQ, NN) \
+  if (Q == QQ && NT == NN) SET_ATTR((zdtf_a2f_smem_kernel<QQ, NN>), (CztSmemShape<QQ>::template smem<NN>()))
   SET_AF(64, 32) SET_AF(128, 32) SET_AF(256, 32) SET_AF(512, 32)
   SET_AF(64, 64) SET_AF(128, 64) SET_AF(256, 64)
 #undef SET_AF
-#define SET_WS(Q, NT)                                                                          \
-  SET_ATTR((zdtf_czt_ws_kernel<Q, NT, kWhole>), (CztWsShape<Q>::template smem<NT>()))           \
-  SET_ATTR((zdtf_czt_ws_kernel<Q, NT, kRounds>), (CztWsShape<Q>::template smem<NT>()))
+#define SET_WS(QQ, NN)                                                                         \
+  if (Q == QQ && NT == NN) {                                                                   \
+    SET_ATTR((zdtf_czt_ws_kernel<QQ, NN, kWhole>), (CztWsShape<QQ>::template smem<NN>()))      \
+    SET_ATTR((zdtf_czt_ws_kernel<QQ, NN, kRounds>), (CztWsShape<QQ>::template smem<NN>()))     \
+  }
   SET_WS(512, 32) SET_WS(256, 32) SET_WS(256, 64)
-  SET_ATTR((zdtf_czt_ws_kernel<512, 32, kSingles>), (CztWsShape<512>::smem<32>()))
 #undef SET_WS
-  SET_ATTR(zdtf_czt_cl_kernel<kWhole>, CztClShape::SMEM)
-  SET_ATTR(zdtf_czt_cl_kernel<kRounds>, CztClShape::SMEM)
-  SET_ATTR(zdtf_a2f_half_kernel, CztClShape::SMEM)
+  if (Q == 512 && NT == 32) SET_ATTR((zdtf_czt_ws_kernel<512, 32, kSingles>), (CztWsShape<512>::smem<32>()))
+  if (Q == CztClShape::Q && NT == 64) {
+    SET_ATTR(zdtf_czt_cl_kernel<kWhole>, CztClShape::SMEM)
+    SET_ATTR(zdtf_czt_cl_kernel<kRounds>, CztClShape::SMEM)
+    SET_ATTR(zdtf_a2f_half_kernel, CztClShape::SMEM)
+  }
 #undef SET_ATTR
-  if (dev < 64) done[dev] = true;
+  if (mark) mark->store(true);
   return FDR_OK;
 }
 
@@ -2906,13 +2913,13 @@ int fused_plan_create(FusedPlan** out, int64_t N, int64_t Nt, int64_t Nr) {
               (long long)N, (long long)Nt);
     return FDR_ERR_UNSUPPORTED_SIZE;
   }
-  FDR_TRY(set_smem_attrs());
   FusedPlan* st = new FusedPlan();
   st->N = N; st->Nt = Nt; st->Nr = Nr;
   st->L = ilog2(N);
   const int Qlog = fused_qlog(st->L, Nt);
   st->Q = 1 << Qlog;
   st->P = (int)(N >> Qlog);
+  if (const int e = set_smem_attrs(st->P, st->Q, Nt)) { delete st; return e; }
   st->NP = cdiv(Nt, 2);
   st->npairs = cdiv(Nr, 2);
   st->half = cdiv(st->npairs, 2);
