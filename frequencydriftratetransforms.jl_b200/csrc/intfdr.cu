@@ -72,12 +72,12 @@ struct alignas(16) TiledTable {  // rel is read four words at a time
   int32_t off[kTiledMaxNt + 1];   // start of time step t's window in shared memory
 };
 
-// T threads with TNV channels each, T apart: TN = TNV * T output channels per CTA.
-template <int TNV, int T>
-__global__ void __launch_bounds__(T)
+// Threads with TNV channels each, T apart: TN = TNV * T output channels per CTA.
+template <int TNV>
+__global__ void __launch_bounds__(kIntfdrThreads)
 intfdr_tiled_kernel(const float* __restrict__ spec, long long Nf, int Nt, int nrates,
                     float* __restrict__ fdr, const __grid_constant__ TiledTable tab) {
-  constexpr int TN = TNV * T;
+  constexpr int T = kIntfdrThreads, TN = TNV * T;
   extern __shared__ float win[];
   const long long n0 = (long long)blockIdx.x * TN;
   // asynchronous copies: every word of the windows is in flight at once
@@ -201,15 +201,15 @@ static bool run_intfdr_tiled(const float* spec, int64_t Nf, int64_t Nt, int64_t 
     for (int64_t t = 0; t < Nt; ++t) tab.rel[j * Ntp + t] += tab.off[t];
   const size_t smem = sizeof(float) * (size_t)tab.off[Nt];
   cudaError_t ea = cudaSuccess;
-#define TILED(V, T)                                                                             \
-  if (TN == V * T) {                                                                            \
-    ea = cudaFuncSetAttribute(intfdr_tiled_kernel<V, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+#define TILED(V)                                                                                \
+  if (TN == V * kIntfdrThreads) {                                                               \
+    ea = cudaFuncSetAttribute(intfdr_tiled_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                               (int)(sizeof(float) * kTiledMaxWords));                           \
     if (ea == cudaSuccess)                                                                      \
-      intfdr_tiled_kernel<V, T><<<(unsigned)cdiv(Nf, TN), T, smem, s>>>(                        \
+      intfdr_tiled_kernel<V><<<(unsigned)cdiv(Nf, TN), kIntfdrThreads, smem, s>>>(             \
           spec, Nf, (int)Nt, (int)nr, fdr + j0 * Nf, tab);                                      \
   }
-  TILED(1, 256) TILED(2, 256) TILED(4, 256)
+  TILED(1) TILED(2) TILED(4)
 #undef TILED
   if (ea != cudaSuccess) { *status = cuda_status(ea, "intfdr tiled attribute"); return true; }
   cudaError_t e = cudaGetLastError();

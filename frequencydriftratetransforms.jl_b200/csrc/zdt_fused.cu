@@ -175,7 +175,6 @@ zdtf_input64_kernel(const float* __restrict__ spec, long long N, int Nt, int NP,
   using SH = In64Shape;
   constexpr int P = SH::P, P1 = SH::P1, P2 = SH::P2, TS = SH::TS, S1 = SH::S1, SSEQ = SH::SSEQ;
   extern __shared__ float2 sm[];
-  let_dependents_start();
   float2* region = sm;           // TS * SSEQ: the transpose
   float2* tw1 = sm + TS * SSEQ;  // w^(nb1 k): P1 rows of S1; rows 3 (mod 4) negated, see pass 2
   float2* tw2 = tw1 + SH::TW1;   // w64^n, n < P1 / 2
@@ -1419,7 +1418,6 @@ zdtf_czt_cl_kernel(CztArgs a) {
   float2* const twr = sm + SH::TWR;
   float2* const gs = sm + SH::GS_OFF;
   float2* const gnyq = gs + NT * QH;
-  let_dependents_start();
   const int tid = threadIdx.x;
   const int rank = (int)cluster.block_rank();  // the side this CTA holds
   const int c = blockIdx.x >> 1;                // residue pair
@@ -1427,7 +1425,6 @@ zdtf_czt_cl_kernel(CztArgs a) {
   const int k1s[2] = {c == 0 ? 0 : c, c == 0 ? P / 2 : P - c};
   for (int i = tid; i < tw_size(Q); i += T) twt[i] = __ldg(a.tab.twQ + i);
   fill_output_twiddles<Q, T>(a, k1s, twr);
-  wait_for_predecessor();
   czt_forward_cluster<Q, NT, T>(a, c, k1s, buf, twt, gs, gnyq, rank, cluster);
   auto bin0 = [&](int bp) { return (unsigned long long)k1s[rank] + (unsigned long long)P * (2 * bp); };
   fold_smem<T>(a, reinterpret_cast<float4*>(gs), QH / 2, bin0);
@@ -1877,7 +1874,6 @@ zdtf_output_tma_kernel(const __grid_constant__ CUtensorMap wmap, long long N, in
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (int i = tid; i < P; i += SH::T) roots[i] = __ldg(rootsP + i);
-  wait_for_predecessor();
   __syncthreads();
   auto issue = [&](int tile) {  // thread 0 only
     const int q = tile / ntna, nat = tile % ntna;
@@ -2022,7 +2018,6 @@ zdtf_output_tma64_kernel(const __grid_constant__ CUtensorMap wmap, long long N, 
     tw1[(i / P2) * S1 + i % P2] = (i / P2) % 4 == 3 ? make_float2(-w.x, -w.y) : w;
   }
   for (int i = tid; i < P1 / 2; i += SH::T) tw2[i] = cconj(__ldg(rootsP + i * (P / P1)));
-  wait_for_predecessor();
   __syncthreads();
   auto issue = [&](int tile) {  // thread 0 only
     const int q = tile / ntna, nat = tile % ntna;
@@ -2858,7 +2853,6 @@ static int set_smem_attrs(int P, int Q, int64_t Nt) {
   if (P == PP && Q == QQ) SET_ATTR(kernel, bytes)
   SET_PQ(1024, 256, (zdtf_output_tma_kernel<32, 32, 8, 256>), (OutTmaShape<32, 32, 8>::SMEM))
   SET_PQ(1024, 512, (zdtf_output_tma_kernel<32, 32, 8, 512>), (OutTmaShape<32, 32, 8>::SMEM))
-  SET_PQ(1024, 1024, (zdtf_output_tma_kernel<32, 32, 8, 1024>), (OutTmaShape<32, 32, 8>::SMEM))
 #define SET_P2048(QQ)                                                                          \
   SET_PQ(2048, QQ, (zdtf_output_tma64_kernel<8, QQ>), OutTma64Shape<8>::SMEM)                  \
   SET_PQ(2048, QQ, zdtf_input64_kernel<QQ>, In64Shape::SMEM)
@@ -2954,7 +2948,8 @@ int64_t fused_plan_table_bytes(const FusedPlan* st) {
 int64_t fused_A_elems(const FusedPlan* st) { return st->N * st->NP; }
 int64_t fused_W_elems(const FusedPlan* st) { return st->N * st->npairs; }
 
-// Whether the czt and output kernels may start before the kernel in front has ended: where launches
+// Whether the czt and output kernels may start before the kernel in front has ended (those of Nf = 2^18
+// and above only, the cluster czt kernel and the TMA output passes, are launched plainly): where launches
 // are a good part of the call (Nf = 2^12, 17 rates 20.5 -> 18.6 us; 2^16, 33 rates 31.5 -> 30.7).
 // Larger grids end in partial waves whose SMs the waiting CTAs would hold (2^18, Nt = 32, 257 rates
 // 409 -> 431 us; a batch of 8 channels on four streams 5.21 -> 5.27 ms).
@@ -3085,7 +3080,7 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
   groups = (int)cdiv(a.nblk, a.blocks_per_group);
   if (st->Nt > 32 && Q == CztClShape::Q) {  // F of 64 steps for 512 bins: two-CTA cluster
     auto kernel = rounds ? zdtf_czt_cl_kernel<kRounds> : zdtf_czt_cl_kernel<kWhole>;
-    FDR_CUDA(launch_dependent(early_launch(st), kernel, dim3(2 * ctas, groups), CztClShape::T, CztClShape::SMEM, s, a));
+    kernel<<<dim3(2 * ctas, groups), CztClShape::T, CztClShape::SMEM, s>>>(a);
     FDR_LAUNCH_CHECK("zdtf_czt_cl_kernel");
     return FDR_OK;
   }
@@ -3240,7 +3235,7 @@ int fused_output_mixed(const FusedPlan* st, const float2* W, float* dest, double
 
 int fused_output(const FusedPlan* st, const float2* W, float* dest, double* acc, cudaStream_t s) {
   const int P = st->P, Q = st->Q;
-  // P = 1024 or 2048: Q is 256 to 1024 (fused_qlog).  (P = 512 through the TMA kernel, half of its
+  // P = 1024 with Q = 256 or 512, P = 2048 with 256 to 1024 (fused_qlog).  (P = 512 through the TMA kernel, half of its
   // threads idle in pass 1, took 130 us against zdtf_output2_kernel's 124 at Nf = 2^18, 257 rates.)
   if ((P == 1024 || P == 2048) && tma_output_enabled()) {
     CUtensorMap map;
@@ -3249,8 +3244,8 @@ int fused_output(const FusedPlan* st, const float2* W, float* dest, double* acc,
 #define LAUNCH_OUT(PP, QQ, SH, KERNEL)                                                         \
       if (P == PP && Q == QQ) {                                                                \
         const int grid = (int)std::min<long long>(ntiles, (long long)SH::MINB * sm_count());   \
-        FDR_CUDA(launch_dependent(early_launch(st), KERNEL, grid, SH::T, SH::SMEM, s, map, st->N, (int)st->Nr,   \
-                                  (int)st->npairs, dest, st->tab.rootsP, acc));                \
+        KERNEL<<<grid, SH::T, SH::SMEM, s>>>(map, st->N, (int)st->Nr, (int)st->npairs, dest,   \
+                                             st->tab.rootsP, acc);                             \
         FDR_LAUNCH_CHECK(#KERNEL);                                                             \
         return FDR_OK;                                                                         \
       }
@@ -3258,7 +3253,6 @@ int fused_output(const FusedPlan* st, const float2* W, float* dest, double* acc,
       using S2048 = OutTma64Shape<8>;
       LAUNCH_OUT(1024, 256, S1024, (zdtf_output_tma_kernel<32, 32, 8, 256>))
       LAUNCH_OUT(1024, 512, S1024, (zdtf_output_tma_kernel<32, 32, 8, 512>))
-      LAUNCH_OUT(1024, 1024, S1024, (zdtf_output_tma_kernel<32, 32, 8, 1024>))
       LAUNCH_OUT(2048, 256, S2048, (zdtf_output_tma64_kernel<8, 256>))
       LAUNCH_OUT(2048, 512, S2048, (zdtf_output_tma64_kernel<8, 512>))
       LAUNCH_OUT(2048, 1024, S2048, (zdtf_output_tma64_kernel<8, 1024>))
