@@ -207,7 +207,9 @@ __device__ __forceinline__ float2 cispi_d(double h) {
 // plainly pass both calls at once.
 // ------------------------------------------------------------------------------------
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_dependents_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void let_dependents_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 template <class... P, class... A>
 inline cudaError_t launch_dependent(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,

@@ -96,20 +96,44 @@ struct DftCoprime {
 
 // cos and sin of 2 pi m / n
 struct CosSin7 {
-  float c[7] = {1.00000000000000000f, 0.62348980185873359f, -0.22252093395631434f, -0.90096886790241903f, -0.90096886790241915f, -0.22252093395631459f, 0.62348980185873337f};
-  float s[7] = {0.00000000000000000f, 0.78183148246802980f, 0.97492791218182362f, 0.43388373911755823f, -0.43388373911755801f, -0.97492791218182362f, -0.78183148246802991f};
+  float c[7] = {
+      1.00000000000000000f, 0.62348980185873359f, -0.22252093395631434f, -0.90096886790241903f,
+      -0.90096886790241915f, -0.22252093395631459f, 0.62348980185873337f};
+  float s[7] = {
+      0.00000000000000000f, 0.78183148246802980f, 0.97492791218182362f, 0.43388373911755823f,
+      -0.43388373911755801f, -0.97492791218182362f, -0.78183148246802991f};
 };
 struct CosSin9 {
-  float c[9] = {1.00000000000000000f, 0.76604444311897801f, 0.17364817766693041f, -0.49999999999999978f, -0.93969262078590832f, -0.93969262078590843f, -0.50000000000000044f, 0.17364817766692997f, 0.76604444311897779f};
-  float s[9] = {0.00000000000000000f, 0.64278760968653925f, 0.98480775301220802f, 0.86602540378443871f, 0.34202014332566888f, -0.34202014332566866f, -0.86602540378443837f, -0.98480775301220813f, -0.64278760968653958f};
+  float c[9] = {
+      1.00000000000000000f, 0.76604444311897801f, 0.17364817766693041f, -0.49999999999999978f,
+      -0.93969262078590832f, -0.93969262078590843f, -0.50000000000000044f, 0.17364817766692997f,
+      0.76604444311897779f};
+  float s[9] = {
+      0.00000000000000000f, 0.64278760968653925f, 0.98480775301220802f, 0.86602540378443871f,
+      0.34202014332566888f, -0.34202014332566866f, -0.86602540378443837f, -0.98480775301220813f,
+      -0.64278760968653958f};
 };
 struct CosSin11 {
-  float c[11] = {1.00000000000000000f, 0.84125353283118121f, 0.41541501300188644f, -0.14231483827328500f, -0.65486073394528499f, -0.95949297361449737f, -0.95949297361449748f, -0.65486073394528521f, -0.14231483827328523f, 0.41541501300188605f, 0.84125353283118121f};
-  float s[11] = {0.00000000000000000f, 0.54064081745559756f, 0.90963199535451833f, 0.98982144188093280f, 0.75574957435425827f, 0.28173255684142967f, -0.28173255684142939f, -0.75574957435425816f, -0.98982144188093268f, -0.90963199535451855f, -0.54064081745559744f};
+  float c[11] = {
+      1.00000000000000000f, 0.84125353283118121f, 0.41541501300188644f, -0.14231483827328500f,
+      -0.65486073394528499f, -0.95949297361449737f, -0.95949297361449748f, -0.65486073394528521f,
+      -0.14231483827328523f, 0.41541501300188605f, 0.84125353283118121f};
+  float s[11] = {
+      0.00000000000000000f, 0.54064081745559756f, 0.90963199535451833f, 0.98982144188093280f,
+      0.75574957435425827f, 0.28173255684142967f, -0.28173255684142939f, -0.75574957435425816f,
+      -0.98982144188093268f, -0.90963199535451855f, -0.54064081745559744f};
 };
 struct CosSin13 {
-  float c[13] = {1.00000000000000000f, 0.88545602565320991f, 0.56806474673115592f, 0.12053668025532301f, -0.35460488704253545f, -0.74851074817110119f, -0.97094181742605201f, -0.97094181742605212f, -0.74851074817110130f, -0.35460488704253590f, 0.12053668025532320f, 0.56806474673115481f, 0.88545602565321002f};
-  float s[13] = {0.00000000000000000f, 0.46472317204376851f, 0.82298386589365635f, 0.99270887409805397f, 0.93501624268541483f, 0.66312265824079519f, 0.23931566428755768f, -0.23931566428755743f, -0.66312265824079497f, -0.93501624268541472f, -0.99270887409805397f, -0.82298386589365702f, -0.46472317204376840f};
+  float c[13] = {
+      1.00000000000000000f, 0.88545602565320991f, 0.56806474673115592f, 0.12053668025532301f,
+      -0.35460488704253545f, -0.74851074817110119f, -0.97094181742605201f, -0.97094181742605212f,
+      -0.74851074817110130f, -0.35460488704253590f, 0.12053668025532320f, 0.56806474673115481f,
+      0.88545602565321002f};
+  float s[13] = {
+      0.00000000000000000f, 0.46472317204376851f, 0.82298386589365635f, 0.99270887409805397f,
+      0.93501624268541483f, 0.66312265824079519f, 0.23931566428755768f, -0.23931566428755743f,
+      -0.66312265824079497f, -0.93501624268541472f, -0.99270887409805397f, -0.82298386589365702f,
+      -0.46472317204376840f};
 };
 
 template <> struct Dft<6> : DftCoprime<2, 3, 3, 4> {};

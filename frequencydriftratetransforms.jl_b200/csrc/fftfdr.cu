@@ -217,14 +217,18 @@ int fdr_fftfdr(fdr_fft_ws* ws, const float* rates, int64_t Nr, float* fdr, fdr_s
       if (!((double)fabsf(rp.r[i]) * (double)ws->Nt < (double)(1 << 19))) large |= 1u << i;
     auto launch = [&](auto rpt) {
       constexpr int RPT = decltype(rpt)::value;
-      auto kernel = large ? (mult ? (pow2 ? phasor_sum_kernel<RPT, true, true, true> : phasor_sum_kernel<RPT, true, false, true>)
-                                  : (pow2 ? phasor_sum_kernel<RPT, false, true, true> : phasor_sum_kernel<RPT, false, false, true>))
-                          : (mult ? (pow2 ? phasor_sum_kernel<RPT, true, true, false> : phasor_sum_kernel<RPT, true, false, false>)
-                                  : (pow2 ? phasor_sum_kernel<RPT, false, true, false> : phasor_sum_kernel<RPT, false, false, false>));
+      auto pick = [&](auto m, auto p2) {
+        constexpr bool M = decltype(m)::value, P = decltype(p2)::value;
+        return large ? phasor_sum_kernel<RPT, M, P, true> : phasor_sum_kernel<RPT, M, P, false>;
+      };
+      const std::true_type yes;
+      const std::false_type no;
+      auto kernel = mult ? (pow2 ? pick(yes, yes) : pick(yes, no)) : (pow2 ? pick(no, yes) : pick(no, no));
       const dim3 grid((unsigned)cdiv(ws->K, 256), (unsigned)cdiv(nr, RPT));
       kernel<<<grid, 256, 0, s>>>(ws->F, ws->K, (int)ws->Nt, ws->Nf, nr, large, ws->S, rp);
     };
-    if (cdiv(ws->K, 256) * cdiv(nr, kRatesPerThread) >= sm_count()) launch(std::integral_constant<int, kRatesPerThread>());
+    const bool full = cdiv(ws->K, 256) * cdiv(nr, kRatesPerThread) >= sm_count();
+    if (full) launch(std::integral_constant<int, kRatesPerThread>());
     else launch(std::integral_constant<int, 2>());
     FDR_LAUNCH_CHECK("phasor_sum_kernel");
     FDR_TRY(irfft_columns(ws->S, ws->K, nr, ws->Nf, fdr + j0 * ws->Nf, ws->Nf, ws->rscratch,

@@ -175,7 +175,8 @@ static int launch_input(const float* spec, int64_t Nf, int64_t Nt, int factor, i
 // grid (X/kConvTile, B), kConvTile / 2 threads: a thread takes two bins and all 32 output
 // channels, two channels per packed multiply-add, so that a 16-byte broadcast load of weights
 // feeds four of them (one scalar weight load per multiply-add bound the scalar form: 190 us a
-// layer at 64 x 4096 bins, 33 channels; now 83 us, FMA pipe 57%, the weights' loads behind it).  Every output sums over (ci, k) in order from its bias.
+// layer at 64 x 4096 bins, 33 channels; now 83 us, FMA pipe 57%, the weights' loads behind it).
+// Every output sums over (ci, k) in order from its bias.
 // HEAD: the last hidden layer also forms the 16 window logits of its bins (the 1x1 layer, same
 // order of sums) and their maximum over the tile's bins, the first bin on ties.
 // odd: per (sample, tile, input channel) the taps that meet an infinity or NaN (bit k), for HEAD
@@ -633,7 +634,8 @@ sparse_weight_grad_kernel(const SparseGrad* __restrict__ sg, const float* __rest
     for (int q = 0; q < 4; ++q)
 #pragma unroll
       for (int k = 0; k < kTaps; ++k)
-        pb[L.woff + ((long long)(4 * cg + q) * cin + ci) * kTaps + k] = (taps >> k & 1) && fabsf(a[q][k]) < INFINITY ? NAN : a[q][k];
+        pb[L.woff + ((long long)(4 * cg + q) * cin + ci) * kTaps + k] =
+            (taps >> k & 1) && fabsf(a[q][k]) < INFINITY ? NAN : a[q][k];
   }
   for (int c = tid; c < kWidth; c += kSparseThreads) {
     float a = 0.f;
@@ -643,7 +645,8 @@ sparse_weight_grad_kernel(const SparseGrad* __restrict__ sg, const float* __rest
 }
 
 // grad[i] = sum over samples (in order) of partial[b][i]
-__global__ void reduce_partials_kernel(const float* __restrict__ partial, int B, long long n, float* __restrict__ grad) {
+__global__ void reduce_partials_kernel(const float* __restrict__ partial, int B, long long n,
+                                       float* __restrict__ grad) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   float s = 0.f;

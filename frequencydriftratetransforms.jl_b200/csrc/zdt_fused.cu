@@ -329,7 +329,8 @@ __device__ __forceinline__ void czt_forward(const CztArgs& a, int c, const int* 
           const int e = tid + i * T;
           const int seq = e / Q, na = e - seq * Q;
           const int pp = p0 + (seq >> 1) - a.pshift, side = seq & 1;
-          v[i] = ((unsigned)pp < (unsigned)a.NP && FDR_DBG_OK(((long long)pp * a.P + k1s[side]) * Q + na < (long long)a.NP * a.P * Q))
+          v[i] = ((unsigned)pp < (unsigned)a.NP &&
+                  FDR_DBG_OK(((long long)pp * a.P + k1s[side]) * Q + na < (long long)a.NP * a.P * Q))
                      ? __ldcs(a.A + ((long long)pp * a.P + k1s[side]) * Q + na)
                              : make_float2(0.f, 0.f);
         }
@@ -439,7 +440,7 @@ __device__ __forceinline__ void nyquist_block(const CztArgs& a, const float2* gn
 // ------------------------------------------------------------------------------------
 // Sums over the time steps at pairs of rates about the grid's centre.
 //
-// Rates 2H + m and 2H - 1 - m of a grid padded to 4h rates (H = 2h; h "super pairs" of two rate
+// Rates H + m and H - 1 - m of a grid padded to 4h rates (H = 2h; h "super pairs" of two rate
 // pairs) lie at +-phi, phi = (2m + 1) k dr / (2 Nf) turns, about its centre.  With the centre's
 // phase theta and a middle step c taken out of F,
 //     F'_t = F_t exp(2 pi i t theta),  G_u = F'_{c+u} + F'_{c-u},  H_u = F'_{c+u} - F'_{c-u},
@@ -574,7 +575,8 @@ __device__ __forceinline__ void fold_factor(const FoldPhase& f, int q, float2& z
 // The phases of a thread of the kernels with F in shared memory: the factors stay in registers.
 struct FoldPhases : FoldPhase {
   float2 fzx[3], fzy[3], frx[3], fry[3];
-  __device__ __forceinline__ void setup(unsigned long long k0, unsigned long long k1, unsigned long long Rh, int middle) {
+  __device__ __forceinline__ void setup(unsigned long long k0, unsigned long long k1, unsigned long long Rh,
+                                        int middle) {
     rh0 = k0 * Rh;
     rh1 = k1 * Rh;
     c = middle;
@@ -1227,6 +1229,7 @@ __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArg
   for (int i = tid; i < tw_size(Q); i += T) twt[i] = __ldg(a.tab.twQ + i);
   fill_output_twiddles<Q, T>(a, k1s, twr);
   wait_for_predecessor();
+  static_assert(2 * 8 * SS <= SH::BUF1 + kRatesPerBlock * SS, "16 sequences: both rate-block buffers");
   czt_forward_smem<Q, NT, T, false, 8>(a, c, k1s, buf0, twt, gs, gnyq);  // ends with a barrier
   auto bin0 = [&](int bp) {
     const int b0 = 2 * bp, side = b0 / (Q / 2);
@@ -1274,8 +1277,10 @@ __global__ void __launch_bounds__(CztWsShape<Q>::T, 1) zdtf_czt_ws_kernel(CztArg
           const int ja = 2 * (a.half + 2 * blk + i);  // rates past the grid's last: zero
           if (ja >= a.Nr) px[2 * i] = py[2 * i] = zero;
           if (ja + 1 >= a.Nr) px[2 * i + 1] = py[2 * i + 1] = zero;
-          put_rate_pair<SS>(hb + 4 * i * SS, side, k20, ms, mk2, dc, win, px[2 * i], py[2 * i], px[2 * i + 1], py[2 * i + 1]);
-          put_rate_pair<SS>(hb + (4 * i + 2) * SS, side, k20, ms, mk2, dc, win, mx[2 * i + 1], my[2 * i + 1], mx[2 * i], my[2 * i]);
+          put_rate_pair<SS>(hb + 4 * i * SS, side, k20, ms, mk2, dc, win,
+                            px[2 * i], py[2 * i], px[2 * i + 1], py[2 * i + 1]);
+          put_rate_pair<SS>(hb + (4 * i + 2) * SS, side, k20, ms, mk2, dc, win,
+                            mx[2 * i + 1], my[2 * i + 1], mx[2 * i], my[2 * i]);
         }
       }
       if (c == 0 && bp < kRatesPerBlock)
@@ -1331,6 +1336,7 @@ __device__ __forceinline__ void czt_forward_cluster(const CztArgs& a, int c, con
                                                     int rank, cg::cluster_group& cluster) {
   constexpr int SS = b_stride<Q>();
   constexpr int PC = 16, QH = Q / 2;
+  static_assert(PC <= 2 * kRatesPerBlock, "both rate-block buffers");
   constexpr int NE = PC * Q, NL = (NE + T - 1) / T;
   const int tid = threadIdx.x;
   if (c == 0 && rank == 0 && tid == 0)
@@ -1413,7 +1419,7 @@ zdtf_czt_cl_kernel(CztArgs a) {
   static_assert(SH::H == QH, "two blocks at a time, a bin pair per thread");
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ float2 sm[];
-  float2* const buf = sm;  // forward pass: 8 sequences; then two buffers of 8 (two rate blocks)
+  float2* const buf = sm;  // forward pass: 16 sequences; then two buffers of 8 (two rate blocks)
   float2* const twt = sm + SH::TWT;
   float2* const twr = sm + SH::TWR;
   float2* const gs = sm + SH::GS_OFF;
@@ -1468,8 +1474,10 @@ zdtf_czt_cl_kernel(CztArgs a) {
             if (ja >= a.Nr) px[2 * i] = py[2 * i] = zero;
             if (ja + 1 >= a.Nr) px[2 * i + 1] = py[2 * i + 1] = zero;
             const int slot = 2 * (2 * bb + i);
-            put_rate_pair<SS>(hb0 + slot * SS, side, k20, ms, mk2, dc, win, px[2 * i], py[2 * i], px[2 * i + 1], py[2 * i + 1]);
-            put_rate_pair<SS>(hb1 + slot * SS, side, k20, ms, mk2, dc, win, mx[2 * i + 1], my[2 * i + 1], mx[2 * i], my[2 * i]);
+            put_rate_pair<SS>(hb0 + slot * SS, side, k20, ms, mk2, dc, win,
+                              px[2 * i], py[2 * i], px[2 * i + 1], py[2 * i + 1]);
+            put_rate_pair<SS>(hb1 + slot * SS, side, k20, ms, mk2, dc, win,
+                              mx[2 * i + 1], my[2 * i + 1], mx[2 * i], my[2 * i]);
           }
         }
         if (c == 0 && rank == 0 && bp < kRatesPerBlock)
@@ -1809,7 +1817,8 @@ __global__ void bounded_wait_selftest_kernel(unsigned long long limit_ns) {
 // both channels of rate j and the odd lane both of rate j + 1 as one 8-byte streaming store
 // each.  Every lane of the warp must call it; p is the even lane's element of rate j or the
 // element before the odd lane's of rate j + 1, live: that rate exists.
-__device__ __forceinline__ void store_rate_pair(float* p, float2 v, bool odd, bool live, const float* dlo, const float* dhi) {
+__device__ __forceinline__ void store_rate_pair(float* p, float2 v, bool odd, bool live, const float* dlo,
+                                                const float* dhi) {
   const float recv = __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
   if (live && FDR_DBG_OK(p >= dlo && p + 2 <= dhi))
     __stcs(reinterpret_cast<float2*>(p), make_float2(odd ? recv : v.x, odd ? v.y : recv));
@@ -1857,7 +1866,8 @@ struct OutTmaShape {
 // 222 us, 1.09 GB read and written, 4.9 TB/s.)
 template <int P1, int P2, int TS, int Q>
 __global__ void __launch_bounds__(OutTmaShape<P1, P2, TS>::T, OutTmaShape<P1, P2, TS>::MINB)
-zdtf_output_tma_kernel(const __grid_constant__ CUtensorMap wmap, long long N, int Nr, int npairs, float* __restrict__ dest, const float2* __restrict__ rootsP,
+zdtf_output_tma_kernel(const __grid_constant__ CUtensorMap wmap, long long N, int Nr, int npairs,
+                       float* __restrict__ dest, const float2* __restrict__ rootsP,
                         double* __restrict__ acc) {
   using SH = OutTmaShape<P1, P2, TS>;
   constexpr int P = SH::P, S1 = SH::S1, SSEQ = SH::SSEQ;
@@ -1994,7 +2004,8 @@ struct OutTma64Shape {
 
 template <int TS_, int Q>
 __global__ void __launch_bounds__(OutTma64Shape<TS_>::T, OutTma64Shape<TS_>::MINB)
-zdtf_output_tma64_kernel(const __grid_constant__ CUtensorMap wmap, long long N, int Nr, int npairs, float* __restrict__ dest, const float2* __restrict__ rootsP,
+zdtf_output_tma64_kernel(const __grid_constant__ CUtensorMap wmap, long long N, int Nr, int npairs,
+                         float* __restrict__ dest, const float2* __restrict__ rootsP,
                          double* __restrict__ acc) {
   using SH = OutTma64Shape<TS_>;
   constexpr int P = SH::P, P1 = SH::P1, P2 = SH::P2, TS = SH::TS, S1 = SH::S1, SSEQ = SH::SSEQ;
@@ -3084,15 +3095,17 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
     FDR_LAUNCH_CHECK("zdtf_czt_cl_kernel");
     return FDR_OK;
   }
-  // 16 < Nt <= 64 with 256 or 512 bins per CTA: the warp-specialised kernel (measured 6-9%
-  // faster than zdtf_czt_smem_kernel at Nf = 2^19..2^20); Nt <= 16 keeps F in registers.
+  // 16 < Nt <= 64 with 256 or 512 bins per CTA: sums and transforms side by side (with Horner's rule 6
+  // to 9% faster at Nf = 2^19 and 2^20 than one after the other, as zdtf_czt_smem_kernel has them for 64
+  // and 128 bins, whose transforms would leave most of a second group idle); Nt <= 16 keeps F in registers.
   if (st->Nt > kFusedMaxNt && ((Q == 512 && st->Nt <= 32) || (Q == 256 && st->Nt <= 64))) {
     const int NT = st->Nt <= 32 ? 32 : 64;
 #define LAUNCH_WS(QQ, NN)                                                                      \
     if (Q == QQ && NT == NN) {                                                                 \
       auto kernel = rounds ? zdtf_czt_ws_kernel<QQ, NN, kRounds> : zdtf_czt_ws_kernel<QQ, NN, kWhole>; \
       if (rounds && !both && QQ == 512) kernel = zdtf_czt_ws_kernel<512, 32, kSingles>;        \
-      FDR_CUDA(launch_dependent(early_launch(st), kernel, dim3(ctas, groups), CztWsShape<QQ>::T, CztWsShape<QQ>::template smem<NN>(), s, a)); \
+      FDR_CUDA(launch_dependent(early_launch(st), kernel, dim3(ctas, groups), CztWsShape<QQ>::T, \
+                                CztWsShape<QQ>::template smem<NN>(), s, a));                   \
       FDR_LAUNCH_CHECK("zdtf_czt_ws_kernel");                                                  \
       return FDR_OK;                                                                           \
     }
@@ -3104,7 +3117,8 @@ int fused_czt_blocks(const FusedPlan* st, const float2* A, float2* W, float r0, 
 #define LAUNCH_BS(QQ, NN)                                                                      \
     if (Q == QQ && NT == NN) {                                                                 \
       auto kernel = rounds ? zdtf_czt_smem_kernel<QQ, NN, kRounds> : zdtf_czt_smem_kernel<QQ, NN, kWhole>; \
-      FDR_CUDA(launch_dependent(early_launch(st), kernel, dim3(ctas, groups), CztSmemShape<QQ>::T, CztSmemShape<QQ>::template smem<NN>(), s, a)); \
+      FDR_CUDA(launch_dependent(early_launch(st), kernel, dim3(ctas, groups), CztSmemShape<QQ>::T, \
+                                CztSmemShape<QQ>::template smem<NN>(), s, a));                 \
       FDR_LAUNCH_CHECK("zdtf_czt_smem_kernel");                                                \
       return FDR_OK;                                                                           \
     }
@@ -3262,8 +3276,9 @@ int fused_output(const FusedPlan* st, const float2* W, float* dest, double* acc,
 #define LAUNCH_C2(PP, P1, P2)                                                                  \
   if (P == PP) {                                                                               \
     using SH = Out2Shape<P1, P2, 8>;                                                           \
-    FDR_CUDA(launch_dependent(early_launch(st), zdtf_output2_kernel<P1, P2, 8>, dim3(Q / 8, (unsigned)st->npairs), \
-                              SH::T, SH::SMEM, s, W, st->N, Q, (int)st->Nr, dest, st->tab.rootsP, acc)); \
+    const dim3 grid(Q / 8, (unsigned)st->npairs);                                              \
+    FDR_CUDA(launch_dependent(early_launch(st), zdtf_output2_kernel<P1, P2, 8>, grid, SH::T,   \
+                              SH::SMEM, s, W, st->N, Q, (int)st->Nr, dest, st->tab.rootsP, acc)); \
     FDR_LAUNCH_CHECK("zdtf_output2_kernel");                                                   \
     return FDR_OK;                                                                             \
   }
@@ -3276,7 +3291,8 @@ int fused_output(const FusedPlan* st, const float2* W, float* dest, double* acc,
 #define LAUNCH_C(PP)                                                                           \
   if (P == PP) {                                                                               \
     constexpr int TC = AcShape<PP>::TILE, T = AcShape<PP>::T;                                  \
-    FDR_CUDA(launch_dependent(early_launch(st), zdtf_output_kernel<PP, TC, T>, dim3(Q / TC, (unsigned)st->npairs), T, \
+    const dim3 grid(Q / TC, (unsigned)st->npairs);                                             \
+    FDR_CUDA(launch_dependent(early_launch(st), zdtf_output_kernel<PP, TC, T>, grid, T,        \
                               AcShape<PP>::SMEM, s, W, st->N, Q, (int)st->Nr, dest, st->tab, acc)); \
     FDR_LAUNCH_CHECK("zdtf_output_kernel");                                                    \
     return FDR_OK;                                                                             \
