@@ -2961,7 +2961,9 @@ int64_t fused_W_elems(const FusedPlan* st) { return st->N * st->npairs; }
 
 // Whether the czt and output kernels may start before the kernel in front has ended (those of Nf = 2^18
 // and above only, the cluster czt kernel and the TMA output passes, are launched plainly): where launches
-// are a good part of the call (Nf = 2^12, 17 rates 20.5 -> 18.6 us; 2^16, 33 rates 31.5 -> 30.7).
+// are a good part of the call, plain launch against this one: Nf = 2^12, 17 rates 20.9 -> 20.4 us (as long as
+// the host takes to issue the calls); 2^15, 33 rates 24.8 -> 20.5; 2^16, 129 rates 53.7 -> 49.3; 2^17, Nt = 64, 33
+// rates 94.3 -> 88.3; the least gain is a loss, 2^16 and 2^17, Nt = 16, 33 rates 28.9 -> 29.5 and 46.3 -> 47.1.
 // Larger grids end in partial waves whose SMs the waiting CTAs would hold (2^18, Nt = 32, 257 rates
 // 409 -> 431 us; a batch of 8 channels on four streams 5.21 -> 5.27 ms).
 static bool early_launch(const FusedPlan* st) { return st->N <= (1 << 17); }
@@ -3249,8 +3251,9 @@ int fused_output_mixed(const FusedPlan* st, const float2* W, float* dest, double
 
 int fused_output(const FusedPlan* st, const float2* W, float* dest, double* acc, cudaStream_t s) {
   const int P = st->P, Q = st->Q;
-  // P = 1024 with Q = 256 or 512, P = 2048 with 256 to 1024 (fused_qlog).  (P = 512 through the TMA kernel, half of its
-  // threads idle in pass 1, took 130 us against zdtf_output2_kernel's 124 at Nf = 2^18, 257 rates.)
+  // P = 1024 with Q = 256 or 512, P = 2048 with 256 to 1024 (fused_qlog).  (P = 512 through the TMA
+  // kernel, half of its threads idle in pass 1, took 130 us against zdtf_output2_kernel's 124 at
+  // Nf = 2^18, 257 rates.)
   if ((P == 1024 || P == 2048) && tma_output_enabled()) {
     CUtensorMap map;
     if (w_tensor_map(&map, W, Q, st->npairs * (int64_t)P, 8)) {
